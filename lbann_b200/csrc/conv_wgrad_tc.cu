@@ -38,6 +38,7 @@ struct WgradParams {
   float alpha;
   float* dW;
   long long s_tap, s_k, s_c;            // output strides in elements
+  float* ws;                            // partial sums: [CTA][G * BN / 4][128 rows][4]
   FastDiv fd_bw, fd_bh, fd_bd;          // brick decode without run-time divisions
 };
 
@@ -61,7 +62,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
 
   // Rows of a stage that no TMA box covers must read as zero: they are part of the
   // reduction.  TMA only ever writes the first rows_used rows, so one clear suffices.
-  {
+  if (p.rows_used < 64) {
     uint8_t* base = smem_raw + (smem_base - smem_u32(smem_raw));
     uint4* q = reinterpret_cast<uint4*>(base);
     const int n16 = S * p.stage_bytes / 16;
@@ -232,25 +233,23 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     if (my_bricks > 0 && !landed && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
     if (landed) {
       tc_fence_after();
+      // Four consecutive columns of a row are one 16-byte unit and the units of a column group
+      // lie row by row, so a warp stores 512 contiguous bytes.  (fp32 atomics straight into dW,
+      // whose rows are taps * 4 bytes apart, touched one sector per lane: with 296 CTAs adding
+      // 64 x 64 x 9 weights each that tail took three quarters of the kernel.)
       const int row = warp * 32 + lane;
+      float4* out = reinterpret_cast<float4*>(p.ws) + (size_t)blockIdx.x * (p.G * p.BN * 32) + row;
       for (int gi = 0; gi < g_count; ++gi) {
-        const int sl = (g_first + gi) * p.spg + row / p.Cb;
-        const int tap = sl / p.cblocks;
-        const int ch = (sl - tap * p.cblocks) * p.Cb + row % p.Cb;
-        const bool row_ok = sl < p.slices_total && ch < g.C;
         for (int c = 0; c < p.BN; c += 32) {
           if (n0 + c >= g.Kout) break;
           uint32_t r[32];
           tmem_ld_32x32(tmem_base + gi * p.BN + c + ((uint32_t)(warp * 32) << 16), r);
           tmem_ld_wait();
-          if (row_ok) {
-            float* dst = p.dW + tap * p.s_tap + ch * p.s_c;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int k = n0 + c + j;
-              if (k < g.Kout) atomicAdd(dst + k * p.s_k, p.alpha * __uint_as_float(r[j]));
-            }
-          }
+          for (int j = 0; j < 8; ++j)
+            __stcg(out + ((gi * p.BN + c) / 4 + j) * 128,
+                   make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                               __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
         }
       }
     }
@@ -263,6 +262,62 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   }
 }
 
+// dW += alpha * sum over the splits of the partial sums.  A block owns four filters (one 16-byte
+// unit of the partials), CH channels and up to kRedTaps taps; its threads are the CH x taps
+// items, times as many split groups as fit, so that the loads of a warp are CH * 16 contiguous
+// bytes and the stores (filter layout: taps innermost) are contiguous too, through shared memory.
+constexpr int kRedThreads = 256, kRedTaps = 32;
+
+__global__ void __launch_bounds__(kRedThreads)
+wgrad_reduce_kernel(const WgradParams p, int CH) {
+  __shared__ float4 part[kRedTaps * 32 > kRedThreads ? kRedTaps * 32 : kRedThreads];
+  const WgradGeom& g = p.g;
+  const int taps = g.kd * g.kh * g.kw;
+  const int k0 = blockIdx.x * 4, c0 = blockIdx.y * CH, t0 = blockIdx.z * kRedTaps;
+  const int nt = min(kRedTaps, taps - t0), nch = min(CH, g.C - c0), items = nt * CH;
+  const int groups = max(1, min(kRedThreads / items, p.splits));   // > 1 only when items <= 128
+  const int n_tile = k0 / p.BN, col = k0 - n_tile * p.BN;
+  const size_t cta_stride = (size_t)p.G * p.BN * 32;               // in float4
+  const float4* ws = reinterpret_cast<const float4*>(p.ws);
+  for (int u = threadIdx.x; u < items * groups; u += kRedThreads) {
+    const int sg = u / items, i = u - sg * items;
+    const int tap = t0 + i / CH, ch = c0 + i % CH;
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (ch < g.C) {
+      const int sl = tap * p.cblocks + ch / p.Cb;
+      const int grp = sl / p.spg, row = (sl - grp * p.spg) * p.Cb + ch % p.Cb;
+      const int gs = grp / p.G, gi = grp - gs * p.G;
+      const float4* src = ws + ((size_t)(gs * p.n_tiles + n_tile) * p.splits) * cta_stride +
+                          ((gi * p.BN + col) / 4) * 128 + row;
+      const int s1 = (sg + 1) * p.splits / groups;
+      int s = sg * p.splits / groups;
+      for (; s + 4 <= s1; s += 4) {
+        float4 q[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[j] = __ldcg(src + (s + j) * cta_stride);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { a.x += q[j].x; a.y += q[j].y; a.z += q[j].z; a.w += q[j].w; }
+      }
+      for (; s < s1; ++s) {
+        const float4 q = __ldcg(src + s * cta_stride);
+        a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
+      }
+    }
+    part[u] = a;
+  }
+  __syncthreads();
+  // element i of the output order: channel i / nt, tap i % nt (adjacent in a packed filter)
+  for (int i = threadIdx.x; i < 4 * nch * nt; i += kRedThreads) {
+    const int kk = i / (nch * nt), r = i - kk * (nch * nt);
+    const int chl = r / nt, tl = r - chl * nt;
+    if (k0 + kk >= g.Kout) continue;
+    float v = 0.f;
+    for (int sg = 0; sg < groups; ++sg)
+      v += reinterpret_cast<const float*>(&part[sg * items + tl * CH + chl])[kk];
+    atomicAdd(p.dW + (t0 + tl) * p.s_tap + (k0 + kk) * p.s_k + (c0 + chl) * p.s_c, p.alpha * v);
+  }
+}
+
 static int wg_largest_tile(int extent, int limit) {
   if (extent <= limit) return extent;
   int best = 1;
@@ -271,27 +326,10 @@ static int wg_largest_tile(int extent, int limit) {
   return best * 2 > limit ? best : limit;
 }
 
-}  // namespace lb
-
-extern "C" {
-
-// x:  [N][D][H][W][C] (strides xs, C contiguous), dy: [N][Do][Ho][Wo][Kout] (strides ys).
-// dW: fp32, element (tap, k, c) at tap*s_tap + k*s_k + c*s_c; the kernel ADDS alpha * grad.
-// geom as in lb_conv_fwd_tc.  Requires C % 8 == 0 and Kout % 8 == 0.
-int lb_conv_wgrad_tc(const void* x, const void* dy, float* dW, const int* geom,
-                     const long long* xs, const long long* ys, long long s_tap, long long s_k,
-                     long long s_c, int in_dtype, float alpha, void* stream_) {
-  using namespace lb;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  WgradParams p;
-  static_assert(sizeof(WgradGeom) == 21 * sizeof(int), "geom layout");
-  memcpy(&p.g, geom, sizeof(WgradGeom));
+// Tiling of a filter gradient; a function of the sizes only.  False: not covered.
+static bool wgrad_plan(WgradParams& p) {
   const WgradGeom& g = p.g;
-  if (g.C % 8 || g.Kout % 8) return -1;
-  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(dy) & 15)) return -1;
-  for (int i = 0; i < 4; ++i)
-    if (xs[i] % 8 || ys[i] % 8) return -1;
-
+  if (g.C % 8 || g.Kout % 8) return false;
   p.Cb = g.C >= 64 ? 64 : (g.C >= 32 ? 32 : 16);
   p.cblocks = (g.C + p.Cb - 1) / p.Cb;
   p.slices_total = g.kd * g.kh * g.kw * p.cblocks;
@@ -299,19 +337,8 @@ int lb_conv_wgrad_tc(const void* x, const void* dy, float* dW, const int* geom,
   p.groups_total = (p.slices_total + p.spg - 1) / p.spg;
   p.BN = g.Kout > 128 ? 256 : (g.Kout > 64 ? 128 : (g.Kout > 32 ? 64 : 32));
   p.n_tiles = (g.Kout + p.BN - 1) / p.BN;
-  p.G = 512 / p.BN < 4 ? 512 / p.BN : 4;
-  if (p.G > p.groups_total) p.G = p.groups_total;
-  p.group_sets = (p.groups_total + p.G - 1) / p.G;
   p.a_layout = p.Cb == 64 ? kLayoutSw128 : (p.Cb == 32 ? kLayoutSw64 : kLayoutSw32);
   p.b_layout = p.BN == 32 ? kLayoutSw64 : kLayoutSw128;
-  p.a_bytes = p.G * 16384;
-  p.stage_bytes = p.a_bytes + 64 * p.BN * 2;
-  p.stages = 200 * 1024 / p.stage_bytes;
-  if (p.stages > 4) p.stages = 4;
-  if (p.stages < 1) return -1;
-  int cols = p.G * p.BN;
-  p.tmem_cols = 32;
-  while (p.tmem_cols < cols) p.tmem_cols *= 2;
 
   p.TW = wg_largest_tile(g.Wo, 64);
   p.TH = wg_largest_tile(g.Ho, 64 / p.TW);
@@ -323,20 +350,82 @@ int lb_conv_wgrad_tc(const void* x, const void* dy, float* dW, const int* geom,
   p.bricks_d = (g.Do + p.TD - 1) / p.TD;
   p.bricks_n = (g.N + p.TN - 1) / p.TN;
   p.bricks_total = p.bricks_w * p.bricks_h * p.bricks_d * p.bricks_n;
-  if ((long long)p.bricks_total * 256 >= (1ll << 32)) return -1;
+  if ((long long)p.bricks_total * 256 >= (1ll << 32)) return false;
   p.fd_bw = FastDiv((uint32_t)p.bricks_w);
   p.fd_bh = FastDiv((uint32_t)p.bricks_h);
   p.fd_bd = FastDiv((uint32_t)p.bricks_d);
 
-  const int base_ctas = p.group_sets * p.n_tiles;
-  int splits = (2 * lbhost::sm_count() + base_ctas - 1) / base_ctas;
-  // keep at least 8 bricks per CTA so the pipeline fill is amortised
-  if (splits > (p.bricks_total + 7) / 8) splits = (p.bricks_total + 7) / 8;
-  if (splits < 1) splits = 1;
-  p.splits = splits;
+  // Accumulators per CTA (G) and splits of the pixels: the choice with the shortest longest CTA.
+  // A brick costs its bytes at the ~58 B/clk that an SM's copies bring in (or ~75 cycles per
+  // box), or its MMAs (44 / 48 / 64 / 128 cycles at N = 32 / 64 / 128 / 256), whichever is
+  // longer; with two stages in flight part of the copies' latency shows, with one all of it.
+  // The workspace (CTAs x G x BN rows) is bounded by one wave of CTAs, except where the filter
+  // alone needs more of them.
+  const int sms = lbhost::sm_count();
+  const int mma = p.BN == 32 ? 44 : (p.BN == 64 ? 48 : (p.BN == 128 ? 64 : 128));
+  const int g_max = min(min(512 / p.BN, 4), p.groups_total);
+  double best = 0.0;
+  for (int G = g_max; G >= 1; --G) {
+    const int stage_bytes = G * 16384 + 64 * p.BN * 2;
+    int stages = (232448 - 2048) / stage_bytes;
+    if (stages > 4) stages = 4;
+    if (stages < 1) continue;
+    const int sets = (p.groups_total + G - 1) / G, base = sets * p.n_tiles;
+    int splits = base < sms ? sms / base : 1;
+    if (splits > (p.bricks_total + 3) / 4) splits = (p.bricks_total + 3) / 4;   // amortise the pipeline fill
+    const int waves = (base * splits + sms - 1) / sms;
+    const double copy = max(stage_bytes / 58.0, 75.0 * (G * p.spg + p.BN / 64));
+    const double brick = max(copy, 4.0 * G * mma) * (stages >= 3 ? 1.0 : (stages == 2 ? 1.25 : 2.0));
+    const double cost = waves * (((p.bricks_total + splits - 1) / splits) * brick + 3000.0);
+    if (best == 0.0 || cost < best) {
+      best = cost;
+      p.G = G; p.group_sets = sets; p.splits = splits; p.stages = stages; p.stage_bytes = stage_bytes;
+    }
+  }
+  if (best == 0.0) return false;
+  p.a_bytes = p.G * 16384;
+  const int cols = p.G * p.BN;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < cols) p.tmem_cols *= 2;
+  return true;
+}
+
+static long long wgrad_ws_floats(const WgradParams& p) {
+  return (long long)p.group_sets * p.n_tiles * p.splits * p.G * p.BN * 128;
+}
+
+}  // namespace lb
+
+extern "C" {
+
+// fp32 words of workspace that lb_conv_wgrad_tc needs for these sizes; -1: not covered.
+long long lb_conv_wgrad_ws(const int* geom) {
+  lb::WgradParams p;
+  memcpy(&p.g, geom, sizeof(lb::WgradGeom));
+  return lb::wgrad_plan(p) ? lb::wgrad_ws_floats(p) : -1;
+}
+
+// x:  [N][D][H][W][C] (strides xs, C contiguous), dy: [N][Do][Ho][Wo][Kout] (strides ys).
+// dW: fp32, element (tap, k, c) at tap*s_tap + k*s_k + c*s_c; the kernel ADDS alpha * grad.
+// geom as in lb_conv_fwd_tc; ws: lb_conv_wgrad_ws(geom) words, 16-byte aligned, whose contents
+// do not matter.  Requires C % 8 == 0 and Kout % 8 == 0.
+int lb_conv_wgrad_tc(const void* x, const void* dy, float* dW, float* ws, const int* geom,
+                     const long long* xs, const long long* ys, long long s_tap, long long s_k,
+                     long long s_c, int in_dtype, float alpha, void* stream_) {
+  using namespace lb;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  WgradParams p;
+  static_assert(sizeof(WgradGeom) == 21 * sizeof(int), "geom layout");
+  memcpy(&p.g, geom, sizeof(WgradGeom));
+  const WgradGeom& g = p.g;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(dy) & 15)) return -1;
+  for (int i = 0; i < 4; ++i)
+    if (xs[i] % 8 || ys[i] % 8) return -1;
+  if (!wgrad_plan(p) || !ws || (reinterpret_cast<uintptr_t>(ws) & 15)) return -1;
   p.in_dtype = in_dtype;
   p.alpha = alpha;
   p.dW = dW;
+  p.ws = ws;
   p.s_tap = s_tap; p.s_k = s_k; p.s_c = s_c;
 
   const uint32_t bw = (p.TW - 1) * g.sw + 1, bh = (p.TH - 1) * g.sh + 1, bd = (p.TD - 1) * g.sd + 1;
@@ -368,6 +457,13 @@ int lb_conv_wgrad_tc(const void* x, const void* dy, float* dW, const int* geom,
   }
   const int grid = p.group_sets * p.n_tiles * p.splits;
   conv_wgrad_kernel<<<grid, 192, smem, stream>>>(tmX, tmDy, p, lbhost::status_word());
+  const int rc = (int)cudaGetLastError();
+  if (rc) return rc;
+  // 32 channels a block where that gives enough blocks to fill the GPU, else fewer
+  const int taps = g.kd * g.kh * g.kw, kq = (g.Kout + 3) / 4, tz = (taps + kRedTaps - 1) / kRedTaps;
+  int CH = 32;
+  while (CH > 8 && (long long)kq * ((g.C + CH - 1) / CH) * tz < 2 * lbhost::sm_count()) CH /= 2;
+  wgrad_reduce_kernel<<<dim3(kq, (g.C + CH - 1) / CH, tz), kRedThreads, 0, stream>>>(p, CH);
   return (int)cudaGetLastError();
 }
 

@@ -32,8 +32,10 @@ def _lib():
             ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
             c_int, c_int, c_float, c_float, c_int, c_float, c_void_p, c_void_p]
         lib.lb_conv_wgrad_tc.restype = c_int
+        lib.lb_conv_wgrad_ws.restype = ctypes.c_longlong
+        lib.lb_conv_wgrad_ws.argtypes = [ctypes.POINTER(c_int)]
         lib.lb_conv_wgrad_tc.argtypes = [
-            c_void_p, c_void_p, c_void_p, ctypes.POINTER(c_int),
+            c_void_p, c_void_p, c_void_p, c_void_p, ctypes.POINTER(c_int),
             ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
             ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, c_int, c_float, c_void_p]
         _configured = True
@@ -175,9 +177,11 @@ def conv_wgrad(x: torch.Tensor, dy: torch.Tensor, ksize, *, pad=0, stride=1, dil
                         dd, dh, dw)
     xs = (ctypes.c_longlong * 4)(x.stride(0), x.stride(1), x.stride(2), x.stride(3))
     ys = (ctypes.c_longlong * 4)(dy.stride(0), dy.stride(1), dy.stride(2), dy.stride(3))
-    rc = _lib().lb_conv_wgrad_tc(x.data_ptr(), dy.data_ptr(), out.data_ptr(), geom, xs, ys,
+    words = _lib().lb_conv_wgrad_ws(geom)       # -1: not covered, reported by the launch
+    ws = torch.empty(words, dtype=torch.float32, device=x.device) if words > 0 else None
+    rc = _lib().lb_conv_wgrad_tc(x.data_ptr(), dy.data_ptr(), out.data_ptr(), native.ptr(ws), geom, xs, ys,
                                  1, C * taps, taps, native.dtype_code(x.dtype), float(alpha),
                                  native.stream_ptr())
     native.check(rc, "lb_conv_wgrad_tc")
-    native.count_launch()
+    native.count_launch(2)
     return out

@@ -102,6 +102,39 @@ def test_conv_wgrad(case):
     torch.testing.assert_close(got, ref, rtol=2e-3, atol=2e-2 * (N * D * H * W) ** 0.5 / 8)
 
 
+@pytest.mark.parametrize("case", [
+    # N, C, D, H, W, K, k: the splits of the pixels and the blocks of the reduction at their edges
+    (1, 8, 1, 4, 4, 8, 1),          # one brick, one tap, 8 channels and filters
+    (1, 48, 1, 9, 17, 40, 3),       # a part of a channel slice, bricks with unused rows
+    (2, 24, 3, 7, 5, 72, 5),        # 125 taps: four tap blocks, the last one ragged
+    (3, 520, 1, 6, 6, 264, 1),      # more channel blocks and filter tiles than fit one of each
+    (8, 64, 1, 40, 56, 64, 3),      # one CTA per SM and split, many split groups
+    (1, 256, 4, 4, 4, 256, 3),      # few bricks, a filter that fills the GPU by itself
+])
+def test_conv_wgrad_reduction(case):
+    """fp32 partial sums of exact products: against 64 bits the error is that of summation, which
+    grows like sqrt(terms) * 2^-24 (below 2e-6 for the largest here); the same call twice gives the same bits."""
+    from lbann_b200.ops.conv import conv_wgrad
+    N, C, D, H, W, K, k = case
+    torch.manual_seed(7)
+    ks = (1 if D == 1 else k, k, k)
+    pd = tuple(v // 2 for v in ks)
+    x = torch.randn(N, D, H, W, C, device="cuda").bfloat16()
+    dy = torch.randn(N, D, H, W, K, device="cuda").bfloat16()
+    got = conv_wgrad(x, dy, ks, pad=pd)
+    again = conv_wgrad(x, dy, ks, pad=pd)
+    assert native.consume_status() == 0
+    xp = F.pad(x.double(), (0, 0, pd[2], pd[2], pd[1], pd[1], pd[0], pd[0]))
+    ref = torch.empty(K, C, *ks, device="cuda", dtype=torch.double)
+    for a in range(ks[0]):
+        for b in range(ks[1]):
+            for c in range(ks[2]):
+                view = xp[:, a:a + D, b:b + H, c:c + W].reshape(-1, C)
+                ref[:, :, a, b, c] = dy.double().reshape(-1, K).t() @ view
+    assert torch.equal(got, again)
+    assert float((got.double() - ref).norm() / ref.norm()) < 4e-6
+
+
 @pytest.mark.parametrize("case", [(2, 256, 8, 8, 8, 256), (1, 128, 4, 16, 16, 200), (3, 64, 1, 12, 12, 96)])
 def test_conv_deep_layers_split_the_reduction(case, monkeypatch):
     """The deep layers of a network on a small batch: a handful of output bricks, thousands of
