@@ -1,4 +1,4 @@
-"""In-tree native build: every ``csrc/*.cu`` / ``csrc/*.cpp`` -> ``_native/liblbann_b200.so``.
+"""In-tree native build: every ``csrc/*.cu`` / ``csrc/*.cpp`` -> ``_native/*.so``.
 
 The kernels are plain CUDA C++ with ``extern "C"`` launchers (no torch headers), so a
 file compiles in seconds and the library can be loaded with ``ctypes`` by any host
@@ -18,6 +18,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "_native")
 LIB_NAME = "liblbann_b200.so"
 HOST_LIB_NAME = "liblbann_b200_host.so"
+NODES_SRC = "autograd_nodes.cpp"            # the one source that is written against PyTorch's headers
+NODES_NAME = "_lbann_autograd.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -44,6 +46,28 @@ def _digest(path: str, extra: str) -> str:
     return h.hexdigest()
 
 
+def _nodes_flags():
+    """Include paths and defines of the autograd nodes (a Python extension module)."""
+    import sysconfig
+
+    import torch
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    return ["-DTORCH_API_INCLUDE_EXTENSION_H", "-DTORCH_EXTENSION_NAME=_lbann_autograd",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", inc, "-I",
+            os.path.join(inc, "torch", "csrc", "api", "include"), "-I", cuda, "-I", sysconfig.get_paths()["include"]]
+
+
+def _link_nodes(obj: str, out: str) -> None:
+    import torch
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-shared", "-o", out, obj, "-L", OUT_DIR, f"-l:{LIB_NAME}", "-L", libs, "-ltorch_python", "-ltorch",
+           "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+
+
 def _compile_one(cmd, src, obj, stamp, digest, verbose):
     if verbose:
         print("[lbann_b200 build]", os.path.basename(src), flush=True)
@@ -63,8 +87,8 @@ def build_native(verbose: bool = False, force: bool = False) -> dict:
     cu_srcs = sorted(f for f in os.listdir(CSRC) if f.endswith(".cu"))
     cpp_srcs = sorted(f for f in os.listdir(CSRC) if f.endswith(".cpp"))
     jobs = []
-    cu_objs, cpp_objs = [], []
-    relink_cu = relink_cpp = force
+    cu_objs, cpp_objs, nodes_obj = [], [], None
+    relink_cu = relink_cpp = relink_nodes = force
     for name in cu_srcs + cpp_srcs:
         src = os.path.join(CSRC, name)
         obj = os.path.join(obj_dir, name + ".o")
@@ -75,13 +99,19 @@ def build_native(verbose: bool = False, force: bool = False) -> dict:
             cu_objs.append(obj)
         else:
             cmd = ["g++"] + CXX_FLAGS + ["-I", CSRC, "-c", src, "-o", obj]
-            cpp_objs.append(obj)
+            if name == NODES_SRC:
+                cmd[1:1] = _nodes_flags()
+                nodes_obj = obj
+            else:
+                cpp_objs.append(obj)
         digest = _digest(src, " ".join(cmd))
         old = open(stamp).read() if os.path.exists(stamp) else ""
         if force or old != digest or not os.path.exists(obj):
             jobs.append((cmd, src, obj, stamp, digest, verbose))
             if is_cu:
                 relink_cu = True
+            elif name == NODES_SRC:
+                relink_nodes = True
             else:
                 relink_cpp = True
     if jobs:
@@ -101,7 +131,10 @@ def build_native(verbose: bool = False, force: bool = False) -> dict:
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    return {"cuda": lib if cu_objs else None, "host": host_lib if cpp_objs else None}
+    nodes = os.path.join(OUT_DIR, NODES_NAME)
+    if nodes_obj and (relink_nodes or not os.path.exists(nodes)):
+        _link_nodes(nodes_obj, nodes)
+    return {"cuda": lib if cu_objs else None, "host": host_lib if cpp_objs else None, "nodes": nodes}
 
 
 if __name__ == "__main__":

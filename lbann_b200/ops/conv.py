@@ -12,35 +12,7 @@ import ctypes
 import torch
 
 from . import native
-from .native import c_float, c_int, c_void_p
-
-_configured = False
-
-
-def _lib():
-    global _configured
-    lib = native.cuda_lib()
-    if not _configured:
-        lib.lb_conv_fwd_tc.restype = c_int
-        lib.lb_conv_fwd_tc.argtypes = [
-            c_void_p, c_void_p, c_void_p, c_void_p, ctypes.POINTER(c_int),
-            ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
-            c_int, c_int, c_float, c_float, c_int, c_float, c_void_p]
-        lib.lb_conv_fwd_halo_tc.restype = c_int
-        lib.lb_conv_fwd_halo_tc.argtypes = [
-            c_void_p, c_void_p, c_void_p, c_void_p, ctypes.POINTER(c_int),
-            ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
-            c_int, c_int, c_float, c_float, c_int, c_float, c_void_p, c_void_p]
-        lib.lb_conv_wgrad_tc.restype = c_int
-        lib.lb_conv_wgrad_ws.restype = ctypes.c_longlong
-        lib.lb_conv_wgrad_ws.argtypes = [ctypes.POINTER(c_int)]
-        lib.lb_conv_wgrad_tc.argtypes = [
-            c_void_p, c_void_p, c_void_p, c_void_p, ctypes.POINTER(c_int),
-            ctypes.POINTER(ctypes.c_longlong), ctypes.POINTER(ctypes.c_longlong),
-            ctypes.c_longlong, ctypes.c_longlong, ctypes.c_longlong, c_int, c_float, c_void_p]
-        _configured = True
-    return lib
-
+from .native import c_void_p
 
 class HaloSyncArgs(ctypes.Structure):
     """Mirror of ``lb::HaloSyncArgs`` (csrc/halo_sync.cuh)."""
@@ -121,29 +93,10 @@ def conv_fwd(x: torch.Tensor, w_taps: torch.Tensor, ksize, *, pad=0, stride=1, d
 
     if x.stride(4) != 1:
         raise ValueError("conv_fwd: channel dimension must be contiguous")
-    if w_taps.dtype != x.dtype or not w_taps.is_contiguous():
-        w_taps = w_taps.to(x.dtype).contiguous()
-    if out is None:
-        out = torch.empty((N, Do, Ho, Wo, Kout), dtype=out_dtype, device=x.device)
-        if beta != 0.0:
-            out.zero_()
-    geom = (c_int * 21)(N, D, H, W, C, Do, Ho, Wo, Kout, kd, kh, kw, pd, ph, pw, sd, sh, sw,
-                        dd, dh, dw)
-    xs = (ctypes.c_longlong * 4)(x.stride(0), x.stride(1), x.stride(2), x.stride(3))
-    ys = (ctypes.c_longlong * 4)(out.stride(0), out.stride(1), out.stride(2), out.stride(3))
-    if bias is not None and bias.dtype != torch.float32:
-        bias = bias.float()
-    scratch = native.offer_splitk(N * Do * Ho * Wo, Kout, x.device) if C * kd * kh * kw >= 512 else None
-    rc = _lib().lb_conv_fwd_halo_tc(x.data_ptr(), w_taps.data_ptr(), out.data_ptr(), native.ptr(bias),
-                                    geom, xs, ys, native.dtype_code(x.dtype),
-                                    native.dtype_code(out.dtype), float(alpha), float(beta), int(act),
-                                    float(act_param),
-                                    ctypes.cast(ctypes.pointer(halo), c_void_p) if halo is not None else None,
-                                    native.stream_ptr())
-    native.check(rc, "lb_conv_fwd_halo_tc")
-    native.count_launch()
-    del scratch
-    return out
+    return native.nodes().conv_fwd(x, w_taps, out, native.dtype_code(out_dtype),
+                                   (kd, kh, kw, pd, ph, pw, sd, sh, sw, dd, dh, dw), (Do, Ho, Wo), float(alpha),
+                                   float(beta), bias, int(act), float(act_param),
+                                   ctypes.addressof(halo) if halo is not None else 0)
 
 
 def conv_wgrad(x: torch.Tensor, dy: torch.Tensor, ksize, *, pad=0, stride=1, dilation=1,
@@ -171,17 +124,5 @@ def conv_wgrad(x: torch.Tensor, dy: torch.Tensor, ksize, *, pad=0, stride=1, dil
         return out
     if out.dtype != torch.float32 or not out.is_contiguous():
         raise ValueError("conv_wgrad: out must be a contiguous fp32 tensor")
-    if dy.dtype != x.dtype:
-        dy = dy.to(x.dtype)
-    geom = (c_int * 21)(N, D, H, W, C, Do, Ho, Wo, Kout, kd, kh, kw, pd, ph, pw, sd, sh, sw,
-                        dd, dh, dw)
-    xs = (ctypes.c_longlong * 4)(x.stride(0), x.stride(1), x.stride(2), x.stride(3))
-    ys = (ctypes.c_longlong * 4)(dy.stride(0), dy.stride(1), dy.stride(2), dy.stride(3))
-    words = _lib().lb_conv_wgrad_ws(geom)       # -1: not covered, reported by the launch
-    ws = torch.empty(words, dtype=torch.float32, device=x.device) if words > 0 else None
-    rc = _lib().lb_conv_wgrad_tc(x.data_ptr(), dy.data_ptr(), out.data_ptr(), native.ptr(ws), geom, xs, ys,
-                                 1, C * taps, taps, native.dtype_code(x.dtype), float(alpha),
-                                 native.stream_ptr())
-    native.check(rc, "lb_conv_wgrad_tc")
-    native.count_launch(2)
+    native.nodes().conv_wgrad(x, dy, out, (kd, kh, kw, pd, ph, pw, sd, sh, sw, dd, dh, dw), float(alpha))
     return out

@@ -12,7 +12,6 @@ import math
 import torch
 
 from . import native
-from .native import c_float, c_int, c_ll, c_void_p
 
 UNARY = ["identity", "logical_not", "abs", "negative", "sign", "round", "ceil", "floor",
          "reciprocal", "square", "sqrt", "rsqrt", "safe_reciprocal", "exp", "expm1", "log",
@@ -135,22 +134,6 @@ _CPU_BINARY = {
     "boolean_false_positive": lambda a, b: ((a >= 0.5) & (b < 0.5)).to(a.dtype),
 }
 
-_configured = False
-
-
-def _lib():
-    global _configured
-    lib = native.cuda_lib()
-    if not _configured:
-        lib.lb_unary.restype = c_int
-        lib.lb_unary.argtypes = [c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_float,
-                                 c_float, c_int, c_void_p]
-        lib.lb_binary.restype = c_int
-        lib.lb_binary.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_int,
-                                  c_int, c_int, c_void_p]
-        _configured = True
-    return lib
-
 
 def _dense(t: torch.Tensor) -> bool:
     return t.is_contiguous() or t.is_contiguous(memory_format=torch.channels_last) or \
@@ -160,86 +143,15 @@ def _dense(t: torch.Tensor) -> bool:
 def unary_raw(code: int, x, dy, p0: float, p1: float, mode: int):
     """Launch the unary kernel on a dense tensor (any memory format); returns a tensor with
     the same strides as ``x``."""
-    out = torch.empty_like(x)
-    rc = _lib().lb_unary(x.data_ptr(), native.ptr(dy), out.data_ptr(), x.numel(), code, mode,
-                         float(p0), float(p1), native.dtype_code(x.dtype), native.stream_ptr())
-    native.check(rc, "lb_unary")
-    native.count_launch()
-    return out
-
-
-class _Unary(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, code, p0, p1):
-        ctx.save_for_backward(x)
-        ctx.args = (code, p0, p1)
-        return unary_raw(code, x, None, p0, p1, 0)
-
-    @staticmethod
-    def backward(ctx, dy):
-        (x,) = ctx.saved_tensors
-        code, p0, p1 = ctx.args
-        if dy.stride() != x.stride():
-            dy = torch.empty_like(x).copy_(dy)
-        return unary_raw(code, x, dy, p0, p1, 1), None, None, None
-
-
-class _Binary(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, a, b, code):
-        ctx.save_for_backward(a, b)
-        ctx.code = code
-        out = torch.empty_like(a)
-        rc = _lib().lb_binary(a.data_ptr(), b.data_ptr(), 0, out.data_ptr(), 0, a.numel(), code,
-                              0, native.dtype_code(a.dtype), native.stream_ptr())
-        native.check(rc, "lb_binary")
-        native.count_launch()
-        return out
-
-    @staticmethod
-    def backward(ctx, dy):
-        a, b = ctx.saved_tensors
-        if ctx.code == BINARY_CODE["add"]:
-            return dy, dy, None          # no kernel, no copies
-        if dy.stride() != a.stride():
-            dy = torch.empty_like(a).copy_(dy)
-        da, db = torch.empty_like(a), torch.empty_like(a)
-        rc = _lib().lb_binary(a.data_ptr(), b.data_ptr(), dy.data_ptr(), da.data_ptr(),
-                              db.data_ptr(), a.numel(), ctx.code, 1,
-                              native.dtype_code(a.dtype), native.stream_ptr())
-        native.check(rc, "lb_binary")
-        native.count_launch()
-        return da, db, None
-
-
-class _AddRelu(torch.autograd.Function):
-    """relu(a + b) in one kernel; backward is one masking pass on the saved output and both
-    inputs receive the same gradient tensor."""
-
-    @staticmethod
-    def forward(ctx, a, b):
-        out = torch.empty_like(a)
-        rc = _lib().lb_binary(a.data_ptr(), b.data_ptr(), 0, out.data_ptr(), 0, a.numel(),
-                              BINARY_CODE["add_relu"], 0, native.dtype_code(a.dtype), native.stream_ptr())
-        native.check(rc, "lb_binary")
-        native.count_launch()
-        ctx.save_for_backward(out)
-        return out
-
-    @staticmethod
-    def backward(ctx, dy):
-        (out,) = ctx.saved_tensors
-        if dy.stride() != out.stride():
-            dy = torch.empty_like(out).copy_(dy)
-        g = unary_raw(UNARY_CODE["relu"], out, dy, 0.0, 0.0, 1)
-        return g, g
+    return native.nodes().unary_raw(code, x, dy, float(p0), float(p1), mode)
 
 
 def add_relu(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
-    """relu(a + b); one native kernel each way for dense same-layout CUDA tensors."""
+    """relu(a + b); one native kernel each way for dense same-layout CUDA tensors (backward is a
+    masking pass on the saved output, and both inputs receive the same gradient tensor)."""
     if (a.is_cuda and a.dtype in _NATIVE_DTYPES and a.dtype == b.dtype and a.shape == b.shape
             and a.stride() == b.stride() and _dense(a) and a.numel() > 0):
-        return _AddRelu.apply(a, b)
+        return native.nodes().add_relu(a, b, BINARY_CODE["add_relu"], UNARY_CODE["relu"])
     return torch.relu(a + b)
 
 
@@ -248,12 +160,12 @@ _NATIVE_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 
 def unary(name: str, x: torch.Tensor, p0: float = 0.0, p1: float = 0.0) -> torch.Tensor:
     if x.is_cuda and x.dtype in _NATIVE_DTYPES and _dense(x) and x.numel() > 0:
-        return _Unary.apply(x, UNARY_CODE[name], float(p0), float(p1))
+        return native.nodes().unary(x, UNARY_CODE[name], float(p0), float(p1))
     return _CPU_UNARY[name](x, p0, p1)
 
 
 def binary(name: str, a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     if (a.is_cuda and a.dtype in _NATIVE_DTYPES and a.shape == b.shape and a.dtype == b.dtype
             and a.stride() == b.stride() and _dense(a) and a.numel() > 0):
-        return _Binary.apply(a, b, BINARY_CODE[name])
+        return native.nodes().binary(a, b, BINARY_CODE[name], name == "add")
     return _CPU_BINARY[name](a, b)

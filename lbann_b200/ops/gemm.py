@@ -10,12 +10,9 @@ scale factors used to accumulate straight into optimizer buffers
 """
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import native
-from .native import c_float, c_int, c_ll, c_void_p
 
 _ACT_FN = {
     native.ACT_NONE: lambda x, p: x,
@@ -25,34 +22,6 @@ _ACT_FN = {
     native.ACT_TANH: lambda x, p: torch.tanh(x),
     native.ACT_SIGMOID: lambda x, p: torch.sigmoid(x),
 }
-
-_configured = False
-
-
-def _lib():
-    global _configured
-    lib = native.cuda_lib()
-    if not _configured:
-        lib.lb_gemm_tc.restype = c_int
-        lib.lb_gemm_tc.argtypes = [
-            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-            c_ll, c_ll, c_ll, c_ll, c_ll, c_ll, c_int, c_int, c_int, c_int,
-            c_float, c_float, c_int, c_int, c_float, c_int, c_void_p]
-        _configured = True
-    return lib
-
-
-def _tma_ready(t: torch.Tensor) -> torch.Tensor:
-    """Return ``t`` or a copy whose rows start on 16-byte boundaries with a legal pitch."""
-    if t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and t.stride(-2) % 8 == 0 and (
-            t.dim() == 2 or (t.stride(0) % 8 == 0 and t.stride(0) >= 0)):
-        return t
-    cols = t.shape[-1]
-    pitch = (cols + 7) // 8 * 8
-    buf = torch.zeros(*t.shape[:-1], pitch, dtype=t.dtype, device=t.device)
-    buf[..., :cols].copy_(t)
-    return buf[..., :cols]
-
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bool = False,
          out: torch.Tensor | None = None, out_dtype: torch.dtype | None = None,
@@ -86,32 +55,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, trans_a: bool = False, trans_b: bo
         out.copy_(acc)
         return out
 
-    if a.dtype not in (torch.float16, torch.bfloat16):
-        a = a.to(torch.bfloat16)
-    if b.dtype != a.dtype:
-        b = b.to(a.dtype)
-    a = _tma_ready(a)
-    b = _tma_ready(b)
-    if out is None:
-        shape = (nb, M, N) if batched else (M, N)
-        out = torch.empty(shape, dtype=out_dtype, device=a.device)
-        if beta != 0.0:
-            out.zero_()
-    elif out.stride(-1) != 1:
+    if out is not None and out.stride(-1) != 1:
         raise ValueError("gemm: output must have unit stride in its last dimension")
-    if bias is not None and bias.dtype != torch.float32:
-        bias = bias.float()
-    scratch = native.offer_splitk(M * nb, N, a.device) if K >= 512 else None
-    rc = _lib().lb_gemm_tc(
-        a.data_ptr(), b.data_ptr(), out.data_ptr(), native.ptr(bias), M, N, K, nb,
-        a.stride(-2), b.stride(-2), out.stride(-2),
-        a.stride(0) if batched else 0, b.stride(0) if batched else 0,
-        out.stride(0) if batched else 0,
-        1 if trans_a else 0, 0 if trans_b else 1,
-        native.dtype_code(a.dtype), native.dtype_code(out.dtype),
-        float(alpha), float(beta), 2 if bias_per_row else 1, int(act), float(act_param),
-        int(bn_hint), native.stream_ptr())
-    native.check(rc, "lb_gemm_tc")
-    native.count_launch()
-    del scratch         # enqueued: the allocator may hand the workspace to later work of this stream
-    return out
+    return native.nodes().gemm(a, b, bool(trans_a), bool(trans_b), out, native.dtype_code(out_dtype), float(alpha),
+                               float(beta), bias, bool(bias_per_row), int(act), float(act_param), int(bn_hint))

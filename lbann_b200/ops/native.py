@@ -18,6 +18,7 @@ _NATIVE = os.path.join(os.path.dirname(_HERE), "_native")
 _lock = threading.Lock()
 _cuda = None
 _host = None
+_nodes = None
 
 c_void_p = ctypes.c_void_p
 c_int = ctypes.c_int
@@ -86,6 +87,27 @@ def host_lib():
     return _host
 
 
+def nodes():
+    """The C++ autograd nodes (``csrc/autograd_nodes.cpp``): the launches of the tensor-core
+    kernels and the forward / backward functions of the layers built on them."""
+    global _nodes
+    if _nodes is None:
+        with_lib = cuda_lib()
+        with _lock:
+            if _nodes is None and with_lib is not None:
+                import importlib.util
+                path = os.path.join(_NATIVE, "_lbann_autograd.so")
+                if not os.path.exists(path):
+                    from .. import _build
+                    _build.build_native()
+                spec = importlib.util.spec_from_file_location("_lbann_autograd", path)
+                mod = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(mod)
+                mod.set_error_type(NativeError)
+                _nodes = mod
+    return _nodes
+
+
 def have_cuda_lib() -> bool:
     return os.path.exists(os.path.join(_NATIVE, "liblbann_b200.so"))
 
@@ -147,33 +169,11 @@ def count_launch(n: int = 1) -> None:
 
 
 def launches() -> int:
-    return _launch_count
+    return _launch_count + (_nodes.launches() if _nodes is not None else 0)
 
 
-# --------------------------------------------------------------------------- split-K scratch
-_splitk_sms: dict = {}      # device index -> SM count
-splitk_offers = 0           # how many launches were lent scratch (tests read it)
-
-
-def offer_splitk(rows: int, cols: int, device) -> "torch.Tensor | None":
-    """Lends scratch memory to the GEMM / convolution launch that the calling thread makes
-    NEXT, so that a product with few output tiles and a long reduction can be cut along the
-    reduction (``csrc/tc_pipeline.cuh``).  Offered only where that can pay: an output of at
-    most half a wave of 128 x 256 tiles.  Returns the workspace tensor; the caller holds it
-    until the launch is enqueued."""
-    global splitk_offers
-    if rows * cols > 74 * 128 * 256 or os.environ.get("LBANN_DISABLE_SPLITK", "") not in ("", "0"):
-        return None
-    device = torch.device(device)
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    lib = cuda_lib()
-    sms = _splitk_sms.get(idx)
-    if sms is None:
-        lib.lb_splitk_offer.restype = c_int
-        lib.lb_splitk_offer.argtypes = [c_void_p, ctypes.c_longlong]
-        sms = _splitk_sms[idx] = int(lib.lb_sm_count())
-    bn = 256 if cols > 128 else 128
-    ws = torch.empty(sms * 128 * bn, dtype=torch.float32, device=device)
-    check(lib.lb_splitk_offer(ws.data_ptr(), ws.numel() * 4), "lb_splitk_offer")
-    splitk_offers += 1
-    return ws
+def __getattr__(name):
+    # how many launches were lent scratch for a split of their reduction (tests read it)
+    if name == "splitk_offers":
+        return _nodes.splitk_offers() if _nodes is not None else 0
+    raise AttributeError(f"module '{__name__}' has no attribute '{name}'")

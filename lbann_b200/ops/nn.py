@@ -49,30 +49,10 @@ def _lib():
         VPP = P(c_void_p)
         lib.lb_bn_fused_ws_floats.restype = c_int
         lib.lb_bn_fused_ws_floats.argtypes = [c_int]
-        lib.lb_bn_fused_fwd.restype = c_int
-        lib.lb_bn_fused_fwd.argtypes = [c_void_p] * 8 + [c_ll, c_int, c_float, c_float, c_float, c_float,
-                                                       c_int, c_float, c_int, VPP, VPP, c_int, c_int, c_ll,
-                                                       c_void_p, c_void_p]
-        lib.lb_bn_fused_bwd.restype = c_int
-        lib.lb_bn_fused_bwd.argtypes = [c_void_p] * 9 + [c_ll, c_int, c_float, c_float, c_float, c_int,
-                                                       c_float, c_int, VPP, VPP, c_int, c_int, c_ll,
-                                                       c_void_p, c_void_p]
         lib.lb_pool_bwd.restype = c_int
         lib.lb_pool_bwd.argtypes = [c_void_p, c_void_p, c_void_p, P(c_int), P(c_ll), c_int, c_void_p]
-        lib.lb_layer_norm_fwd.restype = c_int
-        lib.lb_layer_norm_fwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                          c_ll, c_int, c_float, c_int, c_void_p]
-        lib.lb_layer_norm_bwd.restype = c_int
-        lib.lb_layer_norm_bwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                          c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p]
         lib.lb_bn_partial_sums.restype = c_int
         lib.lb_bn_partial_sums.argtypes = [c_void_p, c_void_p, c_ll, c_int, c_int, c_int, c_int, c_void_p]
-        lib.lb_pack_filter.restype = c_int
-        lib.lb_pack_filter.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
-                                       c_int, c_void_p]
-        lib.lb_outer_accum.restype = c_int
-        lib.lb_outer_accum.argtypes = [c_void_p, c_void_p, c_void_p, c_int, c_int, c_ll, c_float,
-                                       c_float, c_int, c_void_p]
         lib.lb_bn_finalize_apply.restype = c_int
         lib.lb_bn_finalize_apply.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                              c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int,
@@ -210,83 +190,37 @@ def _act_grad_from_output(y: torch.Tensor, dy: torch.Tensor, act: int, p: float)
 
 
 # --------------------------------------------------------------------------- linear
-class _Linear(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w_leaf, b_leaf, wh: WeightHandle, bh: Optional[WeightHandle], act, act_p):
-        x2 = x.reshape(-1, x.shape[-1])
-        if not x2.is_contiguous():
-            x2 = x2.contiguous()
-        w16 = wh.cast(x.dtype)
-        bias = bh.master.detach() if bh is not None else None
-        y = gemm(x2, w16, trans_b=True, bias=bias, act=act, act_param=act_p)
-        ctx.save_for_backward(x2, y if act != native.ACT_NONE else None)
-        ctx.meta = (wh, bh, act, act_p, x.shape)
-        return y.reshape(*x.shape[:-1], w16.shape[0])
-
-    @staticmethod
-    def backward(ctx, dy):
-        x2, y = ctx.saved_tensors
-        wh, bh, act, act_p, xshape = ctx.meta
-        dy2 = dy.reshape(-1, dy.shape[-1])
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        dy2 = _act_grad_from_output(y, dy2, act, act_p) if y is not None else dy2
-        dx = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm(dy2, wh.cast(dy2.dtype)).reshape(xshape)
-        if wh.grad is not None:
-            _weight_grad(dy2, x2, wh.grad.view(wh.master.shape))
-            wh.mark_ready()     # data-parallel runs start reducing this gradient right away
-        if bh is not None and bh.grad is not None:
-            bh.grad.add_(column_sums(dy2))
-            bh.mark_ready()
-        return dx, None, None, None, None, None, None
-
-
 def _pack_both(wh: WeightHandle, dtype: torch.dtype, Kout, Cin, Kp, Cp, ksize) -> None:
     """Fill the handle's cache with the forward and the data-gradient filter layouts in one
     launch (they are valid until the optimizer changes the weights)."""
     if ("fwd", dtype) in wh._cache or not wh.master.is_cuda or wh.master.dtype != torch.float32:
         return
-    m = wh.master.detach()
+    m = wh.master
     if not m.is_contiguous():
         return
     taps = 1
     for k in ksize:
         taps *= int(k)
-    fwd = torch.empty((taps, Kp, Cp), dtype=dtype, device=m.device)
-    dgrad = torch.empty((taps, Cp, Kp), dtype=dtype, device=m.device)
-    rc = _lib().lb_pack_filter(m.data_ptr(), fwd.data_ptr(), dgrad.data_ptr(), Kout, Cin, taps, Kp, Cp,
-                               native.dtype_code(dtype), native.stream_ptr())
-    native.check(rc, "lb_pack_filter")
-    native.count_launch()
-    wh._cache[("fwd", dtype)] = fwd
-    wh._cache[("dgrad", dtype)] = dgrad
+    wh._cache[("fwd", dtype)], wh._cache[("dgrad", dtype)] = native.nodes().pack_filter(
+        m, Kout, Cin, taps, Kp, Cp, native.dtype_code(dtype))
 
 
 def _weight_grad(dy2: torch.Tensor, x2: torch.Tensor, grad: torch.Tensor) -> None:
-    """grad[out, in] += dy2^T x2.  Mini-batches of at most 16 rows make this a rank-K update
-    bound by the fp32 read-modify-write of ``grad``; a plain kernel does it at memory speed,
-    everything else goes to the tensor-core GEMM."""
-    K = dy2.shape[0]
-    if (K in (1, 2, 4, 8, 16) and grad.dtype == torch.float32 and grad.is_contiguous()
-            and x2.shape[1] % 4 == 0 and dy2.dtype == x2.dtype and _native_ok(x2)):
-        rc = _lib().lb_outer_accum(dy2.data_ptr(), x2.data_ptr(), grad.data_ptr(), K, dy2.shape[1],
-                                   x2.shape[1], 1.0, 1.0, native.dtype_code(x2.dtype),
-                                   native.stream_ptr())
-        if rc != -2:
-            native.check(rc, "lb_outer_accum")
-            native.count_launch()
-            return
-    gemm(dy2, x2, trans_a=True, out=grad, beta=1.0)
+    """grad[out, in] += dy2^T x2 (16-bit CUDA tensors)."""
+    native.nodes().weight_grad(dy2, x2, grad)
+
+
+_ACT_OP = {native.ACT_NONE: -1, native.ACT_RELU: UNARY_CODE["relu"], native.ACT_LEAKY: UNARY_CODE["leaky_relu"]}
 
 
 def linear(x, wh: WeightHandle, bh: Optional[WeightHandle] = None, act: int = native.ACT_NONE,
            act_param: float = 0.0):
     """y = act(x @ W^T + b) over the last dimension; W is [out, in]."""
     if _native_ok(x) and act in (native.ACT_NONE, native.ACT_RELU, native.ACT_LEAKY):
-        return _Linear.apply(x, wh.master, bh.master if bh is not None else None, wh, bh, act,
-                             float(act_param))
+        b = bh is not None
+        return native.nodes().linear(x, wh.master, bh.master if b else None, wh.cast(x.dtype),
+                                     None if wh.grad is None else wh.grad.view(wh.master.shape),
+                                     bh.grad if b else None, wh, bh, act, _ACT_OP[act], float(act_param))
     w = wh.master if wh.master.dtype == x.dtype else wh.master.to(x.dtype)
     b = None if bh is None else (bh.master if bh.master.dtype == x.dtype else bh.master.to(x.dtype))
     y = F.linear(x, w, b)
@@ -334,84 +268,26 @@ def _pad_channels(x_cl: torch.Tensor, mult: int = 8) -> torch.Tensor:
     return F.pad(x_cl, (0, mult - C % mult))
 
 
-def _upsample_zero(dy_cl: torch.Tensor, stride, out_dims) -> torch.Tensor:
-    """Insert zeros between the elements of dy (data gradient of a strided convolution)."""
-    N, Do, Ho, Wo, K = dy_cl.shape
-    sd, sh, sw = stride
-    up = torch.zeros((N, (Do - 1) * sd + 1, (Ho - 1) * sh + 1, (Wo - 1) * sw + 1, K),
-                     dtype=dy_cl.dtype, device=dy_cl.device)
-    up[:, ::sd, ::sh, ::sw, :] = dy_cl
-    return up
+def _conv(x, wh, bh, ksize, pad, stride, dil, act, act_p, skip_act_grad):
+    """The general implicit-GEMM convolution (csrc/autograd_nodes.cpp); the filters are packed
+    once per optimizer step."""
+    Kout, Cin = wh.master.shape[0], wh.master.shape[1]
+    Kp, Cp = (Kout + 7) // 8 * 8, (x.shape[1] + 7) // 8 * 8
 
+    def pack(for_dgrad):
+        w = wh.master.detach().reshape(Kout, Cin, -1)
+        if Kp != Kout or Cp != Cin:
+            w = F.pad(w, (0, 0, 0, Cp - Cin, 0, Kp - Kout))
+        return pack_filter(w.reshape(Kp, Cp, *ksize), x.dtype, for_dgrad=for_dgrad)
 
-class _Conv(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, w_leaf, b_leaf, wh, bh, ksize, pad, stride, dil, act, act_p, skip_act_grad):
-        ndim = x.dim()
-        x_cl = _pad_channels(_cl_view(x))
-        Kout, Cin = wh.master.shape[0], wh.master.shape[1]
-        Kp = (Kout + 7) // 8 * 8
-        Cp = x_cl.shape[-1]
-
-        def pack_fwd():
-            w = wh.master.detach().reshape(Kout, Cin, -1)
-            if Kp != Kout or Cp != Cin:
-                w = F.pad(w, (0, 0, 0, Cp - Cin, 0, Kp - Kout))
-            return pack_filter(w.reshape(Kp, Cp, *ksize), x.dtype)
-
-        _pack_both(wh, x.dtype, Kout, Cin, Kp, Cp, ksize)
-        wt = wh.packed("fwd", x.dtype, pack_fwd)
-        bias = None
-        if bh is not None:
-            bias = bh.master.detach()
-            if Kp != Kout:
-                bias = F.pad(bias, (0, Kp - Kout))
-        y = conv_fwd(x_cl, wt, ksize, pad=pad, stride=stride, dilation=dil, bias=bias, act=act,
-                     act_param=act_p)
-        ctx.save_for_backward(x_cl, y if (act != native.ACT_NONE and not skip_act_grad) else None)
-        ctx.meta = (wh, bh, ksize, pad, stride, dil, act, act_p, ndim, Kout, Cin, Kp, Cp)
-        out = y[..., :Kout] if Kp != Kout else y
-        return _from_cl(out, ndim)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x_cl, y = ctx.saved_tensors
-        wh, bh, ksize, pad, stride, dil, act, act_p, ndim, Kout, Cin, Kp, Cp = ctx.meta
-        dy_cl = _cl_view(dy)
-        if Kp != Kout:
-            dy_cl = _pad_channels(dy_cl)
-        if not dy_cl.is_contiguous():
-            dy_cl = dy_cl.contiguous()
-        if y is not None:
-            dy_cl = _act_grad_from_output(y, dy_cl, act, act_p)
-        N, D, H, W, _ = x_cl.shape
-        dx = None
-        if ctx.needs_input_grad[0]:
-            def pack_bwd():
-                w = wh.master.detach().reshape(Kout, Cin, -1)
-                if Kp != Kout or Cp != Cin:
-                    w = F.pad(w, (0, 0, 0, Cp - Cin, 0, Kp - Kout))
-                return pack_filter(w.reshape(Kp, Cp, *ksize), dy.dtype, for_dgrad=True)
-
-            wt = wh.packed("dgrad", dy.dtype, pack_bwd)
-            src = dy_cl if stride == (1, 1, 1) else _upsample_zero(dy_cl, stride, (D, H, W))
-            bpad = tuple(d * (k - 1) - p for d, k, p in zip(dil, ksize, pad))
-            dx_cl = conv_fwd(src, wt, ksize, pad=bpad, stride=1, dilation=dil, out_dims=(D, H, W))
-            if Cp != Cin:
-                dx_cl = dx_cl[..., :Cin]
-            dx = _from_cl(dx_cl, ndim)
-        if wh.grad is not None:
-            if Kp == Kout and Cp == Cin:
-                conv_wgrad(x_cl, dy_cl, ksize, pad=pad, stride=stride, dilation=dil,
-                           out=wh.grad.view(Kout, Cin, *ksize))
-            else:
-                tmp = conv_wgrad(x_cl, dy_cl, ksize, pad=pad, stride=stride, dilation=dil)
-                wh.grad.add_(tmp[:Kout, :Cin].reshape(wh.grad.shape))
-            wh.mark_ready()
-        if bh is not None and bh.grad is not None:
-            bh.grad.add_(column_sums(dy_cl.reshape(-1, dy_cl.shape[-1]))[:Kout])
-            bh.mark_ready()
-        return (dx,) + (None,) * 11
+    _pack_both(wh, x.dtype, Kout, Cin, Kp, Cp, ksize)
+    fwd = wh.packed("fwd", x.dtype, lambda: pack(False))
+    dgrad = wh.packed("dgrad", x.dtype, lambda: pack(True)) if x.requires_grad else None
+    b = bh is not None
+    return native.nodes().convolution(
+        x, wh.master, bh.master if b else None, fwd, dgrad,
+        None if wh.grad is None else wh.grad.view(Kout, Cin, *ksize), bh.grad if b else None, wh, bh,
+        (act, -1 if skip_act_grad else _ACT_OP[act], Kout, Cin, *ksize, *pad, *stride, *dil), act_p)
 
 
 def _first_layer_pixels(x, cr: int):
@@ -643,8 +519,7 @@ def convolution(x, wh: WeightHandle, bh: Optional[WeightHandle], ksize, pad, str
                                          p3, act, float(act_param), fuse_pool.out_alloc)
             return _ConvC8.apply(x, wh.master, bh.master if bh is not None else None, wh, bh, k3,
                                  p3, act, float(act_param), bool(skip_act_grad))
-        return _Conv.apply(x, wh.master, bh.master if bh is not None else None, wh, bh, k3, p3, s3,
-                           d3, act, float(act_param), bool(skip_act_grad))
+        return _conv(x, wh, bh, k3, p3, s3, d3, act, float(act_param), bool(skip_act_grad))
     w = wh.master if wh.master.dtype == x.dtype else wh.master.to(x.dtype)
     b = None if bh is None else (bh.master if bh.master.dtype == x.dtype else bh.master.to(x.dtype))
     fn = {1: F.conv1d, 2: F.conv2d, 3: F.conv3d}[nsp]
@@ -863,65 +738,21 @@ def _bn_fused_peers(reduce_fn):
     return (g.staging._c_ptrs, g.pad._c_ptrs, g.rank, g.world, 4096, g.ctr_ptr)
 
 
-class _BatchNormFused(torch.autograd.Function):
+def _batch_norm_fused(x, sh, bh, run_mean, run_var, eps, decay, correction, count_scale, act, act_p, peers):
     """Training-mode batch norm as one cooperative kernel per direction, statistics over the
     ranks of a symmetric group reduced inside the kernel (csrc/bn_fused.cu)."""
-
-    @staticmethod
-    def forward(ctx, x, s_leaf, b_leaf, sh, bh, run_mean, run_var, eps, decay, correction,
-                reduce_fn, count_scale, act, act_p, peers):
-        ndim = x.dim()
-        x_cl = _cl_view(x)
-        if not x_cl.is_contiguous():
-            x_cl = x_cl.contiguous()
-        C = x_cl.shape[-1]
-        rows = x_cl.numel() // C
-        staging, pads, rank, world, stride, ctr = peers
-        count = float(rows * count_scale)
-        y = torch.empty_like(x_cl)
-        stats = torch.empty(2 * C, dtype=torch.float32, device=x.device)
-        scale = sh.master.detach() if sh is not None else None
-        bias = bh.master.detach() if bh is not None else None
-        owner = sh if sh is not None else (bh if bh is not None else run_mean)
-        ws = _bn_ws(owner, "fwd", rows, C, x.device)
-        rc = _lib().lb_bn_fused_fwd(x_cl.data_ptr(), native.ptr(scale), native.ptr(bias), y.data_ptr(),
-                                    stats.data_ptr(), native.ptr(run_mean), native.ptr(run_var),
-                                    ws.data_ptr(), rows, C, count, float(correction), float(eps),
-                                    float(decay), act, float(act_p), native.dtype_code(x.dtype),
-                                    staging, pads, rank, world, stride, ctr, native.stream_ptr())
-        native.check(rc, "lb_bn_fused_fwd")
-        native.count_launch()
-        ctx.save_for_backward(x_cl, stats, y if act else None)
-        ctx.meta = (sh, bh, eps, correction, count, act, act_p, ndim, peers, owner)
-        return _from_cl(y, ndim)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x_cl, stats, y = ctx.saved_tensors
-        sh, bh, eps, correction, count, act, act_p, ndim, peers, owner = ctx.meta
-        dy_cl = _cl_view(dy)
-        if not dy_cl.is_contiguous():
-            dy_cl = dy_cl.contiguous()
-        C = x_cl.shape[-1]
-        rows = x_cl.numel() // C
-        staging, pads, rank, world, stride, ctr = peers
-        scale = sh.master.detach() if sh is not None else None
-        dscale = sh.grad.view(-1) if (sh is not None and sh.grad is not None) else None
-        dbias = bh.grad.view(-1) if (bh is not None and bh.grad is not None) else None
-        dx = torch.empty_like(x_cl)
-        ws = _bn_ws(owner, "bwd", rows, C, x_cl.device)
-        rc = _lib().lb_bn_fused_bwd(x_cl.data_ptr(), dy_cl.data_ptr(), native.ptr(y), stats.data_ptr(),
-                                    native.ptr(scale), dx.data_ptr(), native.ptr(dscale),
-                                    native.ptr(dbias), ws.data_ptr(), rows, C, count, float(correction),
-                                    float(eps), act, float(act_p), native.dtype_code(x_cl.dtype),
-                                    staging, pads, rank, world, stride, ctr, native.stream_ptr())
-        native.check(rc, "lb_bn_fused_bwd")
-        native.count_launch()
-        if dscale is not None:
-            sh.mark_ready()
-        if dbias is not None:
-            bh.mark_ready()
-        return (_from_cl(dx, ndim),) + (None,) * 14
+    C = x.shape[1]
+    rows = x.numel() // C
+    staging, pads, rank, world, stride, ctr = peers
+    owner = sh if sh is not None else (bh if bh is not None else run_mean)
+    s, b = sh is not None, bh is not None
+    return native.nodes().batch_norm(
+        x, sh.master if s else None, bh.master if b else None, run_mean, run_var,
+        _bn_ws(owner, "fwd", rows, C, x.device), _bn_ws(owner, "bwd", rows, C, x.device),
+        sh.grad if s else None, bh.grad if b else None, sh, bh,
+        (act, ctypes.addressof(staging) if staging is not None else 0,
+         ctypes.addressof(pads) if pads is not None else 0, rank, world, stride, ctr or 0),
+        (float(eps), float(decay), float(correction), float(count_scale), float(act_p)))
 
 
 class _BatchNorm(torch.autograd.Function):
@@ -1009,9 +840,8 @@ def batch_norm(x, sh, bh, run_mean, run_var, training: bool, eps: float, decay: 
             peers = _bn_fused_peers(reduce_fn) if (2 * C <= 4096 and not os.environ.get(
                 "LBANN_BN_SEPARATE_KERNELS")) else None
             if peers is not None:
-                return _BatchNormFused.apply(x, sh.master if sh else None, bh.master if bh else None,
-                                             sh, bh, run_mean, run_var, eps, decay, correction,
-                                             reduce_fn, count_scale, act, float(act_param), peers)
+                return _batch_norm_fused(x, sh, bh, run_mean, run_var, eps, decay, correction, count_scale,
+                                         act, float(act_param), peers)
             return _BatchNorm.apply(x, sh.master if sh else None, bh.master if bh else None, sh, bh,
                                     run_mean, run_var, eps, decay, correction, reduce_fn,
                                     count_scale, act, float(act_param))
@@ -1081,53 +911,13 @@ class _ReduceSum(torch.autograd.Function):
 
 
 # --------------------------------------------------------------------------- layer norm
-class _LayerNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, s_leaf, b_leaf, sh, bh, cols, eps):
-        xc = x.contiguous()
-        rows = xc.numel() // cols
-        y = torch.empty_like(xc)
-        mean = torch.empty(rows, dtype=torch.float32, device=x.device)
-        rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        scale = sh.master.detach().reshape(-1) if sh is not None else None
-        bias = bh.master.detach().reshape(-1) if bh is not None else None
-        native.check(_lib().lb_layer_norm_fwd(xc.data_ptr(), native.ptr(scale), native.ptr(bias),
-                                              y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), rows,
-                                              cols, float(eps), native.dtype_code(x.dtype),
-                                              native.stream_ptr()), "lb_layer_norm_fwd")
-        native.count_launch()
-        ctx.save_for_backward(xc, mean, rstd)
-        ctx.meta = (sh, bh, cols)
-        return y
-
-    @staticmethod
-    def backward(ctx, dy):
-        xc, mean, rstd = ctx.saved_tensors
-        sh, bh, cols = ctx.meta
-        dyc = dy.contiguous()
-        rows = xc.numel() // cols
-        dx = torch.empty_like(xc)
-        scale = sh.master.detach().reshape(-1) if sh is not None else None
-        dscale = sh.grad.view(-1) if (sh is not None and sh.grad is not None) else None
-        dbias = bh.grad.view(-1) if (bh is not None and bh.grad is not None) else None
-        native.check(_lib().lb_layer_norm_bwd(xc.data_ptr(), dyc.data_ptr(), native.ptr(scale),
-                                              mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(),
-                                              native.ptr(dscale), native.ptr(dbias), rows, cols,
-                                              native.dtype_code(xc.dtype), native.stream_ptr()),
-                     "lb_layer_norm_bwd")
-        native.count_launch(2)
-        if dscale is not None:
-            sh.mark_ready()
-        if dbias is not None:
-            bh.mark_ready()
-        return dx, None, None, None, None, None, None
-
-
 def layer_norm(x, normalized_size: int, sh=None, bh=None, eps: float = 1e-5):
     """Normalise over the trailing ``normalized_size`` elements of every sample."""
     if x.is_cuda and x.dtype in (torch.float16, torch.bfloat16, torch.float32):
-        return _LayerNorm.apply(x, sh.master if sh else None, bh.master if bh else None, sh, bh,
-                                int(normalized_size), eps)
+        s, b = sh is not None, bh is not None
+        return native.nodes().layer_norm(x, sh.master if s else None, bh.master if b else None,
+                                         sh.grad if s else None, bh.grad if b else None, sh, bh,
+                                         int(normalized_size), float(eps))
     shape = x.shape
     x2 = x.reshape(-1, normalized_size).float()
     mean = x2.mean(1, keepdim=True)

@@ -84,7 +84,6 @@ class _ModelParallelLinearFused(torch.autograd.Function):
     def forward(ctx, x, w_leaf, b_leaf, tp, layer):
         import ctypes
         from ..ops import native
-        from ..ops.gemm import _lib as gemm_lib
         wh = layer.w.handle
         bh = layer.b.handle if layer.b is not None else None
         P = tp.size
@@ -99,10 +98,11 @@ class _ModelParallelLinearFused(torch.autograd.Function):
         w_loc = wh.cast(dt)[lo:hi]
         bias = bh.master.detach()[lo:hi].float().contiguous() if bh is not None else None
         ptrs = (native.c_void_p * P)(*[ybuf.peer_ptr(q, lo * es) for q in range(P)])
-        lib = gemm_lib()
+        lib = native.cuda_lib()
         lib.lb_gemm_bcast_tc.restype = native.c_int
-        lib.lb_gemm_bcast_tc.argtypes = lib.lb_gemm_tc.argtypes[:-1] + [
-            ctypes.POINTER(native.c_void_p), native.c_int, native.c_void_p]
+        lib.lb_gemm_bcast_tc.argtypes = [native.c_void_p] * 4 + [native.c_int] * 4 + [native.c_ll] * 6 + \
+            [native.c_int] * 4 + [native.c_float] * 2 + [native.c_int] * 2 + [native.c_float, native.c_int] + \
+            [ctypes.POINTER(native.c_void_p), native.c_int, native.c_void_p]
         tp.sg.barrier_device(2)            # every rank is done reading the previous output
         rc = lib.lb_gemm_bcast_tc(x.data_ptr(), w_loc.data_ptr(), ybuf.ptr + lo * es, native.ptr(bias),
                                   tokens, hi - lo, k, 1, k, k, n, 0, 0, 0, 0, 0, native.dtype_code(dt),

@@ -385,3 +385,51 @@ def test_sharded_update_with_state_for_owned_blocks_only():
         if which == 1:      # the second moment exists for the Adam tensor only
             got, want = got[:n1], want[:n1]
         torch.testing.assert_close(got[:want.numel()], want, rtol=1e-6, atol=1e-7)
+
+
+@pytest.mark.parametrize("layer", ["linear", "convolution", "batch_norm", "layer_norm"])
+def test_nodes_report_gradients_and_keep_saved_tensor_hooks(layer):
+    """The C++ autograd nodes: a handle that listens (data-parallel reduction) hears once per
+    backward that its gradient is complete, saved tensors go through the hooks of the context, and
+    the results are those of the plain run, bit for bit."""
+    torch.manual_seed(3)
+    C = 16
+
+    def build():
+        torch.manual_seed(4)
+        shapes = {"linear": ((24, C), (24,)), "convolution": ((8, C, 3, 3), (8,)), "batch_norm": ((C,), (C,)),
+                  "layer_norm": ((C,), (C,))}[layer]
+        hs = []
+        for s in shapes:
+            w = torch.randn(*s, device="cuda", requires_grad=True)
+            hs.append(nn.WeightHandle(w, torch.zeros(*s, device="cuda")))
+        return hs
+
+    def run(hs, x):
+        if layer == "linear":
+            return nn.linear(x, *hs, native.ACT_RELU)
+        if layer == "convolution":
+            return nn.convolution(x, *hs, (3, 3), (1, 1), (1, 1), (1, 1), act=native.ACT_LEAKY, act_param=0.1)
+        if layer == "batch_norm":
+            return nn.batch_norm(x, *hs, torch.zeros(C, device="cuda"), torch.ones(C, device="cuda"), True, 1e-5, 0.9)
+        return nn.layer_norm(x, C, *hs)
+
+    shape = (2, C, 5, 6) if layer in ("convolution", "batch_norm") else (10, C)
+    x0 = torch.randn(*shape, device="cuda").bfloat16()
+    results = []
+    for hooked in (False, True):
+        hs, x, packed, heard = build(), x0.clone().requires_grad_(True), [], []
+        for k, h in enumerate(hs):
+            h.on_grad_ready = (lambda k=k: heard.append(k)) if hooked else None
+        if hooked:
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(1), t.clone())[1], lambda t: t):
+                y = run(hs, x)
+        else:
+            y = run(hs, x)
+        dx, = torch.autograd.grad(y, x, torch.ones_like(y))
+        results.append([y.detach(), dx] + [h.grad for h in hs])
+        assert sorted(heard) == ([0, 1] if hooked else []) and bool(packed) == hooked
+    assert native.consume_status() == 0
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+    assert float(results[0][2].abs().sum()) > 0
