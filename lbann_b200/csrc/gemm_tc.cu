@@ -19,6 +19,7 @@ struct GemmPolicy {
   static constexpr int BN = BN_;
   static constexpr int kEpiGroups = 2;       // two tiles' epilogues in flight (tc_pipeline.cuh)
   using G = StageGeom<BN>;
+  using HasSingleIssue = void;               // one to six boxes a stage, issued by one thread
 
   struct Params {
     int M, N, K, batch;
@@ -47,19 +48,21 @@ struct GemmPolicy {
   }
   __device__ static void load(const Params& p, const Tile& tl, int k, uint32_t sA, uint32_t sB,
                               uint32_t bar, const CUtensorMap* tmA, const CUtensorMap* tmB,
-                              int lane) {
+                              int) {
     const int k0 = k * kBK;
-    // boxes of the A operand go out from lanes 0.., boxes of B from lanes 8..
     if (!p.a_mn) {
-      if (lane == 0) tma_load_3d(sA, tmA, bar, k0, tl.m0, tl.b);  // box {64 k, 128 rows}
-    } else if (lane < kBM / 64) {                                 // box {64 m, 64 k-rows}
-      tma_load_3d(sA + lane * 8192, tmA, bar, tl.m0 + lane * 64, k0, tl.b);
+      tma_load_3d(sA, tmA, bar, k0, tl.m0, tl.b);                 // box {64 k, 128 rows}
+    } else {
+#pragma unroll
+      for (int j = 0; j < kBM / 64; ++j)                          // box {64 m, 64 k-rows}
+        tma_load_3d(sA + j * 8192, tmA, bar, tl.m0 + j * 64, k0, tl.b);
     }
     if (!p.b_mn) {
-      if (lane == 8) tma_load_3d(sB, tmB, bar, k0, tl.n0, tl.b);  // box {64 k, BN rows}
-    } else if (lane >= 8 && lane < 8 + BN / 64) {
-      const int j = lane - 8;
-      tma_load_3d(sB + j * 8192, tmB, bar, tl.n0 + j * 64, k0, tl.b);
+      tma_load_3d(sB, tmB, bar, k0, tl.n0, tl.b);                 // box {64 k, BN rows}
+    } else {
+#pragma unroll
+      for (int j = 0; j < BN / 64; ++j)
+        tma_load_3d(sB + j * 8192, tmB, bar, tl.n0 + j * 64, k0, tl.b);
     }
   }
   __device__ static uint32_t idesc(const Params& p) {
@@ -124,6 +127,52 @@ static int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB,
   return rc;
 }
 
+// gemm_pair_tc.cu
+int gemm_pair_slots();
+int gemm_pair_launch(const void* A, const void* B, void* C, const float* bias, int M, int N, int K, int batch,
+                     long long lda, long long ldb, long long ldc, long long strideA, long long strideB,
+                     long long strideC, int a_mn, int b_mn, int in_dtype, int out_dtype, float alpha, int add,
+                     int bias_mode, int act, float act_param, cudaStream_t stream);
+
+constexpr int kPairHint = 512;
+
+// The tile with the shortest estimate: 256 x 256 on a pair of SMs (kPairHint) or 128 x 256 / 128 /
+// 64 on one.  Per wave of tiles an estimate is k-steps (64 each) x cycles + what the last tile's
+// epilogue shows.  The cycles are slopes measured over K between 1024 and 8192 (0.31 us a step
+// for the pair, 0.48 / 0.30 / 0.27 at 256 / 128 / 64); a product that is cut along K needs its
+// second kernel (which writes whole rows), and the one-SM epilogue reads an accumulated C, and
+// writes rows that do not start on 16 bytes, value by value.
+// Measured, pair against the tile that was taken before: 8192 x 8192 x 2048 167 / 219 us,
+// 4096 x 1024 x 50304 278 / 623 us, fp32 += 4096 x 1024 x 4096 40 / 86 us; the other way,
+// 512 x 1024 x 4096 (8 pair tiles against 128 work items) 31 / 21 us.
+static int gemm_choose(int M, int N, int K, int batch, const lbhost::SplitKOffer& offer, bool pair_ok, bool accumulate,
+                       bool aligned) {
+  const long long k = (K + kBK - 1) / kBK, sms = lbhost::sm_count();
+  int best = 0;
+  long long best_cost = 0;
+  auto consider = [&](int tile, long long cost) {
+    if (best == 0 || cost < best_cost) { best = tile; best_cost = cost; }
+  };
+  const int slots = pair_ok ? gemm_pair_slots() : 0;
+  if (slots > 0) {
+    const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256) * batch;
+    consider(kPairHint, (tiles + slots - 1) / slots * (600 * k + 1500));
+  }
+  const int widths[3] = {256, 128, 64};
+  const long long cycles[3] = {920, 570, 520}, tail[3] = {2500, 1500, 1000};
+  for (int i = 0; i < 3; ++i) {
+    const int bn = widths[i];
+    if (i < 2 && N <= bn / 2) continue;
+    const long long tiles = (long long)((M + 127) / 128) * ((N + bn - 1) / bn) * batch;
+    const int splits = tiles < sms ? lbhost::plan_splitk(offer, (int)tiles, (int)k, bn) : 1;
+    const long long waves = (tiles * splits + sms - 1) / sms;
+    const long long shown = aligned ? tail[i] * (accumulate ? 6 : 1) : 160 * bn;
+    consider(bn, waves * (cycles[i] * ((k + splits - 1) / splits) + (splits > 1 ? tail[i] : shown)) +
+                     (splits > 1 ? 8000 : 0));
+  }
+  return best;
+}
+
 }  // namespace lb
 
 extern "C" {
@@ -171,14 +220,21 @@ int lb_gemm_bcast_tc(const void* A, const void* B, void* C, const float* bias, i
   if ((lda % 8) || (ldb % 8) || (strideA % 8) || (strideB % 8)) return -1;
   if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15)) return -1;
 
+  // Pairs of SMs (gemm_pair_tc.cu) write through TMA: 16-byte rows, and C is only overwritten or,
+  // in fp32, added to.
+  const long long es = out_dtype == kF32 ? 4 : 2;
+  const bool pair_ok = bcast_ranks == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc * es % 16 == 0 &&
+                       strideC * es % 16 == 0 && (batch == 1 || strideC > 0) &&
+                       (beta == 0.f || (beta == 1.f && out_dtype == kF32 && act == kActNone));
   int BN = bn_hint;
-  if (BN != 64 && BN != 128 && BN != 256) {
-    // Heuristic: the widest tile that still gives every SM a tile.
-    const long long t256 = (long long)((M + 127) / 128) * ((N + 255) / 256) * batch;
-    const long long t128 = (long long)((M + 127) / 128) * ((N + 127) / 128) * batch;
-    if (N > 128 && t256 >= lbhost::sm_count()) BN = 256;
-    else if (N > 64 && t128 >= lbhost::sm_count() / 2) BN = 128;
-    else BN = N > 64 ? 128 : 64;
+  if (BN != 64 && BN != 128 && BN != 256 && !(BN == kPairHint && pair_ok))
+    BN = gemm_choose(M, N, K, batch, offer, pair_ok, beta != 0.f,
+                     (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc * es % 16 == 0);
+  if (BN == kPairHint) {
+    const int rc = gemm_pair_launch(A, B, C, bias, M, N, K, batch, lda, ldb, ldc, strideA, strideB, strideC, a_mn, b_mn,
+                                    in_dtype, out_dtype, alpha, beta == 1.f, bias_mode, act, act_param, stream);
+    if (rc != -2) return rc;
+    BN = 256;
   }
 
   CUtensorMap tmA, tmB;

@@ -307,6 +307,12 @@ template <class Policy>
 struct TcEpiGroups<Policy, std::void_t<decltype(Policy::kEpiGroups)>> {
   static constexpr int value = Policy::kEpiGroups;
 };
+// A policy with few boxes per stage (`using HasSingleIssue = void;`) has its producer run by one
+// elected thread; the warp-wide loop below costs ~800 cycles a stage whatever the boxes hold.
+template <class Policy, class = void>
+struct TcSingleIssue { static constexpr bool value = false; };
+template <class Policy>
+struct TcSingleIssue<Policy, typename Policy::HasSingleIssue> { static constexpr bool value = true; };
 template <class Policy>
 constexpr int tc_threads() { return 64 + 128 * TcEpiGroups<Policy>::value; }
 
@@ -373,7 +379,40 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
     if (threadIdx.x == 0) halo_signal(*hs);
   }
 
-  if (warp == 4) {
+  if (TcSingleIssue<Policy>::value && warp == 4) {
+    // --------------------- producer, one elected thread ---------------------
+    if (elect_one()) {
+      uint32_t it = 0;
+      RingPos rp;
+      bool ok = true;
+      for (int w = blockIdx.x; w < num_items && ok; w += n_workers) {
+        const int t = w / splits, sp = w - t * splits;
+        const int k_begin = (int)((long long)sp * k_iters / splits);
+        const int k_end = (int)((long long)(sp + 1) * k_iters / splits);
+        const typename Policy::Tile tile = Policy::decode(p, t);
+        for (int k = k_begin; k < k_end; ++k, ++it) {
+          const uint32_t bar = smem_u32(&sh.full[rp.s]);
+          if (!mbar_wait_bounded(smem_u32(&sh.empty[rp.s]), rp.ph ^ 1, abort_flag)) {
+            raise_status(status, abort_flag, kTimeoutStageEmpty);
+            ok = false;
+            break;
+          }
+          mbar_expect_tx(bar, Policy::stage_bytes(p, tile, k));
+          const uint32_t sA = smem_base + rp.s * G::kStageBytes;
+          Policy::load(p, tile, k, sA, sA + G::kABytes, bar, &tmA, &tmB, -1);
+          rp.advance(S);
+        }
+      }
+      if (!ok || *abort_flag) {      // let the copies in flight land (see below)
+        const uint32_t pending = it < (uint32_t)S ? it : (uint32_t)S;
+        for (uint32_t j = 0; j < pending; ++j) {
+          const uint32_t q = it - 1 - j;
+          mbar_wait_budget_only(smem_u32(&sh.full[q % S]), (q / S) & 1);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 4) {
     // ------------------------------ producer --------------------------------
     // The whole warp runs the loop: lane 0 waits for the stage and arms its barrier, then
     // every lane may issue one of the stage's TMA boxes (Policy::load picks by lane), so
@@ -435,9 +474,9 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
     }
   } else if (warp == 5) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = Policy::idesc(p);
-      uint32_t it = 0;
+      RingPos rp;
       uint32_t local_tile = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < num_items && ok; w += n_workers, ++local_tile) {
@@ -453,10 +492,9 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
         }
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * BN;
-        for (int k = k_begin; k < k_end; ++k, ++it) {
-          const uint32_t s = it % S;
-          const uint32_t ph = (it / S) & 1;
-          if (!mbar_wait_bounded(smem_u32(&sh.full[s]), ph, abort_flag)) {
+        for (int k = k_begin; k < k_end; ++k) {
+          const uint32_t s = rp.s;
+          if (!mbar_wait_bounded(smem_u32(&sh.full[s]), rp.ph, abort_flag)) {
             raise_status(status, abort_flag, kTimeoutTmaFull);
             ok = false;
             break;
@@ -466,6 +504,7 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
           const uint32_t sB = sA + G::kABytes;
           Policy::mma(p, k, sA, sB, tmem_acc, idesc, /*first=*/k == k_begin);
           umma_commit(smem_u32(&sh.empty[s]));  // frees the stage when the MMAs retire
+          rp.advance(S);
         }
         if (ok) umma_commit(smem_u32(&sh.tmem_full[acc]));
       }

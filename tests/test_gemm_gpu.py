@@ -93,3 +93,34 @@ def test_gemm_skinny_products_split_the_reduction(M, N, K, dtype, monkeypatch):
     gemm(a, w, trans_b=True, out=plain, beta=0.5, bias=bias, act=native.ACT_RELU)
     assert native.splitk_offers == before + 2
     torch.testing.assert_close(outs[0].float(), plain.float(), rtol=1e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (264, 776, 72), (130, 2049 * 8, 200), (2304, 520, 136), (1000, 264, 1155)])
+@pytest.mark.parametrize("ta,tb", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("out_dtype,beta", [(torch.bfloat16, 0.0), (torch.float32, 0.0), (torch.float32, 1.0)])
+def test_gemm_on_pairs_of_sms(M, N, K, ta, tb, out_dtype, beta):
+    """The 256 x 256 tile of two SMs at ragged edges of M, N and K, several tiles per pair, every
+    operand layout, plain and accumulating outputs; against 64 bits: products of bf16 are exact in
+    fp32 and the sums of K <= 1155 terms are off by less than 4e-6, a bf16 result by 2^-9."""
+    torch.manual_seed(11)
+    a = torch.randn(*((K, M) if ta else (M, K)), device="cuda").bfloat16()
+    b = torch.randn(*((N, K) if tb else (K, N)), device="cuda").bfloat16()
+    bias = torch.randn(N, device="cuda")
+    prev = torch.randn(M, N, device="cuda").to(out_dtype)
+    ref = 0.5 * ((a.t() if ta else a).double() @ (b.t() if tb else b).double())
+    ref = ref + prev.double() if beta else torch.relu(ref + bias.double())
+    out = prev.clone()
+    gemm(a, b, trans_a=ta, trans_b=tb, out=out, beta=beta, alpha=0.5, bias=None if beta else bias,
+         act=native.ACT_NONE if beta else native.ACT_RELU, bn_hint=512)
+    assert native.consume_status() == 0
+    assert float((out.double() - ref).norm() / ref.norm()) < (2 ** -9 if out_dtype == torch.bfloat16 else 4e-6)
+
+
+def test_gemm_on_pairs_batched():
+    torch.manual_seed(12)
+    a = torch.randn(3, 300, 136, device="cuda").half()
+    b = torch.randn(3, 520, 136, device="cuda").half()
+    out = gemm(a, b, trans_b=True, bn_hint=512)
+    assert native.consume_status() == 0
+    ref = a.double() @ b.double().transpose(1, 2)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2 ** -11
