@@ -27,7 +27,8 @@ int lb_gemm_tc(const void*, const void*, void*, const float*, int, int, int, int
 int lb_splitk_offer(void*, long long);
 int lb_sm_count();
 int lb_outer_accum(const void*, const void*, float*, int, int, long long, float, float, int, void*);
-int lb_bn_partial_sums(const void*, float*, long long, int, int, int, int, void*);
+int lb_grad_prep(const void*, const void*, void*, float*, long long, int, long long, int, float, int, void*);
+int lb_pad_rows(const void*, void*, long long, int, long long, int, void*);
 int lb_unary(const void*, const void*, void*, long long, int, int, float, float, int, void*);
 int lb_binary(const void*, const void*, const void*, void*, void*, long long, int, int, int, void*);
 int lb_attention_fwd(const void*, const void*, const void*, void*, float*, int, int, int, int, const long long*,
@@ -143,8 +144,16 @@ Tensor tma_ready(const Tensor& t) {
       (nd == 2 || (t.stride(0) % 8 == 0 && t.stride(0) >= 0)))
     return t;
   auto shape = t.sizes().vec();
-  const int64_t cols = shape[nd - 1];
-  shape[nd - 1] = (cols + 7) / 8 * 8;
+  const int64_t cols = shape[nd - 1], pitch = (cols + 7) / 8 * 8;
+  shape[nd - 1] = pitch;
+  if (t.stride(nd - 1) == 1 && t.numel() > 0 && t.element_size() == 2 &&
+      (nd == 2 || t.stride(0) == t.size(1) * t.stride(1))) {
+    Tensor buf = at::empty(shape, t.options());
+    check(lb_pad_rows(t.data_ptr(), buf.data_ptr(), t.numel() / cols, cols, t.stride(nd - 2), pitch, stream()),
+          "lb_pad_rows");
+    ++g_launches;
+    return pitch == cols ? buf : buf.narrow(nd - 1, 0, cols);
+  }
   Tensor buf = at::zeros(shape, t.options());
   Tensor view = buf.narrow(nd - 1, 0, cols);
   view.copy_(t);
@@ -192,27 +201,36 @@ Tensor same_strides(const Tensor& dy, const Tensor& x) {
   if (dy.strides() == x.strides()) return dy;
   return at::empty_like(x).copy_(dy);
 }
-// dy * act'(.) for activations whose derivative is a function of the output's sign; act_op is the
-// unary operator of the activation (-1: none).
-Tensor act_grad(const Tensor& y, const Tensor& dy, int64_t act_op, double p) {
-  return act_op < 0 ? dy : unary_raw(act_op, y, same_strides(dy, y), p, 0.0, 1);
-}
-// fp32 sums over the rows of a [rows, C] tensor.
-Tensor column_sums(const Tensor& x) {
-  const int64_t rows = x.size(0), C = x.size(1);
-  if (C % 8 || !x.is_contiguous() || rows == 0) return x.to(at::kFloat).sum(0);
-  const int64_t reps = rows >= 8192 ? 16 : 1;      // copies of the sums that the atomics are spread over
-  Tensor sums = at::zeros({reps, 2 * C}, x.options().dtype(at::kFloat));
-  check(lb_bn_partial_sums(x.data_ptr(), fptr(sums), rows, C, 1, code(x.scalar_type()), reps, stream()),
-        "lb_bn_partial_sums");
+// What the products of a layer's backward read, from the dense rows of dy (csrc/grad_prep.cu):
+// dy * act'(.) where `y`, the layer's output, is given, with a row pitch that TMA takes; the bias
+// gradient (may be undefined) receives the column sums on the way.
+Tensor grad_prep(const Tensor& dy, const Tensor& y, int64_t act, double p, const Tensor& bgrad) {
+  const int64_t C = dy.size(-1), rows = dy.numel() / C, pitch = (C + 7) / 8 * 8;
+  const bool copy = y.defined() || pitch != C;
+  if (!copy && !bgrad.defined()) return dy;
+  Tensor sums = bgrad;
+  const bool direct = bgrad.defined() && bgrad.scalar_type() == at::kFloat && bgrad.is_contiguous() && bgrad.numel() == C;
+  if (bgrad.defined() && !direct) sums = at::zeros({C}, dy.options().dtype(at::kFloat));
+  Tensor g;
+  if (copy) {
+    auto shape = dy.sizes().vec();
+    shape.back() = pitch;
+    g = at::empty(shape, dy.options());
+  }
+  check(lb_grad_prep(dy.data_ptr(), ptr(y), copy ? g.data_ptr() : nullptr, fptr(sums), rows, C, pitch,
+                     y.defined() ? act : 0, p, code(dy.scalar_type()), stream()),
+        "lb_grad_prep");
   ++g_launches;
-  return (reps > 1 ? sums.sum(0) : sums[0]).narrow(0, 0, C);
+  if (bgrad.defined() && !direct) bgrad.add_(sums.narrow(0, 0, bgrad.numel()).view(bgrad.sizes()));
+  if (!copy) return dy;
+  return pitch == C ? g : g.narrow(-1, 0, C);
 }
 // grad[out, in] += dy^T x.  Mini-batches of at most 16 rows make this a rank-K update bound by
 // the read-modify-write of grad (csrc/outer_accum.cu); the rest goes to the tensor cores.
+bool outer_rows(int64_t K) { return K == 1 || K == 2 || K == 4 || K == 8 || K == 16; }
 void weight_grad(const Tensor& dy, const Tensor& x, const Tensor& grad) {
   const int64_t K = dy.size(0);
-  if ((K == 1 || K == 2 || K == 4 || K == 8 || K == 16) && grad.scalar_type() == at::kFloat && grad.is_contiguous() &&
+  if (outer_rows(K) && dy.is_contiguous() && x.is_contiguous() && grad.scalar_type() == at::kFloat && grad.is_contiguous() &&
       x.size(1) % 4 == 0 && dy.scalar_type() == x.scalar_type()) {
     const int rc = lb_outer_accum(dy.data_ptr(), x.data_ptr(), fptr(grad), K, dy.size(1), x.size(1), 1.f, 1.f,
                                   code(x.scalar_type()), stream());
@@ -227,15 +245,19 @@ void weight_grad(const Tensor& dy, const Tensor& x, const Tensor& grad) {
 
 // ----------------------------------------------------------------------------------- linear
 struct LinearNode : torch::autograd::Function<LinearNode> {
-  // state: w = 16-bit weight, wgrad, bgrad; i = {act, act_op}; f = {act_param}
+  // state: w = 16-bit weight, wgrad, bgrad; i = {act}; f = {act_param}
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_leaf, const optional<Tensor>& b_leaf,
                         const c10::intrusive_ptr<State>& s) {
     Tensor x2 = x.reshape({-1, x.size(-1)});
     if (!x2.is_contiguous()) x2 = x2.contiguous();
-    Tensor y = gemm(x2, s->w, false, true, Tensor(), x.scalar_type(), 1.0, 0.0, opt(b_leaf), false, s->i[0], s->f[0], 0);
+    // operands that need another row pitch are copied once for all three products (a few rows:
+    // the weight gradient reads them dense)
+    const Tensor xt = tma_ready(x2);
+    s->w = tma_ready(s->w);
+    Tensor y = gemm(xt, s->w, false, true, Tensor(), x.scalar_type(), 1.0, 0.0, opt(b_leaf), false, s->i[0], s->f[0], 0);
     keep(ctx, s);
     ctx->saved_data["shape"] = x.sizes().vec();
-    ctx->save_for_backward({x2, s->i[1] >= 0 ? y : Tensor()});
+    ctx->save_for_backward({outer_rows(x2.size(0)) ? x2 : xt, s->i[0] ? y : Tensor()});
     auto shape = x.sizes().vec();
     shape.back() = s->w.size(0);
     return x.dim() == 2 ? y : y.reshape(shape);
@@ -246,7 +268,8 @@ struct LinearNode : torch::autograd::Function<LinearNode> {
     const Tensor &x2 = saved[0], &y = saved[1];
     Tensor dy = g[0].reshape({-1, g[0].size(-1)});
     if (!dy.is_contiguous()) dy = dy.contiguous();
-    if (y.defined()) dy = act_grad(y, dy, s->i[1], s->f[0]);
+    dy = grad_prep(dy, y, s->i[0], s->f[0], s->bgrad);
+    if (s->bgrad.defined()) mark_ready(s->bh);
     Tensor dx;
     if (ctx->needs_input_grad(0)) {
       dx = mm(dy, s->w, false, false);
@@ -254,12 +277,8 @@ struct LinearNode : torch::autograd::Function<LinearNode> {
       if (shape.size() != 2) dx = dx.reshape(shape);
     }
     if (s->wgrad.defined()) {
-      weight_grad(dy, x2, s->wgrad);
+      weight_grad(outer_rows(dy.size(0)) && !dy.is_contiguous() ? dy.contiguous() : dy, x2, s->wgrad);
       mark_ready(s->wh);
-    }
-    if (s->bgrad.defined()) {
-      s->bgrad.add_(column_sums(dy));
-      mark_ready(s->bh);
     }
     return {dx, Tensor(), Tensor(), Tensor()};
   }
@@ -349,7 +368,8 @@ Tensor upsample_zero(const Tensor& dy, const int64_t* stride) {
 
 struct ConvNode : torch::autograd::Function<ConvNode> {
   // state: w / w2 = filters of the forward / data-gradient product (w2 undefined: no data
-  // gradient), wgrad, bgrad; i = {act, act_op or -1, Kout, Cin, geom[12]}; f = {act_param}
+  // gradient), wgrad, bgrad; i = {act, act whose gradient is applied here, Kout, Cin, geom[12]};
+  // f = {act_param}
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_leaf, const optional<Tensor>& b_leaf,
                         const c10::intrusive_ptr<State>& s) {
     const int64_t* g = s->i.data() + 4;
@@ -361,7 +381,7 @@ struct ConvNode : torch::autograd::Function<ConvNode> {
     Tensor y = conv_fwd(x_cl, s->w, Tensor(), x.scalar_type(), g, o[0], o[1], o[2], 1.0, 0.0, bias, s->i[0], s->f[0], 0);
     keep(ctx, s);
     ctx->saved_data["ndim"] = x.dim();
-    ctx->save_for_backward({x_cl, s->i[1] >= 0 ? y : Tensor()});
+    ctx->save_for_backward({x_cl, s->i[1] ? y : Tensor()});
     return from_cl(Kp != Kout ? y.narrow(4, 0, Kout) : y, x.dim());
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -374,7 +394,8 @@ struct ConvNode : torch::autograd::Function<ConvNode> {
     Tensor dy = cl_view(grads[0]);
     if (Kp != Kout) dy = pad_channels(dy);
     if (!dy.is_contiguous()) dy = dy.contiguous();
-    if (y.defined()) dy = act_grad(y, dy, s->i[1], s->f[0]);
+    dy = grad_prep(dy, y, s->i[1], s->f[0], s->bgrad);
+    if (s->bgrad.defined()) mark_ready(s->bh);
     Tensor dx;
     if (ctx->needs_input_grad(0)) {
       const bool unit = g[6] == 1 && g[7] == 1 && g[8] == 1;
@@ -398,10 +419,6 @@ struct ConvNode : torch::autograd::Function<ConvNode> {
         s->wgrad.add_(tmp.narrow(0, 0, Kout).narrow(1, 0, Cin).reshape(s->wgrad.sizes()));
       }
       mark_ready(s->wh);
-    }
-    if (s->bgrad.defined()) {
-      s->bgrad.add_(column_sums(dy.reshape({-1, dy.size(-1)})).narrow(0, 0, Kout));
-      mark_ready(s->bh);
     }
     return {dx, Tensor(), Tensor(), Tensor()};
   }
@@ -686,9 +703,9 @@ PYBIND11_MODULE(_lbann_autograd, m) {
   });
   m.def("linear", [](const Tensor& x, const Tensor& w_leaf, const optional<Tensor>& b_leaf, const Tensor& w16,
                      const optional<Tensor>& wgrad, const optional<Tensor>& bgrad, const py::object& wh,
-                     const py::object& bh, int64_t act, int64_t act_op, double act_param) {
+                     const py::object& bh, int64_t act, double act_param) {
     return LinearNode::apply(x, w_leaf, b_leaf,
-                             make_state(w16, {}, wgrad, bgrad, wh, bh, {act, act_op}, {act_param}));
+                             make_state(w16, {}, wgrad, bgrad, wh, bh, {act}, {act_param}));
   });
   m.def("convolution", [](const Tensor& x, const Tensor& w_leaf, const optional<Tensor>& b_leaf, const Tensor& fwd,
                           const optional<Tensor>& dgrad, const optional<Tensor>& wgrad, const optional<Tensor>& bgrad,

@@ -210,9 +210,6 @@ def _weight_grad(dy2: torch.Tensor, x2: torch.Tensor, grad: torch.Tensor) -> Non
     native.nodes().weight_grad(dy2, x2, grad)
 
 
-_ACT_OP = {native.ACT_NONE: -1, native.ACT_RELU: UNARY_CODE["relu"], native.ACT_LEAKY: UNARY_CODE["leaky_relu"]}
-
-
 def linear(x, wh: WeightHandle, bh: Optional[WeightHandle] = None, act: int = native.ACT_NONE,
            act_param: float = 0.0):
     """y = act(x @ W^T + b) over the last dimension; W is [out, in]."""
@@ -220,7 +217,7 @@ def linear(x, wh: WeightHandle, bh: Optional[WeightHandle] = None, act: int = na
         b = bh is not None
         return native.nodes().linear(x, wh.master, bh.master if b else None, wh.cast(x.dtype),
                                      None if wh.grad is None else wh.grad.view(wh.master.shape),
-                                     bh.grad if b else None, wh, bh, act, _ACT_OP[act], float(act_param))
+                                     bh.grad if b else None, wh, bh, act, float(act_param))
     w = wh.master if wh.master.dtype == x.dtype else wh.master.to(x.dtype)
     b = None if bh is None else (bh.master if bh.master.dtype == x.dtype else bh.master.to(x.dtype))
     y = F.linear(x, w, b)
@@ -287,7 +284,7 @@ def _conv(x, wh, bh, ksize, pad, stride, dil, act, act_p, skip_act_grad):
     return native.nodes().convolution(
         x, wh.master, bh.master if b else None, fwd, dgrad,
         None if wh.grad is None else wh.grad.view(Kout, Cin, *ksize), bh.grad if b else None, wh, bh,
-        (act, -1 if skip_act_grad else _ACT_OP[act], Kout, Cin, *ksize, *pad, *stride, *dil), act_p)
+        (act, 0 if skip_act_grad else act, Kout, Cin, *ksize, *pad, *stride, *dil), act_p)
 
 
 def _first_layer_pixels(x, cr: int):

@@ -433,3 +433,28 @@ def test_nodes_report_gradients_and_keep_saved_tensor_hooks(layer):
     for a, b in zip(*results):
         assert torch.equal(a, b)
     assert float(results[0][2].abs().sum()) > 0
+
+
+@pytest.mark.parametrize("rows,C", [(1, 8), (3, 24), (64, 120), (1000, 777), (33, 7), (5000, 264), (2, 4099)])
+@pytest.mark.parametrize("act", [native.ACT_NONE, native.ACT_RELU, native.ACT_LEAKY])
+def test_linear_backward_of_ragged_sizes(rows, C, act):
+    """The pass that masks dy, pads its rows and sums its columns (csrc/grad_prep.cu), inside a
+    linear layer whose sizes are no multiples of eight: bias gradients are fp32 sums of the 16-bit
+    values that the products see, so they agree with 64-bit sums of those to 1e-5."""
+    torch.manual_seed(6)
+    K = 19
+    x = torch.randn(rows, K, device="cuda").bfloat16().requires_grad_(True)
+    w = torch.randn(C, K, device="cuda").requires_grad_(True)
+    b = torch.randn(C, device="cuda").requires_grad_(True)
+    wh = nn.WeightHandle(w, torch.zeros_like(w))
+    bh = nn.WeightHandle(b, torch.ones(C, device="cuda"))
+    y = nn.linear(x, wh, bh, act, 0.25 if act == native.ACT_LEAKY else 0.0)
+    dy = torch.randn(rows, C, device="cuda").bfloat16()
+    dx, = torch.autograd.grad(y, x, dy)
+    assert native.consume_status() == 0
+    slope = {native.ACT_NONE: 1.0, native.ACT_RELU: 0.0, native.ACT_LEAKY: 0.25}[act]
+    g = torch.where(y > 0, dy, (dy.float() * slope).bfloat16()).double()
+    wd = w.detach().bfloat16().double()
+    for got, ref, tol in ((bh.grad - 1, g.sum(0), 1e-5), (wh.grad, g.t() @ x.detach().double(), 1e-5),
+                          (dx, g @ wd, 2 ** -8)):
+        assert float((got.double() - ref).norm()) <= tol * float(ref.norm()) + 1e-6
