@@ -234,7 +234,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const uint32_t tS0 = tmem, tO = tmem + 256;
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(smem_u32(&sh.q_full), kAttTile);
       att_load_tile(sQ, &tmQ, smem_u32(&sh.q_full), h, qb * 128, b);
       int j = 0;
@@ -265,7 +265,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
       const uint32_t idesc_qk = make_idesc_f16(fmt, 0, 0, 128, 128);
       const uint32_t idesc_pv = make_idesc_f16(fmt, 0, 1, 128, 128);
@@ -515,7 +515,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       mbar_expect_tx(smem_u32(&sh.kv_full), 2 * kAttTile);
       att_load_tile(sK, &tmK, smem_u32(&sh.kv_full), h, kb * 128, b);
       att_load_tile(sV, &tmV, smem_u32(&sh.kv_full), h, kb * 128, b);
@@ -542,7 +542,7 @@ attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
       const uint32_t idesc_kk = make_idesc_f16(fmt, 0, 0, 128, 128);
       const uint32_t idesc_kn = make_idesc_f16(fmt, 0, 1, 128, 128);
@@ -682,7 +682,7 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       const float* lse = p.lse + ((long long)b * p.H + h) * p.Sq + qb * 128;
       const float* dl = p.delta + ((long long)b * p.H + h) * p.Sq + qb * 128;
       mbar_expect_tx(smem_u32(&sh.kv_full), 2 * kAttTile + 1024);
@@ -708,7 +708,7 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
       const uint32_t idesc_kk = make_idesc_f16(fmt, 0, 0, 128, 128);
       const uint32_t idesc_kn = make_idesc_f16(fmt, 0, 1, 128, 128);

@@ -221,7 +221,7 @@ conv_c8_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const C8FwdParams p,
   const int chunk_px = p.cr == 4 ? 16 : 8;
 
   if (warp == kProducerWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       // tile index -> (tw, h, d, n), advanced incrementally: no divisions in the loop
@@ -264,7 +264,7 @@ conv_c8_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const C8FwdParams p,
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(p.in_dtype == kBF16 ? 1u : 0u, 0, 0, 128, BN);
       // A (K-major, un-swizzled): core matrix = 8 pixels x 16 B; K chunks 128 B apart (LBO),
       // 8-pixel groups mb_pad * 128 B apart (SBO).  B: [K chunk][BN rows][16 B]: K chunks
@@ -546,7 +546,7 @@ conv_c8_fwd_pool_kernel(const __grid_constant__ CUtensorMap tmX, const C8PoolPar
   const uint32_t tmem_base = sh.tmem_base;
 
   if (warp == kProducerWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       RingPos rp;
@@ -578,7 +578,7 @@ conv_c8_fwd_pool_kernel(const __grid_constant__ CUtensorMap tmX, const C8PoolPar
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(p.in_dtype == kBF16 ? 1u : 0u, 0, 0, 128, BN);
       const uint64_t a_desc0 = make_smem_desc(0, 128, p.mb_pad * 128, kLayoutNone);
       const uint64_t b_desc0 = make_smem_desc(s_filter, BN * 16, 128, kLayoutNone);
@@ -777,7 +777,7 @@ conv_c8_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   const int k_steps = (bw_px + 15) / 16;
 
   if (warp == kProducerWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       RingPos rp;
@@ -812,7 +812,7 @@ conv_c8_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       }
     }
   } else if (warp == kMmaWarp) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = make_idesc_f16(p.in_dtype == kBF16 ? 1u : 0u, 1, 1, 128, (uint32_t)p.BN);
       // A (MN-major, un-swizzled): core matrix = 8 pixels x 16 B; row blocks 128 B apart
       // (SBO), 8-pixel groups mb_pad * 128 B apart (LBO); one UMMA = 2 pixel groups.

@@ -1,6 +1,6 @@
 // Halo-slab forward convolution (stride 1, no dilation) for filters that fit in shared
 // memory: 3x3x3 convolutions with few channels on large images, where the implicit-GEMM
-// kernel of conv_tc.cu is bound by the ~300 cycles that every TMA box costs its issuer.
+// kernel of conv_tc.cu brings every pixel in once per tap.
 //
 // Output pixels of one image plane are numbered along a PADDED row pitch
 // Wp = Wo + kw - 1:  q = h * Wp + w.  A tile is 128 consecutive q (rows with w >= Wo or
@@ -124,7 +124,7 @@ conv_slab_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   }
 
   if (warp == 4) {
-    if (lane == 0) {
+    if (elect_one()) {
       // filter: one box per channel block, [cblock][tap][BN rows][Cb]
       const uint32_t fbar = smem_u32(&sh.filter_ready);
       mbar_expect_tx(fbar, (uint32_t)p.filter_bytes);
@@ -179,7 +179,7 @@ conv_slab_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       // Everything between two tcgen05.mma of this loop is on the critical path of the CTA
       // (one thread issues all of them): descriptors differ in the start-address field of
       // their low word only, and the tap offsets are running sums.

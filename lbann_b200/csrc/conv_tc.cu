@@ -23,6 +23,7 @@ struct ConvFwdPolicy {
   static constexpr int BN = BN_;
   static constexpr int kEpiGroups = 2;       // two tiles' epilogues in flight (tc_pipeline.cuh)
   using G = StageGeom<BN>;
+  using HasSingleIssue = void;               // two boxes a slice, issued by one thread
 
   struct Params {
     ConvGeom g;
@@ -73,16 +74,13 @@ struct ConvFwdPolicy {
   }
   __device__ static void load(const Params& p, const Tile& tl, int k, uint32_t sA, uint32_t sB,
                               uint32_t bar, const CUtensorMap* tmA, const CUtensorMap* tmB,
-                              int lane) {
+                              int) {
     const ConvGeom& g = p.g;
     const int ns = slices_in(p, k);
-    // lane 2j issues the activation box of slice j, lane 2j+1 its filter box
-    const int j = lane >> 1;
-    if (j >= ns) return;
-    const int sl = k * p.slices_per_stage + j;
-    const int tap = (int)p.fd_cblocks.div((uint32_t)sl);
-    const int c0 = (sl - tap * p.cblocks) * p.Cb;
-    if ((lane & 1) == 0) {
+    for (int j = 0; j < ns; ++j) {
+      const int sl = k * p.slices_per_stage + j;
+      const int tap = (int)p.fd_cblocks.div((uint32_t)sl);
+      const int c0 = (sl - tap * p.cblocks) * p.Cb;
       uint32_t ua, rem, ub, uc;
       p.fd_khw.divmod((uint32_t)tap, ua, rem);
       p.fd_kw.divmod(rem, ub, uc);
@@ -91,7 +89,6 @@ struct ConvFwdPolicy {
                   tl.w0 * g.sw - g.pw + c * g.dw,
                   tl.h0 * g.sh - g.ph + b * g.dh,
                   tl.d0 * g.sd - g.pd + a * g.dd, tl.n0);
-    } else {
       tma_load_3d(sB + j * (BN * p.Cb * 2), tmB, bar, c0, tl.col0, tap);
     }
   }

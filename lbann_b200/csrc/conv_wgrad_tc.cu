@@ -182,7 +182,7 @@ conv_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       }
     }
   } else if (warp == 5) {
-    if (lane == 0) {
+    if (elect_one()) {
       // descriptors differ in the start-address field of the low word only; four MMAs per
       // accumulator and stage, issued straight-line (see slab_issue_plane for why)
       const uint32_t idesc =
