@@ -6,12 +6,18 @@
 // all of it:
 //
 //   1. every block adds its partial sums into a small replicated accumulator (L2 atomics);
-//   2. grid barrier; block 0 adds the replicas up and - when the statistics span several
-//      ranks - stores its 2 C floats into its slot of every peer's staging buffer (plain peer
-//      stores over NVLink), meets the peers at a bounded flag rendezvous, sums the slots and
-//      publishes the total; grid barrier;
+//   2. grid barrier; every block adds up the replicas of its own channels.  When the statistics
+//      span several ranks, block 0 does so for all of them, stores its 2 C floats into its slot
+//      of every peer's staging buffer (plain peer stores over NVLink), meets the peers at a
+//      bounded flag rendezvous, sums the slots and publishes the total for the others;
 //   3. every block normalises its rows with the total (the second read of x hits the L2 for
 //      activations that fit).
+//
+// What bounds it at layer sizes (5-50 MB, in L2): the chain load -> block sum -> atomics ->
+// barrier -> totals -> load.  So two blocks an SM with eight (backward: twelve) 16-byte loads in
+// flight a thread instead of four blocks with four, sums over the rows of a warp by shuffles, and no
+// second hop through a block that adds the replicas up one after another.  Measured, bf16, forward /
+// backward: 100352 x 64 40 / 40 -> 16 / 21 us, 25088 x 128 47 / 37 -> 14 / 18 us.
 //
 // Backward: the same shape with (sum g, sum g (x - mean)) as the accumulators; the parameter
 // gradients are added to the gradient arena by block 0, the (dmean, dvar) pair crosses the
@@ -43,20 +49,72 @@ __device__ __forceinline__ void bnf_st8(T* p, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(p) = q;
 }
 
-// Sum of an 8-wide register array over the threads of a block that share threadIdx.x; valid
-// where threadIdx.y == 0.  `sm`: blockDim.y * 8 * blockDim.x floats.
-__device__ __forceinline__ void bnf_reduce_y(float (&a)[8], float* sm) {
-  const int bx = blockDim.x;
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < 8; ++j) sm[(threadIdx.y * 8 + j) * bx + threadIdx.x] = a[j];
-  __syncthreads();
-  if (threadIdx.y == 0) {
+constexpr int kBnSums = 8 * 32 * 16;       // floats of shared memory: 8 warps x up to 32 vectors x 16 sums
+
+// The block's sums of a[8] and b[8] over the threads that share threadIdx.x, added to
+// out[channel] and out[C + channel].  blockDim.x is a power of two <= 32, 256 threads.
+__device__ __forceinline__ void bnf_add_sums(float (&a)[8], float (&b)[8], float* sm, float* out, int C, int cv) {
+  const int bx = blockDim.x, tid = threadIdx.y * bx + threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  for (int off = bx; off < 32; off <<= 1) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      float t = 0.f;
-      for (int w = 0; w < (int)blockDim.y; ++w) t += sm[(w * 8 + j) * bx + threadIdx.x];
-      a[j] = t;
+      a[j] += __shfl_xor_sync(0xffffffffu, a[j], off);
+      b[j] += __shfl_xor_sync(0xffffffffu, b[j], off);
+    }
+  }
+  if (lane < bx) {
+    float4* d = reinterpret_cast<float4*>(sm + (warp * bx + lane) * 16);
+    d[0] = make_float4(a[0], a[1], a[2], a[3]);
+    d[1] = make_float4(a[4], a[5], a[6], a[7]);
+    d[2] = make_float4(b[0], b[1], b[2], b[3]);
+    d[3] = make_float4(b[4], b[5], b[6], b[7]);
+  }
+  __syncthreads();
+  for (int i = tid; i < 16 * bx; i += 256) {
+    const int v = blockIdx.x * bx + (i >> 4), q = i & 15;
+    if (v >= cv) continue;
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += sm[w * bx * 16 + i];
+    atomicAdd(out + (q < 8 ? 0 : C) + v * 8 + (q & 7), t);
+  }
+}
+
+// The two totals of this thread's eight channels: from the replicas `acc` ([replicas][2 C]), or
+// from `total` where another block has added them up.  `sm`: kBnSums floats.
+__device__ __forceinline__ void bnf_totals(float (&a)[8], float (&b)[8], float* sm, const float* acc, const float* total,
+                                           int C, int cv) {
+  const int bx = blockDim.x, tid = threadIdx.y * bx + threadIdx.x, items = 16 * bx;
+  int parts = items < 256 ? 256 / items : 1;           // threads per item, each takes replicas / parts
+  if (parts > kBnReplicas) parts = kBnReplicas;
+  if (total) parts = 1;
+  for (int u = tid; u < items * parts; u += 256) {
+    const int part = u / items, i = u - part * items;
+    const int v = blockIdx.x * bx + (i >> 4), q = i & 15;
+    float t = 0.f;
+    if (v < cv) {
+      const int at = (q < 8 ? 0 : C) + v * 8 + (q & 7);
+      if (total) {
+        t = __ldcg(total + at);
+      } else {
+        const int n = kBnReplicas / parts;
+        const float* src = acc + (size_t)part * n * 2 * C + at;
+        float r[kBnReplicas];
+#pragma unroll
+        for (int k = 0; k < kBnReplicas; ++k) r[k] = k < n ? __ldcg(src + (size_t)k * 2 * C) : 0.f;
+#pragma unroll
+        for (int k = 0; k < kBnReplicas; ++k) t += r[k];
+      }
+    }
+    sm[u] = t;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    a[j] = b[j] = 0.f;
+    for (int k = 0; k < parts; ++k) {
+      a[j] += sm[k * items + threadIdx.x * 16 + j];
+      b[j] += sm[k * items + threadIdx.x * 16 + 8 + j];
     }
   }
 }
@@ -167,22 +225,72 @@ struct BnFusedArgs {
   PeerPtrs pp;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(256)
-bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
-  __shared__ float sm[256 * 8];
-  const int C = a.C, cv = C / 8, width = 2 * C;
-  const int v = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = v < cv;
+// What both kernels do between their passes: publish, meet, and return the totals of this
+// thread's channels (false: a wait ran out).  With several ranks block 0
+// also adds the parameter gradients, which are sums over its own rank.
+__device__ __forceinline__ bool bnf_meet(const BnFusedArgs& a, BnWork& w, unsigned epoch, float* acc, float* sm,
+                                         bool backward, float (&ta)[8], float (&tb)[8], int* status) {
+  const int C = a.C, width = 2 * C;
   const unsigned nblocks = gridDim.x * gridDim.y;
   const bool lead = blockIdx.x == 0 && blockIdx.y == 0;
   const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
+  const bool alone = a.world <= 1;
+  bool ok = bn_grid_arrive_wait(w.ctl, epoch, nblocks, alone || lead, status);
+  if (lead) {
+    if (!alone) {
+      if (ok) {
+        for (int i = tid; i < width; i += nthr) {
+          float t = 0.f;
+          for (int rp = 0; rp < kBnReplicas; ++rp) t += __ldcg(acc + (size_t)rp * width + i);
+          w.total[i] = t;
+        }
+        __syncthreads();
+        if (backward) {
+          // parameter gradients are local sums (the gradient reduction of the step sums the ranks)
+          for (int c = tid; c < C; c += nthr) {
+            const float rstd = rsqrtf(a.stats[C + c] + a.eps);
+            if (a.dscale) a.dscale[c] += w.total[C + c] * rstd;
+            if (a.dbias) a.dbias[c] += w.total[c];
+          }
+          __syncthreads();
+        }
+        ok = bn_cross_rank_sum(a.pp, a.rank, a.world, w.total, width, a.slot_stride, a.ctr, status);
+      }
+      __syncthreads();
+    }
+    if (tid == 0) {
+      __threadfence();
+      atomicAdd(w.ctl + 2, 1u);                 // totals published (also on failure: nobody hangs)
+      atomicAdd(w.ctl, 1u);                     // every block has read the launch count by now
+    }
+  }
+  if (!alone) ok = bn_wait_block(w.ctl + 2, epoch + 1u, status) && ok;
+  if (!ok) return false;
+  bnf_totals(ta, tb, sm, acc, alone ? nullptr : w.total, C, C / 8);
+  return true;
+}
+
+// The accumulators of the next launch: nobody uses them during this one.
+__device__ __forceinline__ void bnf_clear_next(const BnWork& w, unsigned epoch, int width) {
+  if (blockIdx.x != 0 || blockIdx.y != 0) return;
+  float* next = w.acc + (size_t)((epoch + 1u) & 1u) * kBnReplicas * width;
+  for (int i = threadIdx.y * blockDim.x + threadIdx.x; i < kBnReplicas * width; i += 256) next[i] = 0.f;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256, 2)
+bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
+  __shared__ __align__(16) float sm[kBnSums];
+  const int C = a.C, cv = C / 8, width = 2 * C;
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool valid = v < cv;
   BnWork w = bn_work(a.ws, width);
   const unsigned epoch = *reinterpret_cast<volatile unsigned*>(w.ctl);
   float* acc = w.acc + (size_t)(epoch & 1u) * kBnReplicas * width;
   const T* x = reinterpret_cast<const T*>(a.x);
   const long long r0 = (long long)blockIdx.y * a.rows_per_block;
   const long long r1 = min(a.rows, r0 + a.rows_per_block);
+  const long long step = blockDim.y;
 
   // ---- 1. partial sums
   float s[8], ss[8];
@@ -190,14 +298,13 @@ bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
   for (int j = 0; j < 8; ++j) { s[j] = 0.f; ss[j] = 0.f; }
   if (valid) {
     const T* base = x + v * 8;
-    const long long step = blockDim.y;
     long long r = r0 + threadIdx.y;
-    for (; r + 3 * step < r1; r += 4 * step) {
-      uint4 q[4];
+    for (; r + 7 * step < r1; r += 8 * step) {
+      uint4 q[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) q[u] = *reinterpret_cast<const uint4*>(base + (r + u * step) * C);
+      for (int u = 0; u < 8; ++u) q[u] = *reinterpret_cast<const uint4*>(base + (r + u * step) * C);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < 8; ++u) {
         const T* e = reinterpret_cast<const T*>(&q[u]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -207,6 +314,7 @@ bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
         }
       }
     }
+#pragma unroll 4
     for (; r < r1; r += step) {
       float f[8];
       bnf_ld8<T>(base + r * C, f);
@@ -214,41 +322,11 @@ bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
       for (int j = 0; j < 8; ++j) { s[j] += f[j]; ss[j] += f[j] * f[j]; }
     }
   }
-  bnf_reduce_y(s, sm);
-  bnf_reduce_y(ss, sm);
-  if (valid && threadIdx.y == 0) {
-    float* out = acc + (size_t)(blockIdx.y % kBnReplicas) * width;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      atomicAdd(out + v * 8 + j, s[j]);
-      atomicAdd(out + C + v * 8 + j, ss[j]);
-    }
-  }
+  bnf_add_sums(s, ss, sm, acc + (size_t)(blockIdx.y % kBnReplicas) * width, C, cv);
+  bnf_clear_next(w, epoch, width);
 
-  // ---- 2. grid barrier; the lead block forms the total (over the ranks too)
-  bool ok = bn_grid_arrive_wait(w.ctl, epoch, nblocks, lead, status);
-  if (lead) {
-    if (ok) {
-      for (int i = tid; i < width; i += nthr) {
-        float t = 0.f;
-        for (int rp = 0; rp < kBnReplicas; ++rp) {
-          t += __ldcg(acc + (size_t)rp * width + i);
-          acc[(size_t)rp * width + i] = 0.f;          // ready for the launch after the next
-        }
-        w.total[i] = t;
-      }
-      __syncthreads();
-      if (a.world > 1)
-        ok = bn_cross_rank_sum(a.pp, a.rank, a.world, w.total, width, a.slot_stride, a.ctr, status);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(w.ctl + 2, 1u);                 // totals published (also on failure: nobody hangs)
-      atomicAdd(w.ctl, 1u);                     // every block has read the launch count by now
-    }
-  }
-  if (!bn_wait_block(w.ctl + 2, epoch + 1u, status) || !ok) return;
+  // ---- 2. the totals (over the ranks too)
+  if (!bnf_meet(a, w, epoch, acc, sm, false, s, ss, status)) return;
 
   // ---- 3. normalise
   if (!valid) return;
@@ -256,8 +334,8 @@ bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int c = v * 8 + j;
-    const float m = __ldcg(w.total + c) / a.count;
-    const float sq = __ldcg(w.total + C + c) / a.count;
+    const float m = s[j] / a.count;
+    const float sq = ss[j] / a.count;
     float var = a.count * (sq - m * m) / (a.count - a.correction);
     var = var > a.eps ? var : a.eps;
     const float rstd = rsqrtf(var + a.eps);
@@ -275,7 +353,7 @@ bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
   }
   T* y = reinterpret_cast<T*>(a.out);
 #pragma unroll 4
-  for (long long r = r0 + threadIdx.y; r < r1; r += blockDim.y) {
+  for (long long r = r0 + threadIdx.y; r < r1; r += step) {
     float f[8];
     bnf_ld8<T>(x + r * C + v * 8, f);
 #pragma unroll
@@ -289,16 +367,35 @@ bn_fused_fwd_kernel(const BnFusedArgs a, int* status) {
   }
 }
 
+// Rows r, r + step, ... of up to kRows x, dy and (where act) y; the loads come first.
+template <typename T, int kRows>
+struct BnRows {
+  uint4 x[kRows], g[kRows], y[kRows];
+  __device__ __forceinline__ void load(const T* px, const T* pg, const T* py, long long off, long long stride, bool act) {
+#pragma unroll
+    for (int u = 0; u < kRows; ++u) {
+      x[u] = *reinterpret_cast<const uint4*>(px + off + u * stride);
+      g[u] = *reinterpret_cast<const uint4*>(pg + off + u * stride);
+      if (act) y[u] = *reinterpret_cast<const uint4*>(py + off + u * stride);
+    }
+  }
+  // the gradient behind the activation
+  __device__ __forceinline__ float grad(int u, int j, int act, float slope) const {
+    const float v = to_f32<T>(reinterpret_cast<const T*>(&g[u])[j]);
+    if (act == 0) return v;
+    const float o = to_f32<T>(reinterpret_cast<const T*>(&y[u])[j]);
+    return o > 0.f ? v : (act == 1 ? 0.f : slope * v);
+  }
+  __device__ __forceinline__ float in(int u, int j) const { return to_f32<T>(reinterpret_cast<const T*>(&x[u])[j]); }
+};
+
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 bn_fused_bwd_kernel(const BnFusedArgs a, int* status) {
-  __shared__ float sm[256 * 8];
+  __shared__ __align__(16) float sm[kBnSums];
   const int C = a.C, cv = C / 8, width = 2 * C;      // accumulators: S1 = sum g, S2 = sum g (x - mean)
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = v < cv;
-  const unsigned nblocks = gridDim.x * gridDim.y;
-  const bool lead = blockIdx.x == 0 && blockIdx.y == 0;
-  const int tid = threadIdx.y * blockDim.x + threadIdx.x, nthr = blockDim.x * blockDim.y;
   BnWork w = bn_work(a.ws, width);
   const unsigned epoch = *reinterpret_cast<volatile unsigned*>(w.ctl);
   float* acc = w.acc + (size_t)(epoch & 1u) * kBnReplicas * width;
@@ -308,6 +405,7 @@ bn_fused_bwd_kernel(const BnFusedArgs a, int* status) {
   const int act = ya ? a.act : 0;
   const long long r0 = (long long)blockIdx.y * a.rows_per_block;
   const long long r1 = min(a.rows, r0 + a.rows_per_block);
+  const long long step = blockDim.y;
 
   float mean[8], s1[8], s2[8];
 #pragma unroll
@@ -315,64 +413,31 @@ bn_fused_bwd_kernel(const BnFusedArgs a, int* status) {
     mean[j] = a.stats[valid ? v * 8 + j : 0];
     s1[j] = s2[j] = 0.f;
   }
-  if (valid) {
-#pragma unroll 4
-    for (long long r = r0 + threadIdx.y; r < r1; r += blockDim.y) {
-      float fx[8], fg[8], fy[8];
-      bnf_ld8<T>(x + r * C + v * 8, fx);
-      bnf_ld8<T>(dy + r * C + v * 8, fg);
-      if (act) bnf_ld8<T>(ya + r * C + v * 8, fy);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float g = fg[j];
-        if (act == 1) g = fy[j] > 0.f ? g : 0.f;
-        else if (act == 2) g = fy[j] > 0.f ? g : a.act_param * g;
-        s1[j] += g;
-        s2[j] += g * (fx[j] - mean[j]);
-      }
-    }
-  }
-  bnf_reduce_y(s1, sm);
-  bnf_reduce_y(s2, sm);
-  if (valid && threadIdx.y == 0) {
-    float* out = acc + (size_t)(blockIdx.y % kBnReplicas) * width;
+  auto add = [&](const auto& rows, int u) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      atomicAdd(out + v * 8 + j, s1[j]);
-      atomicAdd(out + C + v * 8 + j, s2[j]);
+      const float g = rows.grad(u, j, act, a.act_param);
+      s1[j] += g;
+      s2[j] += g * (rows.in(u, j) - mean[j]);
+    }
+  };
+  if (valid) {
+    long long r = r0 + threadIdx.y;
+    for (; r + 3 * step < r1; r += 4 * step) {
+      BnRows<T, 4> q;
+      q.load(x, dy, ya, r * C + v * 8, step * C, act != 0);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) add(q, u);
+    }
+    for (; r < r1; r += step) {
+      BnRows<T, 1> q;
+      q.load(x, dy, ya, r * C + v * 8, 0, act != 0);
+      add(q, 0);
     }
   }
-
-  bool ok = bn_grid_arrive_wait(w.ctl, epoch, nblocks, lead, status);
-  if (lead) {
-    if (ok) {
-      for (int i = tid; i < width; i += nthr) {
-        float t = 0.f;
-        for (int rp = 0; rp < kBnReplicas; ++rp) {
-          t += __ldcg(acc + (size_t)rp * width + i);
-          acc[(size_t)rp * width + i] = 0.f;
-        }
-        w.total[i] = t;
-      }
-      __syncthreads();
-      // parameter gradients are local sums (the gradient reduction of the step sums the ranks)
-      for (int c = tid; c < C; c += nthr) {
-        const float rstd = rsqrtf(a.stats[C + c] + a.eps);
-        if (a.dscale) a.dscale[c] += w.total[C + c] * rstd;
-        if (a.dbias) a.dbias[c] += w.total[c];
-      }
-      __syncthreads();
-      if (a.world > 1)
-        ok = bn_cross_rank_sum(a.pp, a.rank, a.world, w.total, width, a.slot_stride, a.ctr, status);
-    }
-    __syncthreads();
-    if (tid == 0) {
-      __threadfence();
-      atomicAdd(w.ctl + 2, 1u);
-      atomicAdd(w.ctl, 1u);
-    }
-  }
-  if (!bn_wait_block(w.ctl + 2, epoch + 1u, status) || !ok) return;
+  bnf_add_sums(s1, s2, sm, acc + (size_t)(blockIdx.y % kBnReplicas) * width, C, cv);
+  bnf_clear_next(w, epoch, width);
+  if (!bnf_meet(a, w, epoch, acc, sm, true, s1, s2, status)) return;
   if (!valid) return;
 
   // dx = g scale rstd + dmean / n + dvar 2 (x - mean) / (n - corr), with
@@ -383,26 +448,34 @@ bn_fused_bwd_kernel(const BnFusedArgs a, int* status) {
     const int c = v * 8 + j;
     const float rstd = rsqrtf(a.stats[C + c] + a.eps);
     const float sc = a.scale ? a.scale[c] : 1.f;
-    const float S1 = __ldcg(w.total + c), S2 = __ldcg(w.total + C + c);
+    const float S1 = s1[j], S2 = s2[j];
+    if (a.world <= 1 && blockIdx.y == 0 && threadIdx.y == 0) {
+      if (a.dscale) a.dscale[c] += S2 * rstd;
+      if (a.dbias) a.dbias[c] += S1;
+    }
     k0[j] = sc * rstd;
     k1[j] = -sc * rstd * S1 / a.count;
     k2[j] = -0.5f * sc * rstd * rstd * rstd * S2 * 2.f / (a.count - a.correction);
   }
   T* dx = reinterpret_cast<T*>(a.out);
-#pragma unroll 4
-  for (long long r = r0 + threadIdx.y; r < r1; r += blockDim.y) {
-    float fx[8], fg[8], fy[8];
-    bnf_ld8<T>(x + r * C + v * 8, fx);
-    bnf_ld8<T>(dy + r * C + v * 8, fg);
-    if (act) bnf_ld8<T>(ya + r * C + v * 8, fy);
+  auto put = [&](const auto& rows, int u, long long off) {
+    float f[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float g = fg[j];
-      if (act == 1) g = fy[j] > 0.f ? g : 0.f;
-      else if (act == 2) g = fy[j] > 0.f ? g : a.act_param * g;
-      fx[j] = g * k0[j] + k1[j] + k2[j] * (fx[j] - mean[j]);
-    }
-    bnf_st8<T>(dx + r * C + v * 8, fx);
+    for (int j = 0; j < 8; ++j)
+      f[j] = rows.grad(u, j, act, a.act_param) * k0[j] + k1[j] + k2[j] * (rows.in(u, j) - mean[j]);
+    bnf_st8<T>(dx + off, f);
+  };
+  long long r = r0 + threadIdx.y;
+  for (; r + step < r1; r += 2 * step) {
+    BnRows<T, 2> q;
+    q.load(x, dy, ya, r * C + v * 8, step * C, act != 0);
+    put(q, 0, r * C + v * 8);
+    put(q, 1, (r + step) * C + v * 8);
+  }
+  for (; r < r1; r += step) {
+    BnRows<T, 1> q;
+    q.load(x, dy, ya, r * C + v * 8, 0, act != 0);
+    put(q, 0, r * C + v * 8);
   }
 }
 
@@ -424,7 +497,7 @@ static BnGrid bn_fused_grid(K kernel, long long rows, int C) {
   int per_sm = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, 0);
   if (per_sm < 1) per_sm = 1;
-  if (per_sm > 4) per_sm = 4;
+  if (per_sm > 2) per_sm = 2;
   long long cap = (long long)lbhost::sm_count() * per_sm / gx;
   if (cap < 1) cap = 1;
   long long gy = (rows + by - 1) / by;

@@ -458,3 +458,41 @@ def test_linear_backward_of_ragged_sizes(rows, C, act):
     for got, ref, tol in ((bh.grad - 1, g.sum(0), 1e-5), (wh.grad, g.t() @ x.detach().double(), 1e-5),
                           (dx, g @ wd, 2 ** -8)):
         assert float((got.double() - ref).norm()) <= tol * float(ref.norm()) + 1e-6
+
+
+@pytest.mark.parametrize("N,C,H,W", [(1, 8, 1, 2), (3, 24, 5, 7), (2, 2048, 3, 5), (16, 64, 40, 41), (2, 264, 33, 9)])
+@pytest.mark.parametrize("act", [native.ACT_NONE, native.ACT_RELU])
+def test_batch_norm_fused_edges(N, C, H, W, act):
+    """The one-kernel batch norm from one row of blocks to a full grid, at the smallest and largest
+    channel counts; three passes in a row (its accumulators alternate and are cleared by the
+    launch in between), each against 64 bits: outputs are rounded to 2^-9, sums are fp32."""
+    torch.manual_seed(5)
+    s = (1 + 0.2 * torch.randn(C, device="cuda")).requires_grad_(True)
+    b = (0.1 * torch.randn(C, device="cuda")).requires_grad_(True)
+    sh, bh = nn.WeightHandle(s, torch.zeros(C, device="cuda")), nn.WeightHandle(b, torch.zeros(C, device="cuda"))
+    rm, rv = torch.zeros(C, device="cuda"), torch.ones(C, device="cuda")
+    for _ in range(3):
+        sh.grad.zero_()
+        bh.grad.zero_()
+        x = (torch.randn(N, C, H, W, device="cuda") * 2 + 0.5).bfloat16().contiguous(
+            memory_format=torch.channels_last).requires_grad_(True)
+        dy = torch.randn(N, C, H, W, device="cuda").bfloat16().contiguous(memory_format=torch.channels_last)
+        y = nn.batch_norm(x, sh, bh, rm, rv, True, 1e-5, 0.9, act=act)
+        dx, = torch.autograd.grad(y, x, dy)
+        assert native.consume_status() == 0
+        xd, sd, bd = (t.detach().double().requires_grad_(True) for t in (x, s, b))
+        n = N * H * W
+        mean = xd.mean((0, 2, 3), keepdim=True)
+        var = (((xd - mean) ** 2).sum((0, 2, 3), keepdim=True) / (n - 1)).clamp(min=1e-5)
+        ref = (xd - mean) / torch.sqrt(var + 1e-5) * sd.view(1, -1, 1, 1) + bd.view(1, -1, 1, 1)
+        gd = dy.double()
+        if act:
+            gd = gd * (y > 0)                 # the kernel masks with its own output
+            want_y = torch.relu(ref.detach())
+        else:
+            want_y = ref.detach()
+        refs = torch.autograd.grad(ref, (xd, sd, bd), gd)
+        # two rows: dx is the difference of nearly equal terms, compared with the size of those
+        floor = 0.01 * float((gd * (sd / torch.sqrt(var.view(-1) + 1e-5)).view(1, -1, 1, 1)).norm())
+        for got, want in zip((y, dx, sh.grad, bh.grad), (want_y, *refs)):
+            assert float((got.double() - want).norm()) <= 0.006 * float(want.norm()) + floor * 0.5
