@@ -13,20 +13,16 @@
 // head strides (so the three slices of a packed [B][S][3 H 128] projection are used in
 // place, and the output needs no permute).  Sequence lengths are multiples of 128.
 //
-// Warp roles (320 threads, one CTA per (batch, head, 128 query rows)):
-//   warp 4  TMA producer (Q once, then a two-stage ring of K and V tiles)
-//   warp 5  TMEM allocation + MMA issue (one lane)
-//   warps 0-3 and 6-9  softmax, rescaling of O, epilogue: two threads per query row, one for
-//              key columns 0-63 of a block and one for 64-127 (two warps per scheduler hide
-//              each other's TMEM and MUFU latency); the pair exchanges its row maxima
-//              through shared memory
+// Warp roles (320 threads): warp 4 loads (TMA), warp 5 allocates TMEM and issues the MMAs (one
+// elected thread each), warps 0-3 and 6-9 own the accumulator rows.
 //
-// Backward is two kernels of the same shape, both recomputing P from Q, K and the saved
-// log-sum-exp: attn_bwd_kv_kernel (one CTA per 128 keys, loop over query blocks:
-// dV += P^T dO, dK += dS^T Q) and attn_bwd_q_kernel (one CTA per 128 queries, loop over key
-// blocks: dQ += dS K), with dS = P * (dP - rowsum(dO * O)) * scale.
+// Backward is one launch of two kinds of CTA, both recomputing P from Q, K and the saved
+// log-sum-exp: one per 128 keys (loop over queries: dV += P^T dO, dK += dS^T Q) and one per 128
+// queries (loop over keys: dQ += dS K), with dS = P * (dP - rowsum(dO * O)) * scale.
 //
 // Every wait is bounded; a wait that runs out records a status code and all roles leave.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace lb {
@@ -44,21 +40,22 @@ struct AttnParams {
   // outputs / side inputs (element strides: batch, token, head; head dim contiguous)
   void* o; long long o_sb, o_ss, o_sh;
   float* lse;            // [B][H][Sq], log2 domain: max + log2(sum)
-  const float* delta;    // [B][H][Sq] rowsum(dO * O) (backward)
+  const float* delta;    // [B][H][Sq] scale * rowsum(dO * O) (backward)
   void* dq; long long dq_sb, dq_ss, dq_sh;
   void* dk; long long dk_sb, dk_ss, dk_sh;
   void* dv; long long dv_sb, dv_ss, dv_sh;
 };
 
+constexpr int kFwdSlots = 3;               // ring of K and V tiles: K0 V0 K1 V1 ...
+constexpr int kFwdSmem = (2 + 2 + kFwdSlots) * kAttTile + 1024;
+
 struct AttnShared {
   uint64_t q_full;
-  uint64_t k_full[2], v_full[2], k_empty[2], v_empty[2];
-  uint64_t s_full[2], s_empty[2];
-  uint64_t p_full, pv_done;
-  uint64_t x_full[2], l_full;  // the two threads of a row have published their partial values
+  uint64_t kv_full[kFwdSlots], kv_empty[kFwdSlots];
+  uint64_t s_full[2], s_empty[2];      // scores of a query tile: complete / read by its four warps
+  uint64_t p_full[2], pv_done[2];      // probabilities written by four warps / their product retired
   uint32_t tmem_base;
   int abort_flag;
-  float xch[3][2][128];      // [slot][column half][row]: partial row maxima (0, 1) / sums (2)
 };
 
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
@@ -121,36 +118,15 @@ __device__ __forceinline__ void att_load_tile(uint32_t dst, const CUtensorMap* t
   tma_load_4d(dst + kAttHalf, tm, bar, 64, h, s0, b);
 }
 
-// Packs 32 fp32 values to 16-bit and stores them as columns [c0, c0 + 32) of row `row`.
-__device__ __forceinline__ void att_store_row32(uint32_t tile, int row, int c0, const float (&v)[32],
-                                                int dtype) {
-#pragma unroll
-  for (int j = 0; j < 32; j += 8) {
-    uint4 q;
-    q.x = pack2(v[j], v[j + 1], dtype);
-    q.y = pack2(v[j + 2], v[j + 3], dtype);
-    q.z = pack2(v[j + 4], v[j + 5], dtype);
-    q.w = pack2(v[j + 6], v[j + 7], dtype);
-    sts128(tile + att_tile_off(row, c0 + j), q);
-  }
-}
-
 constexpr int kAttThreads = 320;
 
-// Role of a warp among the 8 that work on accumulator rows: `group` picks the column half,
+// Role of a warp among the 8 that work on accumulator rows: `group` 0 or 1 (four warps each),
 // `quarter` the 32 TMEM lanes (= rows) that the warp may access (warp index modulo 4).
 __device__ __forceinline__ bool att_row_role(int warp, int& group, int& quarter) {
   if (warp == 4 || warp == 5) return false;
   group = warp < 4 ? 0 : 1;
   quarter = warp & 3;
   return true;
-}
-
-// 64 fp32 values of one row -> 16-bit, columns [c0, c0 + 64) of a K-major tile.
-__device__ __forceinline__ void att_store_row64(uint32_t tile, int row, int c0, const uint32_t (&pk)[32]) {
-#pragma unroll
-  for (int j = 0; j < 8; ++j)
-    sts128(tile + att_tile_off(row, c0 + 8 * j), make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]));
 }
 
 // 64 accumulator columns of one row, scaled, -> 16-bit global row (16-byte stores).
@@ -183,38 +159,47 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 // ------------------------------------------------------------------------------------
-// Forward
+// Forward.  A CTA holds two tiles of 128 queries (one, where that gives every SM a CTA) and walks
+// the keys 128 at a time.  Each tile has four warps, one thread per query, and its own scores,
+// probabilities and output accumulator; scores of the next keys are computed as soon as a
+// tile's warps have read the present ones, so a tile's warps never wait for the tensor core and
+// the tensor core works for one tile while the other's exponentials run.  (One tile per CTA
+// with two threads per query left every latency of the chain exposed and cost 5700 cycles a
+// block of 128 x 128, whose MMAs and exponentials take 1024 each.)  B = 2, H = 16, S = 2048,
+// causal, bf16: 89 -> 50 us.
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kAttThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                const __grid_constant__ CUtensorMap tmV, const AttnParams p, int* status) {
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ AttnParams p, int tiles, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ AttnShared sh;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = base, sK = base + kAttTile, sV = base + 3 * kAttTile, sP = base + 5 * kAttTile;
+  const uint32_t sQ = base, sP = base + 2 * kAttTile, sKV = base + 4 * kAttTile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &sh.abort_flag;
 
+  // the longest (late) query blocks first; tile t of this CTA is query block qb0 + t
   const int nqb = p.Sq / 128;
-  const int qb = nqb - 1 - (int)blockIdx.x;            // long (late) query blocks first
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int nkv = p.causal ? qb + 1 : p.Sk / 128;
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int qb0 = ((nqb + tiles - 1) / tiles - 1 - (int)blockIdx.z) * tiles;
+  const int have = min(tiles, nqb - qb0);                // 1 or 2 tiles
+  int n[2];
+#pragma unroll
+  for (int t = 0; t < 2; ++t) n[t] = t < have ? (p.causal ? qb0 + t + 1 : p.Sk / 128) : 0;
+  const int nmax = max(n[0], n[1]);
 
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&sh.q_full), 1);
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(smem_u32(&sh.k_full[s]), 1);
-      mbar_init(smem_u32(&sh.v_full[s]), 1);
-      mbar_init(smem_u32(&sh.k_empty[s]), 1);
-      mbar_init(smem_u32(&sh.v_empty[s]), 1);
-      mbar_init(smem_u32(&sh.s_full[s]), 1);
-      mbar_init(smem_u32(&sh.s_empty[s]), 256);
+    for (int s = 0; s < kFwdSlots; ++s) {
+      mbar_init(smem_u32(&sh.kv_full[s]), 1);
+      mbar_init(smem_u32(&sh.kv_empty[s]), 1);
     }
-    mbar_init(smem_u32(&sh.p_full), 256);
-    mbar_init(smem_u32(&sh.pv_done), 1);
-    mbar_init(smem_u32(&sh.x_full[0]), 256);
-    mbar_init(smem_u32(&sh.x_full[1]), 256);
-    mbar_init(smem_u32(&sh.l_full), 256);
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(smem_u32(&sh.s_full[t]), 1);
+      mbar_init(smem_u32(&sh.s_empty[t]), 4);
+      mbar_init(smem_u32(&sh.p_full[t]), 4);
+      mbar_init(smem_u32(&sh.pv_done[t]), 1);
+    }
     sh.abort_flag = 0;
     mbar_fence_init();
   }
@@ -230,38 +215,32 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = sh.tmem_base;
-  const uint32_t tS0 = tmem, tO = tmem + 256;
+  const uint32_t tmem = sh.tmem_base;                    // scores of tile t at 128 t, outputs at 256 + 128 t
 
   if (warp == 4) {
     if (elect_one()) {
-      mbar_expect_tx(smem_u32(&sh.q_full), kAttTile);
-      att_load_tile(sQ, &tmQ, smem_u32(&sh.q_full), h, qb * 128, b);
-      int j = 0;
+      mbar_expect_tx(smem_u32(&sh.q_full), (uint32_t)have * kAttTile);
+      for (int t = 0; t < have; ++t)
+        att_load_tile(sQ + t * kAttTile, &tmQ, smem_u32(&sh.q_full), h, (qb0 + t) * 128, b);
+      RingPos rp;
+      int seq = 0;
       bool ok = true;
-      for (; j < nkv && ok; ++j) {
-        const int s = j & 1;
-        if (j >= 2) {
-          const uint32_t par = ((j >> 1) - 1) & 1;
-          if (!mbar_wait_bounded(smem_u32(&sh.k_empty[s]), par, abort_flag) ||
-              !mbar_wait_bounded(smem_u32(&sh.v_empty[s]), par, abort_flag)) {
-            raise_status(status, abort_flag, kTimeoutStageEmpty);
-            ok = false;
-            break;
-          }
+      for (; seq < 2 * nmax; ++seq) {                    // K of block seq / 2, then its V
+        if (!mbar_wait_bounded(smem_u32(&sh.kv_empty[rp.s]), rp.ph ^ 1, abort_flag)) {
+          raise_status(status, abort_flag, kTimeoutStageEmpty);
+          ok = false;
+          break;
         }
-        mbar_expect_tx(smem_u32(&sh.k_full[s]), kAttTile);
-        att_load_tile(sK + s * kAttTile, &tmK, smem_u32(&sh.k_full[s]), h, j * 128, b);
-        mbar_expect_tx(smem_u32(&sh.v_full[s]), kAttTile);
-        att_load_tile(sV + s * kAttTile, &tmV, smem_u32(&sh.v_full[s]), h, j * 128, b);
+        const uint32_t bar = smem_u32(&sh.kv_full[rp.s]);
+        mbar_expect_tx(bar, kAttTile);
+        att_load_tile(sKV + rp.s * kAttTile, (seq & 1) ? &tmV : &tmK, bar, h, (seq >> 1) * 128, b);
+        rp.advance(kFwdSlots);
       }
       if (!ok || *abort_flag) {
         // let the copies in flight land before shared memory is released
         mbar_wait_budget_only(smem_u32(&sh.q_full), 0);
-        for (int i = (j >= 2 ? j - 2 : 0); i < j; ++i) {
-          mbar_wait_budget_only(smem_u32(&sh.k_full[i & 1]), (i >> 1) & 1);
-          mbar_wait_budget_only(smem_u32(&sh.v_full[i & 1]), (i >> 1) & 1);
-        }
+        for (int j = seq > kFwdSlots ? seq - kFwdSlots : 0; j < seq; ++j)
+          mbar_wait_budget_only(smem_u32(&sh.kv_full[j % kFwdSlots]), (j / kFwdSlots) & 1);
       }
     }
   } else if (warp == 5) {
@@ -271,158 +250,168 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       const uint32_t idesc_pv = make_idesc_f16(fmt, 0, 1, 128, 128);
       bool ok = mbar_wait_bounded(smem_u32(&sh.q_full), 0, abort_flag);
       if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
-      for (int j = 0; j <= nkv && ok; ++j) {
-        if (j < nkv) {
-          const int s = j & 1;
-          if (!mbar_wait_bounded(smem_u32(&sh.k_full[s]), (j >> 1) & 1, abort_flag)) {
+      RingPos kp, vp;                                    // slots of K(j) and V(j - 1): sequence 2 j and 2 j - 1
+      vp.advance(kFwdSlots);
+      for (int j = 0; j <= nmax && ok; ++j) {
+        if (j < nmax) {
+          if (!mbar_wait_bounded(smem_u32(&sh.kv_full[kp.s]), kp.ph, abort_flag)) {
             raise_status(status, abort_flag, kTimeoutTmaFull);
             ok = false;
             break;
           }
-          if (j >= 2 && !mbar_wait_bounded(smem_u32(&sh.s_empty[s]), ((j >> 1) - 1) & 1, abort_flag)) {
-            raise_status(status, abort_flag, kTimeoutTmemEmpty);
-            ok = false;
-            break;
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (j >= n[t]) continue;
+            if (j >= 1 && !mbar_wait_bounded(smem_u32(&sh.s_empty[t]), (j - 1) & 1, abort_flag)) {
+              raise_status(status, abort_flag, kTimeoutTmemEmpty);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            att_mma_kk(tmem + t * 128, sQ + t * kAttTile, sKV + kp.s * kAttTile, idesc_qk, false);
+            umma_commit(smem_u32(&sh.s_full[t]));
           }
-          tc_fence_after();
-          att_mma_kk(tS0 + s * 128, sQ, sK + s * kAttTile, idesc_qk, false);
-          umma_commit(smem_u32(&sh.k_empty[s]));
-          umma_commit(smem_u32(&sh.s_full[s]));
+          if (!ok) break;
+          umma_commit(smem_u32(&sh.kv_empty[kp.s]));
+          kp.advance(kFwdSlots);
+          kp.advance(kFwdSlots);
         }
         if (j >= 1) {
-          const int jj = j - 1, s = jj & 1;
-          if (!mbar_wait_bounded(smem_u32(&sh.p_full), jj & 1, abort_flag) ||
-              !mbar_wait_bounded(smem_u32(&sh.v_full[s]), (jj >> 1) & 1, abort_flag)) {
+          const int jj = j - 1;
+          if (!mbar_wait_bounded(smem_u32(&sh.kv_full[vp.s]), vp.ph, abort_flag)) {
             raise_status(status, abort_flag, kTimeoutTmaFull);
             ok = false;
             break;
           }
-          tc_fence_after();
-          att_mma_kn(tO, sP, sV + s * kAttTile, idesc_pv, jj > 0);
-          umma_commit(smem_u32(&sh.v_empty[s]));
-          umma_commit(smem_u32(&sh.pv_done));
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            if (jj >= n[t]) continue;
+            if (!mbar_wait_bounded(smem_u32(&sh.p_full[t]), jj & 1, abort_flag)) {
+              raise_status(status, abort_flag, kTimeoutTmemEmpty);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            att_mma_kn(tmem + 256 + t * 128, sP + t * kAttTile, sKV + vp.s * kAttTile, idesc_pv, jj > 0);
+            umma_commit(smem_u32(&sh.pv_done[t]));
+          }
+          if (!ok) break;
+          umma_commit(smem_u32(&sh.kv_empty[vp.s]));
+          vp.advance(kFwdSlots);
+          vp.advance(kFwdSlots);
         }
       }
     }
   } else {
     // ---------------------------------------------------------------- softmax / epilogue
-    int group = 0, quarter = 0;
-    att_row_role(warp, group, quarter);
-    const int row = quarter * 32 + lane;               // query row of this thread
-    const int col0 = group * 64;                       // its half of the key columns / head dim
+    int t = 0, quarter = 0;
+    att_row_role(warp, t, quarter);
+    const int row = quarter * 32 + lane;                 // query row of this thread in tile t
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t tS = tmem + t * 128 + lane_off, tO = tmem + 256 + t * 128 + lane_off;
+    const uint32_t tile = sP + t * kAttTile;
+    const int nt = t == 0 ? n[0] : n[1];
     float m = -1e30f, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < nkv && ok; ++j) {
-      const int s = j & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full[s]), (j >> 1) & 1, abort_flag));
+    for (int j = 0; j < nt && ok; ++j) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full[t]), j & 1, abort_flag));
       if (!ok) {
         if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
         break;
       }
       tc_fence_after();
-      const uint32_t tS = tS0 + s * 128 + lane_off + col0;
-      const int limit = (p.causal && j == qb) ? row : 127;        // last visible key column
-      uint32_t ra[32], rb[32];
-      tmem_ld_32x32(tS, ra);
-      tmem_ld_32x32(tS + 32, rb);
-      tmem_ld_wait();
-      float mx = -1e30f;
+      uint32_t r[4][32];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (col0 + i <= limit) mx = fmaxf(mx, __uint_as_float(ra[i]));
-        if (col0 + 32 + i <= limit) mx = fmaxf(mx, __uint_as_float(rb[i]));
-      }
-      // exchange with the thread that holds the other half of this row (bounded wait)
-      sh.xch[s][group][row] = mx;
-      mbar_arrive(smem_u32(&sh.x_full[s]));
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.x_full[s]), (j >> 1) & 1, abort_flag));
-      if (!ok) {
-        if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-        break;
-      }
-      mx = fmaxf(mx, sh.xch[s][group ^ 1][row]) * p.scale_log2;
+      for (int c = 0; c < 4; ++c) tmem_ld_32x32(tS + 32 * c, r[c]);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.s_empty[t]));
+      const bool diag = p.causal && j == nt - 1;         // columns up to `row` are visible
+      auto row_max = [&](auto masked) {
+        float mx[4] = {-1e30f, -1e30f, -1e30f, -1e30f};
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (!decltype(masked)::value || 32 * c + i <= row) mx[i & 3] = fmaxf(mx[i & 3], __uint_as_float(r[c][i]));
+        return fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      };
+      const float top = (diag ? row_max(std::true_type{}) : row_max(std::false_type{})) * p.scale_log2;
       // the running maximum is only moved when it would grow by more than 2^8: until then
       // the probabilities stay below 256 and O needs no rescaling
       float alpha = 1.f;
-      if (mx > m + 8.f) {
-        alpha = fast_exp2(m - mx);
-        m = mx;
+      if (top > m + 8.f) {
+        alpha = fast_exp2(m - top);
+        m = top;
       }
       l *= alpha;
-      // probabilities, packed to 16 bits in registers (off the critical path: the tensor
-      // core is still busy with the previous block's P V)
-      uint32_t pk[32];
-#pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        float e0 = fast_exp2(__uint_as_float(ra[i]) * p.scale_log2 - m);
-        float e1 = fast_exp2(__uint_as_float(ra[i + 1]) * p.scale_log2 - m);
-        e0 = (col0 + i <= limit) ? e0 : 0.f;
-        e1 = (col0 + i + 1 <= limit) ? e1 : 0.f;
-        l += e0 + e1;
-        pk[i >> 1] = pack2(e0, e1, p.in_dtype);
-      }
-#pragma unroll
-      for (int i = 0; i < 32; i += 2) {
-        float e0 = fast_exp2(__uint_as_float(rb[i]) * p.scale_log2 - m);
-        float e1 = fast_exp2(__uint_as_float(rb[i + 1]) * p.scale_log2 - m);
-        e0 = (col0 + 32 + i <= limit) ? e0 : 0.f;
-        e1 = (col0 + 32 + i + 1 <= limit) ? e1 : 0.f;
-        l += e0 + e1;
-        pk[16 + (i >> 1)] = pack2(e0, e1, p.in_dtype);
-      }
       if (j >= 1) {
         // the previous P V has retired: the P buffer is free and O is consistent
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.pv_done), (j - 1) & 1, abort_flag));
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.pv_done[t]), (j - 1) & 1, abort_flag));
         if (!ok) {
           if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
           break;
         }
-        tc_fence_after();
         if (__any_sync(0xffffffffu, alpha != 1.f)) {
-          uint32_t oa[32], ob[32];
-          tmem_ld_32x32(tO + lane_off + col0, oa);
-          tmem_ld_32x32(tO + lane_off + col0 + 32, ob);
-          tmem_ld_wait();
+          tc_fence_after();
+#pragma unroll 1
+          for (int c = 0; c < 4; ++c) {
+            uint32_t o[32];
+            tmem_ld_32x32(tO + 32 * c, o);
+            tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            oa[i] = __float_as_uint(__uint_as_float(oa[i]) * alpha);
-            ob[i] = __float_as_uint(__uint_as_float(ob[i]) * alpha);
+            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+            tmem_st_32x32(tO + 32 * c, o);
           }
-          tmem_st_32x32(tO + lane_off + col0, oa);
-          tmem_st_32x32(tO + lane_off + col0 + 32, ob);
           tmem_st_wait();
         }
       }
-      att_store_row64(sP, row, col0, pk);
+      auto probabilities = [&](auto masked) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int i = 0; i < 32; i += 8) {
+            float e[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              e[k] = fast_exp2(fmaf(__uint_as_float(r[c][i + k]), p.scale_log2, -m));
+              if (decltype(masked)::value && 32 * c + i + k > row) e[k] = 0.f;
+              sum[k & 3] += e[k];
+            }
+            sts128(tile + att_tile_off(row, 32 * c + i),
+                   make_uint4(pack2(e[0], e[1], p.in_dtype), pack2(e[2], e[3], p.in_dtype),
+                              pack2(e[4], e[5], p.in_dtype), pack2(e[6], e[7], p.in_dtype)));
+          }
+          l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        }
+      };
+      if (diag) probabilities(std::true_type{});
+      else probabilities(std::false_type{});
       tc_fence_before();
       fence_async_smem();
-      mbar_arrive(smem_u32(&sh.s_empty[s]));
-      mbar_arrive(smem_u32(&sh.p_full));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.p_full[t]));
     }
-    if (ok) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.pv_done), (nkv - 1) & 1, abort_flag));
+    if (ok && nt > 0) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.pv_done[t]), (nt - 1) & 1, abort_flag));
       if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
     }
-    if (ok) {
-      // the row sum is the sum of the two halves
-      sh.xch[2][group][row] = l;
-      mbar_arrive(smem_u32(&sh.l_full));
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.l_full), 0, abort_flag));
-      if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-    }
-    if (ok) {
-      l += sh.xch[2][group ^ 1][row];
+    if (ok && nt > 0) {
       tc_fence_after();
       const float inv = 1.f / l;
-      const long long q = (long long)qb * 128 + row;
-      uint16_t* orow = reinterpret_cast<uint16_t*>(p.o) + b * p.o_sb + q * p.o_ss + h * p.o_sh + col0;
-      uint32_t oa[32], ob[32];
-      tmem_ld_32x32(tO + lane_off + col0, oa);
-      tmem_ld_32x32(tO + lane_off + col0 + 32, ob);
-      tmem_ld_wait();
-      att_store_out64(orow, oa, ob, inv, p.in_dtype);
-      if (p.lse && group == 0) p.lse[((long long)b * p.H + h) * p.Sq + q] = m + log2f(l);
+      const long long q = (long long)(qb0 + t) * 128 + row;
+      uint16_t* orow = reinterpret_cast<uint16_t*>(p.o) + b * p.o_sb + q * p.o_ss + h * p.o_sh;
+#pragma unroll
+      for (int c = 0; c < 128; c += 64) {
+        uint32_t oa[32], ob[32];
+        tmem_ld_32x32(tO + c, oa);
+        tmem_ld_32x32(tO + c + 32, ob);
+        tmem_ld_wait();
+        att_store_out64(orow + c, oa, ob, inv, p.in_dtype);
+      }
+      if (p.lse) p.lse[((long long)b * p.H + h) * p.Sq + q] = m + log2f(l);
     }
   }
   tc_fence_before();
@@ -434,240 +423,328 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 }
 
 // ------------------------------------------------------------------------------------
-// delta[b][h][q] = sum_d dO[b][q][h][d] * O[b][q][h][d]     (one warp per row)
+// delta[b][h][q] = scale * sum_d dO[b][q][h][d] * O[b][q][h][d]: 16 lanes of 16 bytes a row, two
+// rows of a warp at a time, four rounds in flight
 // ------------------------------------------------------------------------------------
 template <typename T>
-__global__ void attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout,
-                                  float* __restrict__ delta, int B, int H, int S, long long o_sb,
-                                  long long o_ss, long long o_sh, long long d_sb, long long d_ss,
-                                  long long d_sh) {
-  const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __restrict__ delta, int B, int H, int S,
+                  float scale, long long o_sb, long long o_ss, long long o_sh, long long d_sb, long long d_ss,
+                  long long d_sh) {
   const long long total = (long long)B * H * S;
-  if (warp >= total) return;
-  const int q = (int)(warp % S);
-  const int h = (int)((warp / S) % H);
-  const int b = (int)(warp / ((long long)S * H));
-  const T* po = o + b * o_sb + (long long)q * o_ss + h * o_sh + lane * 4;
-  const T* pd = dout + b * d_sb + (long long)q * d_ss + h * d_sh + lane * 4;
-  const uint2 a = *reinterpret_cast<const uint2*>(po);
-  const uint2 g = *reinterpret_cast<const uint2*>(pd);
-  const T* ea = reinterpret_cast<const T*>(&a);
-  const T* eg = reinterpret_cast<const T*>(&g);
-  float sacc = 0.f;
+  const int half = (threadIdx.x >> 4) & 1, lane = threadIdx.x & 15;
+  const long long row0 = (((long long)blockIdx.x * 256 + threadIdx.x) >> 5) * 8 + half;
+  uint4 a[4], g[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) sacc += to_f32<T>(ea[i]) * to_f32<T>(eg[i]);
-  sacc = warp_sum(sacc);
-  if (lane == 0) delta[((long long)b * H + h) * S + q] = sacc;
+  for (int u = 0; u < 4; ++u) {
+    const long long r = min(row0 + 2 * u, total - 1);
+    // consecutive rows are the heads of a token: they are adjacent in memory
+    const int h = (int)(r % H);
+    const long long t = r / H;
+    const int q = (int)(t % S), b = (int)(t / S);
+    a[u] = *reinterpret_cast<const uint4*>(o + b * o_sb + (long long)q * o_ss + h * o_sh + lane * 8);
+    g[u] = *reinterpret_cast<const uint4*>(dout + b * d_sb + (long long)q * d_ss + h * d_sh + lane * 8);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const T* ea = reinterpret_cast<const T*>(&a[u]);
+    const T* eg = reinterpret_cast<const T*>(&g[u]);
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) s += to_f32<T>(ea[i]) * to_f32<T>(eg[i]);
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    const long long r = row0 + 2 * u;
+    if (lane == 0 && r < total) {
+      const int h = (int)(r % H);
+      const long long t = r / H;
+      const int q = (int)(t % S), b = (int)(t / S);
+      delta[((long long)b * H + h) * S + q] = s * scale;
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------
-// Backward, key / value side: one CTA per (batch, head, 128 keys); rows = keys.
-//   per query block i:  S^T = K Q_i^T, dP^T = V dO_i^T   (TMEM)
-//                       P^T = exp2(S^T * c - lse_i), dS^T = P^T * (dP^T - delta_i) * scale
-//                       dV += P^T dO_i,  dK += dS^T Q_i
+// Backward.  One launch holds two kinds of CTA:
+//   keys    (KV): 128 keys stay, the loop runs over 64 queries at a time; rows = keys
+//       S^T = K Q_i^T, dP^T = V dO_i^T;  dV += P^T dO_i,  dK += dS^T Q_i
+//   queries (Q):  128 queries stay, the loop runs over 64 keys at a time; rows = queries
+//       S = Q K_n^T, dP = dO V_n^T;      dQ += dS K_n
+// with P = exp2(S c - lse) and dS = P * (dP - delta) * scale.  In both, with R0, R1 the operands
+// that stay and T0, T1 the streamed ones: S = R0 T0^T, dP = R1 T1^T, acc1 += dS T0 and for keys
+// acc0 += P T1.
+//
+// The chain S -> exp -> shared memory -> accumulate is 2-3 thousand cycles long and the MMAs of a
+// step 1.0-1.3 thousand, so steps overlap: 64 columns a step leave room in TMEM for two S / dP
+// pairs beside the accumulators and in shared memory for two P / dS pairs and three stages of
+// the streamed operands.  The issuer starts step i + 1's scores before it waits for step i's
+// probabilities, and the two groups of row warps take every other step, so that one computes
+// while the other waits for TMEM, fences and barriers.  One arrival per warp (256 single arrivals
+// on a barrier took longer than the exponentials).  B = 2, H = 16, S = 2048, causal, bf16: 308 us as
+// two kernels with one step in flight -> 161 us; what is left is shared-memory traffic (operands,
+// P and dS: 1.4-1.9 of the 2.6 thousand cycles a step takes).
 // ------------------------------------------------------------------------------------
+constexpr int kBwdCols = 64;                          // streamed rows (= score columns) per step
+constexpr int kBwdTile = kBwdCols * kAttD * 2;        // 16 KB: one streamed operand, or P / dS
+constexpr int kBwdHalf = kBwdTile / 2;                // its two [64 rows][64] halves
+constexpr int kBwdStages = 3;
+constexpr int kBwdSmem = 2 * kAttTile + kBwdStages * 2 * kBwdTile + 4 * kBwdTile + 1024;
+
 struct __align__(128) AttnBwdShared {
-  uint64_t kv_full;        // resident operands loaded
-  uint64_t st_full;        // stage (per-iteration operands) loaded
-  uint64_t st_empty;       // the MMAs that read the stage, P and dS have retired
-  uint64_t s_full;         // score and dP accumulators complete
-  uint64_t p_full;         // P and dS written to shared memory (128 arrivals)
+  float lse[kBwdStages][kBwdCols];     // keys: of the streamed queries
+  float delta[kBwdStages][kBwdCols];
+  uint64_t resident;                   // the operands that stay have landed
+  uint64_t st_full[kBwdStages];        // a stage has landed
+  uint64_t st_empty[kBwdStages];       // the MMAs of a step have retired: stage, P and dS are free
+  uint64_t s_full[2];                  // scores and dP of a step are complete
+  uint64_t p_full[2];                  // P and dS of a step are in shared memory (4 warps)
   uint32_t tmem_base;
   int abort_flag;
-  float lse[128];
-  float delta[128];
 };
 
-__global__ void __launch_bounds__(kAttThreads, 1)
-attn_bwd_kv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                   const AttnParams p, int* status) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ AttnBwdShared sh;
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sK = base, sV = base + kAttTile, sQ = base + 2 * kAttTile, sDO = base + 3 * kAttTile;
-  const uint32_t sP = base + 4 * kAttTile, sDS = base + 5 * kAttTile;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  volatile int* abort_flag = &sh.abort_flag;
-  const int kb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int nqb = p.Sq / 128;
-  const int i0 = p.causal ? kb : 0;                    // first query block that sees these keys
-  const int iters = nqb - i0;
-
-  if (threadIdx.x == 0) {
-    mbar_init(smem_u32(&sh.kv_full), 1);
-    mbar_init(smem_u32(&sh.st_full), 1);
-    mbar_init(smem_u32(&sh.st_empty), 1);
-    mbar_init(smem_u32(&sh.s_full), 1);
-    mbar_init(smem_u32(&sh.p_full), 256);
-    sh.abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 5) {
-    tmem_alloc(smem_u32(&sh.tmem_base), 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = sh.tmem_base;
-  const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
-
-  if (warp == 4) {
-    if (elect_one()) {
-      mbar_expect_tx(smem_u32(&sh.kv_full), 2 * kAttTile);
-      att_load_tile(sK, &tmK, smem_u32(&sh.kv_full), h, kb * 128, b);
-      att_load_tile(sV, &tmV, smem_u32(&sh.kv_full), h, kb * 128, b);
-      int it = 0;
-      bool ok = true;
-      for (; it < iters && ok; ++it) {
-        if (it >= 1 && !mbar_wait_bounded(smem_u32(&sh.st_empty), (it - 1) & 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutStageEmpty);
-          ok = false;
-          break;
-        }
-        const int i = i0 + it;
-        const float* lse = p.lse + ((long long)b * p.H + h) * p.Sq + i * 128;
-        const float* dl = p.delta + ((long long)b * p.H + h) * p.Sq + i * 128;
-        mbar_expect_tx(smem_u32(&sh.st_full), 2 * kAttTile + 1024);
-        att_load_tile(sQ, &tmQ, smem_u32(&sh.st_full), h, i * 128, b);
-        att_load_tile(sDO, &tmDO, smem_u32(&sh.st_full), h, i * 128, b);
-        bulk_load_1d(smem_u32(sh.lse), lse, 512, smem_u32(&sh.st_full));
-        bulk_load_1d(smem_u32(sh.delta), dl, 512, smem_u32(&sh.st_full));
-      }
-      if (!ok || *abort_flag) {
-        mbar_wait_budget_only(smem_u32(&sh.kv_full), 0);
-        if (it >= 1) mbar_wait_budget_only(smem_u32(&sh.st_full), (it - 1) & 1);
-      }
-    }
-  } else if (warp == 5) {
-    if (elect_one()) {
-      const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
-      const uint32_t idesc_kk = make_idesc_f16(fmt, 0, 0, 128, 128);
-      const uint32_t idesc_kn = make_idesc_f16(fmt, 0, 1, 128, 128);
-      bool ok = mbar_wait_bounded(smem_u32(&sh.kv_full), 0, abort_flag);
-      if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
-      for (int it = 0; it < iters && ok; ++it) {
-        if (!mbar_wait_bounded(smem_u32(&sh.st_full), it & 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutTmaFull);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        att_mma_kk(tS, sK, sQ, idesc_kk, false);       // S^T[key][q]
-        att_mma_kk(tDP, sV, sDO, idesc_kk, false);     // dP^T[key][q]
-        umma_commit(smem_u32(&sh.s_full));
-        if (!mbar_wait_bounded(smem_u32(&sh.p_full), it & 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutTmemEmpty);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        att_mma_kn(tDV, sP, sDO, idesc_kn, it > 0);    // dV[key][d] += P^T dO
-        att_mma_kn(tDK, sDS, sQ, idesc_kn, it > 0);    // dK[key][d] += dS^T Q
-        umma_commit(smem_u32(&sh.st_empty));
-      }
-    }
-  } else {
-    int group = 0, quarter = 0;
-    att_row_role(warp, group, quarter);
-    const int row = quarter * 32 + lane;               // key row of this thread
-    const int col0 = group * 64;                       // its half of the query columns / head dim
-    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    bool ok = true;
-    for (int it = 0; it < iters && ok; ++it) {
-      const int i = i0 + it;
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full), it & 1, abort_flag));
-      if (!ok) {
-        if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-        break;
-      }
-      // lse / delta of this query block came with the stage (same barrier as Q and dO)
-      mbar_wait_bounded(smem_u32(&sh.st_full), it & 1, abort_flag);
-      tc_fence_after();
-      // causal, diagonal block: query column c sees key `row` only when c >= row
-      const int first = (p.causal && i == kb) ? row : 0;
-      uint32_t pk[32], dk[32];
+// acc = A . B^T over K = 128: A a K-major tile [2][128 rows][64], B [2][64 rows][64]
+__device__ __forceinline__ void bwd_mma_scores(uint32_t acc, uint32_t a, uint32_t b, uint32_t idesc) {
+  const uint64_t d0 = make_smem_desc(0, 16, 1024, kLayoutSw128);
+  const uint32_t hi = (uint32_t)(d0 >> 32);
+  const uint32_t alo = (uint32_t)d0 + (a >> 4), blo = (uint32_t)d0 + (b >> 4);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int c = col0 + half * 32;
-        uint32_t rs[32], rd[32];
-        tmem_ld_32x32(tS + lane_off + c, rs);
-        tmem_ld_32x32(tDP + lane_off + c, rd);
-        tmem_ld_wait();
+  for (int kk = 0; kk < 8; ++kk)
+    umma_f16_lo(acc, alo + (((kk >> 2) * kAttHalf + (kk & 3) * 32) >> 4), hi,
+                blo + (((kk >> 2) * kBwdHalf + (kk & 3) * 32) >> 4), hi, idesc, kk ? 1u : 0u);
+}
+// acc (+)= A . B over K = 64: A a K-major tile [128 rows][64], B rows of K ([2 halves of N][64][64])
+__device__ __forceinline__ void bwd_mma_accumulate(uint32_t acc, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
+  const uint64_t da = make_smem_desc(0, 16, 1024, kLayoutSw128);
+  const uint64_t db = make_smem_desc(0, kBwdHalf, 1024, kLayoutSw128);
+  const uint32_t ahi = (uint32_t)(da >> 32), bhi = (uint32_t)(db >> 32);
+  const uint32_t alo = (uint32_t)da + (a >> 4), blo = (uint32_t)db + (b >> 4);
 #pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          float e0 = fast_exp2(__uint_as_float(rs[k]) * p.scale_log2 - sh.lse[c + k]);
-          float e1 = fast_exp2(__uint_as_float(rs[k + 1]) * p.scale_log2 - sh.lse[c + k + 1]);
-          e0 = (c + k >= first) ? e0 : 0.f;
-          e1 = (c + k + 1 >= first) ? e1 : 0.f;
-          const float d0 = e0 * (__uint_as_float(rd[k]) - sh.delta[c + k]) * p.scale;
-          const float d1 = e1 * (__uint_as_float(rd[k + 1]) - sh.delta[c + k + 1]) * p.scale;
-          pk[half * 16 + (k >> 1)] = pack2(e0, e1, p.in_dtype);
-          dk[half * 16 + (k >> 1)] = pack2(d0, d1, p.in_dtype);
-        }
-      }
-      att_store_row64(sP, row, col0, pk);
-      att_store_row64(sDS, row, col0, dk);
-      tc_fence_before();
-      fence_async_smem();
-      mbar_arrive(smem_u32(&sh.p_full));
+  for (int kk = 0; kk < 4; ++kk)
+    umma_f16_lo(acc, alo + ((kk * 32) >> 4), ahi, blo + ((kk * 2048) >> 4), bhi, idesc, (accumulate || kk) ? 1u : 0u);
+}
+
+// 32 columns of P and dS of one row, packed: cols[k] of this thread's columns are visible from
+// `first` on (keys) or up to `last` (queries).
+template <bool KV>
+__device__ __forceinline__ void bwd_probabilities(const uint32_t (&rs)[32], const uint32_t (&rd)[32], const float* lse,
+                                                  const float* delta, float my_lse, float my_delta, int first, int last,
+                                                  const AttnParams& p, uint32_t (&pk)[16], uint32_t (&dk)[16]) {
+  const bool masked = first > 0 || last < 31;
+#pragma unroll
+  for (int k = 0; k < 32; k += 4) {
+    float4 l4, d4;
+    if (KV) {
+      l4 = *reinterpret_cast<const float4*>(lse + k);
+      d4 = *reinterpret_cast<const float4*>(delta + k);
+    } else {
+      l4 = make_float4(my_lse, my_lse, my_lse, my_lse);
+      d4 = make_float4(my_delta, my_delta, my_delta, my_delta);
     }
-    if (ok && iters > 0) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty), (iters - 1) & 1, abort_flag));
-      if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+    const float l[4] = {l4.x, l4.y, l4.z, l4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
+    float e[4], d[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      e[j] = fast_exp2(fmaf(__uint_as_float(rs[k + j]), p.scale_log2, -l[j]));
+      if (masked) e[j] = (k + j >= first && k + j <= last) ? e[j] : 0.f;
+      d[j] = e[j] * fmaf(__uint_as_float(rd[k + j]), p.scale, -dl[j]);
     }
-    if (ok) {
-      tc_fence_after();
-      const long long key = (long long)kb * 128 + row;
-      uint16_t* dvrow = reinterpret_cast<uint16_t*>(p.dv) + b * p.dv_sb + key * p.dv_ss + h * p.dv_sh + col0;
-      uint16_t* dkrow = reinterpret_cast<uint16_t*>(p.dk) + b * p.dk_sb + key * p.dk_ss + h * p.dk_sh + col0;
-      uint32_t ra[32], rb[32];
-      tmem_ld_32x32(tDV + lane_off + col0, ra);
-      tmem_ld_32x32(tDV + lane_off + col0 + 32, rb);
-      tmem_ld_wait();
-      att_store_out64(dvrow, ra, rb, 1.f, p.in_dtype);
-      tmem_ld_32x32(tDK + lane_off + col0, ra);
-      tmem_ld_32x32(tDK + lane_off + col0 + 32, rb);
-      tmem_ld_wait();
-      att_store_out64(dkrow, ra, rb, 1.f, p.in_dtype);
+    if (KV) {
+      pk[k / 2] = pack2(e[0], e[1], p.in_dtype);
+      pk[k / 2 + 1] = pack2(e[2], e[3], p.in_dtype);
     }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 5) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    dk[k / 2] = pack2(d[0], d[1], p.in_dtype);
+    dk[k / 2 + 1] = pack2(d[2], d[3], p.in_dtype);
   }
 }
 
-// ------------------------------------------------------------------------------------
-// Backward, query side: one CTA per (batch, head, 128 queries); rows = queries.
-//   per key block n:  S = Q K_n^T, dP = dO V_n^T  (TMEM);  dS = P * (dP - delta) * scale;
-//                     dQ += dS K_n
-// ------------------------------------------------------------------------------------
+template <bool KV>
+__device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUtensorMap* tmR1, const CUtensorMap* tmT0,
+                                             const CUtensorMap* tmT1, const AttnParams& p, int blk, int h, int b,
+                                             uint32_t base, AttnBwdShared& sh, int* status) {
+  const uint32_t sR0 = base, sR1 = base + kAttTile, sT = base + 2 * kAttTile;
+  const uint32_t sP = sT + kBwdStages * 2 * kBwdTile, sDS = sP + 2 * kBwdTile;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int* abort_flag = &sh.abort_flag;
+  const int steps_all = (KV ? p.Sq : p.Sk) / kBwdCols;
+  const int i0 = KV && p.causal ? 2 * blk : 0;                   // first step that sees these rows
+  const int iters = KV ? steps_all - i0 : (p.causal ? 2 * blk + 2 : steps_all);
+  const uint32_t tmem = sh.tmem_base, tAcc0 = tmem + 256, tAcc1 = tmem + 384;
+  const long long stat0 = ((long long)b * p.H + h) * p.Sq;       // this head's lse / delta
+
+  if (warp == 4) {
+    if (elect_one()) {
+      mbar_expect_tx(smem_u32(&sh.resident), 2 * kAttTile);
+      att_load_tile(sR0, tmR0, smem_u32(&sh.resident), h, blk * 128, b);
+      att_load_tile(sR1, tmR1, smem_u32(&sh.resident), h, blk * 128, b);
+      RingPos rp;
+      int it = 0;
+      bool ok = true;
+      for (; it < iters; ++it) {
+        if (!mbar_wait_bounded(smem_u32(&sh.st_empty[rp.s]), rp.ph ^ 1, abort_flag)) {
+          raise_status(status, abort_flag, kTimeoutStageEmpty);
+          ok = false;
+          break;
+        }
+        const uint32_t bar = smem_u32(&sh.st_full[rp.s]), dst = sT + rp.s * 2 * kBwdTile;
+        const int r0 = (i0 + it) * kBwdCols;
+        mbar_expect_tx(bar, 2 * kBwdTile + (KV ? 2 * kBwdCols * 4 : 0));
+        tma_load_4d(dst, tmT0, bar, 0, h, r0, b);
+        tma_load_4d(dst + kBwdHalf, tmT0, bar, 64, h, r0, b);
+        tma_load_4d(dst + kBwdTile, tmT1, bar, 0, h, r0, b);
+        tma_load_4d(dst + kBwdTile + kBwdHalf, tmT1, bar, 64, h, r0, b);
+        if (KV) {
+          bulk_load_1d(smem_u32(sh.lse[rp.s]), p.lse + stat0 + r0, kBwdCols * 4, bar);
+          bulk_load_1d(smem_u32(sh.delta[rp.s]), p.delta + stat0 + r0, kBwdCols * 4, bar);
+        }
+        rp.advance(kBwdStages);
+      }
+      if (!ok || *abort_flag) {        // the copies in flight land before shared memory is released
+        mbar_wait_budget_only(smem_u32(&sh.resident), 0);
+        for (int j = it > kBwdStages ? it - kBwdStages : 0; j < it; ++j)
+          mbar_wait_budget_only(smem_u32(&sh.st_full[j % kBwdStages]), (j / kBwdStages) & 1);
+      }
+    }
+  } else if (warp == 5) {
+    if (elect_one()) {
+      const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
+      const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, 128, kBwdCols);
+      const uint32_t idesc_a = make_idesc_f16(fmt, 0, 1, 128, 128);
+      bool ok = mbar_wait_bounded(smem_u32(&sh.resident), 0, abort_flag);
+      if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
+      RingPos next, cur;               // stages of the scores' step and of the accumulating step
+      for (int it = -1; it < iters && ok; ++it) {
+        if (it + 1 < iters) {          // scores of the next step (its TMEM was read by step it - 1)
+          const int n = it + 1;
+          if (!mbar_wait_bounded(smem_u32(&sh.st_full[next.s]), next.ph, abort_flag)) {
+            raise_status(status, abort_flag, kTimeoutTmaFull);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t t = sT + next.s * 2 * kBwdTile, d = tmem + (n & 1) * 128;
+          bwd_mma_scores(d, sR0, t, idesc_s);
+          bwd_mma_scores(d + kBwdCols, sR1, t + kBwdTile, idesc_s);
+          umma_commit(smem_u32(&sh.s_full[n & 1]));
+          next.advance(kBwdStages);
+        }
+        if (it >= 0) {
+          if (!mbar_wait_bounded(smem_u32(&sh.p_full[it & 1]), (it >> 1) & 1, abort_flag)) {
+            raise_status(status, abort_flag, kTimeoutTmemEmpty);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t t = sT + cur.s * 2 * kBwdTile;
+          if (KV) bwd_mma_accumulate(tAcc0, sP + (it & 1) * kBwdTile, t + kBwdTile, idesc_a, it > 0);
+          bwd_mma_accumulate(tAcc1, sDS + (it & 1) * kBwdTile, t, idesc_a, it > 0);
+          umma_commit(smem_u32(&sh.st_empty[cur.s]));
+          cur.advance(kBwdStages);
+        }
+      }
+    }
+  } else {
+    int group = 0, quarter = 0;
+    att_row_role(warp, group, quarter);
+    const int row = quarter * 32 + lane;               // this thread's key / query
+    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
+    float my_lse = 0.f, my_delta = 0.f;
+    if (!KV) {
+      my_lse = p.lse[stat0 + blk * 128 + row];
+      my_delta = p.delta[stat0 + blk * 128 + row];
+    }
+    bool ok = true;
+    RingPos rp;
+    if (group) rp.advance(kBwdStages);
+    for (int it = group; it < iters && ok; it += 2) {
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full[it & 1]), (it >> 1) & 1, abort_flag));
+      // lse and delta of a step came with its stage; the stage of step it - 2 is empty once the
+      // MMAs that read this P / dS pair have retired
+      if (ok && KV) ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_full[rp.s]), rp.ph, abort_flag));
+      if (ok && it >= 2) {
+        const int j = it - 2;
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1,
+                                                       abort_flag));
+      }
+      if (!ok) {
+        if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t buf = (it & 1) * kBwdTile;
+#pragma unroll
+      for (int c = 0; c < kBwdCols; c += 32) {
+        const uint32_t tS = tmem + (it & 1) * 128 + lane_off + c;
+        uint32_t rs[32], rd[32], pk[16], dk[16];
+        tmem_ld_32x32(tS, rs);
+        tmem_ld_32x32(tS + kBwdCols, rd);
+        tmem_ld_wait();
+        // causal: query >= key; distance of these columns from this CTA's first row
+        const int off = p.causal ? (i0 + it) * kBwdCols + c - blk * 128 : 0;
+        const int first = KV && p.causal ? row - off : 0;
+        const int last = !KV && p.causal ? row - off : 31;
+        bwd_probabilities<KV>(rs, rd, sh.lse[rp.s] + c, sh.delta[rp.s] + c, my_lse, my_delta, first, last, p, pk, dk);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t at = att_tile_off(row, c + 8 * j);
+          if (KV) sts128(sP + buf + at, make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]));
+          sts128(sDS + buf + at, make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]));
+        }
+      }
+      tc_fence_before();
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.p_full[it & 1]));
+      rp.advance(kBwdStages);
+      rp.advance(kBwdStages);
+    }
+    if (ok && iters > 0) {
+      const int j = iters - 1;
+      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1,
+                                                     abort_flag));
+      if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+    }
+    if (ok) {
+      tc_fence_after();
+      const long long r = (long long)blk * 128 + row;
+      const int d0 = group * 64;                       // this thread's half of the head dimension
+      uint32_t ra[32], rb[32];
+      if (KV) {
+        uint16_t* dv = reinterpret_cast<uint16_t*>(p.dv) + b * p.dv_sb + r * p.dv_ss + h * p.dv_sh + d0;
+        tmem_ld_32x32(tAcc0 + lane_off + d0, ra);
+        tmem_ld_32x32(tAcc0 + lane_off + d0 + 32, rb);
+        tmem_ld_wait();
+        att_store_out64(dv, ra, rb, 1.f, p.in_dtype);
+      }
+      uint16_t* out = KV ? reinterpret_cast<uint16_t*>(p.dk) + b * p.dk_sb + r * p.dk_ss + h * p.dk_sh + d0
+                         : reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_sb + r * p.dq_ss + h * p.dq_sh + d0;
+      tmem_ld_32x32(tAcc1 + lane_off + d0, ra);
+      tmem_ld_32x32(tAcc1 + lane_off + d0 + 32, rb);
+      tmem_ld_wait();
+      att_store_out64(out, ra, rb, 1.f, p.in_dtype);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(kAttThreads, 1)
-attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                  const AttnParams p, int* status) {
+attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
+                const __grid_constant__ CUtensorMap tmQ64, const __grid_constant__ CUtensorMap tmK64,
+                const __grid_constant__ CUtensorMap tmV64, const __grid_constant__ CUtensorMap tmDO64,
+                const __grid_constant__ AttnParams p, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ AttnBwdShared sh;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t sQ = base, sDO = base + kAttTile, sK = base + 2 * kAttTile, sV = base + 3 * kAttTile;
-  const uint32_t sDS = base + 4 * kAttTile;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  volatile int* abort_flag = &sh.abort_flag;
-  const int nqb = p.Sq / 128;
-  const int qb = nqb - 1 - (int)blockIdx.x, h = blockIdx.y, b = blockIdx.z;
-  const int iters = p.causal ? qb + 1 : p.Sk / 128;
-
+  const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
-    mbar_init(smem_u32(&sh.kv_full), 1);
-    mbar_init(smem_u32(&sh.st_full), 1);
-    mbar_init(smem_u32(&sh.st_empty), 1);
-    mbar_init(smem_u32(&sh.s_full), 1);
-    mbar_init(smem_u32(&sh.p_full), 256);
+    mbar_init(smem_u32(&sh.resident), 1);
+    for (int s = 0; s < kBwdStages; ++s) {
+      mbar_init(smem_u32(&sh.st_full[s]), 1);
+      mbar_init(smem_u32(&sh.st_empty[s]), 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(smem_u32(&sh.s_full[s]), 1);
+      mbar_init(smem_u32(&sh.p_full[s]), 4);
+    }
     sh.abort_flag = 0;
     mbar_fence_init();
   }
@@ -678,132 +755,29 @@ attn_bwd_q_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = sh.tmem_base;
-  const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
 
-  if (warp == 4) {
-    if (elect_one()) {
-      const float* lse = p.lse + ((long long)b * p.H + h) * p.Sq + qb * 128;
-      const float* dl = p.delta + ((long long)b * p.H + h) * p.Sq + qb * 128;
-      mbar_expect_tx(smem_u32(&sh.kv_full), 2 * kAttTile + 1024);
-      att_load_tile(sQ, &tmQ, smem_u32(&sh.kv_full), h, qb * 128, b);
-      att_load_tile(sDO, &tmDO, smem_u32(&sh.kv_full), h, qb * 128, b);
-      bulk_load_1d(smem_u32(sh.lse), lse, 512, smem_u32(&sh.kv_full));
-      bulk_load_1d(smem_u32(sh.delta), dl, 512, smem_u32(&sh.kv_full));
-      int it = 0;
-      bool ok = true;
-      for (; it < iters && ok; ++it) {
-        if (it >= 1 && !mbar_wait_bounded(smem_u32(&sh.st_empty), (it - 1) & 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutStageEmpty);
-          ok = false;
-          break;
-        }
-        mbar_expect_tx(smem_u32(&sh.st_full), 2 * kAttTile);
-        att_load_tile(sK, &tmK, smem_u32(&sh.st_full), h, it * 128, b);
-        att_load_tile(sV, &tmV, smem_u32(&sh.st_full), h, it * 128, b);
-      }
-      if (!ok || *abort_flag) {
-        mbar_wait_budget_only(smem_u32(&sh.kv_full), 0);
-        if (it >= 1) mbar_wait_budget_only(smem_u32(&sh.st_full), (it - 1) & 1);
-      }
-    }
-  } else if (warp == 5) {
-    if (elect_one()) {
-      const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
-      const uint32_t idesc_kk = make_idesc_f16(fmt, 0, 0, 128, 128);
-      const uint32_t idesc_kn = make_idesc_f16(fmt, 0, 1, 128, 128);
-      bool ok = mbar_wait_bounded(smem_u32(&sh.kv_full), 0, abort_flag);
-      if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
-      for (int it = 0; it < iters && ok; ++it) {
-        if (!mbar_wait_bounded(smem_u32(&sh.st_full), it & 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutTmaFull);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        att_mma_kk(tS, sQ, sK, idesc_kk, false);       // S[q][key]
-        att_mma_kk(tDP, sDO, sV, idesc_kk, false);     // dP[q][key]
-        umma_commit(smem_u32(&sh.s_full));
-        if (!mbar_wait_bounded(smem_u32(&sh.p_full), it & 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutTmemEmpty);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        att_mma_kn(tDQ, sDS, sK, idesc_kn, it > 0);    // dQ[q][d] += dS K
-        umma_commit(smem_u32(&sh.st_empty));
-      }
-    }
-  } else {
-    int group = 0, quarter = 0;
-    att_row_role(warp, group, quarter);
-    const int row = quarter * 32 + lane;               // query row of this thread
-    const int col0 = group * 64;                       // its half of the key columns / head dim
-    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.kv_full), 0, abort_flag));
-    if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmaFull);
-    const float my_lse = ok ? sh.lse[row] : 0.f, my_delta = ok ? sh.delta[row] : 0.f;
-    for (int it = 0; it < iters && ok; ++it) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full), it & 1, abort_flag));
-      if (!ok) {
-        if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-        break;
-      }
-      tc_fence_after();
-      const int limit = (p.causal && it == qb) ? row : 127;
-      uint32_t dk[32];
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int c = col0 + half * 32;
-        uint32_t rs[32], rd[32];
-        tmem_ld_32x32(tS + lane_off + c, rs);
-        tmem_ld_32x32(tDP + lane_off + c, rd);
-        tmem_ld_wait();
-#pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          float e0 = fast_exp2(__uint_as_float(rs[k]) * p.scale_log2 - my_lse);
-          float e1 = fast_exp2(__uint_as_float(rs[k + 1]) * p.scale_log2 - my_lse);
-          e0 = (c + k <= limit) ? e0 : 0.f;
-          e1 = (c + k + 1 <= limit) ? e1 : 0.f;
-          dk[half * 16 + (k >> 1)] = pack2(e0 * (__uint_as_float(rd[k]) - my_delta) * p.scale,
-                                           e1 * (__uint_as_float(rd[k + 1]) - my_delta) * p.scale,
-                                           p.in_dtype);
-        }
-      }
-      att_store_row64(sDS, row, col0, dk);
-      tc_fence_before();
-      fence_async_smem();
-      mbar_arrive(smem_u32(&sh.p_full));
-    }
-    if (ok) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty), (iters - 1) & 1, abort_flag));
-      if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-    }
-    if (ok) {
-      tc_fence_after();
-      const long long q = (long long)qb * 128 + row;
-      uint16_t* dqrow = reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_sb + q * p.dq_ss + h * p.dq_sh + col0;
-      uint32_t ra[32], rb[32];
-      tmem_ld_32x32(tDQ + lane_off + col0, ra);
-      tmem_ld_32x32(tDQ + lane_off + col0 + 32, rb);
-      tmem_ld_wait();
-      att_store_out64(dqrow, ra, rb, 1.f, p.in_dtype);
-    }
-  }
+  // the longest blocks first: keys see the queries behind them, queries the keys before them
+  const int nkb = p.Sk / 128, nqb = p.Sq / 128;
+  const int blk = (int)blockIdx.z, h = blockIdx.x, b = blockIdx.y;
+  if (blk < nkb)
+    attn_bwd_cta<true>(&tmK, &tmV, &tmQ64, &tmDO64, p, blk, h, b, base, sh, status);
+  else
+    attn_bwd_cta<false>(&tmQ, &tmDO, &tmK64, &tmV64, p, nqb - 1 - (blk - nkb), h, b, base, sh, status);
+
   tc_fence_before();
   __syncthreads();
   if (warp == 5) {
     tc_fence_after();
-    tmem_dealloc(tmem, 512);
+    tmem_dealloc(sh.tmem_base, 512);
   }
 }
 
 // Tensor map of a token-major tensor [B][S][H][128] with element strides (sb, ss, sh).
 static bool att_tmap(CUtensorMap* tm, const void* ptr, int dtype, int B, int S, int H, long long sb,
-                     long long ss, long long sh) {
+                     long long ss, long long sh, uint32_t rows = 128) {
   uint64_t dims[4] = {(uint64_t)kAttD, (uint64_t)H, (uint64_t)S, (uint64_t)B};
   uint64_t strides[3] = {(uint64_t)sh * 2, (uint64_t)ss * 2, (uint64_t)sb * 2};
-  uint32_t box[4] = {64, 1, 128, 1};
+  uint32_t box[4] = {64, 1, rows, 1};
   return lbhost::encode_tmap(tm, dtype, 4, ptr, dims, strides, box, nullptr, 128);
 }
 
@@ -838,19 +812,20 @@ int lb_attention_fwd(const void* q, const void* k, const void* v, void* o, float
   p.B = B; p.H = H; p.Sq = Sq; p.Sk = Sk; p.causal = causal; p.in_dtype = dtype;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f;
   p.o = o; p.o_sb = os[0]; p.o_ss = os[1]; p.o_sh = os[2]; p.lse = lse;
-  const int smem = 6 * kAttTile + 1024;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
     configured = true;
   }
-  dim3 grid(Sq / 128, H, B);
-  attn_fwd_kernel<<<grid, kAttThreads, smem, stream>>>(tq, tk, tv, p, lbhost::status_word());
+  // one query tile per CTA where all of them fit on the device at once, else two
+  const int nqb = Sq / 128, tiles = (long long)nqb * H * B <= lbhost::sm_count() ? 1 : 2;
+  attn_fwd_kernel<<<dim3(H, B, (nqb + tiles - 1) / tiles), kAttThreads, kFwdSmem, stream>>>(tq, tk, tv, p, tiles,
+                                                                                       lbhost::status_word());
   return (int)cudaGetLastError();
 }
 
 // Gradients of lb_attention_fwd.  o, dout: [B][Sq][H][128]; lse from the forward call; delta:
-// fp32 workspace [B][H][Sq].  dq, dk, dv are written (not accumulated).
+// fp32 workspace [B][H][Sq], overwritten.  dq, dk, dv are written (not accumulated).
 int lb_attention_bwd(const void* q, const void* k, const void* v, const void* o, const void* dout,
                      const float* lse, float* delta, void* dq, void* dk, void* dv, int B, int H, int Sq,
                      int Sk, const long long* qs, const long long* ks, const long long* vs,
@@ -868,22 +843,25 @@ int lb_attention_bwd(const void* q, const void* k, const void* v, const void* o,
     return -1;
   if ((reinterpret_cast<uintptr_t>(lse) & 15) || (reinterpret_cast<uintptr_t>(delta) & 15)) return -1;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
-  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tq, tk, tv, tdo, tq64, tk64, tv64, tdo64;
   if (!att_tmap(&tq, q, dtype, B, Sq, H, qs[0], qs[1], qs[2]) ||
       !att_tmap(&tk, k, dtype, B, Sk, H, ks[0], ks[1], ks[2]) ||
       !att_tmap(&tv, v, dtype, B, Sk, H, vs[0], vs[1], vs[2]) ||
-      !att_tmap(&tdo, dout, dtype, B, Sq, H, dos[0], dos[1], dos[2])) return -1;
+      !att_tmap(&tdo, dout, dtype, B, Sq, H, dos[0], dos[1], dos[2]) ||
+      !att_tmap(&tq64, q, dtype, B, Sq, H, qs[0], qs[1], qs[2], kBwdCols) ||
+      !att_tmap(&tk64, k, dtype, B, Sk, H, ks[0], ks[1], ks[2], kBwdCols) ||
+      !att_tmap(&tv64, v, dtype, B, Sk, H, vs[0], vs[1], vs[2], kBwdCols) ||
+      !att_tmap(&tdo64, dout, dtype, B, Sq, H, dos[0], dos[1], dos[2], kBwdCols)) return -1;
   {
     const long long rows = (long long)B * H * Sq;
-    const int blocks = (int)((rows * 32 + 255) / 256);
+    const int blocks = (int)((rows + 63) / 64);
     if (dtype == kBF16)
       attn_delta_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(
-          (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, H, Sq, os[0], os[1], os[2],
+          (const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, B, H, Sq, scale, os[0], os[1], os[2],
           dos[0], dos[1], dos[2]);
     else
-      attn_delta_kernel<__half><<<blocks, 256, 0, stream>>>((const __half*)o, (const __half*)dout, delta,
-                                                            B, H, Sq, os[0], os[1], os[2], dos[0],
-                                                            dos[1], dos[2]);
+      attn_delta_kernel<__half><<<blocks, 256, 0, stream>>>((const __half*)o, (const __half*)dout, delta, B, H, Sq,
+                                                            scale, os[0], os[1], os[2], dos[0], dos[1], dos[2]);
   }
   AttnParams p;
   memset(&p, 0, sizeof(p));
@@ -893,17 +871,13 @@ int lb_attention_bwd(const void* q, const void* k, const void* v, const void* o,
   p.dq = dq; p.dq_sb = dqs[0]; p.dq_ss = dqs[1]; p.dq_sh = dqs[2];
   p.dk = dk; p.dk_sb = dks[0]; p.dk_ss = dks[1]; p.dk_sh = dks[2];
   p.dv = dv; p.dv_sb = dvs[0]; p.dv_ss = dvs[1]; p.dv_sh = dvs[2];
-  const int smem_kv = 6 * kAttTile + 1024, smem_q = 5 * kAttTile + 1024;
   static bool configured = false;
   if (!configured) {
-    cudaFuncSetAttribute(attn_bwd_kv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv);
-    cudaFuncSetAttribute(attn_bwd_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q);
+    cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
     configured = true;
   }
-  attn_bwd_kv_kernel<<<dim3(Sk / 128, H, B), kAttThreads, smem_kv, stream>>>(tq, tk, tv, tdo, p,
-                                                                     lbhost::status_word());
-  attn_bwd_q_kernel<<<dim3(Sq / 128, H, B), kAttThreads, smem_q, stream>>>(tq, tk, tv, tdo, p,
-                                                                   lbhost::status_word());
+  attn_bwd_kernel<<<dim3(H, B, Sk / 128 + Sq / 128), kAttThreads, kBwdSmem, stream>>>(
+      tq, tk, tv, tdo, tq64, tk64, tv64, tdo64, p, lbhost::status_word());
   return (int)cudaGetLastError();
 }
 

@@ -539,7 +539,7 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
                          dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), q.size(0), a.H, q.size(1), k.size(1), sq.v, sk.v,
                          sv.v, so.v, sg.v, sdq.v, sdk.v, sdv.v, a.scale, a.causal, code(q.scalar_type()), stream()),
         "lb_attention_bwd");
-  g_launches += 3;
+  g_launches += 2;
 }
 void keep_attn(AutogradContext* ctx, const Attn& a) {
   ctx->saved_data["H"] = a.H;

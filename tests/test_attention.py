@@ -111,3 +111,33 @@ def test_attention_subgraph_is_replaced_by_one_call(monkeypatch):
     assert not plain[1] and len(fused[1]) == 2 and fused[2] >= 2 * 12
     for a, b in zip(plain[0], fused[0]):
         assert abs(a - b) < 1e-4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,Sq,Sk,causal,scale", [
+    (1, 1, 128, 128, True, 0.09),        # one block, one query tile per CTA
+    (6, 5, 640, 640, True, 0.09),        # two tiles per CTA, an odd number of blocks
+    (6, 5, 640, 256, False, 0.09),       # cross attention, fewer keys than queries
+    (2, 2, 256, 896, False, 0.0),        # every key counts the same
+    (1, 3, 384, 384, True, -0.05),       # masked scores must not win where the scale turns them round
+])
+def test_attention_tiles_against_64_bits(B, H, Sq, Sk, causal, scale):
+    """Probabilities are rounded to 16 bits (2^-9) before their products, outputs and gradients
+    once more: 1 % of the norm bounds both, for fp32 accumulation of at most 896 terms."""
+    torch.manual_seed(2)
+    E = H * 128
+    q = torch.randn(B, Sq, E, device="cuda").bfloat16().requires_grad_(True)
+    k, v = (torch.randn(B, Sk, E, device="cuda").bfloat16().requires_grad_(True) for _ in range(2))
+    g = torch.randn(B, Sq, E, device="cuda").bfloat16()
+    assert att.native_ok(q, k, v, H, causal)
+    y = att.attention(q, k, v, H, scale, causal)
+    grads = torch.autograd.grad(y, (q, k, v), g)
+    qd, kd, vd = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    heads = [t.reshape(B, -1, H, 128).transpose(1, 2) for t in (qd, kd, vd)]
+    s = heads[0] @ heads[1].transpose(2, 3) * scale
+    if causal:
+        s = s.masked_fill(torch.ones(Sq, Sk, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = (torch.softmax(s, -1) @ heads[2]).transpose(1, 2).reshape(B, Sq, E)
+    refs = torch.autograd.grad(ref, (qd, kd, vd), g.double())
+    for got, want in zip((y, *grads), (ref, *refs)):
+        assert float((got.double() - want).norm()) <= 0.01 * float(want.norm())
