@@ -69,6 +69,24 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
       "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
       : "memory");
 }
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+      "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem desc]: A has one row per lane, two 16-bit K elements per column.
+__device__ __forceinline__ void umma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t b_hi,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
+      "mov.b64 db, {%2, %3};\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate));
+}
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -474,21 +492,20 @@ attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __
 // that stay and T0, T1 the streamed ones: S = R0 T0^T, dP = R1 T1^T, acc1 += dS T0 and for keys
 // acc0 += P T1.
 //
-// The chain S -> exp -> shared memory -> accumulate is 2-3 thousand cycles long and the MMAs of a
-// step 1.0-1.3 thousand, so steps overlap: 64 columns a step leave room in TMEM for two S / dP
-// pairs beside the accumulators and in shared memory for two P / dS pairs and three stages of
-// the streamed operands.  The issuer starts step i + 1's scores before it waits for step i's
-// probabilities, and the two groups of row warps take every other step, so that one computes
-// while the other waits for TMEM, fences and barriers.  One arrival per warp (256 single arrivals
-// on a barrier took longer than the exponentials).  B = 2, H = 16, S = 2048, causal, bf16: 308 us as
-// two kernels with one step in flight -> 161 us; what is left is shared-memory traffic (operands,
-// P and dS: 1.4-1.9 of the 2.6 thousand cycles a step takes).
+// The chain S -> exp -> P, dS -> accumulate is 2-3 thousand cycles long and the MMAs of a step 1.0
+// to 1.3 thousand, so steps overlap: 64 columns a step leave room in TMEM for two S / dP pairs
+// beside the accumulators.  P and dS overwrite the scores they came from, as 16-bit operands in
+// TMEM: through shared memory they cost as much of its bandwidth as half the MMAs.  The issuer
+// starts step i + 1's scores before it waits for step i's probabilities.  One arrival per warp (256
+// single arrivals on a barrier took longer than the exponentials).
+// B = 2, H = 16, S = 2048, causal, bf16: 308 us as two kernels with one step in flight -> 161 us
+// with P and dS in shared memory -> 154 us; about 25 of them are the CTAs' beginnings and ends.
 // ------------------------------------------------------------------------------------
 constexpr int kBwdCols = 64;                          // streamed rows (= score columns) per step
-constexpr int kBwdTile = kBwdCols * kAttD * 2;        // 16 KB: one streamed operand, or P / dS
+constexpr int kBwdTile = kBwdCols * kAttD * 2;        // 16 KB: one streamed operand
 constexpr int kBwdHalf = kBwdTile / 2;                // its two [64 rows][64] halves
-constexpr int kBwdStages = 3;
-constexpr int kBwdSmem = 2 * kAttTile + kBwdStages * 2 * kBwdTile + 4 * kBwdTile + 1024;
+constexpr int kBwdStages = 4;
+constexpr int kBwdSmem = 2 * kAttTile + kBwdStages * 2 * kBwdTile + 1024;
 
 struct __align__(128) AttnBwdShared {
   float lse[kBwdStages][kBwdCols];     // keys: of the streamed queries
@@ -497,7 +514,7 @@ struct __align__(128) AttnBwdShared {
   uint64_t st_full[kBwdStages];        // a stage has landed
   uint64_t st_empty[kBwdStages];       // the MMAs of a step have retired: stage, P and dS are free
   uint64_t s_full[2];                  // scores and dP of a step are complete
-  uint64_t p_full[2];                  // P and dS of a step are in shared memory (4 warps)
+  uint64_t p_full[2];                  // P and dS of a step are in TMEM (8 warps)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -512,15 +529,14 @@ __device__ __forceinline__ void bwd_mma_scores(uint32_t acc, uint32_t a, uint32_
     umma_f16_lo(acc, alo + (((kk >> 2) * kAttHalf + (kk & 3) * 32) >> 4), hi,
                 blo + (((kk >> 2) * kBwdHalf + (kk & 3) * 32) >> 4), hi, idesc, kk ? 1u : 0u);
 }
-// acc (+)= A . B over K = 64: A a K-major tile [128 rows][64], B rows of K ([2 halves of N][64][64])
+// acc (+)= A . B over K = 64: A in TMEM (two pieces of 16 columns, 32 apart: each group of row
+// warps packs into its own half), B rows of K ([2 halves of N][64][64])
 __device__ __forceinline__ void bwd_mma_accumulate(uint32_t acc, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
-  const uint64_t da = make_smem_desc(0, 16, 1024, kLayoutSw128);
   const uint64_t db = make_smem_desc(0, kBwdHalf, 1024, kLayoutSw128);
-  const uint32_t ahi = (uint32_t)(da >> 32), bhi = (uint32_t)(db >> 32);
-  const uint32_t alo = (uint32_t)da + (a >> 4), blo = (uint32_t)db + (b >> 4);
+  const uint32_t bhi = (uint32_t)(db >> 32), blo = (uint32_t)db + (b >> 4);
 #pragma unroll
   for (int kk = 0; kk < 4; ++kk)
-    umma_f16_lo(acc, alo + ((kk * 32) >> 4), ahi, blo + ((kk * 2048) >> 4), bhi, idesc, (accumulate || kk) ? 1u : 0u);
+    umma_f16_ta(acc, a + (kk >> 1) * 32 + (kk & 1) * 8, blo + ((kk * 2048) >> 4), bhi, idesc, (accumulate || kk) ? 1u : 0u);
 }
 
 // 32 columns of P and dS of one row, packed: cols[k] of this thread's columns are visible from
@@ -562,7 +578,6 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUte
                                              const CUtensorMap* tmT1, const AttnParams& p, int blk, int h, int b,
                                              uint32_t base, AttnBwdShared& sh, int* status) {
   const uint32_t sR0 = base, sR1 = base + kAttTile, sT = base + 2 * kAttTile;
-  const uint32_t sP = sT + kBwdStages * 2 * kBwdTile, sDS = sP + 2 * kBwdTile;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   volatile int* abort_flag = &sh.abort_flag;
   const int steps_all = (KV ? p.Sq : p.Sk) / kBwdCols;
@@ -613,9 +628,10 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUte
       if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
       RingPos next, cur;               // stages of the scores' step and of the accumulating step
       for (int it = -1; it < iters && ok; ++it) {
-        if (it + 1 < iters) {          // scores of the next step (its TMEM was read by step it - 1)
-          const int n = it + 1;
-          if (!mbar_wait_bounded(smem_u32(&sh.st_full[next.s]), next.ph, abort_flag)) {
+        if (it + 1 < iters) {          // scores of the next step, over the P and dS of step it - 1
+          const int n = it + 1, j = n - 2;
+          if (!mbar_wait_bounded(smem_u32(&sh.st_full[next.s]), next.ph, abort_flag) ||
+              (j >= 0 && !mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1, abort_flag))) {
             raise_status(status, abort_flag, kTimeoutTmaFull);
             ok = false;
             break;
@@ -635,8 +651,9 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUte
           }
           tc_fence_after();
           const uint32_t t = sT + cur.s * 2 * kBwdTile;
-          if (KV) bwd_mma_accumulate(tAcc0, sP + (it & 1) * kBwdTile, t + kBwdTile, idesc_a, it > 0);
-          bwd_mma_accumulate(tAcc1, sDS + (it & 1) * kBwdTile, t, idesc_a, it > 0);
+          const uint32_t tP = tmem + (it & 1) * 128;
+          if (KV) bwd_mma_accumulate(tAcc0, tP, t + kBwdTile, idesc_a, it > 0);
+          bwd_mma_accumulate(tAcc1, tP + kBwdCols, t, idesc_a, it > 0);
           umma_commit(smem_u32(&sh.st_empty[cur.s]));
           cur.advance(kBwdStages);
         }
@@ -645,7 +662,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUte
   } else {
     int group = 0, quarter = 0;
     att_row_role(warp, group, quarter);
-    const int row = quarter * 32 + lane;               // this thread's key / query
+    const int row = quarter * 32 + lane;               // this thread's key / query; its half of the columns
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
     float my_lse = 0.f, my_delta = 0.f;
     if (!KV) {
@@ -654,47 +671,33 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUte
     }
     bool ok = true;
     RingPos rp;
-    if (group) rp.advance(kBwdStages);
-    for (int it = group; it < iters && ok; it += 2) {
+    for (int it = 0; it < iters && ok; ++it) {
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full[it & 1]), (it >> 1) & 1, abort_flag));
-      // lse and delta of a step came with its stage; the stage of step it - 2 is empty once the
-      // MMAs that read this P / dS pair have retired
+      // lse and delta of a step came with its stage
       if (ok && KV) ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_full[rp.s]), rp.ph, abort_flag));
-      if (ok && it >= 2) {
-        const int j = it - 2;
-        ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1,
-                                                       abort_flag));
-      }
       if (!ok) {
         if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
         break;
       }
       tc_fence_after();
-      const uint32_t buf = (it & 1) * kBwdTile;
-#pragma unroll
-      for (int c = 0; c < kBwdCols; c += 32) {
-        const uint32_t tS = tmem + (it & 1) * 128 + lane_off + c;
-        uint32_t rs[32], rd[32], pk[16], dk[16];
-        tmem_ld_32x32(tS, rs);
-        tmem_ld_32x32(tS + kBwdCols, rd);
-        tmem_ld_wait();
-        // causal: query >= key; distance of these columns from this CTA's first row
-        const int off = p.causal ? (i0 + it) * kBwdCols + c - blk * 128 : 0;
-        const int first = KV && p.causal ? row - off : 0;
-        const int last = !KV && p.causal ? row - off : 31;
-        bwd_probabilities<KV>(rs, rd, sh.lse[rp.s] + c, sh.delta[rp.s] + c, my_lse, my_delta, first, last, p, pk, dk);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint32_t at = att_tile_off(row, c + 8 * j);
-          if (KV) sts128(sP + buf + at, make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]));
-          sts128(sDS + buf + at, make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]));
-        }
-      }
+      const uint32_t tS = tmem + (it & 1) * 128 + lane_off;
+      const int c = group * 32;
+      uint32_t rs[32], rd[32], pk[16], dk[16];
+      tmem_ld_32x32(tS + c, rs);
+      tmem_ld_32x32(tS + kBwdCols + c, rd);
+      tmem_ld_wait();
+      // causal: query >= key; distance of these columns from this CTA's first row
+      const int off = p.causal ? (i0 + it) * kBwdCols + c - blk * 128 : 0;
+      const int first = KV && p.causal ? row - off : 0;
+      const int last = !KV && p.causal ? row - off : 31;
+      bwd_probabilities<KV>(rs, rd, sh.lse[rp.s] + c, sh.delta[rp.s] + c, my_lse, my_delta, first, last, p, pk, dk);
+      // two to a column, over scores that this thread has read
+      if (KV) tmem_st_32x16(tS + c, pk);
+      tmem_st_32x16(tS + kBwdCols + c, dk);
+      tmem_st_wait();
       tc_fence_before();
-      fence_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sh.p_full[it & 1]));
-      rp.advance(kBwdStages);
       rp.advance(kBwdStages);
     }
     if (ok && iters > 0) {
@@ -743,7 +746,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(smem_u32(&sh.s_full[s]), 1);
-      mbar_init(smem_u32(&sh.p_full[s]), 4);
+      mbar_init(smem_u32(&sh.p_full[s]), 8);
     }
     sh.abort_flag = 0;
     mbar_fence_init();
