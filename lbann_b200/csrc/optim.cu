@@ -284,6 +284,114 @@ fused_optimizer_vec_kernel(float* __restrict__ w, const G* __restrict__ grad,
   }
 }
 
+// The whole arena on one rank.  Memory-bound (30 bytes an element for Adam with a 16-bit copy),
+// so what counts is loads in flight: a block walks a contiguous run of chunks two at a time, eight
+// 16-byte loads a thread, and looks its segment up (a binary search and, for Adam, two powers) only
+// when it enters another one; once per chunk that chain of dependent loads left the memory idle
+// between chunks.  Four elements a thread and chunk; segments start on chunk boundaries.
+template <typename G>
+__device__ __forceinline__ void opt_load_grad4(const G* p, float (&g)[4]) {
+  if (sizeof(G) == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    g[0] = v.x; g[1] = v.y; g[2] = v.z; g[3] = v.w;
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const G* e = reinterpret_cast<const G*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) g[j] = to_f32<G>(e[j]);
+  }
+}
+
+template <typename W16>
+__device__ __forceinline__ void opt_store16(W16* p, float a, float b, float c, float d) {
+  uint2 o;
+  W16* e = reinterpret_cast<W16*>(&o);
+  e[0] = from_f32<W16>(a); e[1] = from_f32<W16>(b); e[2] = from_f32<W16>(c); e[3] = from_f32<W16>(d);
+  *reinterpret_cast<uint2*>(p) = o;
+}
+
+template <typename G, typename W16>
+__global__ void __launch_bounds__(256, 3)
+fused_optimizer_run_kernel(float* __restrict__ w, const G* __restrict__ grad, float* __restrict__ s0,
+                           float* __restrict__ s1, W16* __restrict__ w16, const OptSegment* __restrict__ segs, int nseg,
+                           long long total, float inv_scale, const int* __restrict__ skip_flag,
+                           const int* __restrict__ step_ptr, const float* __restrict__ lr_scale_ptr,
+                           const float* __restrict__ inv_scale_dev, long long chunks_per_block) {
+  if (skip_flag && *skip_flag) return;
+  if (inv_scale_dev) inv_scale *= *inv_scale_dev;
+  const float step_t = step_ptr ? (float)(*step_ptr) : 1.f;
+  const float lr_mul = lr_scale_ptr ? *lr_scale_ptr : 1.f;
+  const long long nchunks = (total + kOptChunk - 1) / kOptChunk;
+  const long long first = (long long)blockIdx.x * chunks_per_block;
+  const long long last = min(nchunks, first + chunks_per_block);
+  const bool has_s1 = s1 != s0;
+  OptSegment sg;
+  long long next = -1, end = 0;               // where the next segment begins, this one's elements end
+  for (long long ch = first; ch < last;) {
+    const long long base = ch * kOptChunk;
+    if (base >= next) {
+      const int si = find_segment(segs, nseg, base);
+      sg = segs[si];
+      next = si + 1 < nseg ? segs[si + 1].offset : total;
+      if (next <= base) next = base + kOptChunk;      // behind the last segment
+      sg.lr *= lr_mul;
+      if (sg.kind == kOptAdam)
+        sg.corr = sg.lr * sqrtf(1.f - powf(sg.p1, step_t)) / (1.f - powf(sg.p0, step_t));
+      end = min(sg.offset + sg.count, total);
+    }
+    const long long i = base + 4 * (long long)threadIdx.x;
+    if (sg.kind >= 0 && ch + 2 <= last && base + 2 * kOptChunk <= end) {
+      float4 x[2], a0[2], a1[2];
+      float g[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        x[u] = *reinterpret_cast<const float4*>(w + i + u * kOptChunk);
+        opt_load_grad4<G>(grad + i + u * kOptChunk, g[u]);
+        a0[u] = *reinterpret_cast<const float4*>(s0 + i + u * kOptChunk);
+        a1[u] = has_s1 ? *reinterpret_cast<const float4*>(s1 + i + u * kOptChunk) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w}, m0[4] = {a0[u].x, a0[u].y, a0[u].z, a0[u].w},
+              m1[4] = {a1[u].x, a1[u].y, a1[u].z, a1[u].w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xs[j] = opt_update_one(sg, xs[j], g[u][j] * inv_scale, m0[j], m1[j]);
+        const long long at = i + u * kOptChunk;
+        *reinterpret_cast<float4*>(s0 + at) = make_float4(m0[0], m0[1], m0[2], m0[3]);
+        if (has_s1 && sg.kind == kOptAdam)
+          *reinterpret_cast<float4*>(s1 + at) = make_float4(m1[0], m1[1], m1[2], m1[3]);
+        *reinterpret_cast<float4*>(w + at) = make_float4(xs[0], xs[1], xs[2], xs[3]);
+        if (w16) opt_store16(w16 + at, xs[0], xs[1], xs[2], xs[3]);
+      }
+      ch += 2;
+      continue;
+    }
+    if (sg.kind < 0 && base + kOptChunk <= end) {           // no optimizer: the 16-bit copy only
+      if (w16) {
+        const float4 x = *reinterpret_cast<const float4*>(w + i);
+        opt_store16(w16 + i, x.x, x.y, x.z, x.w);
+      }
+      ++ch;
+      continue;
+    }
+    // a segment's last chunks: element by element
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+      if (i + j >= end) break;
+      float x = w[i + j];
+      if (sg.kind >= 0) {
+        float m0 = s0[i + j], m1 = has_s1 ? s1[i + j] : 0.f;
+        x = opt_update_one(sg, x, to_f32<G>(grad[i + j]) * inv_scale, m0, m1);
+        s0[i + j] = m0;
+        if (has_s1 && sg.kind == kOptAdam) s1[i + j] = m1;
+        w[i + j] = x;
+      }
+      if (w16) w16[i + j] = from_f32<W16>(x);
+    }
+    ++ch;
+  }
+}
+
 // flag |= any non-finite; optionally g *= inv_scale in place.
 template <typename G>
 __global__ void unscale_check_kernel(G* __restrict__ grad, long long n, float inv_scale,
@@ -459,14 +567,25 @@ int lb_fused_optimizer_sharded2(float* w, const void* grad, float* s0, float* s1
   const long long nchunks = (total + kOptChunk - 1) / kOptChunk;
   const int grid = flat_grid((nchunks + world - 1) / world * kOptChunk, kOptChunk);
   const OptSegment* sg = reinterpret_cast<const OptSegment*>(segs);
-#define LB_OPTV(G, W)                                                                        \
-  fused_optimizer_vec_kernel<G, W><<<grid, 256, 0, s>>>(                                     \
-      w, (const G*)grad, s0, s1, (W*)w16, sg, nseg, total, inv_scale, skip_flag, step_ptr,   \
-      lr_scale_ptr, inv_scale_dev, rank, world, own_chunks, peers, compact_state)
+  const long long most = 3LL * lbhost::sm_count();          // all blocks resident at once
+  const long long per = (nchunks + most - 1) / most;
+  const int runs = (int)((nchunks + per - 1) / per);
+  const bool whole = world == 1 && !compact_state && (reinterpret_cast<uintptr_t>(w16) & 7) == 0;
+#define LB_OPTV(G, W)                                                                                         \
+  {                                                                                                           \
+    if (whole)                                                                                                \
+      fused_optimizer_run_kernel<G, W><<<runs, 256, 0, s>>>(w, (const G*)grad, s0, s1, (W*)w16, sg, nseg, total, \
+                                                            inv_scale, skip_flag, step_ptr, lr_scale_ptr,     \
+                                                            inv_scale_dev, per);                              \
+    else                                                                                                      \
+      fused_optimizer_vec_kernel<G, W><<<grid, 256, 0, s>>>(                                                  \
+          w, (const G*)grad, s0, s1, (W*)w16, sg, nseg, total, inv_scale, skip_flag, step_ptr, lr_scale_ptr,  \
+          inv_scale_dev, rank, world, own_chunks, peers, compact_state);                                      \
+  }
   const bool wb = (w16_dtype == kBF16);
-  if (grad_dtype == kF32) { if (wb) LB_OPTV(float, __nv_bfloat16); else LB_OPTV(float, __half); }
-  else if (grad_dtype == kBF16) { if (wb) LB_OPTV(__nv_bfloat16, __nv_bfloat16); else LB_OPTV(__nv_bfloat16, __half); }
-  else { if (wb) LB_OPTV(__half, __nv_bfloat16); else LB_OPTV(__half, __half); }
+  if (grad_dtype == kF32) { if (wb) LB_OPTV(float, __nv_bfloat16) else LB_OPTV(float, __half) }
+  else if (grad_dtype == kBF16) { if (wb) LB_OPTV(__nv_bfloat16, __nv_bfloat16) else LB_OPTV(__nv_bfloat16, __half) }
+  else { if (wb) LB_OPTV(__half, __nv_bfloat16) else LB_OPTV(__half, __half) }
 #undef LB_OPTV
   return (int)cudaGetLastError();
 }
