@@ -501,7 +501,7 @@ struct LayerNormNode : torch::autograd::Function<LayerNormNode> {
     check(lb_layer_norm_bwd(xc.data_ptr(), dy.data_ptr(), fptr(s->scale), fptr(stat), fptr(stat) + rows, dx.data_ptr(),
                             fptr(s->wgrad), fptr(s->bgrad), rows, cols, code(xc.scalar_type()), stream()),
           "lb_layer_norm_bwd");
-    g_launches += 2;
+    ++g_launches;
     if (s->wgrad.defined()) mark_ready(s->wh);
     if (s->bgrad.defined()) mark_ready(s->bh);
     return {dx, Tensor(), Tensor(), Tensor()};

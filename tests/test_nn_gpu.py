@@ -496,3 +496,24 @@ def test_batch_norm_fused_edges(N, C, H, W, act):
         floor = 0.01 * float((gd * (sd / torch.sqrt(var.view(-1) + 1e-5)).view(1, -1, 1, 1)).norm())
         for got, want in zip((y, dx, sh.grad, bh.grad), (want_y, *refs)):
             assert float((got.double() - want).norm()) <= 0.006 * float(want.norm()) + floor * 0.5
+
+
+@pytest.mark.parametrize("cols", [8, 24, 1000, 1024, 1032, 2048, 4104, 8192, 8200])
+@pytest.mark.parametrize("rows", [1, 9, 700])
+def test_layer_norm_rows_in_registers(rows, cols):
+    """Teams of one to eight warps a row, with and without idle lanes, and the column kernels above
+    8192: outputs round to 2^-9, parameter gradients are fp32 sums of `rows` terms."""
+    torch.manual_seed(8)
+    s, b = (torch.randn(cols, device="cuda").requires_grad_(True) for _ in range(2))
+    sh, bh = nn.WeightHandle(s, torch.ones(cols, device="cuda")), nn.WeightHandle(b, torch.ones(cols, device="cuda"))
+    x = (torch.randn(rows, cols, device="cuda") * 3 + 1).bfloat16().requires_grad_(True)
+    dy = torch.randn(rows, cols, device="cuda").bfloat16()
+    y = nn.layer_norm(x, cols, sh, bh)
+    dx, = torch.autograd.grad(y, x, dy)
+    assert native.consume_status() == 0
+    xd, sd, bd = (t.detach().double().requires_grad_(True) for t in (x, s, b))
+    ref = F.layer_norm(xd, (cols,), sd, bd, 1e-5)
+    refs = torch.autograd.grad(ref, (xd, sd, bd), dy.double())
+    for got, want, tol in ((y, ref, 2 ** -8), (dx, refs[0], 2 ** -8), (sh.grad - 1, refs[1], 2e-5),
+                           (bh.grad - 1, refs[2], 2e-5)):
+        assert float((got.double() - want).norm()) <= tol * float(want.norm()) + 1e-5 * cols ** 0.5
