@@ -49,6 +49,7 @@ int lb_bn_fused_fwd(const void*, const float*, const float*, void*, float*, floa
 int lb_bn_fused_bwd(const void*, const void*, const void*, const float*, const float*, void*, float*, float*, float*,
                     long long, int, float, float, float, int, float, int, void* const*, void* const*, int, int,
                     long long, unsigned*, void*);
+int lb_embedding(const void*, int, float*, void*, long long, int, long long, long long, int, int, void*);
 int lb_layer_norm_fwd(const void*, const float*, const float*, void*, float*, float*, long long, int, float, int,
                       void*);
 int lb_layer_norm_bwd(const void*, const void*, const float*, const float*, const float*, void*, float*, float*,
@@ -508,6 +509,39 @@ struct LayerNormNode : torch::autograd::Function<LayerNormNode> {
   }
 };
 
+// -------------------------------------------------------------------------------- embedding
+struct EmbeddingNode : torch::autograd::Function<EmbeddingNode> {
+  // state: wgrad; i = {padding index, dtype of the output}
+  static int kind(const Tensor& idx) {
+    return idx.scalar_type() == at::kInt ? 0 : (idx.scalar_type() == at::kLong ? 1 : 2);
+  }
+  static Tensor forward(AutogradContext* ctx, const Tensor& idx, const Tensor& table, const c10::intrusive_ptr<State>& s) {
+    auto shape = idx.sizes().vec();
+    shape.push_back(table.size(1));
+    const auto dt = s->i[1] == 0 ? at::kHalf : (s->i[1] == 1 ? at::kBFloat16 : at::kFloat);
+    Tensor out = at::empty(shape, table.options().dtype(dt));
+    check(lb_embedding(idx.data_ptr(), kind(idx), fptr(table), out.data_ptr(), idx.numel(), table.size(1), table.size(0),
+                       s->i[0], s->i[1], 0, stream()),
+          "lb_embedding");
+    ++g_launches;
+    keep(ctx, s);
+    ctx->save_for_backward({idx});
+    return out;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    auto s = state_of(ctx);
+    const Tensor idx = ctx->get_saved_variables()[0];
+    Tensor g = grads[0].contiguous();
+    if (reinterpret_cast<uintptr_t>(g.data_ptr()) % 16) g = g.clone();
+    check(lb_embedding(idx.data_ptr(), kind(idx), fptr(s->wgrad), g.data_ptr(), idx.numel(), s->wgrad.size(1),
+                       s->wgrad.size(0), s->i[0], code(g.scalar_type()), 1, stream()),
+          "lb_embedding");
+    ++g_launches;
+    mark_ready(s->wh);
+    return {Tensor(), Tensor(), Tensor()};
+  }
+};
+
 // -------------------------------------------------------------------------------- attention
 struct Attn {
   int64_t H;
@@ -723,6 +757,10 @@ PYBIND11_MODULE(_lbann_autograd, m) {
                          const optional<Tensor>& sgrad, const optional<Tensor>& bgrad, const py::object& sh,
                          const py::object& bh, int64_t cols, double eps) {
     return LayerNormNode::apply(x, scale, bias, make_state({}, {}, sgrad, bgrad, sh, bh, {cols}, {eps}));
+  });
+  m.def("embedding", [](const Tensor& idx, const Tensor& table, const Tensor& wgrad, const py::object& wh,
+                        int64_t padding, int64_t dtype) {
+    return EmbeddingNode::apply(idx, table, make_state({}, {}, wgrad, {}, wh, py::none(), {padding, dtype}, {}));
   });
   m.def("attention", [](const Tensor& q, const Tensor& k, const Tensor& v, int64_t H, double scale, bool causal) {
     return AttentionNode::apply(q, k, v, H, scale, causal);

@@ -1,0 +1,104 @@
+// Embedding lookup and its gradient (src/layers/learning/embedding.cu of the reference).
+//
+// Forward: one warp per index copies its fp32 table row in the layer's 16-bit type; indices out of
+// range and the padding index give zeros.  Backward adds the rows of the output gradient straight
+// into the table's fp32 gradient buffer with 16-byte atomics.  (Through library operators the
+// gradient was sorted by index, summed into a dense tensor of the table's size and that tensor
+// added to the buffer: 250 us for 4096 tokens of a 50304 x 1024 table, whose rows are 25 MB;
+// here 7 us forward and 8 us backward.)
+#include "common.cuh"
+
+namespace lb {
+
+template <typename T, typename I>
+__global__ void __launch_bounds__(256)
+embedding_fwd_kernel(const I* __restrict__ idx, const float* __restrict__ table, T* __restrict__ out, long long n,
+                     int dim, long long num, long long padding) {
+  const int lane = threadIdx.x & 31;
+  const bool vec = dim % 4 == 0;
+  for (long long r = ((long long)blockIdx.x * 256 + threadIdx.x) >> 5; r < n; r += (long long)gridDim.x * 8) {
+    const long long k = (long long)idx[r];              // floats: towards zero
+    const bool ok = k >= 0 && k < num && k != padding;
+    const float* src = table + (ok ? k : 0) * dim;
+    T* dst = out + r * dim;
+    if (vec) {
+#pragma unroll 4
+      for (int c = lane * 4; c < dim; c += 128) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ok) v = *reinterpret_cast<const float4*>(src + c);
+        __align__(16) T o[4] = {from_f32<T>(v.x), from_f32<T>(v.y), from_f32<T>(v.z), from_f32<T>(v.w)};
+        if (sizeof(T) == 2) *reinterpret_cast<uint2*>(dst + c) = *reinterpret_cast<uint2*>(o);
+        else *reinterpret_cast<uint4*>(dst + c) = *reinterpret_cast<uint4*>(o);
+      }
+    } else {
+      for (int c = lane; c < dim; c += 32) dst[c] = from_f32<T>(ok ? src[c] : 0.f);
+    }
+  }
+}
+
+template <typename T, typename I>
+__global__ void __launch_bounds__(256)
+embedding_bwd_kernel(const I* __restrict__ idx, const T* __restrict__ dout, float* __restrict__ grad, long long n, int dim,
+                     long long num, long long padding) {
+  const int lane = threadIdx.x & 31;
+  const bool vec = dim % 4 == 0;
+  for (long long r = ((long long)blockIdx.x * 256 + threadIdx.x) >> 5; r < n; r += (long long)gridDim.x * 8) {
+    const long long k = (long long)idx[r];
+    if (k < 0 || k >= num || k == padding) continue;
+    const T* src = dout + r * dim;
+    float* dst = grad + k * dim;
+    if (vec) {
+#pragma unroll 4
+      for (int c = lane * 4; c < dim; c += 128) {
+        __align__(16) T e[4];
+        if (sizeof(T) == 2) *reinterpret_cast<uint2*>(e) = *reinterpret_cast<const uint2*>(src + c);
+        else *reinterpret_cast<uint4*>(e) = *reinterpret_cast<const uint4*>(src + c);
+        atomicAdd(reinterpret_cast<float4*>(dst + c),
+                  make_float4(to_f32<T>(e[0]), to_f32<T>(e[1]), to_f32<T>(e[2]), to_f32<T>(e[3])));
+      }
+    } else {
+      for (int c = lane; c < dim; c += 32) atomicAdd(dst + c, to_f32<T>(src[c]));
+    }
+  }
+}
+
+}  // namespace lb
+
+extern "C" {
+
+// idx: n indices, idx_kind 0 int32, 1 int64, 2 fp32.  table, grad: fp32 [num][dim]; out, dout:
+// dense [n][dim] of `dtype`; all of them 16-byte aligned (-2 otherwise).  padding < 0: none.
+// backward = 0: out = table[idx]; 1: grad[idx] += dout.
+int lb_embedding(const void* idx, int idx_kind, float* table, void* out, long long n, int dim, long long num,
+                 long long padding, int dtype, int backward, void* stream_) {
+  using namespace lb;
+  if (n < 1 || dim < 1 || num < 1) return -1;
+  if ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(out)) & 15) return -2;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  long long blocks = (n + 7) / 8;
+  const long long cap = 8LL * lbhost::sm_count();
+  if (blocks > cap) blocks = cap;
+#define LB_EMB(T, I)                                                                                                \
+  {                                                                                                                 \
+    if (backward)                                                                                                   \
+      embedding_bwd_kernel<T, I><<<(int)blocks, 256, 0, s>>>((const I*)idx, (const T*)out, table, n, dim, num, padding); \
+    else                                                                                                            \
+      embedding_fwd_kernel<T, I><<<(int)blocks, 256, 0, s>>>((const I*)idx, table, (T*)out, n, dim, num, padding);   \
+    return (int)cudaGetLastError();                                                                                 \
+  }
+#define LB_EMB_IDX(T)                       \
+  {                                         \
+    if (idx_kind == 0) LB_EMB(T, int)       \
+    if (idx_kind == 1) LB_EMB(T, long long) \
+    if (idx_kind == 2) LB_EMB(T, float)     \
+    return -1;                              \
+  }
+  if (dtype == kBF16) LB_EMB_IDX(__nv_bfloat16)
+  if (dtype == kF16) LB_EMB_IDX(__half)
+  if (dtype == kF32) LB_EMB_IDX(float)
+#undef LB_EMB_IDX
+#undef LB_EMB
+  return -1;
+}
+
+}  // extern "C"

@@ -334,15 +334,7 @@ class Embedding(ExecLayer):
         return [tuple(in_dims[0]) + (self.dim,)]
 
     def forward(self, xs, training):
-        idx = xs[0].long()
-        ok = (idx >= 0) & (idx < self.num)
-        if self.padding_idx >= 0:
-            ok = ok & (idx != self.padding_idx)
-        dt = self.dtype or self.model.default_dtype
-        table = self.w.handle.master
-        out = F.embedding(idx.clamp(0, self.num - 1), table)
-        out = out * ok.unsqueeze(-1).to(out.dtype)
-        return [out.to(dt)]
+        return [nn.embedding(xs[0], self.w.handle, self.padding_idx, self.dtype or self.model.default_dtype)]
 
 
 @register("gru")

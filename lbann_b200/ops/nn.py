@@ -907,6 +907,28 @@ class _ReduceSum(torch.autograd.Function):
         return g, None
 
 
+# --------------------------------------------------------------------------- embedding
+def embedding(idx, wh: WeightHandle, padding_idx: int, dtype):
+    """Rows ``idx`` of the table in ``dtype``; zeros (and no gradient) for indices out of range
+    and for ``padding_idx``.  A trainable fp32 table on a GPU takes the native kernels."""
+    table = wh.master
+    num = table.shape[0]
+    if (table.is_cuda and table.dtype == torch.float32 and table.is_contiguous() and table.data_ptr() % 16 == 0
+            and wh.grad is not None and wh.grad.dtype == torch.float32 and wh.grad.is_contiguous()
+            and wh.grad.data_ptr() % 16 == 0 and idx.numel() > 0 and idx.device == table.device
+            and dtype in (torch.float16, torch.bfloat16, torch.float32)):
+        if idx.dtype not in (torch.int32, torch.int64, torch.float32):
+            idx = idx.long()
+        return native.nodes().embedding(idx.contiguous(), table, wh.grad.view(table.shape), wh, int(padding_idx),
+                                        native.dtype_code(dtype))
+    idx = idx.long()
+    ok = (idx >= 0) & (idx < num)
+    if padding_idx >= 0:
+        ok = ok & (idx != padding_idx)
+    out = F.embedding(idx.clamp(0, num - 1), table)
+    return (out * ok.unsqueeze(-1).to(out.dtype)).to(dtype)
+
+
 # --------------------------------------------------------------------------- layer norm
 def layer_norm(x, normalized_size: int, sh=None, bh=None, eps: float = 1e-5):
     """Normalise over the trailing ``normalized_size`` elements of every sample."""

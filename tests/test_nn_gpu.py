@@ -517,3 +517,24 @@ def test_layer_norm_rows_in_registers(rows, cols):
     for got, want, tol in ((y, ref, 2 ** -8), (dx, refs[0], 2 ** -8), (sh.grad - 1, refs[1], 2e-5),
                            (bh.grad - 1, refs[2], 2e-5)):
         assert float((got.double() - want).norm()) <= tol * float(want.norm()) + 1e-5 * cols ** 0.5
+
+
+@pytest.mark.parametrize("itype", [torch.int32, torch.int64, torch.float32, torch.int16])
+@pytest.mark.parametrize("dim,dtype", [(128, torch.bfloat16), (6, torch.float16), (36, torch.float32)])
+def test_embedding_native(itype, dim, dtype):
+    """Repeated, out-of-range and padding indices; gradients are added to what the buffer holds."""
+    torch.manual_seed(9)
+    num, pad = 23, 5
+    table = torch.randn(num, dim, device="cuda").requires_grad_(True)
+    wh = nn.WeightHandle(table, torch.full((num, dim), 2.0, device="cuda"))
+    idx = torch.randint(-3, num + 3, (7, 40), device="cuda")
+    y = nn.embedding(idx.to(itype), wh, pad, dtype)
+    ok = (idx >= 0) & (idx < num) & (idx != pad)
+    want = (table.detach()[idx.clamp(0, num - 1)] * ok.unsqueeze(-1)).to(dtype)
+    assert y.dtype == dtype and torch.equal(y, want)
+    g = torch.randn_like(y)
+    y.backward(g)
+    ref = torch.zeros(num, dim, device="cuda", dtype=torch.double)
+    ref.index_add_(0, idx.clamp(0, num - 1).reshape(-1), (g.double() * ok.unsqueeze(-1)).reshape(-1, dim))
+    assert native.consume_status() == 0
+    assert float((wh.grad.double() - 2 - ref).abs().max()) < 1e-4      # at most 280 fp32 additions of order one
