@@ -42,6 +42,7 @@ int lb_conv_fwd_halo_tc(const void*, const void*, void*, const float*, const int
 long long lb_conv_wgrad_ws(const int*);
 int lb_conv_wgrad_tc(const void*, const void*, float*, float*, const int*, const long long*, const long long*,
                      long long, long long, long long, int, float, void*);
+int lb_upsample_zero(const void*, void*, const int*, void*);
 int lb_pack_filter(const float*, void*, void*, int, int, int, int, int, int, void*);
 int lb_bn_fused_fwd(const void*, const float*, const float*, void*, float*, float*, float*, float*, long long, int,
                     float, float, float, float, int, float, int, void* const*, void* const*, int, int, long long,
@@ -356,14 +357,18 @@ void conv_wgrad(const Tensor& x, Tensor dy, const Tensor& out, const int64_t* g,
   g_launches += 2;
 }
 
-// Zeros between the elements of dy (data gradient of a strided convolution).
+// Zeros between the elements of dy (data gradient of a strided convolution); dy is dense NDHWC.
 Tensor upsample_zero(const Tensor& dy, const int64_t* stride) {
   std::vector<int64_t> shape{dy.size(0)};
   for (int i = 0; i < 3; ++i) shape.push_back((dy.size(1 + i) - 1) * stride[i] + 1);
   shape.push_back(dy.size(4));
-  Tensor up = at::zeros(shape, dy.options()), view = up;
-  for (int i = 0; i < 3; ++i) view = view.slice(1 + i, 0, INT64_MAX, stride[i]);
-  view.copy_(dy);
+  int geom[8];
+  for (int i = 0; i < 5; ++i) geom[i] = (int)dy.size(i);
+  for (int i = 0; i < 3; ++i) geom[5 + i] = (int)stride[i];
+  Tensor up = at::empty(shape, dy.options());
+  Tensor src = reinterpret_cast<uintptr_t>(dy.data_ptr()) % 16 ? dy.clone() : dy;
+  check(lb_upsample_zero(src.data_ptr(), up.data_ptr(), geom, stream()), "lb_upsample_zero");
+  ++g_launches;
   return up;
 }
 

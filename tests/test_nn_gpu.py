@@ -577,3 +577,21 @@ def test_optimizer_runs_of_chunks(counts, kind):
         # values of up to five: a rounding is 2.4e-7, and 1 - 0.99 in fp32 is 1e-6 off in relation
         assert float((got.double() - x).abs().max()) < 4e-6
         assert torch.equal(a.view(a.compute, s), got.bfloat16())
+
+
+@pytest.mark.parametrize("nd,stride,size", [(2, 2, (9, 14)), (2, 3, (20, 7)), (3, 2, (5, 6, 9))])
+def test_strided_convolution_data_gradient(nd, stride, size):
+    """Zeros between the gradient's pixels, sizes that leave a remainder: against 64 bits."""
+    torch.manual_seed(12)
+    C, K = 16, 24
+    x = torch.randn(2, C, *size, device="cuda").half().requires_grad_(True)
+    w = (torch.randn(K, C, *[3] * nd, device="cuda") / 12).requires_grad_(True)
+    wh = nn.WeightHandle(w, torch.zeros_like(w))
+    y = nn.convolution(x, wh, None, (3,) * nd, (1,) * nd, (stride,) * nd, (1,) * nd)
+    g = torch.randn_like(y)
+    dx, = torch.autograd.grad(y, x, g)
+    assert native.consume_status() == 0
+    xd, wd = x.detach().double().requires_grad_(True), w.detach().half().double()
+    ref = (F.conv2d if nd == 2 else F.conv3d)(xd, wd, None, stride, 1)
+    want, = torch.autograd.grad(ref, xd, g.double())
+    assert float((dx.double() - want).norm()) <= 2 ** -10 * float(want.norm())
