@@ -51,8 +51,7 @@ struct EpiParams {
   // separate work items, so a problem with few output tiles and a long reduction still fills
   // the GPU.  Every item stores its fp32 accumulators into sk_ws[tile][split][128][BN] and is
   // done; tc_splitk_reduce_kernel, launched behind it, sums the partials of every output
-  // element in split order (one warp per output row, lanes along the row), applies the
-  // epilogue and stores.
+  // element in split order, applies the epilogue and stores.
   int k_splits = 1;
   float* sk_ws = nullptr;
 };
@@ -562,17 +561,21 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
   }
 }
 
-// Second half of a split-K product: one warp per output row of a tile, lanes along the row.
-// Sums the k_splits partials of every element in split order, so the result does not depend
-// on how the items were scheduled, then alpha / bias / beta / activation and the store.
+// Second half of a split-K product: one thread per four columns of an output row.  Sums the
+// k_splits partials of every element in split order, so the result does not depend on how the
+// items were scheduled, then alpha / bias / beta / activation and the store.  The loads of eight
+// splits are in flight at once: the partials are in L2, and a skinny product has so few rows that
+// a warp per row (its loads four at a time, twice for 256 columns) took 11 us for 18 splits of one
+// row of 2048.
 constexpr int kSplitReduceThreads = 256;
 
 template <class Policy>
 __global__ void __launch_bounds__(kSplitReduceThreads)
 tc_splitk_reduce_kernel(const __grid_constant__ typename Policy::Params p) {
   constexpr int BN = Policy::BN;
-  const long long wg = (long long)blockIdx.x * (kSplitReduceThreads / 32) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
+  constexpr int kPerRow = BN / 4;                         // threads per row
+  const long long wg = ((long long)blockIdx.x * kSplitReduceThreads + threadIdx.x) / kPerRow;
+  const int c = (int)(threadIdx.x % kPerRow) * 4;
   const int t = (int)(wg / kBM), row = (int)(wg % kBM);
   if (t >= p.num_tiles) return;
   const typename Policy::Tile tile = Policy::decode(p, t);
@@ -580,58 +583,49 @@ tc_splitk_reduce_kernel(const __grid_constant__ typename Policy::Params p) {
   if (!Policy::row_addr(p, tile, row, row_off)) return;
   const int n0 = Policy::col0(p, tile);
   const int n_total = Policy::ncols(p);
+  if (n0 + c >= n_total) return;
   const EpiParams& e = p.epi;
   const int splits = e.k_splits;
   const long long split_stride = (long long)kBM * BN;
-  const float* base = e.sk_ws + ((long long)t * splits * kBM + row) * BN;
+  const float* src = e.sk_ws + ((long long)t * splits * kBM + row) * BN + c;
   const float row_bias = e.bias_mode == 2 ? e.bias[Policy::row_index(p, tile, row)] : 0.f;
-  for (int c = lane * 4; c < BN; c += 128) {
-    if (n0 + c >= n_total) break;
-    const float* src = base + c;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-    int s = 0;
-    for (; s + 4 <= splits; s += 4) {
-      const float4 q0 = __ldcg(reinterpret_cast<const float4*>(src + (s + 0) * split_stride));
-      const float4 q1 = __ldcg(reinterpret_cast<const float4*>(src + (s + 1) * split_stride));
-      const float4 q2 = __ldcg(reinterpret_cast<const float4*>(src + (s + 2) * split_stride));
-      const float4 q3 = __ldcg(reinterpret_cast<const float4*>(src + (s + 3) * split_stride));
-      a.x += q0.x; a.y += q0.y; a.z += q0.z; a.w += q0.w;
-      a.x += q1.x; a.y += q1.y; a.z += q1.z; a.w += q1.w;
-      a.x += q2.x; a.y += q2.y; a.z += q2.z; a.w += q2.w;
-      a.x += q3.x; a.y += q3.y; a.z += q3.z; a.w += q3.w;
-    }
-    for (; s < splits; ++s) {
-      const float4 q = __ldcg(reinterpret_cast<const float4*>(src + s * split_stride));
-      a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
-    }
-    float v[4] = {a.x, a.y, a.z, a.w};
-    const int ncol = min(4, n_total - (n0 + c));
-    const long long off = row_off + n0 + c;
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = 0; s < splits; s += 8) {
+    float4 q[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      if (j >= ncol) break;
-      float x = v[j] * e.alpha + row_bias;
-      if (e.bias_mode == 1) x += __ldg(e.bias + n0 + c + j);
-      if (e.beta != 0.f) x += e.beta * load_as_f32(e.C, off + j, e.out_dtype);
-      v[j] = apply_act(x, e.act, e.act_param);
-    }
-    if (e.out_dtype == kF32) {
-      float* dst = reinterpret_cast<float*>(e.C) + off;
-      if (ncol == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-      } else {
-        for (int j = 0; j < ncol; ++j) dst[j] = v[j];
-      }
+    for (int u = 0; u < 8; ++u)
+      if (s + u < splits) q[u] = __ldcg(reinterpret_cast<const float4*>(src + (s + u) * split_stride));
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (s + u < splits) { a.x += q[u].x; a.y += q[u].y; a.z += q[u].z; a.w += q[u].w; }
+  }
+  float v[4] = {a.x, a.y, a.z, a.w};
+  const int ncol = min(4, n_total - (n0 + c));
+  const long long off = row_off + n0 + c;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (j >= ncol) break;
+    float x = v[j] * e.alpha + row_bias;
+    if (e.bias_mode == 1) x += __ldg(e.bias + n0 + c + j);
+    if (e.beta != 0.f) x += e.beta * load_as_f32(e.C, off + j, e.out_dtype);
+    v[j] = apply_act(x, e.act, e.act_param);
+  }
+  if (e.out_dtype == kF32) {
+    float* dst = reinterpret_cast<float*>(e.C) + off;
+    if (ncol == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+      *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
     } else {
-      uint16_t* dst = reinterpret_cast<uint16_t*>(e.C) + off;
-      const uint32_t lo = pack2(v[0], v[1], e.out_dtype), hi = pack2(v[2], v[3], e.out_dtype);
-      if (ncol == 4 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
-        *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
-      } else {
-        for (int j = 0; j < ncol; ++j) {
-          const uint32_t q = j < 2 ? lo : hi;
-          dst[j] = static_cast<uint16_t>(j & 1 ? q >> 16 : q & 0xffffu);
-        }
+      for (int j = 0; j < ncol; ++j) dst[j] = v[j];
+    }
+  } else {
+    uint16_t* dst = reinterpret_cast<uint16_t*>(e.C) + off;
+    const uint32_t lo = pack2(v[0], v[1], e.out_dtype), hi = pack2(v[2], v[3], e.out_dtype);
+    if (ncol == 4 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
+      *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
+    } else {
+      for (int j = 0; j < ncol; ++j) {
+        const uint32_t q = j < 2 ? lo : hi;
+        dst[j] = static_cast<uint16_t>(j & 1 ? q >> 16 : q & 0xffffu);
       }
     }
   }
@@ -640,9 +634,8 @@ tc_splitk_reduce_kernel(const __grid_constant__ typename Policy::Params p) {
 // Host side: launches the reduction behind a split product.
 template <class Policy>
 static int launch_splitk_reduce(const typename Policy::Params& p, cudaStream_t stream) {
-  const long long rows = (long long)p.num_tiles * kBM;
-  const int per_block = kSplitReduceThreads / 32;
-  const int blocks = (int)((rows + per_block - 1) / per_block);
+  const long long threads = (long long)p.num_tiles * kBM * (Policy::BN / 4);
+  const int blocks = (int)((threads + kSplitReduceThreads - 1) / kSplitReduceThreads);
   tc_splitk_reduce_kernel<Policy><<<blocks, kSplitReduceThreads, 0, stream>>>(p);
   return (int)cudaGetLastError();
 }
