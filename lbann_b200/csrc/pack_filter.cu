@@ -26,6 +26,52 @@ pack_filter_kernel(const float* __restrict__ w, T* __restrict__ fwd, T* __restri
   }
 }
 
+// The same for 16-bit layouts through shared memory, 8 filters x 32 channels x all taps a block.  The
+// master copy is read in runs of 32 * taps floats, eight rows in flight; then a thread owns one
+// (filter, channel) pair and walks the taps: forward rows leave in runs of 64 bytes, data-gradient
+// rows in runs of 16.  (Element by element, lanes were taps * 4 bytes apart on the way in and
+// Kp * 2 on the way out.)
+constexpr int kPackK = 8, kPackC = 32;
+
+template <typename T>
+__global__ void __launch_bounds__(256)
+pack_filter_tiled_kernel(const float* __restrict__ w, T* __restrict__ fwd, T* __restrict__ dgrad, int K, int C, int taps,
+                         int Kp, int Cp) {
+  extern __shared__ __align__(16) uint8_t pack_smem[];
+  T* tile = reinterpret_cast<T*>(pack_smem);                 // [k][c * taps + t], rows two elements further apart
+  const int k0 = blockIdx.y * kPackK, c0 = blockIdx.x * kPackC;
+  const int run = kPackC * taps, pitch = run + 2;
+  const int live = max(0, min(C - c0, kPackC)) * taps;       // elements of a run that exist
+  const float* src = w + ((long long)k0 * C + c0) * taps;
+  const long long row = (long long)C * taps;
+  for (int i = threadIdx.x; i < run; i += 256) {
+    float v[kPackK];
+#pragma unroll
+    for (int k = 0; k < kPackK; ++k) v[k] = i < live && k0 + k < K ? __ldg(src + k * row + i) : 0.f;
+#pragma unroll
+    for (int k = 0; k < kPackK; ++k) tile[k * pitch + i] = from_f32<T>(v[k]);
+  }
+  __syncthreads();
+  if (fwd) {
+    const int c = threadIdx.x & 31, k = threadIdx.x >> 5;
+    if (c0 + c < Cp && k0 + k < Kp) {
+      T* dst = fwd + (long long)(k0 + k) * Cp + c0 + c;
+      const T* from = tile + k * pitch + c * taps;
+#pragma unroll 4
+      for (int t = 0; t < taps; ++t) dst[(long long)t * Kp * Cp] = from[t];
+    }
+  }
+  if (dgrad) {
+    const int k = threadIdx.x & 7, c = threadIdx.x >> 3;
+    if (c0 + c < Cp && k0 + k < Kp) {
+      T* dst = dgrad + (long long)(c0 + c) * Kp + k0 + k;
+      const T* from = tile + k * pitch + c * taps;
+#pragma unroll 4
+      for (int t = 0; t < taps; ++t) dst[(long long)(taps - 1 - t) * Kp * Cp] = from[t];
+    }
+  }
+}
+
 }  // namespace lb
 
 extern "C" int lb_pack_filter(const float* w, void* fwd, void* dgrad, int K, int C, int taps, int Kp,
@@ -33,6 +79,19 @@ extern "C" int lb_pack_filter(const float* w, void* fwd, void* dgrad, int K, int
   using namespace lb;
   if (K < 1 || C < 1 || taps < 1 || Kp < K || Cp < C) return -1;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  // filters of up to 95 taps fit the default 48 KB of shared memory
+  const long long smem = (long long)kPackK * (kPackC * (long long)taps + 2) * 2;
+  if (dtype != kF32 && smem <= 48 * 1024 && (Kp + kPackK - 1) / kPackK <= 65535) {
+    const dim3 grid((Cp + kPackC - 1) / kPackC, (Kp + kPackK - 1) / kPackK);
+    if (dtype == kF16)
+      pack_filter_tiled_kernel<__half><<<grid, 256, (int)smem, s>>>(w, (__half*)fwd, (__half*)dgrad, K, C, taps, Kp, Cp);
+    else if (dtype == kBF16)
+      pack_filter_tiled_kernel<__nv_bfloat16><<<grid, 256, (int)smem, s>>>(w, (__nv_bfloat16*)fwd, (__nv_bfloat16*)dgrad,
+                                                                          K, C, taps, Kp, Cp);
+    else
+      return -1;
+    return (int)cudaGetLastError();
+  }
   const long long total = (long long)taps * Kp * Cp;
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)lbhost::sm_count() * 8;

@@ -595,3 +595,17 @@ def test_strided_convolution_data_gradient(nd, stride, size):
     ref = (F.conv2d if nd == 2 else F.conv3d)(xd, wd, None, stride, 1)
     want, = torch.autograd.grad(ref, xd, g.double())
     assert float((dx.double() - want).norm()) <= 2 ** -10 * float(want.norm())
+
+
+@pytest.mark.parametrize("K,C,ksize", [(8, 8, (1, 1, 1)), (17, 33, (1, 3, 3)), (40, 24, (3, 3, 3)), (16, 16, (5, 5, 5))])
+def test_pack_both_filter_layouts(K, C, ksize):
+    """Tiled packing at ragged filter and channel counts, and the plain kernel beyond 95 taps."""
+    from lbann_b200.ops.conv import pack_filter
+    torch.manual_seed(11)
+    w = torch.randn(K, C, *ksize, device="cuda")
+    Kp, Cp = (K + 7) // 8 * 8, (C + 7) // 8 * 8
+    taps = ksize[0] * ksize[1] * ksize[2]
+    fwd, dgrad = native.nodes().pack_filter(w, K, C, taps, Kp, Cp, native.DT_BF16)
+    padded = F.pad(w.reshape(K, C, taps), (0, 0, 0, Cp - C, 0, Kp - K)).reshape(Kp, Cp, *ksize)
+    assert torch.equal(fwd, pack_filter(padded, torch.bfloat16))
+    assert torch.equal(dgrad, pack_filter(padded, torch.bfloat16, for_dgrad=True))
