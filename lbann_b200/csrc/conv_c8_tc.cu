@@ -923,6 +923,273 @@ conv_c8_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   }
 }
 
+// ------------------------------------------- wgrad + backward of 2 x 2 x 2 max pooling in one pass
+// The filter gradient of a first layer whose output was pooled by conv_c8_fwd_pool_kernel, from the
+// POOLED gradient and the arg-max bytes: the gradient at full resolution (seven eighths of it
+// zeros) is never written.  No operand is unfolded either; what bounds the kernel above is the
+// shared memory traffic of that (900 bytes a pixel, 128 a cycle).
+//
+// A super-tile is 2 planes x 2 rows x 128 pixels of the convolution's output, the tile of the
+// forward kernel, with the same 4 planes x 4 rows slab of the input.  As a product:
+//   M = (output row s of 4) x (32 output channels), N = (slab row t of 16) x (2 pixels x 4 channels),
+//   K = pixel PAIRS along W, so that the rows of B are the 16-byte units of the slab as TMA wrote it.
+// The gradients of even and of odd output pixels are two A operands; with taps -1, 0, 1 an even
+// pixel 2i needs the pairs i - 1 and i, an odd one the pairs i and i + 1: four accumulators of 128
+// columns, all of TMEM, and 16 MMAs of 128 x 128 x 16 a super-tile.  9 of the 16 (s, t) combinations
+// of an accumulator are taps (t - s in 0..2 along depth and height); the others are not read.  Every
+// sum has just the products of its tap, so values that are not finite reach no other tap.
+// Worker warps expand the pooled gradient: a thread takes one pooled pixel and 8 channels and writes
+// its eight positions, two groups of eight warps in turn, their loads one tile ahead.
+// Eight 128^3 volumes of 4 channels, 32 filters, fp16: MEASURED_HERE
+constexpr int kWpBuffers = 4;                       // expanded gradients in shared memory
+constexpr uint32_t kWpOperand = 8u * 2048u;         // one parity: 8 groups of 8 pairs x 16 blocks x 128 B
+constexpr int kWpThreads = 64 + 512;
+constexpr int kWpMaxStages = 4;
+
+struct C8WgradPoolParams {
+  C8Geom g;
+  int tiles_w, Hp, Dp, Wp, num_super;
+  int cin, in_dtype, act;
+  int slab_row_bytes, stage_bytes, stages;
+  float act_param, alpha;
+  const void* dy;               // pooled gradient, [N][Dp][Hp][Wp][Kout]
+  const uint8_t* idx;           // arg-max bytes in the same layout
+  float* dW;
+  long long s_tap, s_k, s_c;
+  FastDiv fd_tiles_w, fd_Hp, fd_Dp;
+};
+
+struct C8WgPoolShared {
+  uint64_t full[kWpMaxStages];
+  uint64_t empty[kWpMaxStages];
+  uint64_t a_ready[kWpBuffers];
+  uint64_t a_free[kWpBuffers];
+  uint64_t done;
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+// One pooled pixel and 8 channels: g (8 x 16 bits) times the activation's derivative, to the eight
+// positions of the window.  Position (a * 2 + b) * 2 + c lies in operand c, blocks of row a * 2 + b.
+template <typename T>
+__device__ __forceinline__ void c8_expand(uint4 q, uint2 b, int act, float act_param, uint32_t dst) {
+  T* e = reinterpret_cast<T*>(&q);
+  if (act != kActNone) {
+    const float low = act == kActLeaky ? act_param : 0.f;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const bool pos = ((c < 4 ? b.x : b.y) >> (8 * (c & 3))) & 0x80u;
+      e[c] = from_f32<T>(to_f32<T>(e[c]) * (pos ? 1.f : low));
+    }
+  }
+  const uint32_t lo = b.x & 0x7f7f7f7fu, hi = b.y & 0x7f7f7f7fu;
+#pragma unroll
+  for (int pos = 0; pos < 8; ++pos) {
+    const uint32_t ml = __vcmpeq4(lo, pos * 0x01010101u), mh = __vcmpeq4(hi, pos * 0x01010101u);
+    sts128(dst + (pos & 1) * kWpOperand + (pos >> 1) * (4 * 128),
+           make_uint4(q.x & __byte_perm(ml, 0, 0x1100), q.y & __byte_perm(ml, 0, 0x3322),
+                      q.z & __byte_perm(mh, 0, 0x1100), q.w & __byte_perm(mh, 0, 0x3322)));
+  }
+}
+
+__global__ void __launch_bounds__(kWpThreads, 1)
+conv_c8_wgrad_pool_kernel(const __grid_constant__ CUtensorMap tmX, const C8WgradPoolParams p, int* status) {
+  constexpr int kWorkers = 16, kProducerWarp = kWorkers, kMmaWarp = kWorkers + 1;
+  constexpr int kTmemCols = 512;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ C8WgPoolShared sh;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t s_a0 = smem_base;                              // kWpBuffers x (even, odd) operands
+  const uint32_t s_stage0 = smem_base + kWpBuffers * 2u * kWpOperand;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int* abort_flag = &sh.abort_flag;
+  const int S = p.stages;
+  const C8Geom& g = p.g;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(smem_u32(&sh.full[s]), 1);
+      mbar_init(smem_u32(&sh.empty[s]), 1);
+    }
+    for (int j = 0; j < kWpBuffers; ++j) {
+      mbar_init(smem_u32(&sh.a_ready[j]), kWorkers / 2);        // one arrive per expanding warp
+      mbar_init(smem_u32(&sh.a_free[j]), 1);
+    }
+    mbar_init(smem_u32(&sh.done), 1);
+    sh.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == kProducerWarp && lane == 0) tma_prefetch_desc(&tmX);
+  if (warp == kMmaWarp) {
+    tmem_alloc(smem_u32(&sh.tmem_base), kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sh.tmem_base;
+
+  if (warp == kProducerWarp) {
+    if (elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      RingPos rp;
+      for (int q = blockIdx.x; q < p.num_super; q += gridDim.x, ++it) {
+        const uint32_t s = rp.s;
+        if (!mbar_wait_bounded(smem_u32(&sh.empty[s]), rp.ph ^ 1, abort_flag)) {
+          raise_status(status, abort_flag, kTimeoutStageEmpty);
+          ok = false;
+          break;
+        }
+        rp.advance((uint32_t)S);
+        uint32_t r, tw, hp, dp, n;
+        p.fd_tiles_w.divmod((uint32_t)q, r, tw);
+        p.fd_Hp.divmod(r, r, hp);
+        p.fd_Dp.divmod(r, n, dp);
+        const uint32_t bar = smem_u32(&sh.full[s]);
+        mbar_expect_tx(bar, (uint32_t)p.stage_bytes);
+        tma_load_5d(s_stage0 + s * p.stage_bytes, &tmX, bar, 0, (int)tw * 8 - 1,
+                    2 * (int)hp - g.ph, 2 * (int)dp - g.pd, (int)n);
+      }
+      if (!ok || *abort_flag) {
+        const uint32_t pending = it < (uint32_t)S ? it : (uint32_t)S;
+        for (uint32_t j = 0; j < pending; ++j) {
+          const uint32_t q = it - 1 - j;
+          mbar_wait_budget_only(smem_u32(&sh.full[q % S]), (q / S) & 1);
+        }
+      }
+    }
+  } else if (warp == kMmaWarp) {
+    if (elect_one()) {
+      const uint32_t idesc = make_idesc_f16(p.in_dtype == kBF16 ? 1u : 0u, 1, 1, 128, 128);
+      // both MN-major, un-swizzled: core matrix = 8 pairs x 16 B.  A: blocks of 8 channels 128 B
+      // apart (SBO), 8-pair groups 2048 B apart (LBO).  B: a block of 8 columns is a slab row.
+      const uint64_t a_desc0 = make_smem_desc(0, 2048, 128, kLayoutNone);
+      const uint64_t b_desc0 = make_smem_desc(0, 128, p.slab_row_bytes, kLayoutNone);
+      const uint32_t a_hi = (uint32_t)(a_desc0 >> 32), b_hi = (uint32_t)(b_desc0 >> 32);
+      const uint32_t a_lo0 = (uint32_t)a_desc0 + (s_a0 >> 4);
+      const uint32_t b_lo0 = (uint32_t)b_desc0 + ((s_stage0 + 128u) >> 4);     // pair 0 of the tile
+      constexpr uint32_t kOdd = kWpOperand >> 4, kAStep = 4096u >> 4, kBStep = 256u >> 4;
+      const uint32_t stage_step = (uint32_t)p.stage_bytes >> 4;
+      uint32_t more = 0;                              // 0 for the MMAs that start the accumulators
+      bool ok = true;
+      RingPos rp;
+      uint32_t it = 0;
+      for (int q = blockIdx.x; q < p.num_super; q += gridDim.x, ++it) {
+        const uint32_t s = rp.s, j = it % kWpBuffers, jph = (it / kWpBuffers) & 1u;
+        if (!mbar_wait_bounded(smem_u32(&sh.full[s]), rp.ph, abort_flag) ||
+            !mbar_wait_bounded(smem_u32(&sh.a_ready[j]), jph, abort_flag)) {
+          raise_status(status, abort_flag, kTimeoutTmaFull);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t ad = a_lo0 + j * (2u * kOdd), bd = b_lo0 + s * stage_step;
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          const uint32_t even = ad + k * kAStep, odd = even + kOdd, b = bd + k * kBStep;
+          const uint32_t acc = k ? 1u : more;
+          umma_f16_lo(tmem_base, even, a_hi, b - 1, b_hi, idesc, acc);
+          umma_f16_lo(tmem_base + 128, even, a_hi, b, b_hi, idesc, acc);
+          umma_f16_lo(tmem_base + 256, odd, a_hi, b, b_hi, idesc, acc);
+          umma_f16_lo(tmem_base + 384, odd, a_hi, b + 1, b_hi, idesc, acc);
+        }
+        more = 1u;
+        umma_commit(smem_u32(&sh.empty[s]));
+        umma_commit(smem_u32(&sh.a_free[j]));
+        rp.advance((uint32_t)S);
+      }
+      if (ok) umma_commit(smem_u32(&sh.done));
+    }
+  } else {
+    const int group = warp >> 3;                    // super-tiles group, group + 2, ... of this CTA
+    const int pair = (warp & 7) * 8 + (lane & 7), block = lane >> 3;
+    const uint32_t dst0 = s_a0 + (uint32_t)(warp & 7) * 2048u + block * 128 + (lane & 7) * 16;
+    const bool chan = block * 8 < g.Kout;
+    uint4 q_next = make_uint4(0, 0, 0, 0);
+    uint2 b_next = make_uint2(0, 0);
+    auto fetch = [&](long long tl) {
+      q_next = make_uint4(0, 0, 0, 0);
+      b_next = make_uint2(0, 0);
+      if (tl >= p.num_super) return;
+      uint32_t r, tw, hp, dp, n;
+      p.fd_tiles_w.divmod((uint32_t)tl, r, tw);
+      p.fd_Hp.divmod(r, r, hp);
+      p.fd_Dp.divmod(r, n, dp);
+      const int wp = (int)tw * 64 + pair;
+      if (!chan || wp >= p.Wp) return;
+      const long long off = ((((long long)n * p.Dp + dp) * p.Hp + hp) * p.Wp + wp) * g.Kout + block * 8;
+      q_next = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.dy) + off));
+      b_next = __ldg(reinterpret_cast<const uint2*>(p.idx + off));
+    };
+    fetch((long long)blockIdx.x + (long long)group * gridDim.x);
+    for (uint32_t it = group;; it += 2) {
+      const long long tl = (long long)blockIdx.x + (long long)it * gridDim.x;
+      if (tl >= p.num_super) break;
+      const uint4 q = q_next;
+      const uint2 b = b_next;
+      fetch(tl + 2ll * gridDim.x);
+      const uint32_t j = it % kWpBuffers, jph = (it / kWpBuffers) & 1u;
+      const bool good = mbar_wait_bounded(smem_u32(&sh.a_free[j]), jph ^ 1, abort_flag);
+      if (!__all_sync(0xffffffffu, good)) {
+        if (lane == 0) raise_status(status, abort_flag, kTimeoutStageEmpty);
+        break;
+      }
+      const uint32_t dst = dst0 + j * (2u * kWpOperand);
+      if (p.in_dtype == kBF16) c8_expand<__nv_bfloat16>(q, b, p.act, p.act_param, dst);
+      else c8_expand<__half>(q, b, p.act, p.act_param, dst);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.a_ready[j]));
+    }
+  }
+  // ---- epilogue: the accumulators' taps are added up in shared memory, then in dW -----------------
+  __syncwarp();
+  const bool landed =
+      __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.done), 0, abort_flag));
+  if (!landed && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+  // per output row s, [tap][channel][32]: the operands' space, every MMA has completed
+  float* sums = reinterpret_cast<float*>(smem_raw + (s_a0 - smem_u32(smem_raw)));
+  constexpr int kSums = 27 * 4 * 32;
+  if (landed && warp < 4) {
+    tc_fence_after();
+    const int sd = warp >> 1, shh = warp & 1;       // this warp's lanes: output row s, lane = channel
+    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
+#pragma unroll 1
+    for (int ab = 0; ab < 9; ++ab) {
+      const int t = (ab / 3 + sd) * 4 + ab % 3 + shh;
+      uint32_t r[4][8];
+#pragma unroll
+      for (int acc = 0; acc < 4; ++acc) tmem_ld_32x8(lane_base + acc * 128 + t * 8, r[acc]);
+      tmem_ld_wait();
+      float* to = sums + warp * kSums + ab * 3 * 128 + lane;
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) {
+        // even output pixels: pairs i - 1 and i; odd ones: pairs i and i + 1
+        to[ch * 32] = __uint_as_float(r[0][4 + ch]) + __uint_as_float(r[2][ch]);
+        to[(4 + ch) * 32] = __uint_as_float(r[1][ch]) + __uint_as_float(r[2][4 + ch]);
+        to[(8 + ch) * 32] = __uint_as_float(r[1][4 + ch]) + __uint_as_float(r[3][ch]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncthreads();
+  if (landed) {
+    // tap fastest: neighbouring threads add to neighbouring elements of a dense filter
+    const int total = 27 * p.cin * g.Kout;
+    for (int i = threadIdx.x; i < total; i += kWpThreads) {
+      const int tap = i % 27, r = i / 27, ch = r % p.cin, k = r / p.cin;
+      const float* v = sums + (tap * 4 + ch) * 32 + k;
+      atomicAdd(p.dW + tap * p.s_tap + ch * p.s_c + k * p.s_k,
+                p.alpha * ((v[0] + v[kSums]) + (v[2 * kSums] + v[3 * kSums])));
+    }
+  }
+  if (warp == kMmaWarp) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
 }  // namespace lb
 
 extern "C" {
@@ -1149,6 +1416,62 @@ int lb_conv_c8_wgrad(const void* x, const void* dy, float* dW, const int* geom,
     configured_smem = smem;
   }
   conv_c8_wgrad_kernel<<<p.splits, 64 + 128 * p.groups, smem, stream>>>(tmX, tmDy, p, lbhost::status_word());
+  return (int)cudaGetLastError();
+}
+
+// The same for a layer computed by lb_conv_c8_fwd_pool: dy and idx are the pooled gradient and the
+// arg-max bytes, both dense [N][Do/2][H/2][W/2][Kout]; act, act_param as in the forward call.
+// Returns -2 when the shape is not covered.
+int lb_conv_c8_wgrad_pool(const void* x, const void* dy, const void* idx, float* dW, const int* geom,
+                          const long long* xs, long long s_tap, long long s_k, long long s_c, int cin,
+                          int in_dtype, int act, float act_param, float alpha, void* stream_) {
+  using namespace lb;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  C8WgradPoolParams p;
+  memcpy(&p.g, geom, sizeof(C8Geom));
+  const C8Geom& g = p.g;
+  if (g.Kout > 32 || g.Kout % 8 || g.Kout <= 0 || cin < 1 || cin > 4) return -2;
+  if (xs[3] != 4 || g.kd != 3 || g.kh != 3 || g.ph != 1) return -2;
+  if (g.W % 16 || g.H % 2 || g.Do % 2) return -2;
+  if (in_dtype != kF16 && in_dtype != kBF16) return -2;
+  if (act != kActNone && act != kActRelu && act != kActLeaky) return -2;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(dy) & 15) ||
+      (reinterpret_cast<uintptr_t>(idx) & 7))
+    return -2;
+  const int nchunks = 10;                            // 128 pixels and one 16-pixel chunk either side
+  p.slab_row_bytes = nchunks * 128;
+  p.stage_bytes = 16 * p.slab_row_bytes;
+  p.stages = kWpMaxStages;
+  p.tiles_w = (g.W + 127) / 128;
+  p.Hp = g.H / 2; p.Dp = g.Do / 2; p.Wp = g.W / 2;
+  const long long num_super = (long long)p.tiles_w * p.Hp * p.Dp * g.N;
+  if (num_super <= 0) return 0;
+  {
+    const long long dmax = std::max(std::max(p.tiles_w, p.Hp), p.Dp);
+    if (num_super * dmax >= (1ll << 32) || num_super >= (1ll << 31)) return -2;
+  }
+  p.num_super = (int)num_super;
+  p.fd_tiles_w = FastDiv((uint32_t)p.tiles_w);
+  p.fd_Hp = FastDiv((uint32_t)p.Hp);
+  p.fd_Dp = FastDiv((uint32_t)p.Dp);
+  p.cin = cin; p.in_dtype = in_dtype; p.act = act; p.act_param = act_param; p.alpha = alpha;
+  p.dy = dy; p.idx = static_cast<const uint8_t*>(idx); p.dW = dW;
+  p.s_tap = s_tap; p.s_k = s_k; p.s_c = s_c;
+  CUtensorMap tmX;
+  {
+    uint64_t dims[5] = {16, (uint64_t)(g.W / 16), (uint64_t)g.H, (uint64_t)g.D, (uint64_t)g.N};
+    uint64_t strides[4] = {128, (uint64_t)xs[2] * 2, (uint64_t)xs[1] * 2, (uint64_t)xs[0] * 2};
+    uint32_t box[5] = {16, (uint32_t)nchunks, 4, 4, 1};
+    if (!lbhost::encode_tmap(&tmX, kI64, 5, x, dims, strides, box, nullptr, 0)) return -1;
+  }
+  const int smem = kWpBuffers * 2 * (int)kWpOperand + p.stages * p.stage_bytes + 1024;
+  static int configured = 0;
+  if (configured < smem) {
+    cudaFuncSetAttribute(conv_c8_wgrad_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    configured = smem;
+  }
+  const int grid = p.num_super < lbhost::sm_count() ? p.num_super : lbhost::sm_count();
+  conv_c8_wgrad_pool_kernel<<<grid, kWpThreads, smem, stream>>>(tmX, p, lbhost::status_word());
   return (int)cudaGetLastError();
 }
 

@@ -100,6 +100,9 @@ def _lib():
         lib.lb_conv_c8_fwd_pool.restype = c_int
         lib.lb_conv_c8_fwd_pool.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, P(c_int),
                                             P(c_ll), P(c_ll), c_int, c_int, c_int, c_float, c_void_p]
+        lib.lb_conv_c8_wgrad_pool.restype = c_int
+        lib.lb_conv_c8_wgrad_pool.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, P(c_int), P(c_ll), c_ll, c_ll,
+                                              c_ll, c_int, c_int, c_int, c_float, c_float, c_void_p]
         lib.lb_conv_c8_wgrad.restype = c_int
         lib.lb_conv_c8_wgrad.argtypes = [c_void_p, c_void_p, c_void_p, P(c_int), P(c_ll), P(c_ll),
                                          c_ll, c_ll, c_ll, c_int, c_int, c_float, c_void_p]
@@ -401,8 +404,9 @@ class PoolFusion:
 class _ConvC8Pool(torch.autograd.Function):
     """First-layer convolution + activation + 2 x 2 x 2 max pooling (stride 2) in one kernel
     (csrc/conv_c8_tc.cu, conv_c8_fwd_pool_kernel): the full-resolution activation is never
-    written.  Backward expands the pooled gradient with the recorded arg-max bytes (the
-    separate pooling layer's kernel) and feeds the first-layer filter-gradient kernel."""
+    written.  Backward: where only the filter gradient is wanted, one kernel takes it from the
+    pooled gradient and the recorded arg-max bytes; otherwise the gradient is expanded (the
+    separate pooling layer's kernel) and feeds the general kernels."""
 
     @staticmethod
     def forward(ctx, x, w_leaf, b_leaf, wh, bh, pad, act, act_p, out_alloc):
@@ -448,6 +452,22 @@ class _ConvC8Pool(torch.autograd.Function):
         if not dyp.is_contiguous():
             dyp = dyp.contiguous()
         N, Do, H, W, _ = full
+        bias_grad = bh is not None and bh.grad is not None
+        if not ctx.needs_input_grad[0] and not bias_grad:
+            # nothing but the filter gradient reads the gradient at full resolution: it is not written
+            rc = -2
+            if wh.grad is None:
+                rc = 0
+            elif wh.grad.is_contiguous() and dyp.dtype == x_cl.dtype:
+                rc = _lib().lb_conv_c8_wgrad_pool(x_cl.data_ptr(), dyp.data_ptr(), idx.data_ptr(), wh.grad.data_ptr(),
+                                                  geom, xs, 1, Cin * 27, 27, Cin, native.dtype_code(x_cl.dtype),
+                                                  int(act), float(act_p), 1.0, native.stream_ptr())
+            if rc != -2:
+                native.check(rc, "lb_conv_c8_wgrad_pool")
+                if wh.grad is not None:
+                    native.count_launch()
+                    wh.mark_ready()
+                return (None,) * 9
         # gradient of pooling and activation at full resolution
         dy_cl = torch.empty(full, dtype=dy.dtype, device=dy.device)
         tg = (c_int * 8)(N, Do, H, W, Kout, 2, 2, 2)
@@ -476,7 +496,7 @@ class _ConvC8Pool(torch.autograd.Function):
                                                  native.stream_ptr()), "lb_conv_c8_wgrad")
             native.count_launch()
             wh.mark_ready()
-        if bh is not None and bh.grad is not None:
+        if bias_grad:
             bh.grad.add_(column_sums(dy_cl.reshape(-1, Kout)))
             bh.mark_ready()
         return (dx,) + (None,) * 8

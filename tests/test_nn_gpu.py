@@ -1,4 +1,6 @@
 """Native differentiable ops (ops/nn.py) against PyTorch fp32 autograd on the same inputs."""
+import ctypes
+
 import pytest
 import torch
 import torch.nn.functional as F
@@ -609,3 +611,48 @@ def test_pack_both_filter_layouts(K, C, ksize):
     padded = F.pad(w.reshape(K, C, taps), (0, 0, 0, Cp - C, 0, Kp - K)).reshape(Kp, Cp, *ksize)
     assert torch.equal(fwd, pack_filter(padded, torch.bfloat16))
     assert torch.equal(dgrad, pack_filter(padded, torch.bfloat16, for_dgrad=True))
+
+
+@pytest.mark.parametrize("shape,pad_d,kout,act,dtype", [
+    ((1, 1, 4, 4, 16), 1, 8, native.ACT_NONE, torch.float16),        # one short row tile, one channel block
+    ((2, 3, 6, 10, 144), 1, 24, native.ACT_RELU, torch.bfloat16),    # ragged second tile, three blocks
+    ((2, 4, 8, 6, 128), 0, 32, native.ACT_LEAKY, torch.float16),     # depth halos come with the input
+    ((3, 2, 14, 34, 272), 1, 32, native.ACT_LEAKY, torch.float16),   # more super-tiles than SMs
+])
+def test_conv_c8_wgrad_from_pooled_gradient(shape, pad_d, kout, act, dtype):
+    """The filter gradient from the pooled gradient and arg-max bytes agrees with the expansion at
+    full resolution followed by the general kernel, and with 64-bit sums.  Products are exact in
+    fp32; the bound is 2^-16 of the sum of their sizes, a hundred roundings that all add up."""
+    N, C, D, H, W = shape
+    Do = D + 2 * pad_d - 2
+    torch.manual_seed(6)
+    x = torch.zeros(N, D, H, W, 4, device="cuda", dtype=dtype)
+    x[..., :C] = torch.randn(N, D, H, W, C, device="cuda").to(dtype)
+    dy = torch.randn(N, Do // 2, H // 2, W // 2, kout, device="cuda").to(dtype)
+    idx = torch.randint(0, 8, dy.shape, device="cuda") + 128 * torch.randint(0, 2, dy.shape, device="cuda")
+    idx = idx.to(torch.uint8)
+    lib, code, stream = nn._lib(), native.dtype_code(dtype), native.stream_ptr()
+    geom = (ctypes.c_int * 10)(N, D, H, W, kout, 3, 3, pad_d, 1, Do)
+    xs = (ctypes.c_longlong * 4)(*x.stride()[:4])
+    dw = torch.zeros(kout, C, 3, 3, 3, device="cuda")
+    native.check(lib.lb_conv_c8_wgrad_pool(x.data_ptr(), dy.data_ptr(), idx.data_ptr(), dw.data_ptr(), geom, xs, 1,
+                                           C * 27, 27, C, code, act, 0.3, 1.0, stream), "lb_conv_c8_wgrad_pool")
+    full = torch.empty(N, Do, H, W, kout, device="cuda", dtype=dtype)
+    tg = (ctypes.c_int * 8)(N, Do, H, W, kout, 2, 2, 2)
+    native.check(lib.lb_pool_bwd_tiled_idx(idx.data_ptr(), dy.data_ptr(), full.data_ptr(), tg, act, 0.3,
+                                           full.stride(0), code, stream), "lb_pool_bwd_tiled_idx")
+    general = torch.zeros_like(dw)
+    ys = (ctypes.c_longlong * 4)(*full.stride()[:4])
+    native.check(lib.lb_conv_c8_wgrad(x.data_ptr(), full.data_ptr(), general.data_ptr(), geom, xs, ys, 1, C * 27, 27,
+                                      C, code, 1.0, stream), "lb_conv_c8_wgrad")
+    assert native.consume_status() == 0
+
+    def sums(a, b):
+        a = F.pad(a.double(), (0, 0, 1, 1, 1, 1, pad_d, pad_d))
+        b = b.double()
+        taps = [torch.einsum("ndhwc,ndhwk->kc", a[:, i:i + Do, j:j + H, k:k + W], b)
+                for i in range(3) for j in range(3) for k in range(3)]
+        return torch.stack(taps, -1).reshape(kout, C, 3, 3, 3)
+    ref, size = sums(x[..., :C], full), sums(x[..., :C].abs(), full.abs())
+    assert bool(((dw - ref).abs() <= 2.0 ** -16 * size + 1e-12).all())
+    assert bool(((general - ref).abs() <= 2.0 ** -16 * size + 1e-12).all())
