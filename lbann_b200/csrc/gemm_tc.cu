@@ -140,7 +140,8 @@ constexpr int kPairHint = 512;
 // 64 on one.  Per wave of tiles an estimate is k-steps (64 each) x cycles + what the last tile's
 // epilogue shows.  The cycles are slopes measured over K between 1024 and 8192 (0.31 us a step
 // for the pair, 0.48 / 0.30 / 0.27 at 256 / 128 / 64); a product that is cut along K needs its
-// second kernel (which writes whole rows), and the one-SM epilogue reads an accumulated C, and
+// second kernel (which writes whole rows; one row of 2048, K 16384: 29.7 us with 18 splits of 8
+// tiles, 27.6 with 9 of 16), and the one-SM epilogue reads an accumulated C, and
 // writes rows that do not start on 16 bytes, value by value.
 // Measured, pair against the tile that was taken before: 8192 x 8192 x 2048 167 / 219 us,
 // 4096 x 1024 x 50304 278 / 623 us, fp32 += 4096 x 1024 x 4096 40 / 86 us; the other way,
@@ -168,7 +169,7 @@ static int gemm_choose(int M, int N, int K, int batch, const lbhost::SplitKOffer
     const long long waves = (tiles * splits + sms - 1) / sms;
     const long long shown = aligned ? tail[i] * (accumulate ? 6 : 1) : 160 * bn;
     consider(bn, waves * (cycles[i] * ((k + splits - 1) / splits) + (splits > 1 ? tail[i] : shown)) +
-                     (splits > 1 ? 8000 : 0));
+                     (splits > 1 ? 6500 + 240 * splits : 0));
   }
   return best;
 }
