@@ -21,6 +21,7 @@
 #include "conv_geom.cuh"
 #include "halo_sync.cuh"
 #include "tc_pipeline.cuh"
+#include <algorithm>
 
 namespace lb {
 
@@ -296,6 +297,267 @@ conv_slab_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant_
   }
 }
 
+// ---------------------------------------------------------------- three depth taps at a time
+// The same convolution for 3 x 3 x 3 filters with at most 64 output channels, where an MMA is bound by
+// its A operand: 128 rows take 32 cycles of shared memory reads whatever N is, so 64 -> 32 channels
+// spent 40 cycles on MMAs worth 16.  A work item is a tile of one plane times L consecutive output
+// planes, and walks the input planes along depth.  Input plane z feeds the outputs z + pd - a,
+// a = 0..2: with the filter laid out as [kh kw][a][Kout] and the accumulators of the L planes in
+// descending order, the three taps of a plane are ONE product with N = 3 BN (less at the two ends).
+// L + 2 slabs are loaded for L outputs instead of three for each.  Accumulators start at zero
+// because the planes of one MMA are at different stages; sums run in the order of the kernel above
+// (depth, height, width tap, channel) and give the same bits.
+// 8 x 64^3, fp16: 64 -> 32 channels 376 -> 199 us, 32 -> 64 272 -> 188 us.
+struct SlabWalkParams {
+  SlabParams s;
+  int L, segments, num_items;
+  FastDiv fd_segments;
+};
+
+template <int KSTEPS>
+__device__ __forceinline__ void slab_walk_plane(uint32_t acc, uint32_t a_line, uint32_t bd, uint32_t line_step,
+                                                uint32_t pix_step, uint32_t tap_step, uint32_t d_hi, uint32_t idesc) {
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int kk = 0; kk < KSTEPS; ++kk)
+        umma_f16_lo(acc, a_line + b * line_step + c * pix_step + 2 * kk, d_hi, bd + (b * 3 + c) * tap_step + 2 * kk,
+                    d_hi, idesc, 1u);
+}
+
+__device__ __forceinline__ void tmem_zero_32(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
+      "%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(0)
+      : "memory");
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kSlabThreads, 1)
+conv_slab_walk_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW,
+                      const SlabWalkParams wp, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ SlabShared sh;
+  const SlabParams& p = wp.s;
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t s_filter = smem_base;
+  const uint32_t s_stage0 = smem_base + p.filter_bytes;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  volatile int* abort_flag = &sh.abort_flag;
+  const int S = p.stages;
+  const ConvGeom& g = p.g;
+  const uint32_t set_cols = (uint32_t)(wp.L * BN);          // columns of one set of accumulators
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(smem_u32(&sh.full[s]), 1);
+      mbar_init(smem_u32(&sh.empty[s]), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(smem_u32(&sh.tmem_full[a]), 1);
+      mbar_init(smem_u32(&sh.tmem_empty[a]), 4);
+    }
+    mbar_init(smem_u32(&sh.filter_ready), 1);
+    sh.abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 4 && lane == 0) {
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW);
+  }
+  if (warp == 5) {
+    tmem_alloc(smem_u32(&sh.tmem_base), 2 * set_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sh.tmem_base;
+
+  if (warp == 4) {
+    if (elect_one()) {
+      const uint32_t fbar = smem_u32(&sh.filter_ready);
+      mbar_expect_tx(fbar, (uint32_t)p.filter_bytes);
+      for (int j = 0; j < p.cblocks; ++j)                  // [cblock][kh kw][a][BN rows][Cb]
+        tma_load_4d(s_filter + j * (p.filter_bytes / p.cblocks), &tmW, fbar, j * p.Cb, 0, 0, 0);
+      uint32_t it = 0;
+      bool ok = true;
+      RingPos rp;
+      for (int t = blockIdx.x; t < wp.num_items && ok; t += gridDim.x) {
+        uint32_t ti, r, seg, nn;
+        p.fd_tiles_plane.divmod((uint32_t)t, r, ti);
+        wp.fd_segments.divmod(r, nn, seg);
+        const int d0 = (int)seg * wp.L, planes = min(wp.L, g.Do - d0) + 2;
+        const int l0 = (int)p.fd_Wp.div(ti * 128u);
+        for (int z = 0; z < planes && ok; ++z) {
+          for (int j = 0; j < p.cblocks; ++j, ++it) {
+            const uint32_t s = rp.s;
+            if (!mbar_wait_bounded(smem_u32(&sh.empty[s]), rp.ph ^ 1, abort_flag)) {
+              raise_status(status, abort_flag, kTimeoutStageEmpty);
+              ok = false;
+              break;
+            }
+            const uint32_t bar = smem_u32(&sh.full[s]);
+            mbar_expect_tx(bar, (uint32_t)p.slab_bytes);
+            tma_load_5d(s_stage0 + s * p.stage_bytes, &tmX, bar, j * p.Cb, -g.pw, l0 - g.ph, d0 - g.pd + z, (int)nn);
+            rp.advance((uint32_t)S);
+          }
+        }
+      }
+      if (!ok || *abort_flag) {
+        const uint32_t pending = it < (uint32_t)S ? it : (uint32_t)S;
+        for (uint32_t j = 0; j < pending; ++j) {
+          const uint32_t q = it - 1 - j;
+          mbar_wait_budget_only(smem_u32(&sh.full[q % S]), (q / S) & 1);
+        }
+        mbar_wait_budget_only(smem_u32(&sh.filter_ready), 0);
+      }
+    }
+  } else if (warp == 5) {
+    if (elect_one()) {
+      const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
+      const uint32_t idesc1 = make_idesc_f16(fmt, 0, 0, 128, BN), idesc2 = make_idesc_f16(fmt, 0, 0, 128, 2 * BN),
+                     idesc3 = make_idesc_f16(fmt, 0, 0, 128, 3 * BN);
+      const uint32_t row_bytes = p.Cb * 2;
+      const uint64_t desc0 = make_smem_desc(0, 16, 8 * row_bytes, p.layout_type);
+      const uint32_t d_lo = (uint32_t)desc0, d_hi = (uint32_t)(desc0 >> 32);
+      const uint32_t depth_step = (BN * row_bytes) >> 4, tap_step = 3 * depth_step;
+      const uint32_t pix_step = row_bytes >> 4;
+      const uint32_t line_step = ((uint32_t)p.Wp * row_bytes) >> 4;
+      const uint32_t fblock = ((uint32_t)p.filter_bytes / (uint32_t)p.cblocks) >> 4;
+      const uint32_t stage_step = (uint32_t)p.stage_bytes >> 4;
+      const uint32_t cblocks = (uint32_t)p.cblocks;
+      const int ksteps = p.Cb / 16;
+      bool ok = mbar_wait_bounded(smem_u32(&sh.filter_ready), 0, abort_flag);
+      if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
+      uint32_t lt = 0;
+      RingPos rp;
+      for (int t = blockIdx.x; t < wp.num_items && ok; t += gridDim.x, ++lt) {
+        uint32_t ti, r, seg, nn;
+        p.fd_tiles_plane.divmod((uint32_t)t, r, ti);
+        wp.fd_segments.divmod(r, nn, seg);
+        const int outs = min(wp.L, g.Do - (int)seg * wp.L);
+        const uint32_t q0 = ti * 128u;
+        const uint32_t row0 = q0 - p.fd_Wp.div(q0) * (uint32_t)p.Wp;
+        const uint32_t acc = lt & 1, acc_ph = (lt >> 1) & 1;
+        // the set is zero: at the start, and again after each item's epilogue
+        if (!mbar_wait_bounded(smem_u32(&sh.tmem_empty[acc]), acc_ph, abort_flag)) {
+          raise_status(status, abort_flag, kTimeoutTmemEmpty);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t set = tmem_base + acc * set_cols;
+        const uint32_t a_tile = d_lo + ((s_stage0 + row0 * row_bytes) >> 4);
+        const uint32_t filter = d_lo + (s_filter >> 4);
+        for (int z = 0; z < outs + 2 && ok; ++z) {
+          // outputs z - a of the segment, a = lo .. hi; output o sits in block outs - 1 - o
+          const int lo = max(0, z - outs + 1), hi = min(2, z);
+          const uint32_t idesc = hi - lo == 2 ? idesc3 : hi - lo == 1 ? idesc2 : idesc1;
+          const uint32_t to = set + (uint32_t)((outs - 1 - z + lo) * BN);
+          uint32_t bd = filter + (uint32_t)lo * depth_step;
+          for (uint32_t j = 0; j < cblocks; ++j, bd += fblock) {
+            if (!mbar_wait_bounded(smem_u32(&sh.full[rp.s]), rp.ph, abort_flag)) {
+              raise_status(status, abort_flag, kTimeoutTmaFull);
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t a_line = a_tile + rp.s * stage_step;
+            if (ksteps == 4) slab_walk_plane<4>(to, a_line, bd, line_step, pix_step, tap_step, d_hi, idesc);
+            else if (ksteps == 2) slab_walk_plane<2>(to, a_line, bd, line_step, pix_step, tap_step, d_hi, idesc);
+            else slab_walk_plane<1>(to, a_line, bd, line_step, pix_step, tap_step, d_hi, idesc);
+            umma_commit(smem_u32(&sh.empty[rp.s]));
+            rp.advance((uint32_t)S);
+          }
+        }
+        if (ok) umma_commit(smem_u32(&sh.tmem_full[acc]));
+      }
+    }
+  } else {
+    // one group of four warps per set of accumulators, as above; it leaves the set at zero
+    const int eg = warp >= 6 ? 1 : 0;
+    const int quarter = warp & 3;
+    uint32_t use = 0;
+    const EpiParams& e = p.epi;
+    const uint32_t taddr = tmem_base + eg * set_cols + (static_cast<uint32_t>(quarter * 32) << 16);
+    auto hand_back = [&]() {
+      __syncwarp();
+      for (uint32_t c = 0; c < set_cols; c += 32) tmem_zero_32(taddr + c);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.tmem_empty[eg]));
+    };
+    hand_back();
+    for (long long tl = (long long)blockIdx.x + (long long)eg * gridDim.x; tl < wp.num_items;
+         tl += 2ll * gridDim.x, ++use) {
+      uint32_t ti, r, seg, nn;
+      p.fd_tiles_plane.divmod((uint32_t)tl, r, ti);
+      wp.fd_segments.divmod(r, nn, seg);
+      const int d0 = (int)seg * wp.L, outs = min(wp.L, g.Do - d0);
+      const bool landed = __all_sync(
+          0xffffffffu, mbar_wait_bounded(smem_u32(&sh.tmem_full[eg]), use & 1u, abort_flag));
+      if (!landed) {
+        if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+        break;
+      }
+      tc_fence_after();
+      const int row = quarter * 32 + lane;
+      const uint32_t q = ti * 128u + (uint32_t)row;
+      const int h = (int)p.fd_Wp.div(q), w = (int)q - h * p.Wp;
+      long long row_off = (long long)nn * p.o_sn + d0 * p.o_sd + h * p.o_sh + (long long)w * p.o_sw;
+      for (int o = 0; o < outs; ++o, row_off += p.o_sd)
+        tc_epilogue_rows<BN>(TmemSrc{taddr + (uint32_t)((outs - 1 - o) * BN)}, h < g.Ho && w < g.Wo, row_off, 0,
+                             g.Kout, row, e);
+      hand_back();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 5) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 2 * set_cols);
+  }
+}
+
+// Output planes per work item of the kernel above, 0 = one tile at a time is faster.  Cycles of an MMA:
+// the larger of its operand reads (32 for A, N / 4 for B) and its arithmetic (N / 2); a wave ends
+// with the epilogue of the last item.  Fewer, longer items lose where they leave SMs idle.  Measured
+// (cold L2, tile by tile / walking), 64 -> 32 channels: one 32^3 volume 16.4 / 14.3 us, four 36.9 / 26.6,
+// 45 x 52 x 60 36.9 / 30.7; 32 -> 64 channels on that volume stays with the tiles (30.7 us).
+static int slab_walk_planes(const SlabParams& p, int BN) {
+  auto mma = [](int n) { return std::max(32 + n / 4, n / 2); };
+  const long long sms = lbhost::sm_count(), steps = 9ll * p.cblocks * (p.Cb / 16);
+  long long best = (p.num_tiles + sms - 1) / sms * (steps * 3 * mma(BN)) + 1500;
+  int L = 0;
+  for (int l = 256 / BN; l >= 2; l /= 2) {
+    const long long items = (long long)p.tiles_plane * ((p.g.Do + l - 1) / l) * p.g.N;
+    const int outs = std::min(l, p.g.Do);
+    long long item = 0;
+    for (int z = 0; z < outs + 2; ++z) item += steps * mma((std::min(2, z) - std::max(0, z - outs + 1) + 1) * BN);
+    const long long cost = (items + sms - 1) / sms * item + 1500ll * outs;
+    if (cost < best) { best = cost; L = l; }
+  }
+  return L;
+}
+
+template <int BN>
+static int launch_slab_walk(const CUtensorMap& tmX, const CUtensorMap& tmW, const SlabWalkParams& p, int smem,
+                            cudaStream_t stream) {
+  static int configured = 0;
+  if (configured < smem) {
+    cudaFuncSetAttribute(conv_slab_walk_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    configured = smem;
+  }
+  const int grid = p.num_items < lbhost::sm_count() ? p.num_items : lbhost::sm_count();
+  conv_slab_walk_kernel<BN><<<grid, kSlabThreads, smem, stream>>>(tmX, tmW, p, lbhost::status_word());
+  return (int)cudaGetLastError();
+}
+
 template <int BN>
 static int launch_slab(const CUtensorMap& tmX, const CUtensorMap& tmW, const SlabParams& p,
                        int smem, cudaStream_t stream) {
@@ -374,6 +636,21 @@ extern "C" int lb_conv_slab_fwd(const void* x, const void* w, void* y, const flo
     if (!lbhost::encode_tmap(&tmW, in_dtype, 3, w, dims, strides, box, nullptr, p.Cb * 2)) return -1;
   }
   const int smem = p.filter_bytes + p.stages * p.stage_bytes + 1024;
+  const int L = !halo && BN <= 64 && g.kd == 3 && g.kh == 3 && g.kw == 3 ? slab_walk_planes(p, BN) : 0;
+  if (L > 0) {
+    SlabWalkParams wp;
+    wp.s = p;
+    wp.L = L;
+    wp.segments = (g.Do + L - 1) / L;
+    wp.num_items = p.tiles_plane * wp.segments * g.N;
+    wp.fd_segments = FastDiv((uint32_t)wp.segments);
+    uint64_t dims[4] = {(uint64_t)g.C, (uint64_t)g.Kout, 3, 9};
+    uint64_t strides[3] = {(uint64_t)g.C * 2, (uint64_t)g.C * g.Kout * 2 * 9, (uint64_t)g.C * g.Kout * 2};
+    uint32_t box[4] = {(uint32_t)p.Cb, (uint32_t)BN, 3, 9};
+    if (!lbhost::encode_tmap(&tmW, in_dtype, 4, w, dims, strides, box, nullptr, p.Cb * 2)) return -1;
+    return BN == 64 ? launch_slab_walk<64>(tmX, tmW, wp, smem, stream)
+                    : launch_slab_walk<32>(tmX, tmW, wp, smem, stream);
+  }
   if (BN == 128) return launch_slab<128>(tmX, tmW, p, smem, stream);
   if (BN == 64) return launch_slab<64>(tmX, tmW, p, smem, stream);
   return launch_slab<32>(tmX, tmW, p, smem, stream);

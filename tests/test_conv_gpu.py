@@ -160,3 +160,35 @@ def test_conv_deep_layers_split_the_reduction(case, monkeypatch):
     plain = conv_fwd(xl, wp, ks, pad=pd, bias=bias, act=native.ACT_LEAKY, act_param=0.01,
                      out_dtype=torch.float32)
     torch.testing.assert_close(ys[0], plain, rtol=1e-4, atol=1e-4)
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, D, H, W, K, depth padding: segments of 8 or 4 planes, ragged ones, one to three channel blocks
+    (8, 64, 19, 40, 64, 32, 1),
+    (6, 32, 21, 64, 48, 64, 1),
+    (9, 16, 12, 56, 50, 24, 0),
+    (8, 96, 17, 40, 40, 32, 1),
+    (16, 48, 10, 30, 60, 40, 2),
+])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_conv_walking_the_depth_gives_the_bits_of_single_planes(case, dtype):
+    """Convolutions large enough for the kernel that takes three depth taps in one product equal,
+    bit for bit, the same computed plane by plane, which is too little work for it; every fourth
+    plane is compared."""
+    N, C, D, H, W, K, pd = case
+    torch.manual_seed(7)
+    x = torch.randn(N, D, H, W, C, device="cuda").to(dtype)
+    wf = (torch.randn(K, C, 3, 3, 3, device="cuda") / (C * 27) ** 0.5).to(dtype)
+    w = pack_filter(wf, dtype)
+    bias = torch.randn(K, device="cuda")
+    y = conv_fwd(x, w, (3, 3, 3), pad=(pd, 1, 1), bias=bias, out_dtype=dtype)
+    Do = D + 2 * pd - 2
+    assert y.shape[1] == Do
+    xp = F.pad(x, (0, 0, 0, 0, 0, 0, pd, pd))
+    for d in sorted({0, 1, *range(2, Do, 4), Do - 2, Do - 1}):
+        one = conv_fwd(xp[:, d:d + 3].contiguous(), w, (3, 3, 3), pad=(0, 1, 1), bias=bias, out_dtype=dtype)
+        assert torch.equal(y[:, d], one[:, 0]), d
+    assert native.consume_status() == 0
+    n = N - 1
+    ref = F.conv3d(x[n:].permute(0, 4, 1, 2, 3).float(), wf.float(), bias, 1, (pd, 1, 1))
+    torch.testing.assert_close(y[n:].permute(0, 4, 1, 2, 3).float(), ref, rtol=2e-2, atol=4e-2)
