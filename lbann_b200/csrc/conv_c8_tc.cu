@@ -3,7 +3,7 @@
 //
 // With so few channels the reduction per tap is tiny, and a tcgen05.mma costs ~104
 // cycles however little of it is used, so the generic implicit-GEMM path (one operand
-// slice per tap) wastes almost all of every instruction here.  Both kernels therefore
+// slice per tap) wastes almost all of every instruction here.  All kernels but the last therefore
 // bring ONE halo slab per tile with TMA and let the four epilogue warps unfold it in
 // shared memory into a dense operand whose rows / columns are (tap, channel):
 //
@@ -385,8 +385,8 @@ conv_c8_fwd_kernel(const __grid_constant__ CUtensorMap tmX, const C8FwdParams p,
 // all four accumulators (the 2 x 2 window in depth and height comes from the four tiles,
 // the one along W from the neighbouring TMEM lane through a shuffle).  Written: the pooled
 // tensor, and one byte per pooled element with the arg-max position in scan order
-// (bits 0-6) and "maximum positive" (bit 7) - the layout pool_bwd_tiled_idx_kernel reads,
-// so the backward pass is the same as for the separate pooling kernel.  Two sets of
+// (bits 0-6) and "maximum positive" (bit 7) - the layout pool_bwd_tiled_idx_kernel and
+// conv_c8_wgrad_pool_kernel read.  Two sets of
 // accumulators alternate between super-tiles.
 // 4-channel pixels, 3 x 3 x 3 filter only.
 struct C8PoolParams {
