@@ -101,6 +101,7 @@ Tensor fp32(const Tensor& t) { return !t.defined() || t.scalar_type() == at::kFl
 // memory that addresses among them point into.
 struct State : torch::CustomClassHolder {
   Tensor w, w2, wgrad, bgrad, scale;
+  Tensor written;            // host flags of gradients that a step's only writer overwrites: set behind the write
   py::object wh, bh, owner;
   std::vector<int64_t> i;
   std::vector<double> f;
@@ -239,14 +240,21 @@ Tensor grad_prep(const Tensor& dy, const Tensor& y, int64_t act, double p, const
   if (!copy) return dy;
   return pitch == C ? g : g.narrow(-1, 0, C);
 }
-// grad[out, in] += dy^T x.  Mini-batches of at most 16 rows make this a rank-K update bound by
-// the read-modify-write of grad (csrc/outer_accum.cu); the rest goes to the tensor cores.
+// grad[out, in] += dy^T x, or = with `overwrite`.  Mini-batches of at most 16 rows make this a rank-K
+// update bound by the read-modify-write of grad (csrc/outer_accum.cu); the rest goes to the tensor
+// cores, in the same tiles and splits either way (the error of a long reduction depends on them).
+constexpr int64_t kTilesAsAdded = 1;
 bool outer_rows(int64_t K) { return K == 1 || K == 2 || K == 4 || K == 8 || K == 16; }
-void weight_grad(const Tensor& dy, const Tensor& x, const Tensor& grad) {
+void weight_grad(const Tensor& dy, const Tensor& x, const Tensor& grad, bool overwrite) {
   const int64_t K = dy.size(0);
+  if (K == 0) {
+    if (overwrite) grad.zero_();
+    return;
+  }
+  const float beta = overwrite ? 0.f : 1.f;
   if (outer_rows(K) && dy.is_contiguous() && x.is_contiguous() && grad.scalar_type() == at::kFloat && grad.is_contiguous() &&
       x.size(1) % 4 == 0 && dy.scalar_type() == x.scalar_type()) {
-    const int rc = lb_outer_accum(dy.data_ptr(), x.data_ptr(), fptr(grad), K, dy.size(1), x.size(1), 1.f, 1.f,
+    const int rc = lb_outer_accum(dy.data_ptr(), x.data_ptr(), fptr(grad), K, dy.size(1), x.size(1), 1.f, beta,
                                   code(x.scalar_type()), stream());
     if (rc != -2) {
       check(rc, "lb_outer_accum");
@@ -254,12 +262,12 @@ void weight_grad(const Tensor& dy, const Tensor& x, const Tensor& grad) {
       return;
     }
   }
-  gemm(dy, x, true, false, grad, grad.scalar_type(), 1.0, 1.0, Tensor(), false, 0, 0.0, 0);
+  gemm(dy, x, true, false, grad, grad.scalar_type(), 1.0, beta, Tensor(), false, 0, 0.0, kTilesAsAdded);
 }
 
 // ----------------------------------------------------------------------------------- linear
 struct LinearNode : torch::autograd::Function<LinearNode> {
-  // state: w = 16-bit weight, wgrad, bgrad; i = {act}; f = {act_param}
+  // state: w = 16-bit weight, wgrad, bgrad, written (may be undefined); i = {act, index into written}; f = {act_param}
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w_leaf, const optional<Tensor>& b_leaf,
                         const c10::intrusive_ptr<State>& s) {
     Tensor x2 = x.reshape({-1, x.size(-1)});
@@ -291,7 +299,8 @@ struct LinearNode : torch::autograd::Function<LinearNode> {
       if (shape.size() != 2) dx = dx.reshape(shape);
     }
     if (s->wgrad.defined()) {
-      weight_grad(outer_rows(dy.size(0)) && !dy.is_contiguous() ? dy.contiguous() : dy, x2, s->wgrad);
+      weight_grad(outer_rows(dy.size(0)) && !dy.is_contiguous() ? dy.contiguous() : dy, x2, s->wgrad, s->written.defined());
+      if (s->written.defined()) s->written.data_ptr<bool>()[s->i[1]] = true;
       mark_ready(s->wh);
     }
     return {dx, Tensor(), Tensor(), Tensor()};
@@ -767,12 +776,13 @@ PYBIND11_MODULE(_lbann_autograd, m) {
   }, NoGil());
   m.def("weight_grad", [](const Tensor& dy, const Tensor& x, const Tensor& grad) {
     at::AutoDispatchBelowAutograd guard;
-    weight_grad(dy, x, grad);
+    weight_grad(dy, x, grad, false);
   }, NoGil());
   m.def("linear", [](const Tensor& x, const Tensor& w_leaf, const optional<Tensor>& b_leaf, const Tensor& w16,
                      const optional<Tensor>& wgrad, const optional<Tensor>& bgrad, const py::object& wh,
-                     const py::object& bh, int64_t act, double act_param) {
-    auto s = make_state(w16, {}, wgrad, bgrad, wh, bh, {act}, {act_param});
+                     const py::object& bh, int64_t act, double act_param, const optional<Tensor>& written, int64_t at) {
+    auto s = make_state(w16, {}, wgrad, bgrad, wh, bh, {act, at}, {act_param});
+    s->written = opt(written);
     py::gil_scoped_release nogil;
     return LinearNode::apply(x, w_leaf, b_leaf, s);
   });

@@ -135,6 +135,7 @@ int gemm_pair_launch(const void* A, const void* B, void* C, const float* bias, i
                      int bias_mode, int act, float act_param, cudaStream_t stream);
 
 constexpr int kPairHint = 512;
+constexpr int kAsAddedHint = 1;       // the choice of an output that is added to
 
 // The tile with the shortest estimate: 256 x 256 on a pair of SMs (kPairHint) or 128 x 256 / 128 /
 // 64 on one.  Per wave of tiles an estimate is k-steps (64 each) x cycles + what the last tile's
@@ -239,7 +240,7 @@ int lb_gemm_bcast_tc(const void* A, const void* B, void* C, const float* bias, i
                        (beta == 0.f || (beta == 1.f && out_dtype == kF32 && act == kActNone));
   int BN = bn_hint;
   if (BN != 64 && BN != 128 && BN != 256 && !(BN == kPairHint && pair_ok))
-    BN = gemm_choose(M, N, K, batch, offer, pair_ok, beta != 0.f,
+    BN = gemm_choose(M, N, K, batch, offer, pair_ok, beta != 0.f || bn_hint == kAsAddedHint,
                      (reinterpret_cast<uintptr_t>(C) & 15) == 0 && ldc * es % 16 == 0, out_dtype == kF32);
   if (BN == kPairHint) {
     const int rc = gemm_pair_launch(A, B, C, bias, M, N, K, batch, lda, ldb, ldc, strideA, strideB, strideC, a_mn, b_mn,

@@ -100,6 +100,7 @@ class ExecModel:
         self._gen = None
         self.sync_layers = False       # debugging: synchronise after every layer
         self._graph_mode = None        # decided at the first training step
+        self._overwrite_cache = None   # (layers, handles), see _overwritten_gradients
         self._graphs = {}
         self.layer_timing = False
         self.is_setup = False
@@ -671,6 +672,36 @@ class ExecModel:
     def clear_gradients(self):
         self.arena.zero_grad()
 
+    _OVERWRITE_MIN = 1 << 20      # elements; below that filling and reading back take under a microsecond
+
+    def _overwritten_gradients(self):
+        """Handles of the large weights whose gradient has one writer in a step, the native
+        fully-connected backward, which can then overwrite the buffer instead of adding to zeros.
+        Steps of one rank only, and none where a callback may look at gradients in between."""
+        from ..callbacks.base import ExecCallback
+        if self.device.type != "cuda" or self.parallel is not None or self.distconv is not None:
+            return []
+        if any(getattr(type(cb), h, None) is not getattr(ExecCallback, h) for cb in self.callbacks
+               for h in self._IN_STEP_HOOKS):
+            return []
+        key = tuple(id(l) for l in self.layers)
+        if self._overwrite_cache is None or self._overwrite_cache[0] != key:
+            uses = defaultdict(int)
+            for l in self.layers:
+                for w in l.weights:
+                    uses[id(w)] += 1
+            found = []
+            for l in self.layers:
+                if l.type not in ("fully_connected", "channelwise_fully_connected") or l.transpose:
+                    continue
+                h, g = l.w.handle, l.w.handle.grad
+                if (uses[id(l.w)] == 1 and not l.w.sharded and g is not None and g.dtype == torch.float32
+                        and g.numel() >= self._OVERWRITE_MIN and g.is_contiguous()
+                        and g.untyped_storage().data_ptr() == self.arena.grad.untyped_storage().data_ptr()):
+                    found.append(h)
+            self._overwrite_cache = (key, found)
+        return self._overwrite_cache[1]
+
     def sync_optimizer_state(self):
         """Collective over the trainer: optimizer state that the ranks hold in shards (the
         sharded update of data-parallel GPU runs) becomes whole on every rank."""
@@ -728,6 +759,7 @@ class ExecModel:
                 (local_obj * self._amp_device_state()[0]).backward()     # no host read of the scale
             else:
                 (local_obj * self._amp_scale_host).backward()
+        self.arena.end_gradients()
         if self.parallel is not None:
             self.parallel.sync_gradients(self)
         for cb in self.callbacks:
@@ -961,7 +993,7 @@ class ExecModel:
         pt = self._phase_timer
         if pt is not None:
             pt.mark("start")
-        self.clear_gradients()
+        self.arena.begin_gradients(self._overwritten_gradients())
         for cb in self.callbacks:
             cb.on_forward_prop_begin(self, "training")
         self.forward_prop(inputs, "training", global_mini_batch_size, mini_batch_offset)

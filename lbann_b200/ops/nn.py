@@ -125,6 +125,13 @@ class WeightHandle:
         self.compute16 = compute16      # kept in sync by the fused optimizer when present
         self.version = 0
         self._cache = {}
+        # (host flags, index) while ``grad`` holds an earlier step's values: the step's only writer
+        # overwrites it instead of adding, and sets its flag (see ParameterArena.begin_gradients)
+        self.overwrite = None
+
+    def take_overwrite(self):
+        o, self.overwrite = self.overwrite, None
+        return o if o is not None else (None, 0)
 
     def bump(self):
         self.version += 1
@@ -220,7 +227,12 @@ def linear(x, wh: WeightHandle, bh: Optional[WeightHandle] = None, act: int = na
         b = bh is not None
         return native.nodes().linear(x, wh.master, bh.master if b else None, wh.cast(x.dtype),
                                      None if wh.grad is None else wh.grad.view(wh.master.shape),
-                                     bh.grad if b else None, wh, bh, act, float(act_param))
+                                     bh.grad if b else None, wh, bh, act, float(act_param),
+                                     *(wh.take_overwrite() if torch.is_grad_enabled() else (None, 0)))
+    if wh.overwrite is not None:             # autograd adds to the gradient
+        flags, at = wh.take_overwrite()
+        wh.grad.zero_()
+        flags[at] = True
     w = wh.master if wh.master.dtype == x.dtype else wh.master.to(x.dtype)
     b = None if bh is None else (bh.master if bh.master.dtype == x.dtype else bh.master.to(x.dtype))
     y = F.linear(x, w, b)

@@ -141,6 +141,10 @@ class ParameterArena:
         self.shard: Optional[ArenaShard] = None   # set when the update is sharded over ranks
         self.state_compact = False    # optimizer state stored for the owned blocks only
         self._full_state = None       # [state0, state1] at full size while a gathered copy is in use
+        self._overwritten = []        # weight handles whose gradient this step overwrites
+        self._begin_key = None
+        self._begin_rest = []
+        self._written = None          # host flags of _overwritten: written by this step's backward
 
     # ---- layout
     def reserve(self, name: str, shape) -> Slot:
@@ -257,7 +261,44 @@ class ParameterArena:
             self.compute.copy_(self.master)
 
     def zero_grad(self):
+        for h in self._overwritten:
+            h.overwrite = None
+        self._overwritten = []
         self.grad.zero_()
+
+    def begin_gradients(self, handles) -> None:
+        """``zero_grad`` for a step in which each of ``handles`` (weights of this arena) has one
+        writer that can overwrite instead of add: their buffers, most of a fully-connected model's
+        arena, are neither filled nor read back.  ``end_gradients`` clears those that the step did
+        not write after all."""
+        if not handles:
+            return self.zero_grad()
+        key = tuple(id(h) for h in handles)
+        if self._begin_key != key:
+            at, rest = 0, []
+            for lo, n in sorted((h.grad.storage_offset() - self.grad.storage_offset(), h.grad.numel()) for h in handles):
+                if lo > at:
+                    rest.append(self.grad[at:lo])
+                at = lo + n
+            if at < self.grad.numel():
+                rest.append(self.grad[at:])
+            self._begin_key, self._begin_rest = key, rest
+            self._written = torch.zeros(len(handles), dtype=torch.bool)
+        if self._begin_rest:
+            torch._foreach_zero_(self._begin_rest)
+        self._written.zero_()
+        self._overwritten = list(handles)
+        for i, h in enumerate(handles):
+            h.overwrite = (self._written, i)
+
+    def end_gradients(self) -> None:
+        if not self._overwritten:
+            return
+        for h, done in zip(self._overwritten, self._written.tolist()):
+            if not done:             # the layer was not on a path of this step's backward
+                h.grad.zero_()
+            h.overwrite = None
+        self._overwritten = []
 
     def gather_sharded_state(self, allreduce_sum) -> None:
         """Make the optimizer state whole on every rank after sharded steps (checkpoints,

@@ -164,3 +164,54 @@ def test_kfac_on_gpu_beats_plain_sgd():
     second = _fit(kfac, cuda=True)
     assert native.consume_status() == 0
     assert math.isfinite(second) and second < plain, (plain, second)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_overwritten_gradients_equal_accumulated_ones(graph, monkeypatch):
+    """Fully-connected gradients with one writer are overwritten instead of cleared and added to: the same
+    gradients and weights after several steps, with a weight that two layers share and one that no objective
+    reaches (cleared: it has stale values, then zeros)."""
+    from lbann_b200.exec.model import ExecModel
+
+    def run(least):
+        monkeypatch.setattr(ExecModel, "_OVERWRITE_MIN", least)
+        o = opts.reset()
+        o.set("default_dtype", "bf16")
+        o.set("use_cuda_graph", graph)
+        x = lbann.Input(data_field="samples")
+        target = lbann.Input(data_field="responses")
+        shared = lbann.Weights(name="shared", initializer=lbann.HeNormalInitializer())
+        h = lbann.Relu(lbann.FullyConnected(x, num_neurons=40, has_bias=True, name="first"))
+        h = lbann.FullyConnected(h, num_neurons=40, has_bias=False, weights=[shared], name="a")
+        h = lbann.FullyConnected(h, num_neurons=40, has_bias=False, weights=[shared], name="b")
+        lbann.FullyConnected(h, num_neurons=16, has_bias=False, name="aside")
+        y = lbann.FullyConnected(h, num_neurons=4, has_bias=True, name="last")
+        loss = lbann.MeanSquaredError(y, target)
+        model = lbann.Model(1, layers=lbann.traverse_layer_graph(x), objective_function=loss)
+        exp = lbann.proto.serialize.build_experiment(
+            trainer=lbann.Trainer(mini_batch_size=8, random_seed=3), model=model,
+            data_reader=_reader(8, [24], "samples:normal responses:normal", response_dims=[4]),
+            optimizer=lbann.SGD(learn_rate=1e-3, momentum=0.9))
+        tr = ExecTrainer(exp)
+        m = tr.build_model(exp.model)
+        m.weights_by_name["aside_linearity_weights"].gradient.fill_(3.0)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        outs = []
+        for step in range(6):
+            rows = 8 if step != 5 else 5
+            batch = {"samples": torch.randn(rows, 24, generator=g, device="cuda"),
+                     "responses": torch.randn(rows, 4, generator=g, device="cuda")}
+            m.train_step(batch, rows)
+            outs += [t.clone() for w in m.weights for t in (w.gradient, w.values)]
+            assert not m.weights_by_name["aside_linearity_weights"].gradient.any()
+        names = {id(w.handle): w.name for w in m.weights}
+        found = {names[id(h)] for h in m._overwritten_gradients()}
+        tr.shutdown()
+        assert native.consume_status() == 0
+        return outs, found
+
+    want, none = run(1 << 40)
+    got, found = run(1)
+    assert not none and found == {"first_linearity_weights", "aside_linearity_weights", "last_linearity_weights"}
+    for a, b in zip(want, got):
+        assert torch.isfinite(a).all() and torch.equal(a, b)
