@@ -270,3 +270,44 @@ def test_conv_wgrad_sums_in_parts(case, bricks):
             ref += dy[n].reshape(-1, K).double().t() @ xp[n, a:a + D, b:b + H, c:c + W].reshape(-1, C).double()
         err = float((got[:, :, a, b, c].double() - ref).norm() / ref.norm())
         assert err < 1.2e-9 * 64 * bricks + 1e-7, err
+
+
+@pytest.mark.parametrize("case", [
+    # N, C, D, H, W, K, k, padding along depth: sizes that take their taps from halo slabs
+    (8, 32, 9, 17, 64, 64, 3, 1),       # 3 x 2 accumulators of four planes and lines, one of the last plane's columns
+    (16, 32, 13, 26, 60, 64, 3, 0),     # bricks that hang over the width, halo planes that come with the input
+    (4, 24, 6, 40, 24, 40, 3, 1),       # a part of a channel slice; groups of eight pixels from two lines
+    (2, 16, 8, 33, 40, 24, 3, 1),       # eight taps an accumulator
+    (16, 64, 1, 56, 56, 64, 3, 0),      # 2-D, pairs of taps
+    (8, 96, 1, 31, 70, 56, 3, 0),       # two channel blocks, a ragged one; ragged filters
+    (8, 64, 32, 32, 32, 128, 3, 1),     # more accumulators than one CTA holds
+    (24, 32, 1, 45, 33, 32, 5, 0),      # five taps a line: one accumulator and one tap over
+    (64, 64, 1, 40, 40, 64, 5, 0),
+    (1, 8, 5, 64, 100, 8, 3, 1),        # 8 channels, 8 filters
+])
+def test_conv_wgrad_from_slabs(case):
+    """fp16 and bf16, added to what the gradient holds.  An accumulator takes at most 56 bricks' worth of 64
+    pixels here, 1.2e-9 of the result a term (test_conv_wgrad_sums_in_parts), and 4e-7 go to the sums of the
+    parts and to adding them: 4.7e-6."""
+    from lbann_b200.ops.conv import conv_wgrad
+    N, C, D, H, W, K, k, pad_d = case
+    ks = (1 if D == 1 else k, k, k)
+    pd = (pad_d if D > 1 else 0, k // 2, k // 2)
+    Do = D + 2 * pd[0] - ks[0] + 1
+    geom = (ctypes.c_int * 21)(N, D, H, W, C, Do, H, W, K, *ks, *pd, 1, 1, 1, 1, 1, 1)
+    assert native.cuda_lib().lb_conv_wgrad_slab(geom) == 1 or native.cuda_lib().lb_sm_count() != 148
+    for dtype in (torch.bfloat16, torch.float16):
+        torch.manual_seed(11)
+        x = torch.randn(N, D, H, W, C, device="cuda").to(dtype)
+        dy = torch.randn(N, Do, H, W, K, device="cuda").to(dtype)
+        prev = torch.randn(K, C, *ks, device="cuda")
+        got = conv_wgrad(x, dy, ks, pad=pd, out=prev.clone(), alpha=0.5)
+        assert native.consume_status() == 0
+        xp = F.pad(x.double(), (0, 0, pd[2], pd[2], pd[1], pd[1], pd[0], pd[0]))
+        ref = torch.empty(K, C, *ks, device="cuda", dtype=torch.double)
+        for a in range(ks[0]):
+            for b in range(ks[1]):
+                for c in range(ks[2]):
+                    view = xp[:, a:a + Do, b:b + H, c:c + W].reshape(-1, C)
+                    ref[:, :, a, b, c] = prev[:, :, a, b, c].double() + 0.5 * (dy.double().reshape(-1, K).t() @ view)
+        assert float((got.double() - ref).norm() / ref.norm()) < 4.7e-6
