@@ -12,6 +12,7 @@
 //   bn_finalize_apply -> mean/var/running stats, y = (x-mean)*rsqrt(var+eps)*scale+bias
 //   bn_bwd_sums       -> dscale, dbias, dmean, dvar partials; bn_bwd_apply -> dx
 // Instance norm reuses the batch-norm kernels with one "batch" per sample.
+#include <algorithm>
 #include <initializer_list>
 
 #include "common.cuh"
@@ -227,19 +228,24 @@ layer_norm_param_grad8_kernel(const T* __restrict__ x, const T* __restrict__ dy,
   }
 }
 
-// Layer norm of 16-bit rows of up to 8192 columns (a multiple of 8): a team of 1, 2, 4 or 8 warps
-// owns a row and keeps it in registers, V 16-byte vectors a lane, so x (and dy) are read once
-// and every load of a row is in flight at the same time; rows of up to 128 columns take LANES = 8 or 16
-// lanes of a warp each.  Backward makes dx and the column sums for scale and bias in the same pass: a
-// lane keeps the sums of its 8 V columns over all rows of its team, the teams of a block meet in shared
-// memory, and one 16-byte atomic per four columns and block follows.  V = 4 for long rows; one vector a
-// lane leaves more rows in flight where that is all a row has, and more warps to a row, with
-// a quarter of the block's closing sums, where there are few rows (ln_plan).
-// 4096 x 1024 bf16, in L2 (one thread per column, two passes, before): forward 13 -> 8 us, backward
-// 17 + 17 -> 23 us.  With four vectors and 32 lanes for every row, and with the plan below: 262144 x 64
-// 152 / 217 -> 26 / 34 us (column kernels 132 / 189), 16 x 1024 10 / 17 -> 7 / 7 (10 / 15).
+// Layer norm of 16-bit rows of up to 8192 columns (a multiple of 8), rows in registers, so x (and dy) are
+// read once and every load of a row is in flight at the same time.  A team of 1, 2, 4 or 8 warps of a
+// block of eight owns a row, V 16-byte vectors a lane; rows of up to 128 columns take LANES = 8 or 16 lanes of
+// a warp each.  V = 2 or 4 for long rows; one vector a lane leaves more rows in flight where that is
+// all a row has, and more warps to a row where there are few rows (ln_plan).  16384 x 512 forward with V = 4
+// 13.9 us, with V = 2 11.1.
+// Backward makes dx and the column sums for scale and bias in the same pass: a lane keeps the sums of its
+// eight columns over all rows that pass it, the teams of a block meet in shared memory, and one 16-byte
+// atomic per four columns and block follows.  Short and few rows as above, V = 1; many rows of several
+// warps in bands: a team takes R rows at a time, their loads are in flight together, their sums meet in
+// one exchange of shuffles and ONE barrier of the team.  (A long row in one warp, four vectors a lane, kept
+// 64 registers of closing sums in 16 warps an SM that each waited for one row, and closed with eight
+// barriers: 4096 x 1024 bf16 17.8 us, in bands 8.5; 65536 x 1024 169 / 106, 16384 x 512 25.6 / 11.7,
+// 1000 x 4096 17.2 / 12.9.)
+// Against four vectors and 32 lanes for every row: 262144 x 64 152 / 217 -> 26 / 34 us (column
+// kernels 132 / 189), 16 x 1024 10 / 17 -> 7 / 7 (10 / 15).
 constexpr int kLnVecs = 4;                   // vectors of eight columns per lane, at most
-constexpr int kLnMaxCols = 8 * 32 * 8 * kLnVecs;
+constexpr int kLnMaxCols = 8192;
 
 // Sum over the team's lanes of two values; `sm`: one float2 per warp.  With more than one warp the
 // whole block calls it the same number of times.
@@ -270,7 +276,7 @@ __device__ __forceinline__ void ln_ld8f(const float* p, float (&f)[8]) {
 }
 
 template <typename T, int V, int LANES>
-__global__ void __launch_bounds__(256, V == 1 ? 4 : 2)
+__global__ void __launch_bounds__(256, V == 1 ? 4 : V == 2 ? 3 : 2)
 layer_norm_fwd_rows_kernel(const T* __restrict__ x, const float* __restrict__ scale, const float* __restrict__ bias,
                            T* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out,
                            long long rows, int cols, float eps, int team_warps) {
@@ -333,8 +339,8 @@ layer_norm_fwd_rows_kernel(const T* __restrict__ x, const float* __restrict__ sc
   }
 }
 
-template <typename T, int V, int LANES>
-__global__ void __launch_bounds__(256, V == 1 ? 4 : 2)
+template <typename T, int LANES>
+__global__ void __launch_bounds__(256, 4)
 layer_norm_bwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ dy, const float* __restrict__ scale,
                            const float* __restrict__ mean_in, const float* __restrict__ rstd_in, T* __restrict__ dx,
                            float* __restrict__ dscale, float* __restrict__ dbias, long long rows, int cols,
@@ -343,38 +349,26 @@ layer_norm_bwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ dy, co
   __shared__ __align__(16) float part[8][32][8];
   constexpr int kPerWarp = 32 / LANES;                 // rows of a warp
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, teams = 8 * kPerWarp / team_warps;
-  const int v0 = (warp % team_warps) * 32 + (lane & (LANES - 1)), vstep = 32 * team_warps, cv = cols / 8;
-  float ds[V][8], db[V][8];
+  const int v = (warp % team_warps) * 32 + (lane & (LANES - 1)), cv = cols / 8;
+  float ds[8], db[8];
 #pragma unroll
-  for (int k = 0; k < V; ++k)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ds[k][j] = db[k][j] = 0.f;
+  for (int j = 0; j < 8; ++j) ds[j] = db[j] = 0.f;
   for (long long r0 = (long long)blockIdx.x * teams; r0 < rows; r0 += (long long)gridDim.x * teams) {
     const long long r = r0 + warp / team_warps * kPerWarp + lane / LANES;
-    const bool live = r < rows;
-    uint4 qx[V], qg[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-      const int v = v0 + k * vstep;
-      const bool on = live && v < cv;
-      qx[k] = on ? *reinterpret_cast<const uint4*>(x + r * cols + v * 8) : make_uint4(0, 0, 0, 0);
-      qg[k] = on ? *reinterpret_cast<const uint4*>(dy + r * cols + v * 8) : make_uint4(0, 0, 0, 0);
-    }
+    const bool live = r < rows, on = live && v < cv;
+    const uint4 qx = on ? *reinterpret_cast<const uint4*>(x + r * cols + v * 8) : make_uint4(0, 0, 0, 0);
+    const uint4 qg = on ? *reinterpret_cast<const uint4*>(dy + r * cols + v * 8) : make_uint4(0, 0, 0, 0);
+    const T* ex = reinterpret_cast<const T*>(&qx);
+    const T* eg = reinterpret_cast<const T*>(&qg);
     const float mean = live ? mean_in[r] : 0.f, rstd = live ? rstd_in[r] : 0.f;
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int k = 0; k < V; ++k) {
-      const int v = v0 + k * vstep;
-      if (v >= cv) continue;
-      const T* ex = reinterpret_cast<const T*>(&qx[k]);
-      const T* eg = reinterpret_cast<const T*>(&qg[k]);
-      float c[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+    float s1 = 0.f, s2 = 0.f, c[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+    if (v < cv) {
       if (scale) ln_ld8f(scale + v * 8, c);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float xh = (to_f32<T>(ex[j]) - mean) * rstd, gy = to_f32<T>(eg[j]);
-        ds[k][j] += gy * xh;
-        db[k][j] += gy;
+        ds[j] += gy * xh;
+        db[j] += gy;
         const float g = gy * c[j];
         s1 += g;
         s2 += g * xh;
@@ -383,83 +377,225 @@ layer_norm_bwd_rows_kernel(const T* __restrict__ x, const T* __restrict__ dy, co
     ln_team_sum<LANES>(s1, s2, team_warps, sm);
     s1 /= cols;
     s2 /= cols;
-    if (!live) continue;
+    if (!on) continue;
+    float o[8];
 #pragma unroll
-    for (int k = 0; k < V; ++k) {
-      const int v = v0 + k * vstep;
-      if (v >= cv) continue;
-      const T* ex = reinterpret_cast<const T*>(&qx[k]);
-      const T* eg = reinterpret_cast<const T*>(&qg[k]);
-      float o[8], c[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-      if (scale) ln_ld8f(scale + v * 8, c);
+    for (int j = 0; j < 8; ++j) {
+      const float xh = (to_f32<T>(ex[j]) - mean) * rstd;
+      const float g = to_f32<T>(eg[j]) * c[j];
+      o[j] = (g - s1 - xh * s2) * rstd;
+    }
+    st8n<T>(dx + r * cols + v * 8, o);
+  }
+  // the teams of the block, one of the two sums at a time
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = (to_f32<T>(ex[j]) - mean) * rstd;
-        const float g = to_f32<T>(eg[j]) * c[j];
-        o[j] = (g - s1 - xh * s2) * rstd;
-      }
-      st8n<T>(dx + r * cols + v * 8, o);
+  for (int which = 0; which < 2; ++which) {
+    float* out = which ? dbias : dscale;
+    if (!out) continue;                                // the same for the whole block
+    __syncthreads();
+    float4* d = reinterpret_cast<float4*>(part[warp][lane]);
+    const float(&a)[8] = which ? db : ds;
+    d[0] = make_float4(a[0], a[1], a[2], a[3]);
+    d[1] = make_float4(a[4], a[5], a[6], a[7]);
+    __syncthreads();
+    // thread -> (warp of a team, lane, half of its vector)
+    for (int i = threadIdx.x; i < team_warps * 2 * LANES; i += 256) {
+      const int tw = i / (2 * LANES), ln = (i >> 1) & (LANES - 1), half = i & 1;
+      const int vec = tw * 32 + ln;
+      if (vec >= cv) continue;
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int w = tw; w < 8; w += team_warps)
+#pragma unroll
+        for (int sub = 0; sub < kPerWarp; ++sub) {
+          const float4 u = *reinterpret_cast<const float4*>(&part[w][sub * LANES + ln][half * 4]);
+          t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+        }
+      atomicAdd(reinterpret_cast<float4*>(out + vec * 8 + half * 4), t);
     }
   }
-  // the teams of the block, one vector slot and one of the two sums at a time
+}
+
+// NV sums over a team of W warps (a power of two from 2 on): lanes hand over half of the values they
+// still have in each step, so that four lanes (NV = 8) end with the warp's sum of one value; the warps
+// meet in shared memory.  `sm` has NV * W floats and alternates between calls: one barrier each.
+template <int NV>
+__device__ __forceinline__ void ln_band_sum(float (&v)[NV], int W, int tw, int lane, int team, float* sm) {
+  int have = NV, index = 0;
 #pragma unroll
-  for (int k = 0; k < V; ++k) {
+  for (int m = 16; m > 0; m >>= 1) {
+    if (m * NV > 16) {                                 // halve the values
+      const bool upper = lane & m;
+      have /= 2;
+#pragma unroll
+      for (int i = 0; i < NV / 2; ++i) {
+        if (i >= have) break;
+        const float give = upper ? v[i] : v[i + have], keep = upper ? v[i + have] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, m);
+      }
+      index += upper ? have : 0;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], m);
+    }
+  }
+  if ((lane & (32 / NV - 1)) == 0) sm[index * W + tw] = v[0];
+  asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "r"(W * 32) : "memory");
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    float t = 0.f;
+    if (W == 2) {
+      const float2 q = *reinterpret_cast<const float2*>(sm + i * 2);
+      t = q.x + q.y;
+    } else {
+      for (int w = 0; w < W; w += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(sm + i * W + w);
+        t += (q.x + q.y) + (q.z + q.w);
+      }
+    }
+    v[i] = t;
+  }
+}
+
+// R rows at a time for a team of W warps; blocks of 256 threads (W <= 8) or, LONG, of one team.
+constexpr int kLnBandR = 4;
+
+template <typename T, bool LONG>
+__global__ void __launch_bounds__(LONG ? 1024 : 256, LONG ? 1 : 2)
+layer_norm_bwd_bands_kernel(const T* __restrict__ x, const T* __restrict__ dy, const float* __restrict__ scale,
+                            const float* __restrict__ mean_in, const float* __restrict__ rstd_in, T* __restrict__ dx,
+                            float* __restrict__ dscale, float* __restrict__ dbias, long long rows, int cols, int W) {
+  constexpr int R = LONG ? 1 : kLnBandR;
+  __shared__ __align__(16) float sm[2][2 * R * 32];
+  __shared__ __align__(16) float part[LONG ? 4 : 8 * 512];       // sums of a block's teams: [team][2][W * 256]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = warp / W, tw = warp - team * W;
+  const int teams = blockDim.x / (32 * W), v = tw * 32 + lane, cv = cols / 8;
+  const bool on = v < cv;
+  float ds[8], db[8], c[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ds[j] = db[j] = 0.f;
+  if (on && scale) ln_ld8f(scale + v * 8, c);
+  const float inv = 1.f / cols;
+  int turn = 0;
+  for (long long r = ((long long)blockIdx.x * teams + team) * R; r < rows; r += (long long)gridDim.x * teams * R, turn ^= 1) {
+    uint4 qx[R], qg[R];
+    float mean[R], rstd[R], s[2 * R];
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const bool there = on && r + u < rows;
+      qx[u] = there ? *reinterpret_cast<const uint4*>(x + (r + u) * cols + v * 8) : make_uint4(0, 0, 0, 0);
+      qg[u] = there ? *reinterpret_cast<const uint4*>(dy + (r + u) * cols + v * 8) : make_uint4(0, 0, 0, 0);
+      mean[u] = there ? __ldg(mean_in + r + u) : 0.f;
+      rstd[u] = there ? __ldg(rstd_in + r + u) : 0.f;
+    }
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      const T* ex = reinterpret_cast<const T*>(&qx[u]);
+      const T* eg = reinterpret_cast<const T*>(&qg[u]);
+      s[2 * u] = s[2 * u + 1] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (to_f32<T>(ex[j]) - mean[u]) * rstd[u], gy = to_f32<T>(eg[j]);
+        ds[j] += gy * xh;
+        db[j] += gy;
+        const float g = gy * c[j];
+        s[2 * u] += g;
+        s[2 * u + 1] += g * xh;
+      }
+    }
+    ln_band_sum<2 * R>(s, W, tw, lane, team, sm[turn] + team * 2 * R * W);
+    if (!on) continue;
+#pragma unroll
+    for (int u = 0; u < R; ++u) {
+      if (r + u >= rows) break;
+      const T* ex = reinterpret_cast<const T*>(&qx[u]);
+      const T* eg = reinterpret_cast<const T*>(&qg[u]);
+      const float s1 = s[2 * u] * inv, s2 = s[2 * u + 1] * inv;
+      float o[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xh = (to_f32<T>(ex[j]) - mean[u]) * rstd[u];
+        o[j] = (to_f32<T>(eg[j]) * c[j] - s1 - xh * s2) * rstd[u];
+      }
+      st8n<T>(dx + (r + u) * cols + v * 8, o);
+    }
+  }
+  if (!dscale && !dbias) return;
+  if (teams == 1) {
 #pragma unroll
     for (int which = 0; which < 2; ++which) {
       float* out = which ? dbias : dscale;
-      if (!out) continue;                              // the same for the whole block
-      __syncthreads();
-      float4* d = reinterpret_cast<float4*>(part[warp][lane]);
-      const float(&a)[8] = which ? db[k] : ds[k];
-      d[0] = make_float4(a[0], a[1], a[2], a[3]);
-      d[1] = make_float4(a[4], a[5], a[6], a[7]);
-      __syncthreads();
-      // thread -> (warp of a team, lane, half of its vector)
-      for (int i = threadIdx.x; i < team_warps * 2 * LANES; i += 256) {
-        const int tw = i / (2 * LANES), ln = (i >> 1) & (LANES - 1), half = i & 1;
-        const int v = tw * 32 + ln + k * vstep;
-        if (v >= cv) continue;
-        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int w = tw; w < 8; w += team_warps)
-#pragma unroll
-          for (int sub = 0; sub < kPerWarp; ++sub) {
-            const float4 u = *reinterpret_cast<const float4*>(&part[w][sub * LANES + ln][half * 4]);
-            t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
-          }
-        atomicAdd(reinterpret_cast<float4*>(out + v * 8 + half * 4), t);
+      const float(&a)[8] = which ? db : ds;
+      if (!out || !on) continue;
+      atomicAdd(reinterpret_cast<float4*>(out + v * 8), make_float4(a[0], a[1], a[2], a[3]));
+      atomicAdd(reinterpret_cast<float4*>(out + v * 8 + 4), make_float4(a[4], a[5], a[6], a[7]));
+    }
+    return;
+  }
+  if constexpr (!LONG) {
+    const int width = W * 256;                         // teams * 2 * width = 4096 floats
+    float4* d = reinterpret_cast<float4*>(part + team * 2 * width + v * 8);
+    d[0] = make_float4(ds[0], ds[1], ds[2], ds[3]);
+    d[1] = make_float4(ds[4], ds[5], ds[6], ds[7]);
+    d[width / 4] = make_float4(db[0], db[1], db[2], db[3]);
+    d[width / 4 + 1] = make_float4(db[4], db[5], db[6], db[7]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < width / 2; i += 256) {
+      const int which = i >= width / 4, col = (i - which * (width / 4)) * 4;
+      float* out = which ? dbias : dscale;
+      if (!out || col >= cols) continue;
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int w = 0; w < teams; ++w) {
+        const float4 u = *reinterpret_cast<const float4*>(part + (w * 2 + which) * width + col);
+        t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
       }
+      atomicAdd(reinterpret_cast<float4*>(out + col), t);
     }
   }
 }
 
 // How the kernels above take a call; team 0: the column kernels take it.
 struct LnPlan {
-  int team, vecs, lanes;
-  int rows_per_block() const { return 8 / team * (32 / lanes); }
+  int team, vecs, lanes;                               // warps of a row, vectors of a lane, lanes of a short row
+  bool bands;                                          // backward
+  int threads() const { return bands && team > 8 ? team * 32 : 256; }
+  int rows_per_block() const {
+    if (!bands) return 8 / team * (32 / lanes);
+    return team > 8 ? 1 : 8 / team * kLnBandR;
+  }
 };
-static LnPlan ln_plan(int dtype, long long rows, int cols, std::initializer_list<const void*> aligned) {
-  LnPlan p = {0, kLnVecs, 32};
+static LnPlan ln_plan(int dtype, long long rows, int cols, bool backward, std::initializer_list<const void*> aligned) {
+  LnPlan p = {0, 1, 32, false};
   if (dtype == kF32 || cols % 8 || cols > kLnMaxCols) return p;
   for (const void* q : aligned)
     if (reinterpret_cast<uintptr_t>(q) & 15) return p;
   int wide = 1;                                        // warps that give a lane one vector
   while (wide * 32 * 8 < cols) wide *= 2;
-  if (wide == 1 || (wide <= 8 && rows * wide <= 8 * 2LL * lbhost::sm_count())) {
-    p.vecs = 1;
-    p.team = wide;
+  p.team = wide;
+  if (wide == 1) {
     p.lanes = cols <= 64 ? 8 : (cols <= 128 ? 16 : 32);
-  } else {
-    p.team = (wide + kLnVecs - 1) / kLnVecs;
+  } else if (wide > 8 || rows * wide > 8 * 2LL * lbhost::sm_count()) {      // fewer rows: more warps to a row
+    p.bands = backward;
+    p.vecs = backward ? 1 : std::min(wide, kLnVecs);
+    p.team = wide / p.vecs;
   }
   return p;
 }
 
-#define LB_LN_LAUNCH(KERNEL, T, GRID, ...)                                                    \
+#define LB_LN_FWD(T, GRID, ...)                                                               \
   {                                                                                           \
-    if (plan.vecs == kLnVecs) KERNEL<T, kLnVecs, 32><<<GRID, 256, 0, s>>>(__VA_ARGS__);       \
-    else if (plan.lanes == 32) KERNEL<T, 1, 32><<<GRID, 256, 0, s>>>(__VA_ARGS__);            \
-    else if (plan.lanes == 16) KERNEL<T, 1, 16><<<GRID, 256, 0, s>>>(__VA_ARGS__);            \
-    else KERNEL<T, 1, 8><<<GRID, 256, 0, s>>>(__VA_ARGS__);                                   \
+    if (plan.vecs == 4) layer_norm_fwd_rows_kernel<T, 4, 32><<<GRID, 256, 0, s>>>(__VA_ARGS__);       \
+    else if (plan.vecs == 2) layer_norm_fwd_rows_kernel<T, 2, 32><<<GRID, 256, 0, s>>>(__VA_ARGS__);  \
+    else if (plan.lanes == 32) layer_norm_fwd_rows_kernel<T, 1, 32><<<GRID, 256, 0, s>>>(__VA_ARGS__);\
+    else if (plan.lanes == 16) layer_norm_fwd_rows_kernel<T, 1, 16><<<GRID, 256, 0, s>>>(__VA_ARGS__);\
+    else layer_norm_fwd_rows_kernel<T, 1, 8><<<GRID, 256, 0, s>>>(__VA_ARGS__);               \
+  }
+#define LB_LN_BWD(T, GRID, ...)                                                               \
+  {                                                                                           \
+    if (plan.bands && plan.team > 8)                                                          \
+      layer_norm_bwd_bands_kernel<T, true><<<GRID, plan.threads(), 0, s>>>(__VA_ARGS__);      \
+    else if (plan.bands) layer_norm_bwd_bands_kernel<T, false><<<GRID, 256, 0, s>>>(__VA_ARGS__);     \
+    else if (plan.lanes == 32) layer_norm_bwd_rows_kernel<T, 32><<<GRID, 256, 0, s>>>(__VA_ARGS__);   \
+    else if (plan.lanes == 16) layer_norm_bwd_rows_kernel<T, 16><<<GRID, 256, 0, s>>>(__VA_ARGS__);   \
+    else layer_norm_bwd_rows_kernel<T, 8><<<GRID, 256, 0, s>>>(__VA_ARGS__);                  \
   }
 
 // ------------------------------- batch norm ---------------------------------
@@ -752,11 +888,11 @@ int lb_layer_norm_fwd(const void* x, const float* scale, const float* bias, void
                       float* rstd, long long rows, int cols, float eps, int dtype, void* stream_) {
   using namespace lb;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  if (const LnPlan plan = ln_plan(dtype, rows, cols, {x, y, scale, bias}); plan.team) {
+  if (const LnPlan plan = ln_plan(dtype, rows, cols, false, {x, y, scale, bias}); plan.team) {
     const int per = plan.rows_per_block();
     const long long need = (rows + per - 1) / per, most = (long long)lbhost::sm_count() * 8;
     const int blocks = (int)(need < most ? need : most);
-    LB_DISPATCH_16(dtype, LB_LN_LAUNCH(layer_norm_fwd_rows_kernel, T, blocks, (const T*)x, scale, bias, (T*)y, mean,
+    LB_DISPATCH_16(dtype, LB_LN_FWD(T, blocks, (const T*)x, scale, bias, (T*)y, mean,
                                        rstd, rows, cols, eps, plan.team));
     return (int)cudaGetLastError();
   }
@@ -774,11 +910,11 @@ int lb_layer_norm_bwd(const void* x, const void* dy, const float* scale, const f
                       int cols, int dtype, void* stream_) {
   using namespace lb;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
-  if (const LnPlan plan = ln_plan(dtype, rows, cols, {x, dy, dx, scale, dscale, dbias}); plan.team) {
+  if (const LnPlan plan = ln_plan(dtype, rows, cols, true, {x, dy, dx, scale, dscale, dbias}); plan.team) {
     const int per = plan.rows_per_block();
-    const long long need = (rows + per - 1) / per, most = (long long)lbhost::sm_count() * (plan.vecs == 1 ? 4 : 2);
+    const long long need = (rows + per - 1) / per, most = (long long)lbhost::sm_count() * (!plan.bands ? 4 : plan.team > 8 ? 1 : 2);
     const int blocks = (int)(need < most ? need : most);       // all resident
-    LB_DISPATCH_16(dtype, LB_LN_LAUNCH(layer_norm_bwd_rows_kernel, T, blocks, (const T*)x, (const T*)dy, scale, mean,
+    LB_DISPATCH_16(dtype, LB_LN_BWD(T, blocks, (const T*)x, (const T*)dy, scale, mean,
                                        rstd, (T*)dx, dscale, dbias, rows, cols, plan.team));
     return (int)cudaGetLastError();
   }
