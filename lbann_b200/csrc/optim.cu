@@ -33,7 +33,7 @@ struct OptSegment {
   float p1;           //                     Adam: beta2
   float eps;
   float wd;           // Adam: decoupled weight decay coefficient (multiplied by lr)
-  float corr;         // unused on entry; the kernel derives it from the device step counter
+  float corr;         // Adam: lr times the bias correction, set on the device (opt_begin_step_kernel)
   float l2;           // L2 regularisation coefficient folded into the gradient (g += l2 * x)
   float pad[3];
 };
@@ -284,13 +284,11 @@ fused_optimizer_vec_kernel(float* __restrict__ w, const G* __restrict__ grad,
   }
 }
 
-// The whole arena on one rank.  Memory-bound (30 bytes an element for Adam with a 16-bit copy),
-// so what counts is loads in flight: a block walks a contiguous run of chunks two at a time, eight
-// 16-byte loads a thread, and looks its segment up (a binary search and, for Adam, two powers) only
-// when it enters another one; once per chunk that chain of dependent loads left the memory idle
-// between chunks.  Four elements a thread and chunk; segments start on chunk boundaries.  A chunk that
-// has no partner (an arena of fewer chunks than blocks, the end of a run or segment) is taken alone, with
-// the same loads (element by element, LeNet's 431080 weights took 8.3 us with Adam instead of 6.4).
+// The whole arena on one rank.  Memory-bound (30 bytes an element for Adam with a 16-bit copy): a block
+// takes ONE chunk, four elements a thread, and its loads go out before anything else; the chunk's segment
+// is found under their latency (Adam's correction, two powers, comes from opt_begin_step_kernel).  Blocks that come and go keep reads and writes in step with the memory: 128 M elements, Adam, 585 us
+// = 6.9 TB/s; resident blocks with strides over the arena took 640 and with a contiguous run each 667
+// (in this kernel's place, with the lookups at the run's segments, 709).
 template <typename G>
 __device__ __forceinline__ void opt_load_grad4(const G* p, float (&g)[4]) {
   if (sizeof(G) == 4) {
@@ -313,84 +311,75 @@ __device__ __forceinline__ void opt_store16(W16* p, float a, float b, float c, f
 }
 
 template <typename G, typename W16>
-__global__ void __launch_bounds__(256, 3)
-fused_optimizer_run_kernel(float* __restrict__ w, const G* __restrict__ grad, float* __restrict__ s0,
-                           float* __restrict__ s1, W16* __restrict__ w16, const OptSegment* __restrict__ segs, int nseg,
-                           long long total, float inv_scale, const int* __restrict__ skip_flag,
-                           const int* __restrict__ step_ptr, const float* __restrict__ lr_scale_ptr,
-                           const float* __restrict__ inv_scale_dev, long long chunks_per_block) {
-  if (skip_flag && *skip_flag) return;
-  if (inv_scale_dev) inv_scale *= *inv_scale_dev;
-  const float step_t = step_ptr ? (float)(*step_ptr) : 1.f;
-  const float lr_mul = lr_scale_ptr ? *lr_scale_ptr : 1.f;
-  const long long nchunks = (total + kOptChunk - 1) / kOptChunk;
-  const long long first = (long long)blockIdx.x * chunks_per_block;
-  const long long last = min(nchunks, first + chunks_per_block);
+__global__ void __launch_bounds__(256)
+fused_optimizer_chunk_kernel(float* __restrict__ w, const G* __restrict__ grad, float* __restrict__ s0,
+                             float* __restrict__ s1, W16* __restrict__ w16, const OptSegment* __restrict__ segs, int nseg,
+                             long long total, float inv_scale, const int* __restrict__ skip_flag,
+                             const int* __restrict__ step_ptr, const float* __restrict__ lr_scale_ptr,
+                             const float* __restrict__ inv_scale_dev) {
+  const long long base = (long long)blockIdx.x * kOptChunk, i = base + 4 * (long long)threadIdx.x;
   const bool has_s1 = s1 != s0;
-  OptSegment sg;
-  long long next = -1, end = 0;               // where the next segment begins, this one's elements end
-  // four elements from i on of n (one or two) chunks: every load comes first.  Frozen: the 16-bit copy only.
-  auto update = [&](int n, long long i) {
-    float4 x[2], a0[2], a1[2];
-    float g[2][4];
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f), a0 = x, a1 = x;
+  float g[4] = {0.f, 0.f, 0.f, 0.f};
+  if (i + 4 <= total) {                          // what lies behind a segment in its last chunk is the arena's too
+    x = *reinterpret_cast<const float4*>(w + i);
+    opt_load_grad4<G>(grad + i, g);
+    a0 = *reinterpret_cast<const float4*>(s0 + i);
+    if (has_s1) a1 = *reinterpret_cast<const float4*>(s1 + i);
+  }
+  const float lr_mul = lr_scale_ptr ? *lr_scale_ptr : 1.f;
+  if (inv_scale_dev) inv_scale *= *inv_scale_dev;
+  const bool skip = skip_flag && *skip_flag;
+  // the last segment that begins here or before: all offsets at once, not one by one
+  int before = 0;
+  for (int t = 0; t < nseg; t += 256)
+    before += __syncthreads_count(t + (int)threadIdx.x < nseg && segs[t + threadIdx.x].offset <= base);
+  if (skip) return;
+  OptSegment sg = segs[max(before, 1) - 1];
+  sg.lr *= lr_mul;
+  if (sg.kind == kOptAdam && sg.corr == 0.f) {   // a table that opt_begin_step_kernel has not seen
+    const float step_t = step_ptr ? (float)(*step_ptr) : 1.f;
+    sg.corr = sg.lr * sqrtf(1.f - powf(sg.p1, step_t)) / (1.f - powf(sg.p0, step_t));
+  }
+  const long long end = min(sg.offset + sg.count, total);
+  if (i + 4 <= end) {
+    float xs[4] = {x.x, x.y, x.z, x.w};
+    if (sg.kind >= 0) {                          // frozen: the 16-bit copy only
+      float m0[4] = {a0.x, a0.y, a0.z, a0.w}, m1[4] = {a1.x, a1.y, a1.z, a1.w};
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u >= n) continue;
-      x[u] = *reinterpret_cast<const float4*>(w + i + u * kOptChunk);
-      if (sg.kind < 0) continue;
-      opt_load_grad4<G>(grad + i + u * kOptChunk, g[u]);
-      a0[u] = *reinterpret_cast<const float4*>(s0 + i + u * kOptChunk);
-      a1[u] = has_s1 ? *reinterpret_cast<const float4*>(s1 + i + u * kOptChunk) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int j = 0; j < 4; ++j) xs[j] = opt_update_one(sg, xs[j], g[j] * inv_scale, m0[j], m1[j]);
+      *reinterpret_cast<float4*>(s0 + i) = make_float4(m0[0], m0[1], m0[2], m0[3]);
+      if (has_s1 && sg.kind == kOptAdam) *reinterpret_cast<float4*>(s1 + i) = make_float4(m1[0], m1[1], m1[2], m1[3]);
+      *reinterpret_cast<float4*>(w + i) = make_float4(xs[0], xs[1], xs[2], xs[3]);
     }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (u >= n) continue;
-      const long long at = i + u * kOptChunk;
-      float xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
-      if (sg.kind >= 0) {
-        float m0[4] = {a0[u].x, a0[u].y, a0[u].z, a0[u].w}, m1[4] = {a1[u].x, a1[u].y, a1[u].z, a1[u].w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) xs[j] = opt_update_one(sg, xs[j], g[u][j] * inv_scale, m0[j], m1[j]);
-        *reinterpret_cast<float4*>(s0 + at) = make_float4(m0[0], m0[1], m0[2], m0[3]);
-        if (has_s1 && sg.kind == kOptAdam)
-          *reinterpret_cast<float4*>(s1 + at) = make_float4(m1[0], m1[1], m1[2], m1[3]);
-        *reinterpret_cast<float4*>(w + at) = make_float4(xs[0], xs[1], xs[2], xs[3]);
-      }
-      if (w16) opt_store16(w16 + at, xs[0], xs[1], xs[2], xs[3]);
-    }
-  };
-  for (long long ch = first; ch < last;) {
-    const long long base = ch * kOptChunk;
-    if (base >= next) {
-      const int si = find_segment(segs, nseg, base);
-      sg = segs[si];
-      next = si + 1 < nseg ? segs[si + 1].offset : total;
-      if (next <= base) next = base + kOptChunk;      // behind the last segment
-      sg.lr *= lr_mul;
-      if (sg.kind == kOptAdam)
-        sg.corr = sg.lr * sqrtf(1.f - powf(sg.p1, step_t)) / (1.f - powf(sg.p0, step_t));
-      end = min(sg.offset + sg.count, total);
-    }
-    const long long i = base + 4 * (long long)threadIdx.x;
-    // two chunks where both are whole; else one, whose elements may end inside a thread's four
-    const int n = ch + 2 <= last && base + 2 * kOptChunk <= end ? 2 : 1;
-    ch += n;
-    if (i + 4 <= end) {
-      update(n, i);
-      continue;
-    }
+    if (w16) opt_store16(w16 + i, xs[0], xs[1], xs[2], xs[3]);
+    return;
+  }
 #pragma unroll 1
-    for (long long j = i; j < end; ++j) {
-      float x = w[j];
-      if (sg.kind >= 0) {
-        float m0 = s0[j], m1 = has_s1 ? s1[j] : 0.f;
-        x = opt_update_one(sg, x, to_f32<G>(grad[j]) * inv_scale, m0, m1);
-        s0[j] = m0;
-        if (has_s1 && sg.kind == kOptAdam) s1[j] = m1;
-        w[j] = x;
-      }
-      if (w16) w16[j] = from_f32<W16>(x);
+  for (long long j = i; j < end; ++j) {          // the segment ends inside this thread's four
+    float v = w[j];
+    if (sg.kind >= 0) {
+      float m0 = s0[j], m1 = has_s1 ? s1[j] : 0.f;
+      v = opt_update_one(sg, v, to_f32<G>(grad[j]) * inv_scale, m0, m1);
+      s0[j] = m0;
+      if (has_s1 && sg.kind == kOptAdam) s1[j] = m1;
+      w[j] = v;
     }
+    if (w16) w16[j] = from_f32<W16>(v);
+  }
+}
+
+// Before an update: the step is counted unless AMP skips it, and every Adam segment of the table gets its
+// bias correction times the learning rate, which the kernel above would take from two powers in every block.
+__global__ void opt_begin_step_kernel(OptSegment* __restrict__ segs, int nseg, int* __restrict__ step_ptr,
+                                      const int* __restrict__ skip_flag, const float* __restrict__ lr_scale_ptr) {
+  const int step = *step_ptr + (skip_flag && *skip_flag ? 0 : 1);
+  const float step_t = (float)step, lr_mul = lr_scale_ptr ? *lr_scale_ptr : 1.f;
+  __syncthreads();
+  if (threadIdx.x == 0) *step_ptr = step;
+  for (int t = threadIdx.x; t < nseg; t += blockDim.x) {
+    if (segs[t].kind != kOptAdam) continue;
+    segs[t].corr = segs[t].lr * lr_mul * sqrtf(1.f - powf(segs[t].p1, step_t)) / (1.f - powf(segs[t].p0, step_t));
   }
 }
 
@@ -409,6 +398,36 @@ __global__ void unscale_check_kernel(G* __restrict__ grad, long long n, float in
     if (!isfinite(g)) bad = true;
     if (write_back) grad[i] = from_f32<G>(g);
   }
+  if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
+}
+
+// The check alone on one rank, 16-byte aligned gradients: one block per 4096 elements, four loads of four a
+// thread, from the END of the arena on.  The gradients that backward wrote last are still in the L2,
+// and the optimizer, which starts at the front, finds there what this kernel read last.
+// 35 M fp32 gradients 33 us with a grid of resident blocks and single floats.
+constexpr int kCheckBlock = 4096;
+template <typename G>
+__global__ void __launch_bounds__(256)
+finite_check_kernel(const G* __restrict__ grad, long long n, float inv_scale, const float* __restrict__ inv_scale_dev,
+                    int* __restrict__ flag) {
+  const long long base = (long long)(gridDim.x - 1 - blockIdx.x) * kCheckBlock + 4 * threadIdx.x;
+  float g[4][4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const long long i = base + u * 1024;
+    if (i + 4 <= n) {
+      opt_load_grad4<G>(grad + i, g[u]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) g[u][j] = i + j < n ? to_f32<G>(grad[i + j]) : 0.f;
+    }
+  }
+  if (inv_scale_dev) inv_scale = *inv_scale_dev;
+  bool bad = false;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bad = bad || !isfinite(g[u][j] * inv_scale);
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(flag, 1);
 }
 
@@ -513,6 +532,16 @@ int lb_fused_optimizer(float* w, const void* grad, float* s0, float* s1, void* w
   return (int)cudaGetLastError();
 }
 
+// Counts the step in *step_ptr unless *skip_flag and fills in the table's corrections, before
+// lb_fused_optimizer_sharded2 on the same stream (which computes those that are zero).
+int lb_opt_begin_step(void* segs, int nseg, int* step_ptr, const int* skip_flag, const float* lr_scale_ptr,
+                      void* stream_) {
+  if (nseg <= 0 || !step_ptr) return -1;
+  lb::opt_begin_step_kernel<<<1, 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(
+      reinterpret_cast<lb::OptSegment*>(segs), nseg, step_ptr, skip_flag, lr_scale_ptr);
+  return (int)cudaGetLastError();
+}
+
 int lb_amp_update(float* state, const float* reduced, int* flag, float growth, float backoff,
                   float interval, void* stream_) {
   lb::amp_update_kernel<<<1, 32, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(
@@ -528,6 +557,13 @@ int lb_unscale_check_owned(void* grad, long long n, float inv_scale, const float
   if (n <= 0) return 0;
   if (world < 1 || rank < 0 || rank >= world || own_chunks < 1) return -1;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
+  if (world == 1 && !write_back && (reinterpret_cast<uintptr_t>(grad) & 15) == 0 && n <= (1ll << 40)) {
+    const int blocks = (int)((n + kCheckBlock - 1) / kCheckBlock);
+    if (dtype == kF32) finite_check_kernel<float><<<blocks, 256, 0, s>>>((const float*)grad, n, inv_scale, inv_scale_dev, flag);
+    else if (dtype == kBF16) finite_check_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>((const __nv_bfloat16*)grad, n, inv_scale, inv_scale_dev, flag);
+    else finite_check_kernel<__half><<<blocks, 256, 0, s>>>((const __half*)grad, n, inv_scale, inv_scale_dev, flag);
+    return (int)cudaGetLastError();
+  }
   const int grid = flat_grid(n, 2048);
   if (dtype == kF32) unscale_check_kernel<float><<<grid, 256, 0, s>>>((float*)grad, n, inv_scale, inv_scale_dev, write_back, flag, rank, world, own_chunks);
   else if (dtype == kBF16) unscale_check_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((__nv_bfloat16*)grad, n, inv_scale, inv_scale_dev, write_back, flag, rank, world, own_chunks);
@@ -569,16 +605,13 @@ int lb_fused_optimizer_sharded2(float* w, const void* grad, float* s0, float* s1
   const long long nchunks = (total + kOptChunk - 1) / kOptChunk;
   const int grid = flat_grid((nchunks + world - 1) / world * kOptChunk, kOptChunk);
   const OptSegment* sg = reinterpret_cast<const OptSegment*>(segs);
-  const long long most = 3LL * lbhost::sm_count();          // all blocks resident at once
-  const long long per = (nchunks + most - 1) / most;
-  const int runs = (int)((nchunks + per - 1) / per);
-  const bool whole = world == 1 && !compact_state && (reinterpret_cast<uintptr_t>(w16) & 7) == 0;
+  const bool whole = world == 1 && !compact_state && (reinterpret_cast<uintptr_t>(w16) & 7) == 0 && nchunks < (1ll << 31);
 #define LB_OPTV(G, W)                                                                                         \
   {                                                                                                           \
     if (whole)                                                                                                \
-      fused_optimizer_run_kernel<G, W><<<runs, 256, 0, s>>>(w, (const G*)grad, s0, s1, (W*)w16, sg, nseg, total, \
-                                                            inv_scale, skip_flag, step_ptr, lr_scale_ptr,     \
-                                                            inv_scale_dev, per);                              \
+      fused_optimizer_chunk_kernel<G, W><<<(int)nchunks, 256, 0, s>>>(w, (const G*)grad, s0, s1, (W*)w16, sg, nseg, \
+                                                                      total, inv_scale, skip_flag, step_ptr,  \
+                                                                      lr_scale_ptr, inv_scale_dev);           \
     else                                                                                                      \
       fused_optimizer_vec_kernel<G, W><<<grid, 256, 0, s>>>(                                                  \
           w, (const G*)grad, s0, s1, (W*)w16, sg, nseg, total, inv_scale, skip_flag, step_ptr, lr_scale_ptr,  \
