@@ -307,6 +307,50 @@ __global__ void unary_kernel(const T* __restrict__ x, const T* __restrict__ dy, 
   UnaryDispatch<T, 0, U_COUNT - 1>::run(op, x, dy, out, n, mode, p0, p1, aligned);
 }
 
+// The activations that models are made of, and additions and products, have kernels of their own: one that
+// holds every operator runs each of them with the registers of the greediest.  Blocks of 512 vectors that
+// come and go, two a thread, both loads first.  16.8 M bf16 values: GELU 23.5 -> 15.3 us, its gradient
+// 38 -> 21; an addition of 4 M 6.0 -> 4.6.
+constexpr int kHotVecs = 2;
+template <typename T, int OP, int MODE>
+__global__ void __launch_bounds__(256)
+unary_hot_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restrict__ out, long long n, float p0, float p1) {
+  constexpr int V = 16 / sizeof(T);
+  const long long i0 = ((long long)blockIdx.x * (256 * kHotVecs) + threadIdx.x) * V;
+  float fx[kHotVecs][8], fd[kHotVecs][8];
+#pragma unroll
+  for (int u = 0; u < kHotVecs; ++u) {
+    load_vec<T>(x, i0 + u * 256 * V, n, fx[u], true);
+    if (MODE) load_vec<T>(dy, i0 + u * 256 * V, n, fd[u], true);
+  }
+#pragma unroll
+  for (int u = 0; u < kHotVecs; ++u) {
+    float fo[8];
+#pragma unroll
+    for (int j = 0; j < V; ++j) fo[j] = MODE ? unary_bwd(OP, fx[u][j], fd[u][j], p0, p1) : unary_fwd(OP, fx[u][j], p0, p1);
+    store_vec<T>(out, i0 + u * 256 * V, n, fo, true);
+  }
+}
+template <typename T, int OP>
+__global__ void __launch_bounds__(256)
+binary_hot_kernel(const T* __restrict__ a, const T* __restrict__ b, T* __restrict__ out, long long n) {
+  constexpr int V = 16 / sizeof(T);
+  const long long i0 = ((long long)blockIdx.x * (256 * kHotVecs) + threadIdx.x) * V;
+  float fa[kHotVecs][8], fb[kHotVecs][8];
+#pragma unroll
+  for (int u = 0; u < kHotVecs; ++u) {
+    load_vec<T>(a, i0 + u * 256 * V, n, fa[u], true);
+    load_vec<T>(b, i0 + u * 256 * V, n, fb[u], true);
+  }
+#pragma unroll
+  for (int u = 0; u < kHotVecs; ++u) {
+    float fo[8];
+#pragma unroll
+    for (int j = 0; j < V; ++j) fo[j] = binary_fwd(OP, fa[u][j], fb[u][j]);
+    store_vec<T>(out, i0 + u * 256 * V, n, fo, true);
+  }
+}
+
 template <typename T, int OP>
 __device__ __forceinline__ void binary_body(const T* __restrict__ a, const T* __restrict__ b,
                                             const T* __restrict__ dy, T* __restrict__ out0,
@@ -378,6 +422,39 @@ static int grid_for(long long n, int vec) {
   return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
+// Blocks of the kernels of single operators; 0: too many for one launch.
+static int hot_grid(long long n, int vec) {
+  const long long blocks = (n + 256LL * kHotVecs * vec - 1) / (256LL * kHotVecs * vec);
+  return blocks < (1LL << 31) ? (int)blocks : 0;
+}
+template <typename T>
+static bool unary_hot(const void* x, const void* dy, void* out, long long n, int op, int mode, float p0, float p1,
+                      cudaStream_t s) {
+  const int grid = hot_grid(n, 16 / (int)sizeof(T));
+  if (!grid) return false;
+  switch (op) {
+#define LB_HOT(OP)                                                                                                 \
+  case OP:                                                                                                         \
+    if (mode) unary_hot_kernel<T, OP, 1><<<grid, 256, 0, s>>>((const T*)x, (const T*)dy, (T*)out, n, p0, p1);      \
+    else unary_hot_kernel<T, OP, 0><<<grid, 256, 0, s>>>((const T*)x, nullptr, (T*)out, n, p0, p1);                \
+    return true;
+    LB_HOT(U_GELU) LB_HOT(U_GELU_TANH) LB_HOT(U_SIGMOID) LB_HOT(U_TANH) LB_HOT(U_RELU) LB_HOT(U_LEAKY_RELU) LB_HOT(U_SCALE)
+#undef LB_HOT
+  }
+  return false;
+}
+template <typename T>
+static bool binary_hot(const void* a, const void* b, void* out, long long n, int op, cudaStream_t s) {
+  const int grid = hot_grid(n, 16 / (int)sizeof(T));
+  if (!grid) return false;
+  switch (op) {
+#define LB_HOT(OP) case OP: binary_hot_kernel<T, OP><<<grid, 256, 0, s>>>((const T*)a, (const T*)b, (T*)out, n); return true;
+    LB_HOT(B_ADD) LB_HOT(B_MUL) LB_HOT(B_ADD_RELU)
+#undef LB_HOT
+  }
+  return false;
+}
+
 static int all_aligned(std::initializer_list<const void*> ps) {
   for (const void* p : ps)
     if (p && (reinterpret_cast<uintptr_t>(p) & 15)) return 0;
@@ -394,6 +471,11 @@ int lb_unary(const void* x, const void* dy, void* out, long long n, int op, int 
   if (n <= 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   const int al = all_aligned({x, dy, out});
+  if (al && (mode == 0 || mode == 1) &&
+      (dtype == kF32    ? unary_hot<float>(x, dy, out, n, op, mode, p0, p1, s)
+       : dtype == kBF16 ? unary_hot<__nv_bfloat16>(x, dy, out, n, op, mode, p0, p1, s)
+                        : unary_hot<__half>(x, dy, out, n, op, mode, p0, p1, s)))
+    return (int)cudaGetLastError();
   if (dtype == kF32)
     unary_kernel<float><<<grid_for(n, 4), 256, 0, s>>>((const float*)x, (const float*)dy,
                                                        (float*)out, n, op, mode, p0, p1, al);
@@ -412,6 +494,11 @@ int lb_binary(const void* a, const void* b, const void* dy, void* out0, void* ou
   if (n <= 0) return 0;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream_);
   const int al = all_aligned({a, b, dy, out0, out1});
+  if (al && mode == 0 &&
+      (dtype == kF32    ? binary_hot<float>(a, b, out0, n, op, s)
+       : dtype == kBF16 ? binary_hot<__nv_bfloat16>(a, b, out0, n, op, s)
+                        : binary_hot<__half>(a, b, out0, n, op, s)))
+    return (int)cudaGetLastError();
   if (dtype == kF32)
     binary_kernel<float><<<grid_for(n, 4), 256, 0, s>>>((const float*)a, (const float*)b,
                                                         (const float*)dy, (float*)out0,

@@ -138,22 +138,30 @@ __global__ void softmax_ce_bwd_kernel(const T* __restrict__ x, const long long* 
   }
 }
 
-// Long rows of 16-bit logits (a vocabulary): one pass with 16-byte loads and a running
+// Long rows of 16-bit logits (a vocabulary): one pass with 16-byte loads, four in flight, and a running
 // (max, sum) pair per thread; the two-pass scalar kernel above read a 100 KB row twice, two
 // bytes per load, and ran at a tenth of the copy rate.  cols % 8 == 0, rows 16-byte aligned.
+// 4096 x 50304 bf16: 89 us with one load in flight, 68 so.
 template <typename T>
-__global__ void softmax_ce_fwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ labels,
-                                          float* __restrict__ loss, float* __restrict__ lse_out,
-                                          long long rows, int cols) {
+__global__ void __launch_bounds__(256)
+softmax_ce_fwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ labels, float* __restrict__ loss,
+                          float* __restrict__ lse_out, long long rows, int cols) {
   __shared__ float scratch[32];
+  constexpr int U = 4;
   const int nv = cols / 8;
-  for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-    const T* xr = x + r * cols;
-    const uint4* xv = reinterpret_cast<const uint4*>(xr);
-    float m = -INFINITY, s = 0.f;
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      const uint4 q = xv[i];
-      const T* e = reinterpret_cast<const T*>(&q);
+  const long long r = blockIdx.x;
+  const T* xr = x + r * cols;
+  const uint4* xv = reinterpret_cast<const uint4*>(xr);
+  float m = -INFINITY, s = 0.f;
+  for (int i0 = threadIdx.x; i0 < nv; i0 += U * 256) {
+    uint4 q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * 256 < nv) q[u] = xv[i0 + u * 256];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (i0 + u * 256 >= nv) break;
+      const T* e = reinterpret_cast<const T*>(&q[u]);
       float f[8];
       float lm = -INFINITY;
 #pragma unroll
@@ -165,42 +173,54 @@ __global__ void softmax_ce_fwd_vec_kernel(const T* __restrict__ x, const long lo
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
     }
-    const float M = block_reduce_max(m, scratch);
-    s = (m == -INFINITY) ? 0.f : s * __expf(m - M);
-    s = block_reduce_sum(s, scratch);
-    if (threadIdx.x == 0) {
-      const float lse = M + logf(s);
-      lse_out[r] = lse;
-      const long long lab = labels[r];
-      loss[r] = (lab >= 0 && lab < cols) ? lse - to_f32<T>(xr[lab]) : 0.f;
-    }
+  }
+  const float M = block_reduce_max(m, scratch);
+  s = (m == -INFINITY) ? 0.f : s * __expf(m - M);
+  s = block_reduce_sum(s, scratch);
+  if (threadIdx.x == 0) {
+    const float lse = M + logf(s);
+    lse_out[r] = lse;
+    const long long lab = labels[r];
+    loss[r] = (lab >= 0 && lab < cols) ? lse - to_f32<T>(xr[lab]) : 0.f;
   }
 }
+// A block takes 1024 vectors of one row, four a thread, and is gone: 4096 x 50304 bf16 132 us with
+// resident blocks that walk rows, 121 so.
+constexpr int kCeBlock = 1024;
 template <typename T>
-__global__ void softmax_ce_bwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ labels,
-                                          const float* __restrict__ lse, const float* __restrict__ dloss,
-                                          float dloss_scalar, T* __restrict__ dx, long long rows,
-                                          int cols) {
+__global__ void __launch_bounds__(256)
+softmax_ce_bwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ labels, const float* __restrict__ lse,
+                          const float* __restrict__ dloss, float dloss_scalar, T* __restrict__ dx, int cols,
+                          FastDiv blocks_row) {
+  constexpr int U = kCeBlock / 256;
   const int nv = cols / 8;
-  for (long long r = blockIdx.x; r < rows; r += gridDim.x) {
-    const uint4* xv = reinterpret_cast<const uint4*>(x + r * cols);
-    uint4* dv = reinterpret_cast<uint4*>(dx + r * cols);
-    const long long lab = labels[r];
-    const bool ok = lab >= 0 && lab < cols;
-    const float g = ok ? (dloss ? dloss[r] : dloss_scalar) : 0.f;
-    const float l = lse[r];
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-      const uint4 q = xv[i];
-      const T* e = reinterpret_cast<const T*>(&q);
-      uint4 o;
-      T* oe = reinterpret_cast<T*>(&o);
+  uint32_t r, part;
+  blocks_row.divmod(blockIdx.x, r, part);
+  const uint4* xv = reinterpret_cast<const uint4*>(x + (long long)r * cols);
+  uint4* dv = reinterpret_cast<uint4*>(dx + (long long)r * cols);
+  const int i0 = (int)part * kCeBlock + threadIdx.x;
+  uint4 q[U];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float p = __expf(to_f32<T>(e[j]) - l);
-        oe[j] = from_f32<T>(g * (p - ((long long)i * 8 + j == lab ? 1.f : 0.f)));
-      }
-      dv[i] = o;
+  for (int u = 0; u < U; ++u)
+    if (i0 + u * 256 < nv) q[u] = xv[i0 + u * 256];
+  const long long lab = labels[r];
+  const bool ok = lab >= 0 && lab < cols;
+  const float g = ok ? (dloss ? dloss[r] : dloss_scalar) : 0.f;
+  const float l = lse[r];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int i = i0 + u * 256;
+    if (i >= nv) break;
+    const T* e = reinterpret_cast<const T*>(&q[u]);
+    const int mine = lab >= i * 8ll && lab < i * 8ll + 8 ? (int)(lab - i * 8ll) : 8;     // the label's place in this vector
+    uint4 o;
+    T* oe = reinterpret_cast<T*>(&o);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float p = __expf(to_f32<T>(e[j]) - l);
+      oe[j] = from_f32<T>(g * (p - (j == mine ? 1.f : 0.f)));
     }
+    dv[i] = o;
   }
 }
 
@@ -370,13 +390,13 @@ int lb_softmax_ce_fwd(const void* x, const long long* labels, float* loss, float
                                (const T*)x, labels, loss, lse, rows, cols)));
     return (int)cudaGetLastError();
   }
-  if (dtype != kF32 && cols % 8 == 0 && cols >= 2048 && (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+  if (dtype != kF32 && cols % 8 == 0 && cols >= 2048 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && rows > 0 &&
+      rows < (1ll << 31)) {
     if (dtype == kBF16)
-      softmax_ce_fwd_vec_kernel<__nv_bfloat16><<<row_grid(rows), 256, 0, s>>>(
-          (const __nv_bfloat16*)x, labels, loss, lse, rows, cols);
+      softmax_ce_fwd_vec_kernel<__nv_bfloat16><<<(int)rows, 256, 0, s>>>((const __nv_bfloat16*)x, labels, loss, lse,
+                                                                          rows, cols);
     else
-      softmax_ce_fwd_vec_kernel<__half><<<row_grid(rows), 256, 0, s>>>((const __half*)x, labels, loss,
-                                                                        lse, rows, cols);
+      softmax_ce_fwd_vec_kernel<__half><<<(int)rows, 256, 0, s>>>((const __half*)x, labels, loss, lse, rows, cols);
     return (int)cudaGetLastError();
   }
   LB_DISPATCH_ALL(dtype, (softmax_ce_fwd_kernel<T><<<row_grid(rows), row_threads(cols), 0, s>>>(
@@ -393,14 +413,16 @@ int lb_softmax_ce_bwd(const void* x, const long long* labels, const float* lse, 
                                (const T*)x, labels, lse, dloss, dloss_scalar, (T*)dx, rows, cols)));
     return (int)cudaGetLastError();
   }
-  if (dtype != kF32 && cols % 8 == 0 && cols >= 2048 &&
+  const long long ce_blocks = rows * ((cols / 8 + kCeBlock - 1) / kCeBlock);
+  if (dtype != kF32 && cols % 8 == 0 && cols >= 2048 && rows > 0 && ce_blocks * (cols / 8192 + 2) < (1ll << 31) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0) {
+    const FastDiv per((uint32_t)((cols / 8 + kCeBlock - 1) / kCeBlock));
     if (dtype == kBF16)
-      softmax_ce_bwd_vec_kernel<__nv_bfloat16><<<row_grid(rows), 256, 0, s>>>(
-          (const __nv_bfloat16*)x, labels, lse, dloss, dloss_scalar, (__nv_bfloat16*)dx, rows, cols);
+      softmax_ce_bwd_vec_kernel<__nv_bfloat16><<<(int)rows * per.d, 256, 0, s>>>(
+          (const __nv_bfloat16*)x, labels, lse, dloss, dloss_scalar, (__nv_bfloat16*)dx, cols, per);
     else
-      softmax_ce_bwd_vec_kernel<__half><<<row_grid(rows), 256, 0, s>>>(
-          (const __half*)x, labels, lse, dloss, dloss_scalar, (__half*)dx, rows, cols);
+      softmax_ce_bwd_vec_kernel<__half><<<(int)rows * per.d, 256, 0, s>>>((const __half*)x, labels, lse, dloss,
+                                                                          dloss_scalar, (__half*)dx, cols, per);
     return (int)cudaGetLastError();
   }
   LB_DISPATCH_ALL(dtype, (softmax_ce_bwd_kernel<T><<<row_grid(rows), row_threads(cols), 0, s>>>(

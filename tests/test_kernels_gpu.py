@@ -290,3 +290,24 @@ def test_unary_operators_on_16_bit_tensors(name, dtype):
     ref.backward(g.float())
     assert native.consume_status() == 0
     torch.testing.assert_close(xa.grad.float(), xr.grad, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("n", [1, 8, 4095, 4096, 4097, 12296])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_operators_with_kernels_of_their_own(n, dtype):
+    """The edges of a block (512 vectors of 16 bytes) and of a vector, and the same values as the kernel of all
+    operators, which takes tensors that do not start on 16 bytes."""
+    torch.manual_seed(2)
+    a, b, dy = (torch.randn(n + 1, device="cuda").to(dtype) for _ in range(3))
+    for name, p0 in (("gelu", 0.0), ("tanh", 0.0), ("leaky_relu", 0.3), ("scale", 1.7)):
+        got, want = [], []
+        for out, cut in ((got, slice(0, n)), (want, slice(1, n + 1))):
+            x = torch.cat([a.new_zeros(cut.start), a[:n]])[cut].requires_grad_(True)
+            g = torch.cat([a.new_zeros(cut.start), dy[:n]])[cut]
+            y = ew.unary(name, x, p0, 0.0)
+            out += [y.detach(), torch.autograd.grad(y, x, g)[0]]
+        for u, v in zip(got, want):
+            assert torch.equal(u, v), name
+    for name in ("add", "multiply"):
+        x = torch.cat([a.new_zeros(1), a[:n]])[1:]
+        assert torch.equal(ew.binary(name, a[:n], b[:n]), ew.binary(name, x, b[:n])), name
