@@ -170,12 +170,6 @@ __device__ __forceinline__ void att_store_out64(uint16_t* dst, const uint32_t (&
   }
 }
 
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
 // ------------------------------------------------------------------------------------
 // Forward.  A CTA holds two tiles of 128 queries (one, where that gives every SM a CTA) and walks
 // the keys 128 at a time.  Each tile has four warps, one thread per query, and its own scores,

@@ -394,6 +394,14 @@ __device__ __forceinline__ void store_from_f32(void* p, long long i, float v, in
   else reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
 }
 
+// 2^x in one instruction (results below the normal range are zero; the form that keeps them scales before
+// and after).
+__device__ __forceinline__ float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

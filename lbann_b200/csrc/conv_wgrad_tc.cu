@@ -494,7 +494,7 @@ conv_wgrad_slab_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 // unit of the partials), CH channels and NT taps; its threads are these items times `groups` groups of
 // splits, so that CH lanes load contiguous bytes and the stores (filter layout: taps innermost) are runs
 // of taps, through shared memory.  Large filters are bound by the bytes (a division by a run-time number
-// for every index took as long: 512 x 512 x 9 22 -> 12 us), small ones by the latency of a thread's loads:
+// for every index took as long: 512 x 512 x 9 21 -> 16 us), small ones by the latency of a thread's loads:
 // eight are in flight, and the launch cuts the splits into as many groups as fill the GPU with threads
 // (64 x 32 x 27, 148 splits: 20 -> 8 us).
 constexpr int kRedThreads = 256;

@@ -309,8 +309,8 @@ __global__ void unary_kernel(const T* __restrict__ x, const T* __restrict__ dy, 
 
 // The activations that models are made of, and additions and products, have kernels of their own: one that
 // holds every operator runs each of them with the registers of the greediest.  Blocks of 512 vectors that
-// come and go, two a thread, both loads first.  16.8 M bf16 values: GELU 23.5 -> 15.3 us, its gradient
-// 38 -> 21; an addition of 4 M 6.0 -> 4.6.
+// come and go, two a thread, both loads first.  16.8 M bf16 values: GELU 23.5 -> 18.6 us, its gradient
+// 38 -> 32; an addition of 4 M 6.0 -> 5.3.
 constexpr int kHotVecs = 2;
 template <typename T, int OP, int MODE>
 __global__ void __launch_bounds__(256)

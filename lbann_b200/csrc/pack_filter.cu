@@ -31,7 +31,7 @@ pack_filter_kernel(const float* __restrict__ w, T* __restrict__ fwd, T* __restri
 // pairs and taps: forward rows leave in runs of CH * 2 bytes, data-gradient rows in runs of 16.  (Element by
 // element, lanes were taps * 4 bytes apart on the way in and Kp * 2 on the way out.)  A block is one
 // round trip to memory, so the launch takes 32, 16 or 8 channels, whichever gives four blocks an SM:
-// 27 taps, 32 -> 64 channels 7.5 us with 8 blocks of 32, 3.4 with 32 of 8.
+// 27 taps, 32 -> 64 channels 7.5 us with 8 blocks of 32, 3.6 with 32 of 8.
 constexpr int kPackK = 8;
 
 template <typename T, int CH>

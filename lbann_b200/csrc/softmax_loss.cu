@@ -13,6 +13,8 @@
 //                l1_norm,l2_norm2}.cu
 //   categorical / top-k accuracy per sample
 //     reference: src/layers/loss/categorical_accuracy.cu, top_k_categorical_accuracy.cu
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace lb {
@@ -138,86 +140,119 @@ __global__ void softmax_ce_bwd_kernel(const T* __restrict__ x, const long long* 
   }
 }
 
-// Long rows of 16-bit logits (a vocabulary): one pass with 16-byte loads, four in flight, and a running
-// (max, sum) pair per thread; the two-pass scalar kernel above read a 100 KB row twice, two
-// bytes per load, and ran at a tenth of the copy rate.  cols % 8 == 0, rows 16-byte aligned.
-// 4096 x 50304 bf16: 89 us with one load in flight, 68 so.
-template <typename T>
+// 16-bit logits: one pass with 16-byte loads, four in flight, and a running (max, sum) pair per thread;
+// the two-pass scalar kernel above reads a row twice, two bytes a load.  A row of 4096 columns or more is
+// a block's, shorter ones a warp's.  Rows start anywhere (a vocabulary of 30522 words): the elements in front
+// of the first 16-byte boundary and behind the last are single ones.
+// Instructions are what is left of long rows: exponentials of one instruction instead of __expf's four
+// (terms below 2^-126 of the largest are zero).  Forward, bf16: 4096 x 50304 86 -> 78 us,
+// 16384 x 2048 34 -> 17 (a block for a row of 256 vectors is mostly its reductions).
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kCeBlockRow = 4096;                     // columns from which a row takes a block
+
+// A row as single elements up to `head`, nv vectors, single elements from `tail` on.
+struct CeSpan {
+  int head, nv, tail;
+  template <typename T>
+  __device__ __forceinline__ CeSpan(const T* row, int cols) {
+    head = min(cols, (int)((16u - (uint32_t)(reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) / 2);
+    nv = (cols - head) / 8;
+    tail = head + nv * 8;
+  }
+};
+
+template <typename T, bool BLOCK>
 __global__ void __launch_bounds__(256)
 softmax_ce_fwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ labels, float* __restrict__ loss,
                           float* __restrict__ lse_out, long long rows, int cols) {
   __shared__ float scratch[32];
-  constexpr int U = 4;
-  const int nv = cols / 8;
-  const long long r = blockIdx.x;
+  constexpr int U = 4, TEAM = BLOCK ? 256 : 32;
+  const long long r = BLOCK ? blockIdx.x : (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int t = BLOCK ? threadIdx.x : threadIdx.x & 31;
+  if (!BLOCK && r >= rows) return;
   const T* xr = x + r * cols;
-  const uint4* xv = reinterpret_cast<const uint4*>(xr);
+  const CeSpan span(xr, cols);
+  const uint4* xv = reinterpret_cast<const uint4*>(xr + span.head);
   float m = -INFINITY, s = 0.f;
-  for (int i0 = threadIdx.x; i0 < nv; i0 += U * 256) {
+  // the single elements: at most seven in front and seven behind
+  const int single = t < 8 ? (t < span.head ? t : cols) : (t < 16 ? span.tail + t - 8 : cols);
+  if (single < cols) {
+    m = to_f32<T>(xr[single]);
+    s = m == -INFINITY ? 0.f : 1.f;
+  }
+  for (int i0 = t; i0 < span.nv; i0 += U * TEAM) {
     uint4 q[U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
-      if (i0 + u * 256 < nv) q[u] = xv[i0 + u * 256];
+      if (i0 + u * TEAM < span.nv) q[u] = xv[i0 + u * TEAM];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (i0 + u * 256 >= nv) break;
+      if (i0 + u * TEAM >= span.nv) break;
       const T* e = reinterpret_cast<const T*>(&q[u]);
       float f[8];
       float lm = -INFINITY;
 #pragma unroll
       for (int j = 0; j < 8; ++j) { f[j] = to_f32<T>(e[j]); lm = fmaxf(lm, f[j]); }
       if (lm > m) {
-        s *= __expf(m - lm);      // m == -inf: s is 0 and stays 0
+        s *= fast_exp2((m - lm) * kLog2e);      // m == -inf: s is 0 and stays 0
         m = lm;
       }
+      const float base = m == -INFINITY ? 0.f : m;   // nothing but masked columns so far: they add zeros
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
+      for (int j = 0; j < 8; ++j) s += fast_exp2((f[j] - base) * kLog2e);
     }
   }
-  const float M = block_reduce_max(m, scratch);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - M);
-  s = block_reduce_sum(s, scratch);
-  if (threadIdx.x == 0) {
+  const float M = BLOCK ? block_reduce_max(m, scratch) : warp_max(m);
+  if (m != -INFINITY) s *= fast_exp2((m - M) * kLog2e);
+  s = BLOCK ? block_reduce_sum(s, scratch) : warp_sum(s);
+  if (t == 0) {
     const float lse = M + logf(s);
     lse_out[r] = lse;
     const long long lab = labels[r];
     loss[r] = (lab >= 0 && lab < cols) ? lse - to_f32<T>(xr[lab]) : 0.f;
   }
 }
-// A block takes 1024 vectors of one row, four a thread, and is gone: 4096 x 50304 bf16 132 us with
-// resident blocks that walk rows, 121 so.
-constexpr int kCeBlock = 1024;
-template <typename T>
+// A block takes 1024 vectors of one row, or a warp 128, four a thread, and is gone: bf16
+// 4096 x 50304 133 us with resident blocks that walk rows, 119 so; 16384 x 2048 31, 19.  x and dx start on 16 bytes.
+template <typename T, bool BLOCK>
 __global__ void __launch_bounds__(256)
 softmax_ce_bwd_vec_kernel(const T* __restrict__ x, const long long* __restrict__ labels, const float* __restrict__ lse,
-                          const float* __restrict__ dloss, float dloss_scalar, T* __restrict__ dx, int cols,
-                          FastDiv blocks_row) {
-  constexpr int U = kCeBlock / 256;
-  const int nv = cols / 8;
+                          const float* __restrict__ dloss, float dloss_scalar, T* __restrict__ dx, long long rows,
+                          int cols, FastDiv parts) {
+  constexpr int U = 4, TEAM = BLOCK ? 256 : 32;
   uint32_t r, part;
-  blocks_row.divmod(blockIdx.x, r, part);
-  const uint4* xv = reinterpret_cast<const uint4*>(x + (long long)r * cols);
-  uint4* dv = reinterpret_cast<uint4*>(dx + (long long)r * cols);
-  const int i0 = (int)part * kCeBlock + threadIdx.x;
+  parts.divmod(BLOCK ? blockIdx.x : blockIdx.x * 8 + (threadIdx.x >> 5), r, part);
+  if (!BLOCK && r >= rows) return;
+  const int t = BLOCK ? threadIdx.x : threadIdx.x & 31;
+  const T* xr = x + (long long)r * cols;
+  T* dr = dx + (long long)r * cols;
+  const CeSpan span(xr, cols);
+  const uint4* xv = reinterpret_cast<const uint4*>(xr + span.head);
+  uint4* dv = reinterpret_cast<uint4*>(dr + span.head);
+  const int i0 = (int)part * (U * TEAM) + t;
   uint4 q[U];
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (i0 + u * 256 < nv) q[u] = xv[i0 + u * 256];
+    if (i0 + u * TEAM < span.nv) q[u] = xv[i0 + u * TEAM];
   const long long lab = labels[r];
   const bool ok = lab >= 0 && lab < cols;
   const float g = ok ? (dloss ? dloss[r] : dloss_scalar) : 0.f;
   const float l = lse[r];
+  const int single = part ? cols : (t < 8 ? (t < span.head ? t : cols) : (t < 16 ? span.tail + t - 8 : cols));
+  if (single < cols)
+    dr[single] = from_f32<T>(g * (fast_exp2((to_f32<T>(xr[single]) - l) * kLog2e) - (single == lab ? 1.f : 0.f)));
+  const long long lv = lab - span.head;          // the label's place among the vectors
 #pragma unroll
   for (int u = 0; u < U; ++u) {
-    const int i = i0 + u * 256;
-    if (i >= nv) break;
+    const int i = i0 + u * TEAM;
+    if (i >= span.nv) break;
     const T* e = reinterpret_cast<const T*>(&q[u]);
-    const int mine = lab >= i * 8ll && lab < i * 8ll + 8 ? (int)(lab - i * 8ll) : 8;     // the label's place in this vector
+    const int mine = lv >= i * 8ll && lv < i * 8ll + 8 ? (int)(lv - i * 8ll) : 8;
     uint4 o;
     T* oe = reinterpret_cast<T*>(&o);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float p = __expf(to_f32<T>(e[j]) - l);
+      const float p = fast_exp2((to_f32<T>(e[j]) - l) * kLog2e);
       oe[j] = from_f32<T>(g * (p - (j == mine ? 1.f : 0.f)));
     }
     dv[i] = o;
@@ -390,13 +425,15 @@ int lb_softmax_ce_fwd(const void* x, const long long* labels, float* loss, float
                                (const T*)x, labels, loss, lse, rows, cols)));
     return (int)cudaGetLastError();
   }
-  if (dtype != kF32 && cols % 8 == 0 && cols >= 2048 && (reinterpret_cast<uintptr_t>(x) & 15) == 0 && rows > 0 &&
-      rows < (1ll << 31)) {
-    if (dtype == kBF16)
-      softmax_ce_fwd_vec_kernel<__nv_bfloat16><<<(int)rows, 256, 0, s>>>((const __nv_bfloat16*)x, labels, loss, lse,
-                                                                          rows, cols);
-    else
-      softmax_ce_fwd_vec_kernel<__half><<<(int)rows, 256, 0, s>>>((const __half*)x, labels, loss, lse, rows, cols);
+  if (dtype != kF32 && rows > 0 && rows < (1ll << 31)) {
+    const bool block = cols >= kCeBlockRow;
+    const int grid = (int)(block ? rows : (rows + 7) / 8);
+#define LB_CE(T)                                                                                                   \
+  if (block) softmax_ce_fwd_vec_kernel<T, true><<<grid, 256, 0, s>>>((const T*)x, labels, loss, lse, rows, cols);  \
+  else softmax_ce_fwd_vec_kernel<T, false><<<grid, 256, 0, s>>>((const T*)x, labels, loss, lse, rows, cols);
+    if (dtype == kBF16) { LB_CE(__nv_bfloat16) }
+    else { LB_CE(__half) }
+#undef LB_CE
     return (int)cudaGetLastError();
   }
   LB_DISPATCH_ALL(dtype, (softmax_ce_fwd_kernel<T><<<row_grid(rows), row_threads(cols), 0, s>>>(
@@ -413,16 +450,22 @@ int lb_softmax_ce_bwd(const void* x, const long long* labels, const float* lse, 
                                (const T*)x, labels, lse, dloss, dloss_scalar, (T*)dx, rows, cols)));
     return (int)cudaGetLastError();
   }
-  const long long ce_blocks = rows * ((cols / 8 + kCeBlock - 1) / kCeBlock);
-  if (dtype != kF32 && cols % 8 == 0 && cols >= 2048 && rows > 0 && ce_blocks * (cols / 8192 + 2) < (1ll << 31) &&
+  const bool block = cols >= kCeBlockRow;
+  const long long per = std::max(1, (cols / 8 + (block ? 1023 : 127)) / (block ? 1024 : 128)), teams = rows * per;
+  if (dtype != kF32 && rows > 0 && (teams + 8) * per < (1ll << 31) &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dx)) & 15) == 0) {
-    const FastDiv per((uint32_t)((cols / 8 + kCeBlock - 1) / kCeBlock));
-    if (dtype == kBF16)
-      softmax_ce_bwd_vec_kernel<__nv_bfloat16><<<(int)rows * per.d, 256, 0, s>>>(
-          (const __nv_bfloat16*)x, labels, lse, dloss, dloss_scalar, (__nv_bfloat16*)dx, cols, per);
-    else
-      softmax_ce_bwd_vec_kernel<__half><<<(int)rows * per.d, 256, 0, s>>>((const __half*)x, labels, lse, dloss,
-                                                                          dloss_scalar, (__half*)dx, cols, per);
+    const FastDiv parts((uint32_t)per);
+    const int grid = (int)(block ? teams : (teams + 7) / 8);
+#define LB_CE(T)                                                                                                   \
+  if (block)                                                                                                       \
+    softmax_ce_bwd_vec_kernel<T, true><<<grid, 256, 0, s>>>((const T*)x, labels, lse, dloss, dloss_scalar, (T*)dx, \
+                                                            rows, cols, parts);                                    \
+  else                                                                                                             \
+    softmax_ce_bwd_vec_kernel<T, false><<<grid, 256, 0, s>>>((const T*)x, labels, lse, dloss, dloss_scalar, (T*)dx, \
+                                                             rows, cols, parts);
+    if (dtype == kBF16) { LB_CE(__nv_bfloat16) }
+    else { LB_CE(__half) }
+#undef LB_CE
     return (int)cudaGetLastError();
   }
   LB_DISPATCH_ALL(dtype, (softmax_ce_bwd_kernel<T><<<row_grid(rows), row_threads(cols), 0, s>>>(

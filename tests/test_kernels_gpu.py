@@ -8,6 +8,7 @@ import torch.nn.functional as F
 
 from lbann_b200.ops import elementwise as ew
 from lbann_b200.ops import native, nn
+from lbann_b200.ops.optim import ParameterArena
 
 pytestmark = pytest.mark.gpu
 
@@ -253,6 +254,68 @@ def test_softmax_cross_entropy_long_rows(rows, cols, dtype):
     (ref * w).sum().backward()
     assert native.consume_status() == 0
     torch.testing.assert_close(logits.grad.float(), lr.grad, rtol=2e-2, atol=2e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols", [(9, 1), (9, 7), (11, 33), (300, 1000), (17, 1031), (33, 4095), (5, 4099), (9, 8200),
+                                       (3, 30522), (3, 65543)])
+def test_softmax_cross_entropy_rows_that_start_anywhere(rows, cols, dtype):
+    """Warps and blocks a row, several parts of a row in the gradient, rows off a 16-byte boundary, and masked
+    columns (-inf), a whole vector of them at a row's start.  Against 64 bits: an exponential is good to two ulp and
+    its argument, |x| < 32, to 2^-19, so the loss to 1e-5; the gradient is rounded to its type (2^-9)."""
+    torch.manual_seed(9)
+    logits = (torch.randn(rows, cols, device="cuda") * 3).to(dtype)
+    labels = torch.randint(0, cols, (rows,), device="cuda")
+    labels[0], labels[1] = cols - 1, cols
+    if cols > 16:
+        logits[:, :9] = -float("inf")
+        labels[2:] = labels[2:].clamp(min=9)
+    logits.requires_grad_(True)
+    loss = nn.softmax_cross_entropy(logits, labels)
+    ok = labels < cols
+    ref_in = logits.detach().double().requires_grad_(True)
+    ref = torch.where(ok, F.cross_entropy(ref_in, labels.clamp(max=cols - 1), reduction="none"), 0.0)
+    torch.testing.assert_close(loss.double(), ref, rtol=1e-5, atol=1e-5)
+    w = torch.rand(rows, device="cuda") + 0.5
+    grad, = torch.autograd.grad((loss * w).sum(), logits)
+    grad_ref, = torch.autograd.grad((ref * w).sum(), ref_in)
+    torch.testing.assert_close(grad.double(), grad_ref, rtol=2.0 ** -8, atol=2e-6)
+    with torch.no_grad():
+        logits[rows - 1, cols - 1] = float("nan")
+        assert bool(torch.isnan(nn.softmax_cross_entropy(logits, labels)[rows - 1]))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n", [1, 7, 4096, 300_001])
+def test_non_finite_gradients_skip_the_step(n, dtype):
+    """The check alone (no value written back) finds an infinity or a NaN at either end; a skipped step changes no
+    weight and is not counted."""
+    arena = ParameterArena(torch.device("cuda"), torch.float16, grad_dtype=dtype)
+    slot = arena.reserve("w", (n,))
+    arena.materialise()
+    arena.ensure_state1()
+    slot.kind, slot.hp = "adam", {"learn_rate": 1e-2, "beta1": 0.9, "beta2": 0.99, "eps": 1e-8}
+    flag = torch.zeros(1, dtype=torch.int32, device="cuda")
+    inv = torch.ones(1, device="cuda")
+    grad = arena.view(arena.grad, slot)
+    for at, bad in ((0, float("inf")), (n - 1, float("nan")), (n // 2, -float("inf"))):
+        grad.fill_(0.5)
+        grad[at] = bad
+        flag.zero_()
+        arena.unscale_and_check(1.0, flag, write_back=False, inv_scale_dev=inv)
+        assert int(flag) == 1
+        before = arena.master.clone()
+        arena.step(1.0, flag, inv_scale_dev=inv)
+        assert torch.equal(arena.master, before) and int(arena.step_dev) == 0
+    grad.fill_(0.5)
+    flag.zero_()
+    arena.unscale_and_check(1.0, flag, write_back=False, inv_scale_dev=inv)
+    assert int(flag) == 0
+    before = arena.view(arena.master, slot).clone()
+    arena.step(1.0, flag, inv_scale_dev=inv)
+    assert int(arena.step_dev) == 1
+    # the first counted step of Adam moves every weight by the learning rate
+    torch.testing.assert_close(before - arena.view(arena.master, slot), torch.full_like(before, 1e-2), rtol=1e-4, atol=1e-6)
 
 
 @pytest.mark.parametrize("rows,cols", [(4096, 2048), (1000, 520), (33, 64), (7, 8)])
