@@ -11,7 +11,9 @@ from __future__ import annotations
 
 import os
 import time
+import weakref
 from collections import OrderedDict, defaultdict
+from collections.abc import Mapping
 from typing import Callable, Dict, List, Optional
 
 import torch
@@ -44,6 +46,29 @@ class ModeStats:
         self.samples = 0
         for m in self.metric_sums:
             m.zero_()
+
+
+class ReplayedActivations(Mapping):
+    """A replayed step's activations by layer name.  The graph's own tensors are overwritten by its
+    next replay, so what is asked for is copied out, once, and stays as it is."""
+
+    def __init__(self, static):
+        self._static, self._own = static, {}
+
+    def __getitem__(self, name):
+        if name not in self._own:
+            self._own[name] = [t.clone() if torch.is_tensor(t) else t for t in self._static[name]]
+        return self._own[name]
+
+    def __iter__(self):
+        return iter(self._static)
+
+    def __len__(self):
+        return len(self._static)
+
+    def keep(self):
+        for name in self._static:
+            self[name]
 
 
 class ExecMetric:
@@ -102,6 +127,7 @@ class ExecModel:
         self._graph_mode = None        # decided at the first training step
         self._overwrite_cache = None   # (layers, handles), see _overwritten_gradients
         self._graphs = {}
+        self._eval_graphs = OrderedDict()
         self.layer_timing = False
         self.is_setup = False
 
@@ -1055,6 +1081,14 @@ class ExecModel:
     @torch.no_grad()
     def evaluate_step(self, inputs, mode="validation", global_mini_batch_size=None,
                       mini_batch_offset=0):
+        """Forward pass, objective and statistics.  With the ``use_cuda_graph`` option small steps are
+        captured once per input signature and replayed, as training steps are."""
+        key = self._eval_graph_key(inputs, mode, global_mini_batch_size, mini_batch_offset)
+        if key is not None:
+            return self._evaluate_step_graph(key, inputs, mode, global_mini_batch_size, mini_batch_offset)
+        return self._evaluate_step_eager(inputs, mode, global_mini_batch_size, mini_batch_offset)
+
+    def _evaluate_step_eager(self, inputs, mode, global_mini_batch_size, mini_batch_offset):
         for cb in self.callbacks:
             cb.on_forward_prop_begin(self, mode)
         if self.distconv is not None:
@@ -1068,6 +1102,91 @@ class ExecModel:
         self.last_objective = obj.detach()
         self.record_statistics(mode, obj)
         return self.last_objective
+
+    # A forward pass of two GPT blocks over 512 tokens takes the host 740 us to launch, and 260 us as a replay.
+    # Steps with more activations than this (all graphs of a model together) run longer than the host takes,
+    # and would hold their memory for good; so would copies of that many weights be repeated by each replay.
+    _EVAL_GRAPH_BYTES = 2 << 30
+    _EVAL_GRAPH_CASTS = 4 << 20     # elements of weights copied or packed for the step
+    _EVAL_GRAPHS = 8
+
+    def _eval_graph_key(self, inputs, mode, gmb, offset):
+        """What a captured evaluation step depends on, or None where the step is launched from the host."""
+        if (self.device.type != "cuda" or self.parallel is not None or self.distconv is not None
+                or self.subgrid is not None or self._phase_timer is not None or not inputs
+                or torch.cuda.is_current_stream_capturing() or not self._graph_capable()
+                or not all(torch.is_tensor(v) and v.is_cuda and v.is_contiguous() for v in inputs.values())):
+            return None
+        return (mode, gmb, offset, torch.cuda.current_stream(self.device).cuda_stream, self.arena.master.data_ptr(),
+                tuple((k, tuple(v.shape), v.dtype, v.device) for k, v in sorted(inputs.items())))
+
+    def _evaluate_step_graph(self, key, inputs, mode, gmb, offset):
+        entry = self._eval_graphs.get(key)
+        if entry is None:
+            entry = self._eval_graphs[key] = {"warm": 0, "bytes": 0}
+            while len(self._eval_graphs) > self._EVAL_GRAPHS:
+                self._drop_eval_graph(next(iter(self._eval_graphs)))
+        self._eval_graphs.move_to_end(key)
+        st = self.stats[mode]
+        if "graph" not in entry:
+            entry["warm"] += 1
+            if entry["warm"] <= 3 or entry.get("eager"):
+                return self._evaluate_step_eager(inputs, mode, gmb, offset)
+            storages = {t.untyped_storage().data_ptr(): t.untyped_storage().nbytes()
+                        for ts in self.acts.values() for t in ts if torch.is_tensor(t)}
+            entry["bytes"] = sum(storages.values())
+            casts = sum(t.numel() for w in self.weights for t in w.handle._cache.values() if torch.is_tensor(t))
+            if entry["bytes"] > self._EVAL_GRAPH_BYTES or casts > self._EVAL_GRAPH_CASTS:
+                entry.update(eager=True, bytes=0)
+                return self._evaluate_step_eager(inputs, mode, gmb, offset)
+            for k in list(self._eval_graphs):
+                if k != key and sum(e["bytes"] for e in self._eval_graphs.values()) > self._EVAL_GRAPH_BYTES:
+                    self._drop_eval_graph(k)
+            static = {k: torch.empty_like(v) for k, v in inputs.items()}
+            samples0, launches0 = st.samples, native.launches()
+            graph = torch.cuda.CUDAGraph()
+            # the weights may change between replays: their 16-bit and packed copies are made inside
+            # the graph, and those made there are nobody else's
+            for w in self.weights:
+                w.handle.bump()
+            torch.cuda.synchronize(self.device)
+            try:
+                with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+                    out = self._evaluate_step_eager(static, mode, gmb, offset)
+                entry.update(graph=graph, static=static, out=out, acts=self.acts, samples=self._global_mb,
+                             launches=native.launches() - launches0)
+            except Exception:           # something in this model cannot be captured
+                entry.update(eager=True, bytes=0)
+                torch.cuda.synchronize(self.device)
+            for w in self.weights:
+                w.handle.bump()
+            st.samples = samples0
+            native.count_launch(launches0 - native.launches())
+            if entry.get("eager"):
+                return self._evaluate_step_eager(inputs, mode, gmb, offset)
+        self.acts = {}
+        last = entry["last"]() if "last" in entry else None
+        if last is not None:
+            last.keep()                 # a caller holds the activations of the step before
+        for k, v in inputs.items():
+            self._copy_into_static(entry["static"][k], v)
+        entry["graph"].replay()
+        first = next(iter(inputs.values()))
+        self.current_inputs = inputs
+        self.current_mini_batch_size = int(first.shape[0])
+        self._global_mb = entry["samples"]
+        self._global_mb_given, self._mb_offset, self._mean_cache = bool(gmb), offset, {}
+        self.acts = ReplayedActivations(entry["acts"])
+        entry["last"] = weakref.ref(self.acts)
+        st.samples += entry["samples"]
+        native.count_launch(entry["launches"])
+        self.last_objective = entry["out"].clone()
+        return self.last_objective
+
+    def _drop_eval_graph(self, key):
+        if isinstance(self.acts, ReplayedActivations):
+            self.acts.keep()
+        del self._eval_graphs[key]
 
     # ------------------------------------------------------------------ reporting
     def reduce_statistics(self, mode: str):

@@ -215,3 +215,53 @@ def test_overwritten_gradients_equal_accumulated_ones(graph, monkeypatch):
     assert not none and found == {"first_linearity_weights", "aside_linearity_weights", "last_linearity_weights"}
     for a, b in zip(want, got):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+def test_evaluation_replays_equal_eager_steps():
+    """Evaluation steps as graphs: losses and activations of several steps are held and compared at the end (a
+    replay must not write over what a caller holds), weights and running statistics change in between, a ragged
+    last mini-batch has a graph of its own, and the statistics add up."""
+    def run(graph):
+        o = opts.reset()
+        o.set("default_dtype", "bf16")
+        o.set("use_cuda_graph", graph)
+        x = lbann.Input(data_field="samples")
+        target = lbann.Input(data_field="responses")
+        h = lbann.Reshape(x, dims=[8, 6, 6])
+        h = lbann.Convolution(h, num_dims=2, out_channels=16, kernel_size=3, padding=1, has_bias=False, name="conv")
+        h = lbann.Relu(lbann.BatchNormalization(h))
+        h = lbann.FullyConnected(h, num_neurons=4, has_bias=True, name="last")
+        loss = lbann.MeanSquaredError(h, target, name="mse")
+        model = lbann.Model(1, layers=lbann.traverse_layer_graph(x), objective_function=loss,
+                            metrics=[lbann.Metric(loss, name="mse")])
+        exp = lbann.proto.serialize.build_experiment(
+            trainer=lbann.Trainer(mini_batch_size=8, random_seed=3), model=model,
+            data_reader=_reader(8, [288], "samples:normal responses:normal", response_dims=[4]),
+            optimizer=lbann.SGD(learn_rate=1e-2, momentum=0.9))
+        tr = ExecTrainer(exp)
+        m = tr.build_model(exp.model)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        losses, outs, held = [], [], []
+        for step in range(16):
+            rows = 5 if step % 5 == 4 else 8
+            batch = {"samples": torch.randn(rows, 288, generator=g, device="cuda"),
+                     "responses": torch.randn(rows, 4, generator=g, device="cuda")}
+            if step % 4 == 1:
+                m.train_step(batch, rows)
+            losses.append(m.evaluate_step(batch, "validation" if step % 3 else "testing", rows))
+            outs.append(m.activation("last"))
+            held.append(m.acts)
+            assert m.current_mini_batch_size == rows and m.current_inputs["samples"] is batch["samples"]
+        held = [a["conv"][0] for a in held]
+        stats = [m.reduce_statistics(mode) for mode in ("validation", "testing")]
+        graphs = sum("graph" in e for e in m._eval_graphs.values())
+        tr.shutdown()
+        assert native.consume_status() == 0
+        return losses, outs, held, stats, graphs
+
+    want, got = run(False), run(True)
+    assert want[4] == 0 and got[4] >= 2
+    for a, b in zip(want[:3], got[:3]):
+        for t, u in zip(a, b):
+            assert torch.equal(t, u)
+    assert want[3] == got[3]
