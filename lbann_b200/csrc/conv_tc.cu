@@ -21,7 +21,7 @@ namespace lb {
 template <int BN_>
 struct ConvFwdPolicy {
   static constexpr int BN = BN_;
-  static constexpr int kEpiGroups = 2;       // two tiles' epilogues in flight (tc_pipeline.cuh)
+  static constexpr int kEpiGroups = BN == 32 ? 1 : 2;   // share a tile's columns (tc_pipeline.cuh)
   using G = StageGeom<BN>;
   using HasSingleIssue = void;               // two boxes a slice, issued by one thread
 

@@ -17,7 +17,7 @@ namespace lb {
 template <int BN_>
 struct GemmPolicy {
   static constexpr int BN = BN_;
-  static constexpr int kEpiGroups = 2;       // two tiles' epilogues in flight (tc_pipeline.cuh)
+  static constexpr int kEpiGroups = BN / 32 < 4 ? BN / 32 : 4;   // share a tile's columns (tc_pipeline.cuh)
   using G = StageGeom<BN>;
   using HasSingleIssue = void;               // one to six boxes a stage, issued by one thread
 

@@ -113,6 +113,12 @@ struct TmemSrc {                 // this warp's lanes of a TMEM accumulator
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
   }
 };
+// 32 bytes, a whole sector, of a lane's row; the address on 32 bytes.
+__device__ __forceinline__ void st_global_32(void* p, const uint32_t* q) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(q[0]), "r"(q[1]), "r"(q[2]),
+               "r"(q[3]), "r"(q[4]), "r"(q[5]), "r"(q[6]), "r"(q[7])
+               : "memory");
+}
 template <int BN, class Src>
 __device__ __forceinline__ void tc_epilogue_rows(const Src& src, bool row_ok, long long row_off,
                                                  int n0, int n_total, int row_index,
@@ -174,7 +180,10 @@ __device__ __forceinline__ void tc_epilogue_rows(const Src& src, bool row_ok, lo
     tc_apply_act32(v, act, e.act_param);
     if (out_dtype == kF32) {
       float* dst = reinterpret_cast<float*>(e.C) + off;
-      if (full && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
+      if (full && ((reinterpret_cast<uintptr_t>(dst) & 31) == 0)) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 8) st_global_32(dst + j, reinterpret_cast<const uint32_t*>(v) + j);
+      } else if (full && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4)
           *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
@@ -204,6 +213,9 @@ __device__ __forceinline__ void tc_epilogue_rows(const Src& src, bool row_ok, lo
             *reinterpret_cast<uint4*>(pd + 8 * j) =
                 make_uint4(q[4 * j], q[4 * j + 1], q[4 * j + 2], q[4 * j + 3]);
         }
+      } else if (full && ((reinterpret_cast<uintptr_t>(dst) & 31) == 0)) {
+        st_global_32(dst, q);
+        st_global_32(dst + 16, q + 8);
       } else if (full && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -230,11 +242,8 @@ __device__ __forceinline__ void tc_splitk_store(uint32_t taddr, float* row, bool
     tmem_ld_32x32(taddr + c, r);
     tmem_ld_wait();
     if (!row_ok) continue;
-    float4* dst = reinterpret_cast<float4*>(row + c);
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      __stcg(dst + j, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                  __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
+    for (int j = 0; j < 32; j += 8) st_global_32(row + c + j, r + j);      // the workspace starts on 32 bytes
   }
 }
 
@@ -280,26 +289,29 @@ struct TcHalo<Policy, typename Policy::HasHalo> {
 template <class Policy, class = void>
 struct TcEpilogue {
   static constexpr bool kSplitK = true;     // the default epilogue can finish a split-K tile
+  template <int CW>                         // the group's columns of the tile
   __device__ static void run(uint32_t taddr, bool row_ok, long long row_off, int n0, int n_total,
                              int row_index, const EpiParams& e, const typename Policy::Params&) {
-    tc_epilogue_rows<Policy::BN>(TmemSrc{taddr}, row_ok, row_off, n0, n_total, row_index, e);
+    tc_epilogue_rows<CW>(TmemSrc{taddr}, row_ok, row_off, n0, n_total, row_index, e);
   }
 };
 template <class Policy>
 struct TcEpilogue<Policy, typename Policy::HasEpilogue> {
   static constexpr bool kSplitK = false;
+  template <int CW>
   __device__ static void run(uint32_t taddr, bool row_ok, long long row_off, int n0, int n_total,
                              int row_index, const EpiParams& e, const typename Policy::Params& p) {
     Policy::epilogue(taddr, row_ok, row_off, n0, n_total, row_index, e, p);
   }
 };
 
-// Epilogue groups of a policy: four warps each (0-3, and 6-9 for the second).  With two
-// groups each owns one of the two accumulators and drains every other tile of the CTA, so
-// that two tiles' epilogues are in flight: with a single warp per scheduler the TMEM load,
-// conversion and row stores of a tile show their full latency, which outlasts the MMAs of
-// tiles with a short reduction (convolutions with few channels, 1x1 convolutions).
-// A policy opts in with `static constexpr int kEpiGroups = 2`.
+// Epilogue groups of a policy: four warps each (0-3, 6-9, ...).  They share the columns of every
+// tile: a TMEM load, the conversion and the row stores of 32 columns show their full latency with a
+// single warp per scheduler, about 1 us, which is what a product of one wave ends with.  bf16, one group
+// a tile -> four (two 64 columns wide): 512 x 3072 x 1024 in tiles of 128 columns 10.8 -> 9.2 us, K 64 in tiles of 256
+// 11.4 -> 7.2, of 128 7.4 -> 5.5.  Convolutions have many tiles a block and keep two groups: 29 us either way
+// for 128 channels at stride 2, 30 with four; their split deep layers 11.4 -> 10.5.
+// A policy opts in with `static constexpr int kEpiGroups`.
 template <class Policy, class = void>
 struct TcEpiGroups { static constexpr int value = 1; };
 template <class Policy>
@@ -350,7 +362,7 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&sh.tmem_full[a]), 1);
-      mbar_init(smem_u32(&sh.tmem_empty[a]), 4);  // one arrive per epilogue warp
+      mbar_init(smem_u32(&sh.tmem_empty[a]), 4 * TcEpiGroups<Policy>::value);  // one arrive per epilogue warp
     }
     sh.abort_flag = 0;
     mbar_fence_init();
@@ -509,18 +521,19 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
     }
   } else {
     // ------------------------------- epilogue -------------------------------
-    constexpr int EG = TcEpiGroups<Policy>::value;
-    const int eg = (EG > 1 && warp >= 6) ? 1 : 0;
+    constexpr int CW = BN / TcEpiGroups<Policy>::value;      // this group's columns of a tile
+    const int eg = warp < 4 ? 0 : (warp - 2) >> 2;
     const int quarter = warp & 3;                    // TMEM lane quarter this warp may read
-    uint32_t local_tile = (uint32_t)eg;
+    uint32_t local_tile = 0;
     bool ok = true;
-    for (long long wl = (long long)blockIdx.x + (long long)eg * n_workers; wl < num_items && ok;
-         wl += (long long)EG * n_workers, local_tile += EG) {
-      const int w = (int)wl;
+    for (int w = blockIdx.x; w < num_items && ok; w += n_workers, ++local_tile) {
       const int t = w / splits;
       const typename Policy::Tile tile = Policy::decode(p, t);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
+      const int n0 = Policy::col0(p, tile) + eg * CW, n_total = Policy::ncols(p);
+      if (TcEpilogue<Policy>::kSplitK && p.epi.bias_mode == 1 && lane * 32 < CW && n0 + lane * 32 < n_total)
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.epi.bias + n0 + lane * 32));   // while the MMAs run
       // The verdict is made warp-uniform: tcgen05.ld below is a warp-collective.
       const bool landed = __all_sync(
           0xffffffffu, mbar_wait_bounded(smem_u32(&sh.tmem_full[acc]), acc_ph, abort_flag));
@@ -533,18 +546,16 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
       const int row = quarter * 32 + lane;
       long long row_off = 0;
       const bool row_ok = Policy::row_addr(p, tile, row, row_off);
-      const int n0 = Policy::col0(p, tile);
-      const int n_total = Policy::ncols(p);
       const int row_index = Policy::row_index(p, tile, row);
       const EpiParams& e = p.epi;
-      const uint32_t taddr = tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16);
+      const uint32_t taddr = tmem_base + acc * BN + eg * CW + (static_cast<uint32_t>(quarter * 32) << 16);
       if (splits == 1) {
-        TcEpilogue<Policy>::run(taddr, row_ok, row_off, n0, n_total, row_index, e, p);
+        TcEpilogue<Policy>::template run<CW>(taddr, row_ok, row_off, n0, n_total, row_index, e, p);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sh.tmem_empty[acc]));
       } else {
-        tc_splitk_store<BN>(taddr, e.sk_ws + ((long long)w * kBM + row) * BN, row_ok, n0, n_total);
+        tc_splitk_store<CW>(taddr, e.sk_ws + ((long long)w * kBM + row) * BN + eg * CW, row_ok, n0, n_total);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sh.tmem_empty[acc]));
