@@ -267,13 +267,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     RingPos acc;
     bool ok = true;
     for (int t = first; t < p.num_tiles && ok; t += step, acc.advance(2)) {
+      const PairTile tl = pair_tile(p, t);
+      LaneBias<128> bias;
+      bias.load(p.bias_mode == 1 ? p.bias : nullptr, tl.n0 + eg * 128, p.N, lane);
       ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.tmem_full[acc.s]), acc.ph, abort_flag));
       if (!ok) {
         if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
         break;
       }
       tc_fence_after();
-      const PairTile tl = pair_tile(p, t);
       const int row0 = tl.m0 + (int)rank * 128 + quarter * 32;
       const bool rows_ok = row0 < p.M;
       const uint32_t taddr = tmem + acc.s * 256 + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -282,26 +284,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       for (int c = eg * 128; c < eg * 128 + 128 && rows_ok; c += width) {
         const int n = tl.n0 + c;
         if (n >= p.N) break;
+        uint32_t q[2][32];
+        tmem_ld_32x32(taddr + c, q[0]);
+        if (width == 64) tmem_ld_32x32(taddr + c + 32, q[1]);
         if (lane == 0) bulk_wait_read<0>();                      // the staging rows have been read
         __syncwarp();
-#pragma unroll 1
-        for (int h = 0; h < width; h += 32) {
-          uint32_t r[32];
-          tmem_ld_32x32(taddr + c + h, r);
-          tmem_ld_wait();
+        tmem_ld_wait();
+#pragma unroll
+        for (int hh = 0; hh < 2; ++hh) {
+          const int h = hh * 32;
+          if (h >= width) break;
           float v[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha + row_bias;
-          if (p.bias_mode == 1) {
-            if (n + h + 32 <= p.N) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) v[j] += __ldg(p.bias + n + h + j);
-            } else {
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (n + h + j < p.N) v[j] += __ldg(p.bias + n + h + j);
-            }
-          }
+          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(q[hh][j]) * p.alpha + row_bias;
+          if (p.bias_mode == 1) bias.add(v, (c - eg * 128 + h) / 32);
           tc_apply_act32(v, p.act, p.act_param);
           if (p.out_dtype == kF32) {
 #pragma unroll
@@ -331,7 +327,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(empty0 + acc.s * 8u);
     }
-    if (lane == 0) bulk_wait<0>();
+    if (lane == 0) bulk_wait_read<0>();      // the rows are written when the grid is through
     __syncwarp();
   }
   tc_fence_before();

@@ -113,6 +113,24 @@ struct TmemSrc {                 // this warp's lanes of a TMEM accumulator
     for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
   }
 };
+// Bias of a group's columns: lane l holds that of column 32 i + l, loaded while the MMAs run and handed round by
+// shuffles.  (Loaded where it is added, a value at a time, 1.2 us more for a 256 x 256 tile: each 32 columns wait for
+// L2 again.)
+template <int CW>
+struct LaneBias {
+  float v[CW / 32];
+  __device__ __forceinline__ void load(const float* bias, int n0, int n_total, int lane) {
+#pragma unroll
+    for (int i = 0; i < CW / 32; ++i) v[i] = bias && n0 + i * 32 + lane < n_total ? __ldg(bias + n0 + i * 32 + lane) : 0.f;
+  }
+  __device__ __forceinline__ void add(float (&x)[32], int chunk) const {        // all lanes of the warp
+    float b = v[0];
+#pragma unroll
+    for (int i = 1; i < CW / 32; ++i) b = chunk == i ? v[i] : b;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) x[j] += __shfl_sync(0xffffffffu, b, j);
+  }
+};
 // 32 bytes, a whole sector, of a lane's row; the address on 32 bytes.
 __device__ __forceinline__ void st_global_32(void* p, const uint32_t* q) {
   asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(q[0]), "r"(q[1]), "r"(q[2]),
@@ -122,7 +140,7 @@ __device__ __forceinline__ void st_global_32(void* p, const uint32_t* q) {
 template <int BN, class Src>
 __device__ __forceinline__ void tc_epilogue_rows(const Src& src, bool row_ok, long long row_off,
                                                  int n0, int n_total, int row_index,
-                                                 const EpiParams& e) {
+                                                 const EpiParams& e, const LaneBias<BN>* lane_bias = nullptr) {
   const float alpha = e.alpha, beta = e.beta;
   const int bias_mode = e.bias_mode, act = e.act, out_dtype = e.out_dtype;
   const float row_bias = bias_mode == 2 ? e.bias[row_index] : 0.f;
@@ -131,9 +149,10 @@ __device__ __forceinline__ void tc_epilogue_rows(const Src& src, bool row_ok, lo
     if (n0 + c >= n_total) break;  // warp-uniform
     float v[32];
     src.load(c, v);
-    if (!row_ok) continue;
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = v[j] * alpha + row_bias;
+    if (lane_bias && bias_mode == 1) lane_bias->add(v, c / 32);
+    if (!row_ok) continue;
     const long long off = row_off + n0 + c;
     const int ncol = min(32, n_total - (n0 + c));
     const bool full = ncol == 32;
@@ -161,7 +180,7 @@ __device__ __forceinline__ void tc_epilogue_rows(const Src& src, bool row_ok, lo
       }
       continue;
     }
-    if (bias_mode == 1) {
+    if (!lane_bias && bias_mode == 1) {
       const float* bp = e.bias + n0 + c;
       if (full) {
 #pragma unroll
@@ -291,8 +310,9 @@ struct TcEpilogue {
   static constexpr bool kSplitK = true;     // the default epilogue can finish a split-K tile
   template <int CW>                         // the group's columns of the tile
   __device__ static void run(uint32_t taddr, bool row_ok, long long row_off, int n0, int n_total,
-                             int row_index, const EpiParams& e, const typename Policy::Params&) {
-    tc_epilogue_rows<CW>(TmemSrc{taddr}, row_ok, row_off, n0, n_total, row_index, e);
+                             int row_index, const EpiParams& e, const typename Policy::Params&,
+                             const LaneBias<CW>& bias) {
+    tc_epilogue_rows<CW>(TmemSrc{taddr}, row_ok, row_off, n0, n_total, row_index, e, &bias);
   }
 };
 template <class Policy>
@@ -300,7 +320,7 @@ struct TcEpilogue<Policy, typename Policy::HasEpilogue> {
   static constexpr bool kSplitK = false;
   template <int CW>
   __device__ static void run(uint32_t taddr, bool row_ok, long long row_off, int n0, int n_total,
-                             int row_index, const EpiParams& e, const typename Policy::Params& p) {
+                             int row_index, const EpiParams& e, const typename Policy::Params& p, const LaneBias<CW>&) {
     Policy::epilogue(taddr, row_ok, row_off, n0, n_total, row_index, e, p);
   }
 };
@@ -308,8 +328,8 @@ struct TcEpilogue<Policy, typename Policy::HasEpilogue> {
 // Epilogue groups of a policy: four warps each (0-3, 6-9, ...).  They share the columns of every
 // tile: a TMEM load, the conversion and the row stores of 32 columns show their full latency with a
 // single warp per scheduler, about 1 us, which is what a product of one wave ends with.  bf16, one group
-// a tile -> four (two 64 columns wide): 512 x 3072 x 1024 in tiles of 128 columns 10.8 -> 9.2 us, K 64 in tiles of 256
-// 11.4 -> 7.2, of 128 7.4 -> 5.5.  Convolutions have many tiles a block and keep two groups: 29 us either way
+// a tile -> four (two 64 columns wide): 512 x 3072 x 1024 in tiles of 128 columns 10.8 -> 9.0 us, K 64 in tiles of 256
+// 11.4 -> 6.8, of 128 7.4 -> 5.3.  Convolutions have many tiles a block and keep two groups: 29 us either way
 // for 128 channels at stride 2, 30 with four; their split deep layers 11.4 -> 10.5.
 // A policy opts in with `static constexpr int kEpiGroups`.
 template <class Policy, class = void>
@@ -532,8 +552,8 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_ph = (local_tile >> 1) & 1;
       const int n0 = Policy::col0(p, tile) + eg * CW, n_total = Policy::ncols(p);
-      if (TcEpilogue<Policy>::kSplitK && p.epi.bias_mode == 1 && lane * 32 < CW && n0 + lane * 32 < n_total)
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(p.epi.bias + n0 + lane * 32));   // while the MMAs run
+      LaneBias<CW> bias;
+      bias.load(TcEpilogue<Policy>::kSplitK && splits == 1 && p.epi.bias_mode == 1 ? p.epi.bias : nullptr, n0, n_total, lane);
       // The verdict is made warp-uniform: tcgen05.ld below is a warp-collective.
       const bool landed = __all_sync(
           0xffffffffu, mbar_wait_bounded(smem_u32(&sh.tmem_full[acc]), acc_ph, abort_flag));
@@ -550,7 +570,7 @@ tc_persistent_kernel(const __grid_constant__ CUtensorMap tmA,
       const EpiParams& e = p.epi;
       const uint32_t taddr = tmem_base + acc * BN + eg * CW + (static_cast<uint32_t>(quarter * 32) << 16);
       if (splits == 1) {
-        TcEpilogue<Policy>::template run<CW>(taddr, row_ok, row_off, n0, n_total, row_index, e, p);
+        TcEpilogue<Policy>::template run<CW>(taddr, row_ok, row_off, n0, n_total, row_index, e, p, bias);
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sh.tmem_empty[acc]));
