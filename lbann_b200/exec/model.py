@@ -18,7 +18,7 @@ from typing import Callable, Dict, List, Optional
 
 import torch
 
-from ..ops import native
+from ..ops import native, nn
 from ..ops.optim import ParameterArena
 from ..proto import lbann_pb2 as pb
 from . import layers_core, layers_misc  # noqa: F401  (populate the registry)
@@ -642,25 +642,25 @@ class ExecModel:
         self.acts = acts
         return acts
 
-    def _layer_mean(self, layer_name: str) -> torch.Tensor:
-        """Sum over the local mini-batch divided by the global mini-batch size."""
+    def _layer_mean(self, layer_name: str, scale: float = 1.0, scaled: bool = False) -> torch.Tensor:
+        """Sum over the local mini-batch divided by the global mini-batch size (``scaled``: times ``scale``)."""
         hit = self._mean_cache.get(layer_name)      # objective term and metric often coincide
         if hit is not None:
-            return hit
+            return hit * scale if scaled else hit
         layer = self.layers_by_name[layer_name]
         y = self.acts[layer_name][0] if self.acts[layer_name] else self.acts[layer.parent_names[0]][0]
         if y is None:        # computed on a sub-grid this rank does not belong to
             val = torch.zeros((), device=self.device)
             self._mean_cache[layer_name] = val
             return val
-        val = y.float().sum() / float(self._global_mb)
+        val, term = nn.objective_term(y, self._global_mb, scale)
         self._mean_cache[layer_name] = val
-        return val
+        return term if scaled else val
 
     def local_objective(self) -> torch.Tensor:
         total = None
         for name, scale in self.objective_terms:
-            v = self._layer_mean(name) * scale
+            v = self._layer_mean(name, scale, scaled=True)
             total = v if total is None else total + v
         if total is None:
             total = torch.zeros((), device=self.device)
@@ -689,11 +689,13 @@ class ExecModel:
         st = self.stats[mode]
         n = self._global_mb
         with torch.no_grad():
-            st.obj_sum.add_(local_obj.detach(), alpha=n)
+            sums, values = [st.obj_sum], [local_obj.detach()]
             st.samples += n
             for i, m in enumerate(self.metrics):
                 if getattr(m, "layer_name", None):
-                    st.metric_sums[i].add_(self._layer_mean(m.layer_name).detach(), alpha=n)
+                    sums.append(st.metric_sums[i])
+                    values.append(self._layer_mean(m.layer_name).detach())
+            nn.add_statistics(sums, values, n)
 
     def clear_gradients(self):
         self.arena.zero_grad()
@@ -782,7 +784,8 @@ class ExecModel:
             if not self.amp_enabled:
                 local_obj.backward()
             elif self.device.type == "cuda":
-                (local_obj * self._amp_device_state()[0]).backward()     # no host read of the scale
+                # the scale as the objective's gradient: no host read of it, and no product
+                local_obj.backward(self._amp_device_state()[0].to(local_obj.dtype))
             else:
                 (local_obj * self._amp_scale_host).backward()
         self.arena.end_gradients()

@@ -92,6 +92,14 @@ def _lib():
         lib.lb_pool_bwd_tiled.restype = c_int
         lib.lb_pool_bwd_tiled.argtypes = [c_void_p, c_void_p, c_void_p, P(c_int), c_int, c_float,
                                           c_int, c_void_p]
+        lib.lb_pack_first.restype = c_int
+        lib.lb_pack_first.argtypes = [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]
+        lib.lb_objective_fwd.restype = c_int
+        lib.lb_objective_fwd.argtypes = [c_void_p, c_ll, c_float, c_float, c_void_p, c_int, c_void_p]
+        lib.lb_objective_bwd.restype = c_int
+        lib.lb_objective_bwd.argtypes = [c_void_p, c_float, c_float, c_void_p, c_ll, c_int, c_void_p]
+        lib.lb_add_statistics.restype = c_int
+        lib.lb_add_statistics.argtypes = [P(c_void_p), P(c_void_p), c_int, ctypes.c_double, c_void_p]
         lib.lb_conv_c8_fwd.restype = c_int
         lib.lb_conv_c8_fwd.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, P(c_int), P(c_ll),
                                        P(c_ll), c_int, c_int, c_int, c_float, c_void_p]
@@ -326,6 +334,22 @@ def _first_layer_pixels(x, cr: int):
     return x_cl if x_cl.is_contiguous() else x_cl.contiguous()
 
 
+def _pack_first(wh, Kout: int, Cin: int, taps: int, cr: int, dtype) -> torch.Tensor:
+    """Filters of a first-layer kernel: K index = tap * cr + channel, padded to a multiple of 16; rows
+    padded to 32; [K chunk][32 rows][8 elements]."""
+    m, kpad = wh.master.detach(), (taps * cr + 15) // 16 * 16
+    if m.is_cuda and m.dtype == torch.float32 and m.is_contiguous():
+        out = torch.empty(kpad // 8, 32, 8, dtype=dtype, device=m.device)
+        native.check(_lib().lb_pack_first(m.data_ptr(), out.data_ptr(), Kout, Cin, taps, cr, kpad,
+                                          native.dtype_code(dtype), native.stream_ptr()), "lb_pack_first")
+        native.count_launch()
+        return out
+    w = m.reshape(Kout, Cin, taps).permute(0, 2, 1)   # K, tap, C
+    w = F.pad(w, (0, cr - Cin)).reshape(Kout, -1)
+    w = F.pad(w, (0, kpad - w.shape[1], 0, 32 - Kout))
+    return w.reshape(32, kpad // 8, 8).permute(1, 0, 2).contiguous().to(dtype)
+
+
 class _ConvC8(torch.autograd.Function):
     """First-layer convolution: at most 8 input channels, kernel (kd, kh, 3), stride 1, no
     dilation, "same" padding along W.  Forward and filter gradient use the dedicated
@@ -343,17 +367,7 @@ class _ConvC8(torch.autograd.Function):
         x_bwd = x_cl
         Kout = wh.master.shape[0]
         kd, kh, _ = ksize
-
-        def pack():
-            # K index = tap * cr + channel, padded to a multiple of 16; rows padded to 32
-            w = wh.master.detach().reshape(Kout, Cin, kd * kh * 3).permute(0, 2, 1)   # K, tap, C
-            w = F.pad(w, (0, cr - Cin)).reshape(Kout, -1)
-            kpad = (w.shape[1] + 15) // 16 * 16
-            w = F.pad(w, (0, kpad - w.shape[1], 0, 32 - Kout))
-            # [K chunk][32 rows][8 elements]
-            return w.reshape(32, kpad // 8, 8).permute(1, 0, 2).contiguous().to(x.dtype)
-
-        wt = wh.packed("c8fwd", x.dtype, pack)
+        wt = wh.packed("c8fwd", x.dtype, lambda: _pack_first(wh, Kout, Cin, kd * kh * 3, cr, x.dtype))
         N, D, H, W, _ = x_cl.shape
         Do = D + 2 * pad[0] - kd + 1
         y = torch.empty((N, Do, H, W, Kout), dtype=x.dtype, device=x.device)
@@ -429,15 +443,7 @@ class _ConvC8Pool(torch.autograd.Function):
         Cin = x.shape[1]
         x_cl = _first_layer_pixels(x, 4)
         Kout = wh.master.shape[0]
-
-        def pack():
-            w = wh.master.detach().reshape(Kout, Cin, 27).permute(0, 2, 1)
-            w = F.pad(w, (0, 4 - Cin)).reshape(Kout, -1)
-            kpad = (w.shape[1] + 15) // 16 * 16
-            w = F.pad(w, (0, kpad - w.shape[1], 0, 32 - Kout))
-            return w.reshape(32, kpad // 8, 8).permute(1, 0, 2).contiguous().to(x.dtype)
-
-        wt = wh.packed("c8fwd", x.dtype, pack)
+        wt = wh.packed("c8fwd", x.dtype, lambda: _pack_first(wh, Kout, Cin, 27, 4, x.dtype))
         N, D, H, W, _ = x_cl.shape
         Do = D + 2 * pad[0] - 2
         shape = (N, Do // 2, H // 2, W // 2, Kout)
@@ -1076,6 +1082,63 @@ def softmax_cross_entropy(logits, labels):
     lp = F.log_softmax(logits.float().reshape(-1, C), -1)
     picked = lp.gather(1, lab.clamp(0, C - 1)[:, None])[:, 0]
     return torch.where(ok, -picked, torch.zeros_like(picked)).reshape(logits.shape[:-1])
+
+
+class _ObjectiveTerm(torch.autograd.Function):
+    """(sum of y / mini-batch, that times scale): csrc/objective.cu."""
+
+    @staticmethod
+    def forward(ctx, y, mini_batch, scale):
+        out = torch.empty(2, dtype=torch.float32, device=y.device)
+        inv = 1.0 / mini_batch
+        native.check(_lib().lb_objective_fwd(y.data_ptr(), y.numel(), inv, scale, out.data_ptr(),
+                                             native.dtype_code(y.dtype), native.stream_ptr()), "lb_objective_fwd")
+        native.count_launch()
+        ctx.set_materialize_grads(False)
+        ctx.meta = (y.shape, y.dtype, inv, scale)
+        return out[0], out[1]
+
+    @staticmethod
+    def backward(ctx, g_mean, g_term):
+        shape, dtype, inv, scale = ctx.meta
+        if g_mean is None and g_term is None:
+            return None, None, None
+        if g_mean is not None:        # somebody differentiates the mean itself
+            g = g_mean if g_term is None else g_mean + g_term * scale
+            scale = 1.0
+        else:
+            g = g_term
+        g = g.float().contiguous()
+        dy = torch.empty(shape, dtype=dtype, device=g.device)
+        native.check(_lib().lb_objective_bwd(g.data_ptr(), scale, inv, dy.data_ptr(), dy.numel(),
+                                             native.dtype_code(dtype), native.stream_ptr()), "lb_objective_bwd")
+        native.count_launch()
+        return dy, None, None
+
+
+def objective_term(y, mini_batch: float, scale: float):
+    """-> (sum over ``y`` / ``mini_batch``, the same times ``scale``), fp32 scalars."""
+    # one block adds them up: 65536 values take it 10 us
+    if y.is_cuda and y.is_contiguous() and 0 < y.numel() <= 65536 and \
+            y.dtype in (torch.float16, torch.bfloat16, torch.float32):
+        return _ObjectiveTerm.apply(y, float(mini_batch), float(scale))
+    mean = y.float().sum() / float(mini_batch)
+    return mean, mean * scale
+
+
+def add_statistics(sums, values, weight: float) -> None:
+    """sums[i] += weight * values[i] (fp64 and fp32 scalars)."""
+    if not all(s.is_cuda and s.dtype == torch.float64 and v.is_cuda and v.dtype == torch.float32
+               for s, v in zip(sums, values)):
+        for s, v in zip(sums, values):
+            s.add_(v, alpha=weight)
+        return
+    for i in range(0, len(sums), 8):
+        part = list(zip(sums[i:i + 8], values[i:i + 8]))
+        ptrs = [(c_void_p * len(part))(*(t.data_ptr() for t in col)) for col in zip(*part)]
+        native.check(_lib().lb_add_statistics(ptrs[0], ptrs[1], len(part), float(weight), native.stream_ptr()),
+                     "lb_add_statistics")
+        native.count_launch()
 
 
 _LOSS_KIND = {"cross_entropy": 0, "mean_squared_error": 1, "mean_absolute_error": 2,
