@@ -23,6 +23,8 @@
 // Every wait is bounded; a wait that runs out records a status code and all roles leave.
 #include <type_traits>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace lb {
@@ -491,8 +493,13 @@ attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __
 // TMEM: through shared memory they cost as much of its bandwidth as half the MMAs.  The issuer
 // starts step i + 1's scores before it waits for step i's probabilities.  One arrival per warp (256
 // single arrivals on a barrier took longer than the exponentials).
-// B = 2, H = 16, S = 2048, causal, bf16: 308 us as two kernels with one step in flight -> 161 us
-// with P and dS in shared memory -> 154 us; about 25 of them are the CTAs' beginnings and ends.
+// The CTAs stay and take items in turn: the next item's operands arrive and its first scores run while
+// the rows of the last one are written.
+// B = 2, H = 16, S = 2048, bf16: causal 308 us as two kernels with one step in flight -> 161 with P and dS in
+// shared memory -> 153 with a CTA an item -> 142; not causal 242 -> 226.  What is left is a step's 16 MMAs of
+// N = 64, which read 128 rows of A for half the arithmetic (48-58 cycles for 32), and about 400 cycles from the
+// end of an accumulation to the scores that overwrite its operands: rows that do nothing leave 124 us.
+// (Waiting for P and dS separately: 143; scores read into registers first, P and dS elsewhere: 157; 16 row warps: no change.)
 // ------------------------------------------------------------------------------------
 constexpr int kBwdCols = 64;                          // streamed rows (= score columns) per step
 constexpr int kBwdTile = kBwdCols * kAttD * 2;        // 16 KB: one streamed operand
@@ -504,6 +511,8 @@ struct __align__(128) AttnBwdShared {
   float lse[kBwdStages][kBwdCols];     // keys: of the streamed queries
   float delta[kBwdStages][kBwdCols];
   uint64_t resident;                   // the operands that stay have landed
+  uint64_t res_empty;                  // their last scores have retired
+  uint64_t acc_empty;                  // the accumulators have been read (8 warps)
   uint64_t st_full[kBwdStages];        // a stage has landed
   uint64_t st_empty[kBwdStages];       // the MMAs of a step have retired: stage, P and dS are free
   uint64_t s_full[2];                  // scores and dP of a step are complete
@@ -566,159 +575,190 @@ __device__ __forceinline__ void bwd_probabilities(const uint32_t (&rs)[32], cons
   }
 }
 
-template <bool KV>
-__device__ __forceinline__ void attn_bwd_cta(const CUtensorMap* tmR0, const CUtensorMap* tmR1, const CUtensorMap* tmT0,
-                                             const CUtensorMap* tmT1, const AttnParams& p, int blk, int h, int b,
-                                             uint32_t base, AttnBwdShared& sh, int* status) {
-  const uint32_t sR0 = base, sR1 = base + kAttTile, sT = base + 2 * kAttTile;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  volatile int* abort_flag = &sh.abort_flag;
-  const int steps_all = (KV ? p.Sq : p.Sk) / kBwdCols;
-  const int i0 = KV && p.causal ? 2 * blk : 0;                   // first step that sees these rows
-  const int iters = KV ? steps_all - i0 : (p.causal ? 2 * blk + 2 : steps_all);
-  const uint32_t tmem = sh.tmem_base, tAcc0 = tmem + 256, tAcc1 = tmem + 384;
-  const long long stat0 = ((long long)b * p.H + h) * p.Sq;       // this head's lse / delta
-
-  if (warp == 4) {
-    if (elect_one()) {
-      mbar_expect_tx(smem_u32(&sh.resident), 2 * kAttTile);
-      att_load_tile(sR0, tmR0, smem_u32(&sh.resident), h, blk * 128, b);
-      att_load_tile(sR1, tmR1, smem_u32(&sh.resident), h, blk * 128, b);
-      RingPos rp;
-      int it = 0;
-      bool ok = true;
-      for (; it < iters; ++it) {
-        if (!mbar_wait_bounded(smem_u32(&sh.st_empty[rp.s]), rp.ph ^ 1, abort_flag)) {
-          raise_status(status, abort_flag, kTimeoutStageEmpty);
-          ok = false;
-          break;
-        }
-        const uint32_t bar = smem_u32(&sh.st_full[rp.s]), dst = sT + rp.s * 2 * kBwdTile;
-        const int r0 = (i0 + it) * kBwdCols;
-        mbar_expect_tx(bar, 2 * kBwdTile + (KV ? 2 * kBwdCols * 4 : 0));
-        tma_load_4d(dst, tmT0, bar, 0, h, r0, b);
-        tma_load_4d(dst + kBwdHalf, tmT0, bar, 64, h, r0, b);
-        tma_load_4d(dst + kBwdTile, tmT1, bar, 0, h, r0, b);
-        tma_load_4d(dst + kBwdTile + kBwdHalf, tmT1, bar, 64, h, r0, b);
-        if (KV) {
-          bulk_load_1d(smem_u32(sh.lse[rp.s]), p.lse + stat0 + r0, kBwdCols * 4, bar);
-          bulk_load_1d(smem_u32(sh.delta[rp.s]), p.delta + stat0 + r0, kBwdCols * 4, bar);
-        }
-        rp.advance(kBwdStages);
-      }
-      if (!ok || *abort_flag) {        // the copies in flight land before shared memory is released
-        mbar_wait_budget_only(smem_u32(&sh.resident), 0);
-        for (int j = it > kBwdStages ? it - kBwdStages : 0; j < it; ++j)
-          mbar_wait_budget_only(smem_u32(&sh.st_full[j % kBwdStages]), (j / kBwdStages) & 1);
-      }
-    }
-  } else if (warp == 5) {
-    if (elect_one()) {
-      const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
-      const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, 128, kBwdCols);
-      const uint32_t idesc_a = make_idesc_f16(fmt, 0, 1, 128, 128);
-      bool ok = mbar_wait_bounded(smem_u32(&sh.resident), 0, abort_flag);
-      if (!ok) raise_status(status, abort_flag, kTimeoutTmaFull);
-      RingPos next, cur;               // stages of the scores' step and of the accumulating step
-      for (int it = -1; it < iters && ok; ++it) {
-        if (it + 1 < iters) {          // scores of the next step, over the P and dS of step it - 1
-          const int n = it + 1, j = n - 2;
-          if (!mbar_wait_bounded(smem_u32(&sh.st_full[next.s]), next.ph, abort_flag) ||
-              (j >= 0 && !mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1, abort_flag))) {
-            raise_status(status, abort_flag, kTimeoutTmaFull);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t t = sT + next.s * 2 * kBwdTile, d = tmem + (n & 1) * 128;
-          bwd_mma_scores(d, sR0, t, idesc_s);
-          bwd_mma_scores(d + kBwdCols, sR1, t + kBwdTile, idesc_s);
-          umma_commit(smem_u32(&sh.s_full[n & 1]));
-          next.advance(kBwdStages);
-        }
-        if (it >= 0) {
-          if (!mbar_wait_bounded(smem_u32(&sh.p_full[it & 1]), (it >> 1) & 1, abort_flag)) {
-            raise_status(status, abort_flag, kTimeoutTmemEmpty);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t t = sT + cur.s * 2 * kBwdTile;
-          const uint32_t tP = tmem + (it & 1) * 128;
-          if (KV) bwd_mma_accumulate(tAcc0, tP, t + kBwdTile, idesc_a, it > 0);
-          bwd_mma_accumulate(tAcc1, tP + kBwdCols, t, idesc_a, it > 0);
-          umma_commit(smem_u32(&sh.st_empty[cur.s]));
-          cur.advance(kBwdStages);
-        }
-      }
-    }
+// One work item: 128 keys (KV) or queries of a head.
+struct BwdItem {
+  bool kv;
+  int blk, h, b, i0, iters;            // first step that sees these rows, steps
+};
+// Items in the order of their lengths, the longest first, and dealt to the CTAs forwards and backwards in turn, so
+// that the sums of the lengths are nearly the same.  False: this CTA's rounds are over.
+__device__ __forceinline__ bool bwd_item(const AttnParams& p, int round, BwdItem& w) {
+  const int nkb = p.Sk / 128, nqb = p.Sq / 128, heads = p.H * p.B, total = (nkb + nqb) * heads;
+  const int base = round * (int)gridDim.x;
+  const int idx = base + ((round & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  if (base >= total) return false;
+  w.iters = 0;
+  if (idx >= total) return true;       // an incomplete last round
+  const int z = idx / heads, hb = idx - z * heads;
+  w.b = hb / p.H;
+  w.h = hb - w.b * p.H;
+  if (p.causal) {                      // keys see the queries behind them, queries the keys before them
+    w.kv = (z & 1) == 0;
+    w.blk = w.kv ? z >> 1 : nqb - 1 - (z >> 1);
+  } else if (p.Sq >= p.Sk) {           // keys walk the queries
+    w.kv = z < nkb;
+    w.blk = w.kv ? z : z - nkb;
   } else {
-    int group = 0, quarter = 0;
-    att_row_role(warp, group, quarter);
-    const int row = quarter * 32 + lane;               // this thread's key / query; its half of the columns
-    const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    float my_lse = 0.f, my_delta = 0.f;
-    if (!KV) {
-      my_lse = p.lse[stat0 + blk * 128 + row];
-      my_delta = p.delta[stat0 + blk * 128 + row];
+    w.kv = z >= nqb;
+    w.blk = w.kv ? z - nqb : z;
+  }
+  const int all = (w.kv ? p.Sq : p.Sk) / kBwdCols;
+  w.i0 = w.kv && p.causal ? 2 * w.blk : 0;
+  w.iters = w.kv ? all - w.i0 : (p.causal ? 2 * w.blk + 2 : all);
+  return true;
+}
+
+struct BwdMaps {
+  const CUtensorMap *r0, *r1, *t0, *t1;
+};
+
+// The producer's part of an item; `step` counts the CTA's steps, `item` its items.
+template <bool KV>
+__device__ __forceinline__ bool bwd_produce(const BwdMaps& m, const AttnParams& p, const BwdItem& w, int item, uint32_t base,
+                                            AttnBwdShared& sh, RingPos& rp, int& step, volatile int* abort_flag, int* status) {
+  const uint32_t sT = base + 2 * kAttTile;
+  const long long stat0 = ((long long)w.b * p.H + w.h) * p.Sq;     // this head's lse / delta
+  if (!mbar_wait_bounded(smem_u32(&sh.res_empty), (item & 1) ^ 1, abort_flag)) {
+    raise_status(status, abort_flag, kTimeoutStageEmpty);
+    return false;
+  }
+  mbar_expect_tx(smem_u32(&sh.resident), 2 * kAttTile);
+  att_load_tile(base, m.r0, smem_u32(&sh.resident), w.h, w.blk * 128, w.b);
+  att_load_tile(base + kAttTile, m.r1, smem_u32(&sh.resident), w.h, w.blk * 128, w.b);
+  for (int it = 0; it < w.iters; ++it, ++step) {
+    if (!mbar_wait_bounded(smem_u32(&sh.st_empty[rp.s]), rp.ph ^ 1, abort_flag)) {
+      raise_status(status, abort_flag, kTimeoutStageEmpty);
+      return false;
     }
-    bool ok = true;
-    RingPos rp;
-    for (int it = 0; it < iters && ok; ++it) {
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full[it & 1]), (it >> 1) & 1, abort_flag));
-      // lse and delta of a step came with its stage
-      if (ok && KV) ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_full[rp.s]), rp.ph, abort_flag));
-      if (!ok) {
-        if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-        break;
+    const uint32_t bar = smem_u32(&sh.st_full[rp.s]), dst = sT + rp.s * 2 * kBwdTile;
+    const int r0 = (w.i0 + it) * kBwdCols;
+    mbar_expect_tx(bar, 2 * kBwdTile + (KV ? 2 * kBwdCols * 4 : 0));
+    tma_load_4d(dst, m.t0, bar, 0, w.h, r0, w.b);
+    tma_load_4d(dst + kBwdHalf, m.t0, bar, 64, w.h, r0, w.b);
+    tma_load_4d(dst + kBwdTile, m.t1, bar, 0, w.h, r0, w.b);
+    tma_load_4d(dst + kBwdTile + kBwdHalf, m.t1, bar, 64, w.h, r0, w.b);
+    if (KV) {
+      bulk_load_1d(smem_u32(sh.lse[rp.s]), p.lse + stat0 + r0, kBwdCols * 4, bar);
+      bulk_load_1d(smem_u32(sh.delta[rp.s]), p.delta + stat0 + r0, kBwdCols * 4, bar);
+    }
+    rp.advance(kBwdStages);
+  }
+  return true;
+}
+
+// The issuer's part: scores of step it + 1 before the accumulation of step it.
+template <bool KV>
+__device__ __forceinline__ bool bwd_issue(const AttnParams& p, const BwdItem& w, int item, uint32_t base, uint32_t tmem,
+                                          AttnBwdShared& sh, RingPos& next, RingPos& cur, int& step,
+                                          volatile int* abort_flag, int* status) {
+  const uint32_t sR0 = base, sR1 = base + kAttTile, sT = base + 2 * kAttTile, tAcc0 = tmem + 256, tAcc1 = tmem + 384;
+  const uint32_t fmt = p.in_dtype == kBF16 ? 1u : 0u;
+  const uint32_t idesc_s = make_idesc_f16(fmt, 0, 0, 128, kBwdCols);
+  const uint32_t idesc_a = make_idesc_f16(fmt, 0, 1, 128, 128);
+  if (!mbar_wait_bounded(smem_u32(&sh.resident), item & 1, abort_flag)) {
+    raise_status(status, abort_flag, kTimeoutTmaFull);
+    return false;
+  }
+  for (int it = -1; it < w.iters; ++it) {
+    if (it + 1 < w.iters) {          // over the P and dS of two steps before
+      const int n = step + it + 1, j = n - 2;
+      if (!mbar_wait_bounded(smem_u32(&sh.st_full[next.s]), next.ph, abort_flag) ||
+          (j >= 0 && !mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1, abort_flag))) {
+        raise_status(status, abort_flag, kTimeoutTmaFull);
+        return false;
       }
       tc_fence_after();
-      const uint32_t tS = tmem + (it & 1) * 128 + lane_off;
-      const int c = group * 32;
-      uint32_t rs[32], rd[32], pk[16], dk[16];
-      tmem_ld_32x32(tS + c, rs);
-      tmem_ld_32x32(tS + kBwdCols + c, rd);
-      tmem_ld_wait();
-      // causal: query >= key; distance of these columns from this CTA's first row
-      const int off = p.causal ? (i0 + it) * kBwdCols + c - blk * 128 : 0;
-      const int first = KV && p.causal ? row - off : 0;
-      const int last = !KV && p.causal ? row - off : 31;
-      bwd_probabilities<KV>(rs, rd, sh.lse[rp.s] + c, sh.delta[rp.s] + c, my_lse, my_delta, first, last, p, pk, dk);
-      // two to a column, over scores that this thread has read
-      if (KV) tmem_st_32x16(tS + c, pk);
-      tmem_st_32x16(tS + kBwdCols + c, dk);
-      tmem_st_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sh.p_full[it & 1]));
-      rp.advance(kBwdStages);
+      const uint32_t t = sT + next.s * 2 * kBwdTile, d = tmem + (n & 1) * 128;
+      bwd_mma_scores(d, sR0, t, idesc_s);
+      bwd_mma_scores(d + kBwdCols, sR1, t + kBwdTile, idesc_s);
+      umma_commit(smem_u32(&sh.s_full[n & 1]));
+      if (it + 2 == w.iters) umma_commit(smem_u32(&sh.res_empty));
+      next.advance(kBwdStages);
     }
-    if (ok && iters > 0) {
-      const int j = iters - 1;
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1,
-                                                     abort_flag));
-      if (!ok && lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
-    }
-    if (ok) {
-      tc_fence_after();
-      const long long r = (long long)blk * 128 + row;
-      const int d0 = group * 64;                       // this thread's half of the head dimension
-      uint32_t ra[32], rb[32];
-      if (KV) {
-        uint16_t* dv = reinterpret_cast<uint16_t*>(p.dv) + b * p.dv_sb + r * p.dv_ss + h * p.dv_sh + d0;
-        tmem_ld_32x32(tAcc0 + lane_off + d0, ra);
-        tmem_ld_32x32(tAcc0 + lane_off + d0 + 32, rb);
-        tmem_ld_wait();
-        att_store_out64(dv, ra, rb, 1.f, p.in_dtype);
+    if (it >= 0) {
+      const int n = step + it;
+      if ((it == 0 && !mbar_wait_bounded(smem_u32(&sh.acc_empty), (item & 1) ^ 1, abort_flag)) ||
+          !mbar_wait_bounded(smem_u32(&sh.p_full[n & 1]), (n >> 1) & 1, abort_flag)) {
+        raise_status(status, abort_flag, kTimeoutTmemEmpty);
+        return false;
       }
-      uint16_t* out = KV ? reinterpret_cast<uint16_t*>(p.dk) + b * p.dk_sb + r * p.dk_ss + h * p.dk_sh + d0
-                         : reinterpret_cast<uint16_t*>(p.dq) + b * p.dq_sb + r * p.dq_ss + h * p.dq_sh + d0;
-      tmem_ld_32x32(tAcc1 + lane_off + d0, ra);
-      tmem_ld_32x32(tAcc1 + lane_off + d0 + 32, rb);
-      tmem_ld_wait();
-      att_store_out64(out, ra, rb, 1.f, p.in_dtype);
+      tc_fence_after();
+      const uint32_t t = sT + cur.s * 2 * kBwdTile;
+      const uint32_t tP = tmem + (n & 1) * 128;
+      if (KV) bwd_mma_accumulate(tAcc0, tP, t + kBwdTile, idesc_a, it > 0);
+      bwd_mma_accumulate(tAcc1, tP + kBwdCols, t, idesc_a, it > 0);
+      umma_commit(smem_u32(&sh.st_empty[cur.s]));
+      cur.advance(kBwdStages);
     }
   }
+  step += w.iters;
+  return true;
+}
+
+// A row warp's part: probabilities and dS of every step, then the accumulators' rows.
+template <bool KV>
+__device__ __forceinline__ bool bwd_rows(const AttnParams& p, const BwdItem& w, int group, int quarter, uint32_t tmem,
+                                         AttnBwdShared& sh, RingPos& rp, int& step, float my_lse, float my_delta,
+                                         volatile int* abort_flag, int* status) {
+  const int lane = threadIdx.x & 31;
+  const int row = quarter * 32 + lane;               // this thread's key / query; its half of the columns
+  const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
+  for (int it = 0; it < w.iters; ++it, ++step) {
+    bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.s_full[step & 1]), (step >> 1) & 1, abort_flag));
+    // lse and delta of a step came with its stage
+    if (ok && KV) ok = __all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_full[rp.s]), rp.ph, abort_flag));
+    if (!ok) {
+      if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+      return false;
+    }
+    tc_fence_after();
+    const uint32_t tS = tmem + (step & 1) * 128 + lane_off;
+    const int c = group * 32;
+    uint32_t rs[32], rd[32], pk[16], dk[16];
+    tmem_ld_32x32(tS + c, rs);
+    tmem_ld_32x32(tS + kBwdCols + c, rd);
+    tmem_ld_wait();
+    // causal: query >= key; distance of these columns from this item's first row
+    const int off = p.causal ? (w.i0 + it) * kBwdCols + c - w.blk * 128 : 0;
+    const int first = KV && p.causal ? row - off : 0;
+    const int last = !KV && p.causal ? row - off : 31;
+    bwd_probabilities<KV>(rs, rd, sh.lse[rp.s] + c, sh.delta[rp.s] + c, my_lse, my_delta, first, last, p, pk, dk);
+    // two to a column, over scores that this thread has read
+    if (KV) tmem_st_32x16(tS + c, pk);
+    tmem_st_32x16(tS + kBwdCols + c, dk);
+    tmem_st_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sh.p_full[step & 1]));
+    rp.advance(kBwdStages);
+  }
+  const int j = step - 1;
+  if (!__all_sync(0xffffffffu, mbar_wait_bounded(smem_u32(&sh.st_empty[j % kBwdStages]), (j / kBwdStages) & 1, abort_flag))) {
+    if (lane == 0) raise_status(status, abort_flag, kTimeoutTmemFull);
+    return false;
+  }
+  tc_fence_after();
+  const long long r = (long long)w.blk * 128 + row;
+  const int d0 = group * 64;                         // this thread's half of the head dimension
+  const uint32_t tAcc = tmem + 256 + lane_off + d0;
+  uint16_t* out = KV ? reinterpret_cast<uint16_t*>(p.dk) + w.b * p.dk_sb + r * p.dk_ss + w.h * p.dk_sh + d0
+                     : reinterpret_cast<uint16_t*>(p.dq) + w.b * p.dq_sb + r * p.dq_ss + w.h * p.dq_sh + d0;
+  uint32_t ra[32], rb[32];
+  if (KV) {
+    uint16_t* dv = reinterpret_cast<uint16_t*>(p.dv) + w.b * p.dv_sb + r * p.dv_ss + w.h * p.dv_sh + d0;
+    tmem_ld_32x32(tAcc, ra);
+    tmem_ld_32x32(tAcc + 32, rb);
+    tmem_ld_wait();
+    att_store_out64(dv, ra, rb, 1.f, p.in_dtype);
+  }
+  tmem_ld_32x32(tAcc + 128, ra);
+  tmem_ld_32x32(tAcc + 160, rb);
+  tmem_ld_wait();
+  tc_fence_before();
+  __syncwarp();
+  if (lane == 0) mbar_arrive(smem_u32(&sh.acc_empty));
+  att_store_out64(out, ra, rb, 1.f, p.in_dtype);
+  return true;
 }
 
 __global__ void __launch_bounds__(kAttThreads, 1)
@@ -731,8 +771,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __shared__ AttnBwdShared sh;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int warp = threadIdx.x >> 5;
+  volatile int* abort_flag = &sh.abort_flag;
   if (threadIdx.x == 0) {
     mbar_init(smem_u32(&sh.resident), 1);
+    mbar_init(smem_u32(&sh.res_empty), 1);
+    mbar_init(smem_u32(&sh.acc_empty), 8);
     for (int s = 0; s < kBwdStages; ++s) {
       mbar_init(smem_u32(&sh.st_full[s]), 1);
       mbar_init(smem_u32(&sh.st_empty[s]), 1);
@@ -751,20 +794,58 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  const uint32_t tmem = sh.tmem_base;
 
-  // the longest blocks first: keys see the queries behind them, queries the keys before them
-  const int nkb = p.Sk / 128, nqb = p.Sq / 128;
-  const int blk = (int)blockIdx.z, h = blockIdx.x, b = blockIdx.y;
-  if (blk < nkb)
-    attn_bwd_cta<true>(&tmK, &tmV, &tmQ64, &tmDO64, p, blk, h, b, base, sh, status);
-  else
-    attn_bwd_cta<false>(&tmQ, &tmDO, &tmK64, &tmV64, p, nqb - 1 - (blk - nkb), h, b, base, sh, status);
+  BwdItem w;
+  int step = 0, item = 0;
+  bool ok = true;
+  if (warp == 4) {
+    if (elect_one()) {
+      const BwdMaps keys = {&tmK, &tmV, &tmQ64, &tmDO64}, queries = {&tmQ, &tmDO, &tmK64, &tmV64};
+      RingPos rp;
+      for (int r = 0; ok && bwd_item(p, r, w); ++r) {
+        if (w.iters == 0) continue;
+        ok = w.kv ? bwd_produce<true>(keys, p, w, item, base, sh, rp, step, abort_flag, status)
+                  : bwd_produce<false>(queries, p, w, item, base, sh, rp, step, abort_flag, status);
+        ++item;
+      }
+      if (!ok || *abort_flag) {        // the copies in flight land before shared memory is released
+        for (int k = max(0, item - 2); k < item; ++k) mbar_wait_budget_only(smem_u32(&sh.resident), k & 1);
+        for (int j = max(0, step - kBwdStages); j < step; ++j)
+          mbar_wait_budget_only(smem_u32(&sh.st_full[j % kBwdStages]), (j / kBwdStages) & 1);
+      }
+    }
+  } else if (warp == 5) {
+    if (elect_one()) {
+      RingPos next, cur;               // stages of the scores' step and of the accumulating step
+      for (int r = 0; ok && bwd_item(p, r, w); ++r) {
+        if (w.iters == 0) continue;
+        ok = w.kv ? bwd_issue<true>(p, w, item, base, tmem, sh, next, cur, step, abort_flag, status)
+                  : bwd_issue<false>(p, w, item, base, tmem, sh, next, cur, step, abort_flag, status);
+        ++item;
+      }
+    }
+  } else {
+    int group = 0, quarter = 0;
+    att_row_role(warp, group, quarter);
+    const int row = quarter * 32 + (threadIdx.x & 31);
+    RingPos rp;
+    for (int r = 0; ok && bwd_item(p, r, w); ++r) {
+      if (w.iters == 0) continue;
+      if (w.kv) {
+        ok = bwd_rows<true>(p, w, group, quarter, tmem, sh, rp, step, 0.f, 0.f, abort_flag, status);
+      } else {
+        const long long at = ((long long)w.b * p.H + w.h) * p.Sq + w.blk * 128 + row;
+        ok = bwd_rows<false>(p, w, group, quarter, tmem, sh, rp, step, p.lse[at], p.delta[at], abort_flag, status);
+      }
+    }
+  }
 
   tc_fence_before();
   __syncthreads();
   if (warp == 5) {
     tc_fence_after();
-    tmem_dealloc(sh.tmem_base, 512);
+    tmem_dealloc(tmem, 512);
   }
 }
 
@@ -874,7 +955,10 @@ int lb_attention_bwd(const void* q, const void* k, const void* v, const void* o,
     cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
     configured = true;
   }
-  attn_bwd_kernel<<<dim3(H, B, Sk / 128 + Sq / 128), kAttThreads, kBwdSmem, stream>>>(
+  const long long items = (long long)H * B * (Sk / 128 + Sq / 128);
+  if (items > (1ll << 30)) return -2;
+  const int grid = (int)std::min<long long>(items, lbhost::sm_count());
+  attn_bwd_kernel<<<grid, kAttThreads, kBwdSmem, stream>>>(
       tq, tk, tv, tdo, tq64, tk64, tv64, tdo64, p, lbhost::status_word());
   return (int)cudaGetLastError();
 }

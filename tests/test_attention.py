@@ -141,3 +141,13 @@ def test_attention_tiles_against_64_bits(B, H, Sq, Sk, causal, scale):
     refs = torch.autograd.grad(ref, (qd, kd, vd), g.double())
     for got, want in zip((y, *grads), (ref, *refs)):
         assert float((got.double() - want).norm()) <= 0.01 * float(want.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,H,Sq,Sk,causal", [
+    (7, 5, 256, 640, False),             # two rounds of items a CTA, the second incomplete; queries walk more than keys
+    (5, 10, 384, 384, True),             # three rounds, the last of four items
+    (37, 4, 128, 128, True),             # exactly two rounds, two steps an item
+])
+def test_attention_gradient_over_several_items(B, H, Sq, Sk, causal):
+    test_attention_tiles_against_64_bits(B, H, Sq, Sk, causal, 0.09)
