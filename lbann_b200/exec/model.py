@@ -945,6 +945,9 @@ class ExecModel:
             counts0 = [s.step_count for s in self.arena.slots]
             launches0 = native.launches()
             graph = torch.cuda.CUDAGraph()
+            # an evaluation step since the last update has left packed filters: the graph packs its own
+            for w in self.weights:
+                w.handle.bump()
             torch.cuda.synchronize(self.device)
             try:
                 if self._phase_graphs:
@@ -979,6 +982,8 @@ class ExecModel:
         # optimizer kernel through its device-side table, refreshed here when they change
         self.arena._segments()
         entry["graph"].replay()
+        for w in self.weights:          # what evaluation steps packed or cast is of older values now
+            w.handle.bump()
         self.stats["training"].samples += entry["samples"]
         for s in self.arena.slots:
             if s.kind != "none":

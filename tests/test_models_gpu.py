@@ -242,7 +242,7 @@ def test_evaluation_replays_equal_eager_steps():
         m = tr.build_model(exp.model)
         g = torch.Generator(device="cuda").manual_seed(1)
         losses, outs, held = [], [], []
-        for step in range(16):
+        for step in range(30):
             rows = 5 if step % 5 == 4 else 8
             batch = {"samples": torch.randn(rows, 288, generator=g, device="cuda"),
                      "responses": torch.randn(rows, 4, generator=g, device="cuda")}
