@@ -49,16 +49,16 @@ class ModeStats:
 
 
 class ReplayedActivations(Mapping):
-    """A replayed step's activations by layer name.  The graph's own tensors are overwritten by its
-    next replay, so what is asked for is copied out, once, and stays as it is."""
+    """A replayed step's activations by layer name.  What is asked for shares the graph's memory: the model
+    does not replay the graph again while somebody holds it, or this mapping."""
 
     def __init__(self, static):
-        self._static, self._own = static, {}
+        self._static, self._out = static, {}
 
     def __getitem__(self, name):
-        if name not in self._own:
-            self._own[name] = [t.clone() if torch.is_tensor(t) else t for t in self._static[name]]
-        return self._own[name]
+        if name not in self._out:
+            self._out[name] = [t.detach() if torch.is_tensor(t) else t for t in self._static[name]]
+        return self._out[name]
 
     def __iter__(self):
         return iter(self._static)
@@ -66,9 +66,30 @@ class ReplayedActivations(Mapping):
     def __len__(self):
         return len(self._static)
 
-    def keep(self):
-        for name in self._static:
-            self[name]
+
+class EvaluationGraph:
+    """A captured evaluation step with its inputs, results and bookkeeping."""
+
+    def __init__(self, graph, static, out, acts, tensors, samples, launches):
+        self.graph, self.static, self.out, self.acts = graph, static, out, acts
+        self.samples, self.launches, self._last = samples, launches, None
+        self._tensors, self._uses = tensors, native.nodes().storage_uses(tensors)
+        self.bytes = storage_bytes(tensors)
+
+    def activations(self):
+        acts = ReplayedActivations(self.acts)
+        self._last = weakref.ref(acts)
+        return acts
+
+    def held(self):
+        """Whether a caller has the last step's mapping, or anything that shares an activation's memory."""
+        uses, least = native.nodes().storage_uses(self._tensors), self._uses
+        self._uses = [min(a, b) for a, b in zip(uses, least)]
+        return (self._last is not None and self._last() is not None) or any(a > b for a, b in zip(uses, least))
+
+
+def storage_bytes(tensors):
+    return sum({t.untyped_storage().data_ptr(): t.untyped_storage().nbytes() for t in tensors}.values())
 
 
 class ExecMetric:
@@ -1111,7 +1132,7 @@ class ExecModel:
         self.record_statistics(mode, obj)
         return self.last_objective
 
-    # A forward pass of two GPT blocks over 512 tokens takes the host 740 us to launch, and 260 us as a replay.
+    # A forward pass of two GPT blocks over 512 tokens takes the host 740 us to launch, and 225 us as a replay.
     # Steps with more activations than this (all graphs of a model together) run longer than the host takes,
     # and would hold their memory for good; so would copies of that many weights be repeated by each replay.
     _EVAL_GRAPH_BYTES = 2 << 30
@@ -1131,70 +1152,79 @@ class ExecModel:
     def _evaluate_step_graph(self, key, inputs, mode, gmb, offset):
         entry = self._eval_graphs.get(key)
         if entry is None:
-            entry = self._eval_graphs[key] = {"warm": 0, "bytes": 0}
+            entry = self._eval_graphs[key] = {"warm": 0, "graphs": []}
             while len(self._eval_graphs) > self._EVAL_GRAPHS:
-                self._drop_eval_graph(next(iter(self._eval_graphs)))
+                self._eval_graphs.popitem(last=False)
         self._eval_graphs.move_to_end(key)
-        st = self.stats[mode]
-        if "graph" not in entry:
-            entry["warm"] += 1
-            if entry["warm"] <= 3 or entry.get("eager"):
-                return self._evaluate_step_eager(inputs, mode, gmb, offset)
-            storages = {t.untyped_storage().data_ptr(): t.untyped_storage().nbytes()
-                        for ts in self.acts.values() for t in ts if torch.is_tensor(t)}
-            entry["bytes"] = sum(storages.values())
-            casts = sum(t.numel() for w in self.weights for t in w.handle._cache.values() if torch.is_tensor(t))
-            if entry["bytes"] > self._EVAL_GRAPH_BYTES or casts > self._EVAL_GRAPH_CASTS:
-                entry.update(eager=True, bytes=0)
-                return self._evaluate_step_eager(inputs, mode, gmb, offset)
-            for k in list(self._eval_graphs):
-                if k != key and sum(e["bytes"] for e in self._eval_graphs.values()) > self._EVAL_GRAPH_BYTES:
-                    self._drop_eval_graph(k)
-            static = {k: torch.empty_like(v) for k, v in inputs.items()}
-            samples0, launches0 = st.samples, native.launches()
-            graph = torch.cuda.CUDAGraph()
-            # the weights may change between replays: their 16-bit and packed copies are made inside
-            # the graph, and those made there are nobody else's
-            for w in self.weights:
-                w.handle.bump()
-            torch.cuda.synchronize(self.device)
-            try:
-                with torch.cuda.graph(graph, capture_error_mode="thread_local"):
-                    out = self._evaluate_step_eager(static, mode, gmb, offset)
-                entry.update(graph=graph, static=static, out=out, acts=self.acts, samples=self._global_mb,
-                             launches=native.launches() - launches0)
-            except Exception:           # something in this model cannot be captured
-                entry.update(eager=True, bytes=0)
-                torch.cuda.synchronize(self.device)
-            for w in self.weights:
-                w.handle.bump()
-            st.samples = samples0
-            native.count_launch(launches0 - native.launches())
-            if entry.get("eager"):
-                return self._evaluate_step_eager(inputs, mode, gmb, offset)
         self.acts = {}
-        last = entry["last"]() if "last" in entry else None
-        if last is not None:
-            last.keep()                 # a caller holds the activations of the step before
+        graph = next((g for g in entry["graphs"] if not g.held()), None)
+        if graph is None:
+            # the second graph is for callers that hold a step's activations during the next one
+            entry["warm"] += 1
+            if entry["warm"] <= 3 or len(entry["graphs"]) == 2 or entry.get("eager"):
+                out = self._evaluate_step_eager(inputs, mode, gmb, offset)
+                if entry["warm"] == 3:
+                    entry["bytes"] = storage_bytes(self._step_tensors(self.acts))
+                    entry["casts"] = sum(t.numel() for w in self.weights for t in w.handle._cache.values()
+                                         if torch.is_tensor(t))
+                return out
+            graph = self._capture_evaluation(entry, key, inputs, mode, gmb, offset)
+            if graph is None:
+                entry["eager"] = True
+                return self._evaluate_step_eager(inputs, mode, gmb, offset)
+            entry["graphs"].append(graph)
         for k, v in inputs.items():
-            self._copy_into_static(entry["static"][k], v)
-        entry["graph"].replay()
+            self._copy_into_static(graph.static[k], v)
+        graph.graph.replay()
         first = next(iter(inputs.values()))
         self.current_inputs = inputs
         self.current_mini_batch_size = int(first.shape[0])
-        self._global_mb = entry["samples"]
+        self._global_mb = graph.samples
         self._global_mb_given, self._mb_offset, self._mean_cache = bool(gmb), offset, {}
-        self.acts = ReplayedActivations(entry["acts"])
-        entry["last"] = weakref.ref(self.acts)
-        st.samples += entry["samples"]
-        native.count_launch(entry["launches"])
-        self.last_objective = entry["out"].clone()
+        self.acts = graph.activations()
+        self.stats[mode].samples += graph.samples
+        native.count_launch(graph.launches)
+        self.last_objective = graph.out.clone()
         return self.last_objective
 
-    def _drop_eval_graph(self, key):
-        if isinstance(self.acts, ReplayedActivations):
-            self.acts.keep()
-        del self._eval_graphs[key]
+    def _step_tensors(self, acts):
+        """Activations in memory of the step's own: not those that are views of the weights."""
+        a = self.arena
+        weights = {t.untyped_storage().data_ptr() for t in (a.master, a.compute) if t is not None}
+        return [t for ts in acts.values() for t in ts
+                if torch.is_tensor(t) and t.untyped_storage().data_ptr() not in weights]
+
+    def _capture_evaluation(self, entry, key, inputs, mode, gmb, offset):
+        """The step as a graph; None where it cannot or should not be one."""
+        st = self.stats[mode]
+        samples0, launches0 = st.samples, native.launches()
+        need = entry["bytes"]
+        for k in list(self._eval_graphs):
+            total = sum(g.bytes for e in self._eval_graphs.values() for g in e["graphs"])
+            if k != key and total + need > self._EVAL_GRAPH_BYTES:
+                del self._eval_graphs[k]
+        if sum(g.bytes for g in entry["graphs"]) + need > self._EVAL_GRAPH_BYTES or entry["casts"] > self._EVAL_GRAPH_CASTS:
+            return None
+        graph, static = None, {k: torch.empty_like(v) for k, v in inputs.items()}
+        cuda_graph = torch.cuda.CUDAGraph()
+        # the weights may change between replays: their 16-bit and packed copies are made inside
+        # the graph, and those made there are nobody else's
+        for w in self.weights:
+            w.handle.bump()
+        torch.cuda.synchronize(self.device)
+        try:
+            with torch.cuda.graph(cuda_graph, capture_error_mode="thread_local"):
+                out = self._evaluate_step_eager(static, mode, gmb, offset)
+            acts, self.acts, self._mean_cache = self.acts, {}, {}
+            graph = EvaluationGraph(cuda_graph, static, out, acts, self._step_tensors(acts), self._global_mb,
+                                    native.launches() - launches0)
+        except Exception:           # something in this model cannot be captured
+            torch.cuda.synchronize(self.device)
+        for w in self.weights:
+            w.handle.bump()
+        st.samples = samples0
+        native.count_launch(launches0 - native.launches())
+        return graph
 
     # ------------------------------------------------------------------ reporting
     def reduce_statistics(self, mode: str):

@@ -230,7 +230,9 @@ def test_evaluation_replays_equal_eager_steps():
         h = lbann.Reshape(x, dims=[8, 6, 6])
         h = lbann.Convolution(h, num_dims=2, out_channels=16, kernel_size=3, padding=1, has_bias=False, name="conv")
         h = lbann.Relu(lbann.BatchNormalization(h))
-        h = lbann.FullyConnected(h, num_neurons=4, has_bias=True, name="last")
+        h = lbann.FullyConnected(h, num_neurons=4, has_bias=True, name="last_product")
+        shift = lbann.WeightsLayer(dims=[4], weights=[lbann.Weights(initializer=lbann.ConstantInitializer(value=0.1))])
+        h = lbann.Add(h, shift, name="last")       # an activation that is a view of the weights
         loss = lbann.MeanSquaredError(h, target, name="mse")
         model = lbann.Model(1, layers=lbann.traverse_layer_graph(x), objective_function=loss,
                             metrics=[lbann.Metric(loss, name="mse")])
@@ -249,18 +251,22 @@ def test_evaluation_replays_equal_eager_steps():
             if step % 4 == 1:
                 m.train_step(batch, rows)
             losses.append(m.evaluate_step(batch, "validation" if step % 3 else "testing", rows))
-            outs.append(m.activation("last"))
-            held.append(m.acts)
+            # held for good, as it is and by the step's mapping; later for the next step only
+            outs.append(m.activation("last") if step < 16 else m.activation("last").clone())
+            last = m.activation("conv")[1:]
+            if step < 16:
+                held.append(m.acts)
             assert m.current_mini_batch_size == rows and m.current_inputs["samples"] is batch["samples"]
         held = [a["conv"][0] for a in held]
         stats = [m.reduce_statistics(mode) for mode in ("validation", "testing")]
-        graphs = sum("graph" in e for e in m._eval_graphs.values())
+        graphs = sum(len(e["graphs"]) for e in m._eval_graphs.values())
+        assert last.shape[0] == rows - 1
         tr.shutdown()
         assert native.consume_status() == 0
         return losses, outs, held, stats, graphs
 
     want, got = run(False), run(True)
-    assert want[4] == 0 and got[4] >= 2
+    assert want[4] == 0 and got[4] >= 5
     for a, b in zip(want[:3], got[:3]):
         for t, u in zip(a, b):
             assert torch.equal(t, u)
