@@ -6,11 +6,10 @@
 // pipeline stage); both operands are "MN-major" (pixel rows, channels contiguous), so
 // x and dy are consumed exactly as they sit in memory.  The accumulator rows stack
 // several (tap, channel-block) slices: with Cb = 16/32/64 channels per slice an M = 128
-// accumulator holds 8/4/2 slices, and a CTA keeps up to four such accumulators in TMEM,
-// so one pass over its pixels yields up to 32 taps x 16 channels (CosmoFlow's first
-// layer needs a single pass for all 27 taps).  The pixel range is split over CTAs and
-// the partial results are added with fp32 atomics into the (pre-scaled) gradient buffer,
-// matching the reference's dst_scale / grad_scale accumulation contract
+// accumulator holds 8/4/2 slices.  Where the sizes allow it, all taps of a brick are read
+// from one halo slab of x (conv_wgrad_slab_kernel).  The pixel range is split over CTAs, whose
+// partial results go to a workspace; wgrad_reduce_kernel adds them up and into the (pre-scaled)
+// gradient buffer, matching the reference's dst_scale / grad_scale accumulation contract
 // (src/layers/learning/base_convolution.cpp:1397-1445).
 #include <algorithm>
 
