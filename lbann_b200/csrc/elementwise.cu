@@ -266,49 +266,6 @@ __device__ __forceinline__ void store_vec(T* p, long long i, long long n, const 
 // copies of all ~60 operators' code (GELU on 134 M bf16 values ran at 1.5 TB/s instead of the
 // copy rate).  Dispatch is a compile-time binary search over the operator codes; each leaf is
 // the grid-stride loop with the operator as a constant.
-// The normal distribution's density and distribution function at x, for tensors of 16 bits: with t = |x| / sqrt 2 and
-// u = 1 / (1 + 0.325 t), erfc(t) = exp(-t^2) u P(u), P of degree 7 fitted (least squares, reweighted towards the
-// largest error) to erfcx(t) / u for |x| < 9.5 with a relative error of 3.7e-8.  One reciprocal and one exponential, which the
-// density shares; erff and expf take three times the instructions and were what bounded GELU.  In fp32 the
-// distribution function is within 1.2e-7 (a 16-bit value rounds by 2.4e-4 of itself) and keeps its digits in the lower
-// tail, where 1 + erff(x) loses them.
-__device__ __forceinline__ void normal16(float x, float& pdf, float& cdf) {
-  float u;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(u) : "f"(fmaf(0.325f * 0.70710678118654752f, fabsf(x), 1.f)));
-  const float e = fast_exp2(x * x * -0.72134752044448170f);
-  float q = -0.15455902990f;
-  q = fmaf(q, u, 0.56927351324f);
-  q = fmaf(q, u, -0.52721550174f);
-  q = fmaf(q, u, 0.56347892999f);
-  q = fmaf(q, u, -0.03389809253f);
-  q = fmaf(q, u, 0.22294988872f);
-  q = fmaf(q, u, 0.17615700056f);
-  q = fmaf(q, u, 0.18381325449f);
-  q = 0.5f * e * u * q;
-  cdf = x >= 0.f ? 1.f - q : q;
-  pdf = 0.3989422804014327f * e;
-}
-template <typename T, int OP>
-__device__ __forceinline__ float op_fwd(float x, float p0, float p1) {
-  if constexpr (OP == U_GELU && sizeof(T) == 2) {
-    float pdf, cdf;
-    normal16(x, pdf, cdf);
-    return x * cdf;
-  } else {
-    return unary_fwd(OP, x, p0, p1);
-  }
-}
-template <typename T, int OP>
-__device__ __forceinline__ float op_bwd(float x, float dy, float p0, float p1) {
-  if constexpr (OP == U_GELU && sizeof(T) == 2) {
-    float pdf, cdf;
-    normal16(x, pdf, cdf);
-    return dy * fmaf(x, pdf, cdf);
-  } else {
-    return unary_bwd(OP, x, dy, p0, p1);
-  }
-}
-
 template <typename T, int OP>
 __device__ __forceinline__ void unary_body(const T* __restrict__ x, const T* __restrict__ dy,
                                            T* __restrict__ out, long long n, int mode, float p0,
@@ -320,11 +277,11 @@ __device__ __forceinline__ void unary_body(const T* __restrict__ x, const T* __r
     load_vec<T>(x, i, n, fx, aligned);
     if (mode == 0) {
 #pragma unroll
-      for (int j = 0; j < V; ++j) fo[j] = op_fwd<T, OP>(fx[j], p0, p1);
+      for (int j = 0; j < V; ++j) fo[j] = unary_fwd(OP, fx[j], p0, p1);
     } else {
       load_vec<T>(dy, i, n, fd, aligned);
 #pragma unroll
-      for (int j = 0; j < V; ++j) fo[j] = op_bwd<T, OP>(fx[j], fd[j], p0, p1);
+      for (int j = 0; j < V; ++j) fo[j] = unary_bwd(OP, fx[j], fd[j], p0, p1);
     }
     store_vec<T>(out, i, n, fo, aligned);
   }
@@ -352,8 +309,8 @@ __global__ void unary_kernel(const T* __restrict__ x, const T* __restrict__ dy, 
 
 // The activations that models are made of, and additions and products, have kernels of their own: one that
 // holds every operator runs each of them with the registers of the greediest.  Blocks of 512 vectors that
-// come and go, two a thread, both loads first.  16.8 M bf16 values: GELU 21.4 -> 14.1 us, its gradient
-// 31.6 -> 19.8 (18.9 and 29.5 with erff); an addition of 4 M 6.0 -> 5.3.
+// come and go, two a thread, both loads first.  16.8 M bf16 values: GELU 21.4 -> 18.9 us, its gradient
+// 31.6 -> 29.5; an addition of 4 M 6.0 -> 5.3.
 constexpr int kHotVecs = 2;
 template <typename T, int OP, int MODE>
 __global__ void __launch_bounds__(256)
@@ -370,7 +327,7 @@ unary_hot_kernel(const T* __restrict__ x, const T* __restrict__ dy, T* __restric
   for (int u = 0; u < kHotVecs; ++u) {
     float fo[8];
 #pragma unroll
-    for (int j = 0; j < V; ++j) fo[j] = MODE ? op_bwd<T, OP>(fx[u][j], fd[u][j], p0, p1) : op_fwd<T, OP>(fx[u][j], p0, p1);
+    for (int j = 0; j < V; ++j) fo[j] = MODE ? unary_bwd(OP, fx[u][j], fd[u][j], p0, p1) : unary_fwd(OP, fx[u][j], p0, p1);
     store_vec<T>(out, i0 + u * 256 * V, n, fo, true);
   }
 }

@@ -355,6 +355,19 @@ def test_unary_operators_on_16_bit_tensors(name, dtype):
     torch.testing.assert_close(xa.grad.float(), xr.grad, rtol=2e-2, atol=2e-2)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gelu_of_every_16_bit_value(dtype):
+    """16-bit tensors get the fp32 operator's value, rounded once: all bit patterns, forward and gradient."""
+    x = torch.arange(-32768, 32768, dtype=torch.int32, device="cuda").to(torch.int16).view(dtype)
+    x = x[torch.isfinite(x)]
+    for name in ("gelu", "gelu_tanh"):
+        a, b = x.clone().requires_grad_(True), x.float().requires_grad_(True)
+        y, z = ew.unary(name, a, 0.0, 0.0), ew.unary(name, b, 0.0, 0.0)
+        assert torch.equal(y, z.to(dtype)), name
+        dy, dz = torch.autograd.grad(y.sum(), a)[0], torch.autograd.grad(z.sum(), b)[0].to(dtype)
+        assert torch.equal(dy.nan_to_num(7.0), dz.nan_to_num(7.0)), name
+
+
 @pytest.mark.parametrize("n", [1, 8, 4095, 4096, 4097, 12296])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
 def test_operators_with_kernels_of_their_own(n, dtype):
