@@ -65,6 +65,10 @@ def broadcast_list(values, n: int, default: int) -> Tuple[int, ...]:
     return tuple(v)
 
 
+_MISSING = object()
+_PLAIN = (bool, int, float, str, tuple, type(None))
+
+
 class ExecLayer:
     """Executable counterpart of one layer message."""
 
@@ -100,6 +104,22 @@ class ExecLayer:
         self.out_dims: List[Tuple[int, ...]] = []
         self.fp_time = 0.0
         self.bp_time = 0.0
+
+    def __setattr__(self, name, value):
+        """The model hears of changes: steps that it has captured may no longer be what the layers compute."""
+        old = type(self) if name == "__class__" else self.__dict__.get(name, _MISSING)
+        object.__setattr__(self, name, value)
+        if old is value or (type(old) is type(value) and isinstance(value, _PLAIN) and old == value):
+            return
+        heard = getattr(self.__dict__.get("model"), "layer_changed", None)
+        if heard is not None and name not in ("fp_time", "bp_time"):
+            heard(name)
+
+    def __delattr__(self, name):
+        object.__delattr__(self, name)
+        heard = getattr(self.__dict__.get("model"), "layer_changed", None)
+        if heard is not None:
+            heard(name)
 
     # ---- set-up
     def setup(self, in_dims: List[Tuple[int, ...]]) -> List[Tuple[int, ...]]:

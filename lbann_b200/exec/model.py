@@ -149,6 +149,9 @@ class ExecModel:
         self._overwrite_cache = None   # (layers, handles), see _overwritten_gradients
         self._graphs = {}
         self._eval_graphs = OrderedDict()
+        # what captured steps depend on beside their inputs, see layer_state
+        self._layer_changes, self._layers_seen, self._frozen_seen, self._in_forward = 0, None, None, False
+        self._graph_changes = self._eval_changes = -1
         self.layer_timing = False
         self.is_setup = False
 
@@ -583,7 +586,6 @@ class ExecModel:
     # ------------------------------------------------------------------ execution
     def forward_prop(self, inputs: Dict[str, torch.Tensor], mode: str = "training",
                      global_mini_batch_size: Optional[int] = None, mini_batch_offset: int = 0):
-        training = mode == "training"
         self.current_inputs = inputs
         first = next(iter(inputs.values())) if inputs else None
         self.current_mini_batch_size = int(first.shape[0]) if first is not None else 0
@@ -591,6 +593,14 @@ class ExecModel:
         self._global_mb = global_mini_batch_size or self.current_mini_batch_size * dp
         self._global_mb_given = bool(global_mini_batch_size)
         self._mb_offset = mini_batch_offset
+        self._in_forward = True
+        try:
+            return self._forward_layers(inputs, mode)
+        finally:
+            self._in_forward = False
+
+    def _forward_layers(self, inputs, mode):
+        training = mode == "training"
         acts = {}
         self.acts = acts          # visible to callbacks while it fills up
         self._mean_cache = {}
@@ -929,6 +939,31 @@ class ExecModel:
             return False
         return True
 
+    # ------------------------------------------------------------------ what captured steps depend on
+    def layer_changed(self, name):
+        """An attribute of a layer was set (ExecLayer.__setattr__)."""
+        if self._in_forward:            # a layer's own notes for the step
+            return
+        if name == "frozen":
+            self._frozen_seen = None
+        else:
+            self._layer_changes += 1
+
+    def layer_state(self):
+        """(number of changes to the layers and to what they compute, which of them are frozen).  Layers may be
+        changed between two steps: a mutation replaces an activation, a callback freezes one side of a GAN.
+        Captured steps are kept per state of the second, which comes back, and dropped with the first."""
+        live = (self.layers, [l.params for l in self.layers], [w.handle for w in self.weights], self.objective_terms,
+                [getattr(m, "layer_name", None) for m in self.metrics])
+        if live != self._layers_seen:
+            params = [None if p is None else type(p).FromString(p.SerializePartialToString()) for p in live[1]]
+            self._layers_seen = (list(live[0]), params, live[2], list(live[3]), live[4])
+            self._layer_changes += 1
+            self._frozen_seen = None
+        if self._frozen_seen is None:
+            self._frozen_seen = tuple(bool(l.frozen) for l in self.layers)
+        return self._layer_changes, self._frozen_seen
+
     _HOST_STATE_LAYERS = frozenset({"mini_batch_index", "dropout", "selu_dropout", "bernoulli", "gaussian",
                                     "uniform", "dist_embedding", "external", "python"})
 
@@ -949,7 +984,14 @@ class ExecModel:
             static.copy_(v)
 
     def _train_step_graph(self, inputs, gmb, offset):
-        key = (tuple((k, tuple(v.shape), v.dtype) for k, v in sorted(inputs.items())), gmb)
+        changes, frozen = self.layer_state()
+        if changes != self._graph_changes:
+            self._graphs.clear()
+            if self._graph_changes >= 0 and not self._graph_capable():
+                self._graph_mode = False
+                return self._train_step_eager(inputs, gmb, offset)
+            self._graph_changes = changes
+        key = (tuple((k, tuple(v.shape), v.dtype) for k, v in sorted(inputs.items())), gmb, frozen)
         entry = self._graphs.get(key)
         if entry is None:
             entry = self._graphs[key] = {"warm": 0}
@@ -1138,6 +1180,7 @@ class ExecModel:
     _EVAL_GRAPH_BYTES = 2 << 30
     _EVAL_GRAPH_CASTS = 4 << 20     # elements of weights copied or packed for the step
     _EVAL_GRAPHS = 8
+    _EVAL_LAYER_MODULES = (layers_core.__name__, layers_misc.__name__)
 
     def _eval_graph_key(self, inputs, mode, gmb, offset):
         """What a captured evaluation step depends on, or None where the step is launched from the host."""
@@ -1146,7 +1189,15 @@ class ExecModel:
                 or torch.cuda.is_current_stream_capturing() or not self._graph_capable()
                 or not all(torch.is_tensor(v) and v.is_cuda and v.is_contiguous() for v in inputs.values())):
             return None
-        return (mode, gmb, offset, torch.cuda.current_stream(self.device).cuda_stream, self.arena.master.data_ptr(),
+        changes, frozen = self.layer_state()
+        if changes != self._eval_changes:
+            self._eval_graphs.clear()
+            self._eval_changes = changes
+            # layers from elsewhere may keep anything on the host
+            self._eval_own_layers = all(type(l).__module__ in self._EVAL_LAYER_MODULES for l in self.layers)
+        if not self._eval_own_layers:
+            return None
+        return (mode, gmb, offset, torch.cuda.current_stream(self.device).cuda_stream, self.arena.master.data_ptr(), frozen,
                 tuple((k, tuple(v.shape), v.dtype, v.device) for k, v in sorted(inputs.items())))
 
     def _evaluate_step_graph(self, key, inputs, mode, gmb, offset):

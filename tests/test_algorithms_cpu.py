@@ -452,3 +452,53 @@ def test_kfac_use_interval_switches_between_sgd_and_kfac_by_epoch(capsys):
     assert abs(off - plain) <= 1e-6 * max(1.0, abs(plain)), (off, plain)
     assert on < plain
     assert "(factors only)" in out and "K-FAC fc1: A (9, 9)" in out
+
+
+def test_changes_of_the_layers_are_seen_between_steps():
+    """What captured steps depend on: steps and settings to the same value leave it as it is, a replaced activation,
+    a parameter set in place or another weight of the objective change it, freezing comes back to what it was."""
+    from lbann_b200.exec.ltfb import Mutation
+    o = opts.reset()
+    o.set("disable_cuda", True)
+    x = lbann.Input(data_field="samples")
+    target = lbann.Input(data_field="responses")
+    h = lbann.Relu(lbann.Identity(lbann.FullyConnected(x, num_neurons=8, has_bias=True)), name="act")
+    y = lbann.FullyConnected(h, num_neurons=4, has_bias=True)
+    loss = lbann.IdentityZero(lbann.MeanSquaredError(y, target), name="switch")
+    exp = lbann.proto.serialize.build_experiment(
+        trainer=lbann.Trainer(mini_batch_size=4), model=lbann.Model(1, layers=lbann.traverse_layer_graph(x),
+                                                                    objective_function=loss),
+        data_reader=_reader(4, [6], "samples:normal responses:normal", response_dims=[4]),
+        optimizer=lbann.SGD(learn_rate=1e-2))
+    tr = ExecTrainer(exp)
+    m = tr.build_model(exp.model)
+    batch = {"samples": torch.randn(4, 6), "responses": torch.randn(4, 4)}
+
+    def stays():
+        before = m.layer_state()
+        m.train_step(batch, 4)
+        m.evaluate_step(batch, "validation", 4)
+        m.layer("act").name = "act"
+        return m.layer_state() == before
+
+    assert stays()
+    states = [m.layer_state()]
+    Mutation("replace_activation", seed=1).mutate(m, 0)
+    assert m.layer("act").type != "relu"
+    states.append(m.layer_state())
+    Mutation("replace_activation", seed=2).mutate(m, 0)
+    m.layer("act").params.CopyFrom(type(m.layer("act").params)())
+    states.append(m.layer_state())
+    next(l for l in m.layers if l.type == "fully_connected").params.num_neurons = 9
+    states.append(m.layer_state())
+    m.objective_terms[0] = (m.objective_terms[0][0], 0.5)
+    states.append(m.layer_state())
+    m.layer("act").dtype = torch.float64
+    states.append(m.layer_state())
+    assert len({s[0] for s in states}) == len(states) and stays()
+    before = m.layer_state()
+    m.layer("switch").frozen = True
+    assert m.layer_state()[0] == before[0] and m.layer_state() != before and stays()
+    m.layer("switch").frozen = False
+    assert m.layer_state() == before
+    tr.shutdown()

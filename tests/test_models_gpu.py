@@ -271,3 +271,67 @@ def test_evaluation_replays_equal_eager_steps():
         for t, u in zip(a, b):
             assert torch.equal(t, u)
     assert want[3] == got[3]
+
+
+def _switching_model(graph):
+    """A model with an activation that a mutation replaces and a loss term that freezing switches off."""
+    o = opts.reset()
+    o.set("default_dtype", "bf16")
+    o.set("use_cuda_graph", graph)
+    x = lbann.Input(data_field="samples")
+    target = lbann.Input(data_field="responses")
+    h = lbann.FullyConnected(x, num_neurons=24, has_bias=True, name="first")
+    h = lbann.Relu(lbann.Identity(h), name="act")
+    y = lbann.FullyConnected(h, num_neurons=4, has_bias=True, name="last")
+    terms = [lbann.IdentityZero(lbann.MeanSquaredError(y, target), name="switch"),
+             lbann.IdentityZero(lbann.MeanAbsoluteError(y, target), name="other")]
+    model = lbann.Model(1, layers=lbann.traverse_layer_graph(x), objective_function=lbann.ObjectiveFunction(terms))
+    exp = lbann.proto.serialize.build_experiment(
+        trainer=lbann.Trainer(mini_batch_size=8, random_seed=3), model=model,
+        data_reader=_reader(8, [24], "samples:normal responses:normal", response_dims=[4]),
+        optimizer=lbann.SGD(learn_rate=1e-2, momentum=0.9))
+    tr = ExecTrainer(exp)
+    return tr, tr.build_model(exp.model)
+
+
+@pytest.mark.parametrize("training", [False, True])
+@pytest.mark.parametrize("change", ["mutation", "params", "phases"])
+def test_replays_follow_changes_of_the_layers(change, training):
+    """A layer changes between steps, after they have been captured: replayed steps equal ordinary ones.  A
+    mutation replaces an activation, a parameter is set in place, a callback freezes one loss and then the other."""
+    from lbann_b200.exec.ltfb import Mutation
+
+    def run(graph):
+        tr, m = _switching_model(graph)
+        assert not getattr(m.layer("act"), "fused_into_parent", False)
+        mutation = Mutation("replace_activation", seed=1)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        losses, types = [], set()
+        for step in range(38):
+            batch = {"samples": torch.randn(8, 24, generator=g, device="cuda"),
+                     "responses": torch.randn(8, 4, generator=g, device="cuda")}
+            if change == "mutation" and step % 8 == 7:
+                mutation.mutate(m, step)
+            elif change == "params" and step % 8 == 7:
+                while m.layer("act").type != "leaky_relu":
+                    mutation.mutate(m, step)
+                m.layer("act").params.negative_slope = 0.1 * step
+            elif change == "phases":
+                for name, on in (("switch", step // 4 % 2), ("other", 1 - step // 4 % 2)):
+                    m.layer(name).frozen = bool(on)
+            types.add(m.layer("act").type)
+            if training:
+                losses.append(m.train_step(batch, 8).clone())
+            else:
+                losses.append(m.evaluate_step(batch, "validation", 8).clone())
+        entries = m._graphs if training else m._eval_graphs
+        captured = sum("graph" in e if training else bool(e["graphs"]) for e in entries.values())
+        tr.shutdown()
+        assert native.consume_status() == 0
+        return torch.stack(losses), captured, types
+
+    want, none, _ = run(False)
+    got, captured, types = run(True)
+    assert not none and captured == (2 if change == "phases" else 1)
+    assert change == "phases" or len(types) > 1
+    assert torch.equal(want, got), (want - got).abs()
