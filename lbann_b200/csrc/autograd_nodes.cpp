@@ -745,13 +745,6 @@ PYBIND11_MODULE(_lbann_autograd, m) {
   m.attr("abi_version") = LB_ABI_VERSION;
   m.def("launches", [] { return (long long)g_launches; });
   m.def("splitk_offers", [] { return (long long)g_offers; });
-  // how many tensors share the storage of each of these
-  m.def("storage_uses", [](const std::vector<Tensor>& ts) {
-    std::vector<int64_t> n;
-    n.reserve(ts.size());
-    for (const Tensor& t : ts) n.push_back((int64_t)t.storage().use_count());
-    return n;
-  });
   m.def("gemm", [](const Tensor& a, const Tensor& b, bool ta, bool tb, const optional<Tensor>& out, int64_t out_code,
                    double alpha, double beta, const optional<Tensor>& bias, bool per_row, int64_t act, double act_param,
                    int64_t bn_hint) {

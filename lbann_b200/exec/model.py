@@ -49,43 +49,62 @@ class ModeStats:
 
 
 class ReplayedActivations(Mapping):
-    """A replayed step's activations by layer name.  What is asked for shares the graph's memory: the model
-    does not replay the graph again while somebody holds it, or this mapping."""
+    """A replayed step's activations by layer name: copies, made when they are asked for, or before the graph
+    is replayed again while somebody holds the mapping."""
 
-    def __init__(self, static):
-        self._static, self._out = static, {}
+    def __init__(self, graph):
+        self._graph, self._names, self._out = graph, graph.acts.keys(), {}
 
     def __getitem__(self, name):
         if name not in self._out:
-            self._out[name] = [t.detach() if torch.is_tensor(t) else t for t in self._static[name]]
+            self._out[name] = self._graph.copies(name)
         return self._out[name]
 
     def __iter__(self):
-        return iter(self._static)
+        return iter(self._names)
 
     def __len__(self):
-        return len(self._static)
+        return len(self._names)
+
+    def keep(self):
+        for name in self._names:
+            self[name]
+        self._graph = None
 
 
 class EvaluationGraph:
     """A captured evaluation step with its inputs, results and bookkeeping."""
 
-    def __init__(self, graph, static, out, acts, tensors, samples, launches):
-        self.graph, self.static, self.out, self.acts = graph, static, out, acts
-        self.samples, self.launches, self._last = samples, launches, None
-        self._tensors, self._uses = tensors, native.nodes().storage_uses(tensors)
-        self.bytes = storage_bytes(tensors)
+    def __init__(self, graph, static, out, acts, borrowed, samples, launches, nbytes):
+        self.graph, self.static, self.out, self.acts, self.bytes = graph, static, out, acts, nbytes
+        self.samples, self.launches = samples, launches
+        self._borrowed = borrowed       # storages that activations share with the model: its weights
+        self._last, self._readers = None, []
+        self._stream = torch.cuda.current_stream(out.device)
 
-    def activations(self):
-        acts = ReplayedActivations(self.acts)
+    def copies(self, name):
+        """One layer's activations in memory of their own, that of the current stream."""
+        ts = [t if not torch.is_tensor(t) else t.detach() if t.untyped_storage().data_ptr() in self._borrowed
+              else t.clone() for t in self.acts[name]]
+        stream = torch.cuda.current_stream(self.out.device)
+        if stream != self._stream and not torch.cuda.is_current_stream_capturing():
+            # the next replay waits for these copies
+            self._readers.append(stream.record_event())
+        return ts
+
+    def replay(self, inputs, copy):
+        last = self._last() if self._last is not None else None
+        if last is not None:
+            last.keep()
+        for event in self._readers:
+            self._stream.wait_event(event)
+        self._readers = []
+        for k, v in inputs.items():
+            copy(self.static[k], v)
+        self.graph.replay()
+        acts = ReplayedActivations(self)
         self._last = weakref.ref(acts)
         return acts
-
-    def held(self):
-        """Whether a caller has the last step's mapping, or anything that shares an activation's memory."""
-        uses, least = native.nodes().storage_uses(self._tensors), self._uses
-        self._uses = [min(a, b) for a, b in zip(uses, least)]
-        return (self._last is not None and self._last() is not None) or any(a > b for a, b in zip(uses, least))
 
 
 def storage_bytes(tensors):
@@ -1203,16 +1222,15 @@ class ExecModel:
     def _evaluate_step_graph(self, key, inputs, mode, gmb, offset):
         entry = self._eval_graphs.get(key)
         if entry is None:
-            entry = self._eval_graphs[key] = {"warm": 0, "graphs": []}
+            entry = self._eval_graphs[key] = {"warm": 0, "graph": None}
             while len(self._eval_graphs) > self._EVAL_GRAPHS:
                 self._eval_graphs.popitem(last=False)
         self._eval_graphs.move_to_end(key)
         self.acts = {}
-        graph = next((g for g in entry["graphs"] if not g.held()), None)
+        graph = entry["graph"]
         if graph is None:
-            # the second graph is for callers that hold a step's activations during the next one
             entry["warm"] += 1
-            if entry["warm"] <= 3 or len(entry["graphs"]) == 2 or entry.get("eager"):
+            if entry["warm"] <= 3 or entry.get("eager"):
                 out = self._evaluate_step_eager(inputs, mode, gmb, offset)
                 if entry["warm"] == 3:
                     entry["bytes"] = storage_bytes(self._step_tensors(self.acts))
@@ -1223,25 +1241,24 @@ class ExecModel:
             if graph is None:
                 entry["eager"] = True
                 return self._evaluate_step_eager(inputs, mode, gmb, offset)
-            entry["graphs"].append(graph)
-        for k, v in inputs.items():
-            self._copy_into_static(graph.static[k], v)
-        graph.graph.replay()
+            entry["graph"] = graph
+        self.acts = graph.replay(inputs, self._copy_into_static)
         first = next(iter(inputs.values()))
         self.current_inputs = inputs
         self.current_mini_batch_size = int(first.shape[0])
         self._global_mb = graph.samples
         self._global_mb_given, self._mb_offset, self._mean_cache = bool(gmb), offset, {}
-        self.acts = graph.activations()
         self.stats[mode].samples += graph.samples
         native.count_launch(graph.launches)
         self.last_objective = graph.out.clone()
         return self.last_objective
 
+    def _weight_storages(self):
+        return {t.untyped_storage().data_ptr() for t in (self.arena.master, self.arena.compute) if t is not None}
+
     def _step_tensors(self, acts):
         """Activations in memory of the step's own: not those that are views of the weights."""
-        a = self.arena
-        weights = {t.untyped_storage().data_ptr() for t in (a.master, a.compute) if t is not None}
+        weights = self._weight_storages()
         return [t for ts in acts.values() for t in ts
                 if torch.is_tensor(t) and t.untyped_storage().data_ptr() not in weights]
 
@@ -1251,10 +1268,10 @@ class ExecModel:
         samples0, launches0 = st.samples, native.launches()
         need = entry["bytes"]
         for k in list(self._eval_graphs):
-            total = sum(g.bytes for e in self._eval_graphs.values() for g in e["graphs"])
+            total = sum(e["graph"].bytes for e in self._eval_graphs.values() if e["graph"] is not None)
             if k != key and total + need > self._EVAL_GRAPH_BYTES:
                 del self._eval_graphs[k]
-        if sum(g.bytes for g in entry["graphs"]) + need > self._EVAL_GRAPH_BYTES or entry["casts"] > self._EVAL_GRAPH_CASTS:
+        if need > self._EVAL_GRAPH_BYTES or entry["casts"] > self._EVAL_GRAPH_CASTS:
             return None
         graph, static = None, {k: torch.empty_like(v) for k, v in inputs.items()}
         cuda_graph = torch.cuda.CUDAGraph()
@@ -1267,8 +1284,8 @@ class ExecModel:
             with torch.cuda.graph(cuda_graph, capture_error_mode="thread_local"):
                 out = self._evaluate_step_eager(static, mode, gmb, offset)
             acts, self.acts, self._mean_cache = self.acts, {}, {}
-            graph = EvaluationGraph(cuda_graph, static, out, acts, self._step_tensors(acts), self._global_mb,
-                                    native.launches() - launches0)
+            graph = EvaluationGraph(cuda_graph, static, out, acts, self._weight_storages(), self._global_mb,
+                                    native.launches() - launches0, storage_bytes(self._step_tensors(acts)))
         except Exception:           # something in this model cannot be captured
             torch.cuda.synchronize(self.device)
         for w in self.weights:

@@ -259,14 +259,14 @@ def test_evaluation_replays_equal_eager_steps():
             assert m.current_mini_batch_size == rows and m.current_inputs["samples"] is batch["samples"]
         held = [a["conv"][0] for a in held]
         stats = [m.reduce_statistics(mode) for mode in ("validation", "testing")]
-        graphs = sum(len(e["graphs"]) for e in m._eval_graphs.values())
+        graphs = sum(e["graph"] is not None for e in m._eval_graphs.values())
         assert last.shape[0] == rows - 1
         tr.shutdown()
         assert native.consume_status() == 0
         return losses, outs, held, stats, graphs
 
     want, got = run(False), run(True)
-    assert want[4] == 0 and got[4] >= 5
+    assert want[4] == 0 and got[4] >= 3        # of four signatures
     for a, b in zip(want[:3], got[:3]):
         for t, u in zip(a, b):
             assert torch.equal(t, u)
@@ -325,7 +325,7 @@ def test_replays_follow_changes_of_the_layers(change, training):
             else:
                 losses.append(m.evaluate_step(batch, "validation", 8).clone())
         entries = m._graphs if training else m._eval_graphs
-        captured = sum("graph" in e if training else bool(e["graphs"]) for e in entries.values())
+        captured = sum("graph" in e if training else e["graph"] is not None for e in entries.values())
         tr.shutdown()
         assert native.consume_status() == 0
         return torch.stack(losses), captured, types
@@ -335,3 +335,63 @@ def test_replays_follow_changes_of_the_layers(change, training):
     assert not none and captured == (2 if change == "phases" else 1)
     assert change == "phases" or len(types) > 1
     assert torch.equal(want, got), (want - got).abs()
+
+
+@pytest.mark.parametrize("where", ["main", "side", "mapping"])
+def test_activations_of_replays_may_be_read_on_other_streams(where):
+    """What a replayed evaluation step hands out obeys the allocator's rules: read late on another stream (asked for
+    here, there, or through the step's mapping), marked with record_stream and dropped, while the next step runs."""
+    tr, m = _switching_model(True)
+    side = torch.cuda.Stream()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    batches = [{"samples": torch.randn(8, 24, generator=g, device="cuda"),
+                "responses": torch.randn(8, 4, generator=g, device="cuda")} for _ in range(10)]
+    want, got = [], []
+    for b in batches:
+        m._evaluate_step_eager(b, "testing", 8, 0)
+        want.append(m.activation("last").clone())
+    for b in batches:
+        m.evaluate_step(b, "validation", 8)
+        main = torch.cuda.current_stream()
+        y = m.activation("last") if where == "main" else m.acts if where == "mapping" else None
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)            # the next step starts meanwhile
+            if where != "main":
+                y = (y["last"][0] if where == "mapping" else m.activation("last"))
+            got.append(y * 1)
+        y.record_stream(side)
+        del y
+    torch.cuda.synchronize()
+    assert m._eval_graphs
+    tr.shutdown()
+    assert native.consume_status() == 0
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
+
+
+def test_evaluation_whose_activations_are_kept_is_replayed():
+    """A list of all steps' logits: every step beyond the first four is a replay, none writes over what is kept."""
+    tr, m = _switching_model(True)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    kept, want, ordinary, eager = [], [], 0, m._evaluate_step_eager
+
+    def counted(*args):
+        nonlocal ordinary
+        ordinary += 1
+        return eager(*args)
+
+    for step in range(50):
+        b = {"samples": torch.randn(8, 24, generator=g, device="cuda"),
+             "responses": torch.randn(8, 4, generator=g, device="cuda")}
+        eager(b, "testing", 8, 0)
+        want.append(m.activation("last").clone())
+        m._evaluate_step_eager = counted
+        m.evaluate_step(b, "validation", 8)
+        m._evaluate_step_eager = eager
+        kept.append(m.activation("last"))
+    assert ordinary == 4                  # three and the capture
+    tr.shutdown()
+    assert native.consume_status() == 0
+    for a, b in zip(want, kept):
+        assert torch.equal(a, b)
