@@ -395,3 +395,35 @@ def test_evaluation_whose_activations_are_kept_is_replayed():
     assert native.consume_status() == 0
     for a, b in zip(want, kept):
         assert torch.equal(a, b)
+
+
+def test_capture_of_an_evaluation_step_leaves_the_allocator_alone():
+    """Blocks that the allocator keeps are still there after a capture."""
+    tr, m = _switching_model(True)
+    block = torch.empty(64 << 20, device="cuda")
+    del block
+    frees = torch.cuda.memory_stats()["num_device_free"]
+    batch = {"samples": torch.ones(8, 24, device="cuda"), "responses": torch.ones(8, 4, device="cuda")}
+    losses = [float(m.evaluate_step(batch, "validation", 8)) for _ in range(6)]
+    assert any(e["graph"] is not None for e in m._eval_graphs.values())
+    assert torch.cuda.memory_stats()["num_device_free"] == frees
+    tr.shutdown()
+    assert native.consume_status() == 0 and len(set(losses)) == 1
+
+
+def test_evaluation_steps_that_cannot_be_captured(capsys):
+    tr, m = _switching_model(True)
+    eager = m._evaluate_step_eager
+
+    def step(*args):
+        out = eager(*args)
+        if torch.cuda.is_current_stream_capturing():
+            raise RuntimeError("not this one")
+        return out
+
+    m._evaluate_step_eager = step
+    batch = {"samples": torch.ones(8, 24, device="cuda"), "responses": torch.ones(8, 4, device="cuda")}
+    losses = [float(m.evaluate_step(batch, "validation", 8)) for _ in range(6)]
+    tr.shutdown()
+    assert len(set(losses)) == 1 and m.stats["validation"].samples == 48 and native.consume_status() == 0
+    assert capsys.readouterr().out.count("not this one") == 1
