@@ -155,6 +155,11 @@ int lb_splitk_offer(void* ws, long long ws_bytes) {
   return 0;
 }
 
+// A stream that nobody else has; it does not wait for the legacy default stream.
+int lb_stream_create(void** out) {
+  return (int)cudaStreamCreateWithFlags(reinterpret_cast<cudaStream_t*>(out), cudaStreamNonBlocking);
+}
+
 int lb_abi_version() { return LB_ABI_VERSION; }
 
 }  // extern "C"

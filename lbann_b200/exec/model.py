@@ -1279,17 +1279,9 @@ class ExecModel:
         # the graph, and those made there are nobody else's
         for w in self.weights:
             w.handle.bump()
-        # not by torch.cuda.graph: that waits for the GPU and gives every cached block of the allocator back, which
-        # the next steps of all models then allocate again
-        current, side = torch.cuda.current_stream(self.device), torch.cuda.Stream(self.device)
-        side.wait_stream(current)
         try:
-            with torch.cuda.stream(side):
-                cuda_graph.capture_begin(capture_error_mode="thread_local")
-                try:
-                    out = self._evaluate_step_eager(static, mode, gmb, offset)
-                finally:
-                    cuda_graph.capture_end()
+            with native.capture(cuda_graph, self.device):
+                out = self._evaluate_step_eager(static, mode, gmb, offset)
             acts, self.acts, self._mean_cache = self.acts, {}, {}
             graph = EvaluationGraph(cuda_graph, static, out, acts, self._weight_storages(), self._global_mb,
                                     native.launches() - launches0, storage_bytes(self._step_tensors(acts)))
@@ -1297,7 +1289,6 @@ class ExecModel:
             torch.cuda.synchronize(self.device)
             print(f"WARNING: an evaluation step could not be captured as a CUDA graph ({e}); "
                   "kernels are launched from the host", flush=True)
-        current.wait_stream(side)
         for w in self.weights:
             w.handle.bump()
         st.samples = samples0

@@ -7,7 +7,9 @@ thread pool, graph utilities), which also works on CPU-only machines.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
+import gc
 import os
 import threading
 
@@ -74,8 +76,47 @@ def cuda_lib():
                 lib.lb_consume_status.argtypes = [c_void_p]
                 lib.lb_status_ptr.restype = c_void_p
                 lib.lb_sm_count.restype = c_int
+                lib.lb_stream_create.restype = c_int
+                lib.lb_stream_create.argtypes = [ctypes.POINTER(c_void_p)]
                 _cuda = lib
     return _cuda
+
+
+_idle_streams = {}       # by device; as many as there were captures at the same time
+
+
+@contextlib.contextmanager
+def capture(graph, device):
+    """``with capture(graph, device)`` records into a ``torch.cuda.CUDAGraph``.  ``torch.cuda.graph`` would wait for
+    the GPU and give every cached block of the allocator back, which the next steps of all models allocate again.
+    The stream is nobody else's: PyTorch hands its 32 streams out again and again, and pinned memory that is freed
+    meanwhile has an event recorded on each stream that read it, in whatever that stream is capturing."""
+    key = torch.device(device).index or 0
+    current = torch.cuda.current_stream(device)
+    with _lock:
+        idle = _idle_streams.setdefault(key, [])
+        stream = idle.pop() if idle else None
+    if stream is None:
+        handle = c_void_p()
+        with torch.cuda.device(key):
+            check(cuda_lib().lb_stream_create(ctypes.byref(handle)), "lb_stream_create")
+        stream = torch.cuda.ExternalStream(handle.value, device=key)
+    stream.wait_stream(current)
+    collecting = gc.isenabled()
+    gc.disable()              # what a collection frees here may not be allowed in a capture
+    try:
+        with torch.cuda.stream(stream):
+            graph.capture_begin(capture_error_mode="thread_local")
+            try:
+                yield
+            finally:
+                graph.capture_end()
+    finally:
+        if collecting:
+            gc.enable()
+    current.wait_stream(stream)
+    with _lock:
+        idle.append(stream)
 
 
 def host_lib():

@@ -427,3 +427,32 @@ def test_evaluation_steps_that_cannot_be_captured(capsys):
     tr.shutdown()
     assert len(set(losses)) == 1 and m.stats["validation"].samples == 48 and native.consume_status() == 0
     assert capsys.readouterr().out.count("not this one") == 1
+
+
+def test_memory_freed_while_an_evaluation_step_is_captured():
+    """Pinned memory that any stream of PyTorch's pool has read may be freed, and reference cycles come apart, during
+    a capture: neither becomes part of it, and both allocators work behind it."""
+    import gc
+    tr, m = _switching_model(True)
+    pinned = []
+    for _ in range(64):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            pinned.append(torch.zeros(1 << 20).pin_memory())
+            pinned[-1].to("cuda", non_blocking=True)
+    eager, seen = m._evaluate_step_eager, []
+
+    def step(*args):
+        if torch.cuda.is_current_stream_capturing():
+            seen.append(gc.isenabled())
+            pinned.clear()
+        return eager(*args)
+
+    m._evaluate_step_eager = step
+    batch = {"samples": torch.ones(8, 24, device="cuda"), "responses": torch.ones(8, 4, device="cuda")}
+    losses = [float(m.evaluate_step(batch, "validation", 8)) for _ in range(6)]
+    again = [torch.zeros(1 << 20).pin_memory() for _ in range(64)]
+    assert seen == [False] and gc.isenabled() and len(again) == 64 and len(set(losses)) == 1
+    assert any(e["graph"] is not None for e in m._eval_graphs.values())
+    tr.shutdown()
+    assert native.consume_status() == 0
