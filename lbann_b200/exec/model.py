@@ -1036,7 +1036,7 @@ class ExecModel:
                     graph = self._capture_phase_graphs(static, gmb, offset)
                     out = self.last_objective
                 else:
-                    with torch.cuda.graph(graph, capture_error_mode="thread_local"):
+                    with native.capture(graph, self.device, empty_cache=True):
                         out = self._train_step_eager(static, gmb, offset)
             except Exception as e:      # something in this model cannot be captured
                 self._graph_mode = False
@@ -1084,15 +1084,15 @@ class ExecModel:
         graphs = [torch.cuda.CUDAGraph() for _ in range(3)]
         pt, self._phase_timer = self._phase_timer, None       # no event records inside a capture
         try:
-            with torch.cuda.graph(graphs[0], pool=pool, capture_error_mode="thread_local"):
+            with native.capture(graphs[0], self.device, pool, empty_cache=True):
                 self.clear_gradients()
                 self.forward_prop(static, "training", gmb, offset)
                 obj = self.local_objective()
                 self.last_objective = obj.detach()
                 self.record_statistics("training", obj)
-            with torch.cuda.graph(graphs[1], pool=pool, capture_error_mode="thread_local"):
+            with native.capture(graphs[1], self.device, pool, empty_cache=True):
                 self.backward_prop(obj)
-            with torch.cuda.graph(graphs[2], pool=pool, capture_error_mode="thread_local"):
+            with native.capture(graphs[2], self.device, pool, empty_cache=True):
                 self.update_weights()
         finally:
             self._phase_timer = pt

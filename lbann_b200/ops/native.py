@@ -86,11 +86,12 @@ _idle_streams = {}       # by device; as many as there were captures at the same
 
 
 @contextlib.contextmanager
-def capture(graph, device):
-    """``with capture(graph, device)`` records into a ``torch.cuda.CUDAGraph``.  ``torch.cuda.graph`` would wait for
-    the GPU and give every cached block of the allocator back, which the next steps of all models allocate again.
-    The stream is nobody else's: PyTorch hands its 32 streams out again and again, and pinned memory that is freed
-    meanwhile has an event recorded on each stream that read it, in whatever that stream is capturing."""
+def capture(graph, device, pool=None, empty_cache=False):
+    """``with capture(graph, device)`` records into a ``torch.cuda.CUDAGraph``.  ``torch.cuda.graph`` always waits for
+    the GPU and gives every cached block of the allocator back, which the next steps of all models allocate again:
+    ``empty_cache``, for steps that need the memory.  Nor is its stream anybody's own: PyTorch hands 32 streams out
+    again and again, and pinned memory that is freed meanwhile has an event recorded on each stream that read it, in
+    whatever that stream is capturing."""
     key = torch.device(device).index or 0
     current = torch.cuda.current_stream(device)
     with _lock:
@@ -101,12 +102,16 @@ def capture(graph, device):
         with torch.cuda.device(key):
             check(cuda_lib().lb_stream_create(ctypes.byref(handle)), "lb_stream_create")
         stream = torch.cuda.ExternalStream(handle.value, device=key)
+    if empty_cache:
+        gc.collect()
+        torch.cuda.synchronize(device)
+        torch.cuda.empty_cache()
     stream.wait_stream(current)
     collecting = gc.isenabled()
-    gc.disable()              # what a collection frees here may not be allowed in a capture
+    gc.disable()              # what a collection frees may not be allowed in a capture
     try:
         with torch.cuda.stream(stream):
-            graph.capture_begin(capture_error_mode="thread_local")
+            graph.capture_begin(*(() if pool is None else (pool,)), capture_error_mode="thread_local")
             try:
                 yield
             finally:

@@ -202,10 +202,12 @@ def test_overwritten_gradients_equal_accumulated_ones(graph, monkeypatch):
             batch = {"samples": torch.randn(rows, 24, generator=g, device="cuda"),
                      "responses": torch.randn(rows, 4, generator=g, device="cuda")}
             m.train_step(batch, rows)
-            outs += [t.clone() for w in m.weights for t in (w.gradient, w.values)]
+            # (detached: a copy that remembers the weights keeps the step from being captured)
+            outs += [t.detach().clone() for w in m.weights for t in (w.gradient, w.values)]
             assert not m.weights_by_name["aside_linearity_weights"].gradient.any()
         names = {id(w.handle): w.name for w in m.weights}
         found = {names[id(h)] for h in m._overwritten_gradients()}
+        assert not graph or any("graph" in e for e in m._graphs.values())
         tr.shutdown()
         assert native.consume_status() == 0
         return outs, found
@@ -429,18 +431,20 @@ def test_evaluation_steps_that_cannot_be_captured(capsys):
     assert capsys.readouterr().out.count("not this one") == 1
 
 
-def test_memory_freed_while_an_evaluation_step_is_captured():
+@pytest.mark.parametrize("training", [False, True])
+def test_memory_freed_while_a_step_is_captured(training):
     """Pinned memory that any stream of PyTorch's pool has read may be freed, and reference cycles come apart, during
     a capture: neither becomes part of it, and both allocators work behind it."""
     import gc
     tr, m = _switching_model(True)
-    pinned = []
+    pinned, seen = [], []
     for _ in range(64):
         stream = torch.cuda.Stream()
         with torch.cuda.stream(stream):
             pinned.append(torch.zeros(1 << 20).pin_memory())
             pinned[-1].to("cuda", non_blocking=True)
-    eager, seen = m._evaluate_step_eager, []
+    name = "_train_step_eager" if training else "_evaluate_step_eager"
+    eager = getattr(m, name)
 
     def step(*args):
         if torch.cuda.is_current_stream_capturing():
@@ -448,11 +452,11 @@ def test_memory_freed_while_an_evaluation_step_is_captured():
             pinned.clear()
         return eager(*args)
 
-    m._evaluate_step_eager = step
+    setattr(m, name, step)
     batch = {"samples": torch.ones(8, 24, device="cuda"), "responses": torch.ones(8, 4, device="cuda")}
-    losses = [float(m.evaluate_step(batch, "validation", 8)) for _ in range(6)]
+    losses = [float(m.train_step(batch, 8) if training else m.evaluate_step(batch, "validation", 8)) for _ in range(6)]
     again = [torch.zeros(1 << 20).pin_memory() for _ in range(64)]
-    assert seen == [False] and gc.isenabled() and len(again) == 64 and len(set(losses)) == 1
-    assert any(e["graph"] is not None for e in m._eval_graphs.values())
+    assert seen == [False] and gc.isenabled() and len(again) == 64 and all(math.isfinite(v) for v in losses)
+    assert any(e.get("graph") is not None for e in (m._graphs if training else m._eval_graphs).values())
     tr.shutdown()
     assert native.consume_status() == 0
