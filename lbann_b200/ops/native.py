@@ -103,7 +103,6 @@ def capture(graph, device, pool=None, empty_cache=False):
             check(cuda_lib().lb_stream_create(ctypes.byref(handle)), "lb_stream_create")
         stream = torch.cuda.ExternalStream(handle.value, device=key)
     if empty_cache:
-        gc.collect()
         torch.cuda.synchronize(device)
         torch.cuda.empty_cache()
     stream.wait_stream(current)
