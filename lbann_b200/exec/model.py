@@ -168,6 +168,7 @@ class ExecModel:
         self._overwrite_cache = None   # (layers, handles), see _overwritten_gradients
         self._graphs = {}
         self._eval_graphs = OrderedDict()
+        self._eval_steps, self._eval_refused = 0, set()
         # what captured steps depend on beside their inputs, see layer_state
         self._layer_changes, self._layers_seen, self._frozen_seen, self._in_forward = 0, None, None, False
         self._graph_changes = self._eval_changes = -1
@@ -935,7 +936,7 @@ class ExecModel:
                       "on_layer_forward_end", "on_backward_prop_begin", "on_backward_prop_end",
                       "on_optimize_begin", "on_optimize_end")
 
-    def _graph_capable(self) -> bool:
+    def _graph_capable(self, layers=True) -> bool:
         """Graph replay is used when asked for, on a GPU, and when nothing needs the host
         inside a step: no callback overrides an in-step hook, no per-layer timing."""
         from ..callbacks.base import ExecCallback
@@ -951,7 +952,7 @@ class ExecModel:
                     return False
         # layers whose output depends on a host-side value that changes from step to step
         # (position in the epoch, host random streams, user code)
-        if any(l.type in self._HOST_STATE_LAYERS for l in self.layers):
+        if layers and any(l.type in self._HOST_STATE_LAYERS for l in self.layers):
             return False
         # hypergradient Adam moves its learning rate on the host every step
         if any(s.kind == "hypergradient_adam" for s in self.arena.slots):
@@ -1173,7 +1174,8 @@ class ExecModel:
                       mini_batch_offset=0):
         """Forward pass, objective and statistics.  With the ``use_cuda_graph`` option small steps are
         captured once per input signature and replayed, as training steps are."""
-        key = self._eval_graph_key(inputs, mode, global_mini_batch_size, mini_batch_offset)
+        refused = self._eval_refused and self._eval_signature(inputs, mode, global_mini_batch_size) in self._eval_refused
+        key = None if refused else self._eval_graph_key(inputs, mode, global_mini_batch_size, mini_batch_offset)
         if key is not None:
             return self._evaluate_step_graph(key, inputs, mode, global_mini_batch_size, mini_batch_offset)
         return self._evaluate_step_eager(inputs, mode, global_mini_batch_size, mini_batch_offset)
@@ -1193,19 +1195,28 @@ class ExecModel:
         self.record_statistics(mode, obj)
         return self.last_objective
 
-    # A forward pass of two GPT blocks over 512 tokens takes the host 740 us to launch, and 225 us as a replay.
-    # Steps with more activations than this (all graphs of a model together) run longer than the host takes,
-    # and would hold their memory for good; so would copies of that many weights be repeated by each replay.
-    _EVAL_GRAPH_BYTES = 2 << 30
-    _EVAL_GRAPH_CASTS = 4 << 20     # elements of weights copied or packed for the step
-    _EVAL_GRAPHS = 8
+    # A forward pass of two GPT blocks over 512 tokens takes the host 740 us to launch, and 240 us as a replay.
+    # The host needs 10 to 20 us for a layer.  Layers with more activations than this take the GPU as long, and
+    # a replay's copies of its inputs and weights only come on top.  Ordinary step / replay: CosmoFlow 64^3, one volume,
+    # 0.5 MB a layer, 458 / 137 us, 16 volumes, 8 MB, 477 / 469; GPT of 1024 tokens, two sequences, 9 MB, 722 / 454.
+    _EVAL_LAYER_BYTES = 16 << 20
+    _EVAL_GRAPH_CASTS = 4 << 20     # elements of weights that every replay copies or packs anew
+    # Memory and number of the graphs that a model keeps.  A graph makes room for another signature's when it
+    # has not been used for that many steps: signatures that take turns do not drive one another out.
+    _EVAL_GRAPH_BYTES = 1 << 30
+    _EVAL_GRAPHS, _EVAL_IDLE = 8, 256
+    _EVAL_SIGNATURES = 64
     _EVAL_LAYER_MODULES = (layers_core.__name__, layers_misc.__name__)
+
+    @staticmethod
+    def _eval_signature(inputs, mode, gmb):
+        return (mode, gmb, tuple((k, v.shape) for k, v in inputs.items() if torch.is_tensor(v)))
 
     def _eval_graph_key(self, inputs, mode, gmb, offset):
         """What a captured evaluation step depends on, or None where the step is launched from the host."""
         if (self.device.type != "cuda" or self.parallel is not None or self.distconv is not None
                 or self.subgrid is not None or self._phase_timer is not None or not inputs
-                or torch.cuda.is_current_stream_capturing() or not self._graph_capable()
+                or torch.cuda.is_current_stream_capturing() or not self._graph_capable(layers=False)
                 or not all(torch.is_tensor(v) and v.is_cuda and v.is_contiguous() for v in inputs.values())):
             return None
         changes, frozen = self.layer_state()
@@ -1213,8 +1224,9 @@ class ExecModel:
             self._eval_graphs.clear()
             self._eval_changes = changes
             # layers from elsewhere may keep anything on the host
-            self._eval_own_layers = all(type(l).__module__ in self._EVAL_LAYER_MODULES for l in self.layers)
-        if not self._eval_own_layers:
+            self._eval_layers = all(type(l).__module__ in self._EVAL_LAYER_MODULES and l.type not in self._HOST_STATE_LAYERS
+                                    for l in self.layers)
+        if not self._eval_layers:
             return None
         return (mode, gmb, offset, torch.cuda.current_stream(self.device).cuda_stream, self.arena.master.data_ptr(), frozen,
                 tuple((k, tuple(v.shape), v.dtype, v.device) for k, v in sorted(inputs.items())))
@@ -1222,26 +1234,29 @@ class ExecModel:
     def _evaluate_step_graph(self, key, inputs, mode, gmb, offset):
         entry = self._eval_graphs.get(key)
         if entry is None:
-            entry = self._eval_graphs[key] = {"warm": 0, "graph": None}
-            while len(self._eval_graphs) > self._EVAL_GRAPHS:
-                self._eval_graphs.popitem(last=False)
+            entry = self._eval_graphs[key] = {"warm": 0, "graph": None, "eager": False}
+            if len(self._eval_graphs) > self._EVAL_SIGNATURES:
+                del self._eval_graphs[next(k for k, e in self._eval_graphs.items() if e["graph"] is None)]
         self._eval_graphs.move_to_end(key)
+        self._eval_steps += 1
+        entry["used"] = self._eval_steps
         self.acts = {}
-        graph = entry["graph"]
-        if graph is None:
-            entry["warm"] += 1
-            if entry["warm"] <= 3 or entry.get("eager"):
+        if entry["graph"] is None:
+            if entry["warm"] == 3 and not entry["eager"] and self._eval_room(entry):
+                entry["graph"] = self._capture_evaluation(inputs, mode, gmb, offset)
+                entry["eager"] = entry["graph"] is None
+            if entry["graph"] is None:
                 out = self._evaluate_step_eager(inputs, mode, gmb, offset)
-                if entry["warm"] == 3:
-                    entry["bytes"] = storage_bytes(self._step_tensors(self.acts))
-                    entry["casts"] = sum(t.numel() for w in self.weights for t in w.handle._cache.values()
-                                         if torch.is_tensor(t))
+                if entry["warm"] < 3:
+                    entry["warm"] += 1
+                    if entry["warm"] == 3:
+                        self._eval_decide(entry)
+                if entry["eager"]:       # for good, without another look (80 us of a step)
+                    if len(self._eval_refused) >= self._EVAL_SIGNATURES:
+                        self._eval_refused.clear()
+                    self._eval_refused.add(self._eval_signature(inputs, mode, gmb))
                 return out
-            graph = self._capture_evaluation(entry, key, inputs, mode, gmb, offset)
-            if graph is None:
-                entry["eager"] = True
-                return self._evaluate_step_eager(inputs, mode, gmb, offset)
-            entry["graph"] = graph
+        graph = entry["graph"]
         self.acts = graph.replay(inputs, self._copy_into_static)
         first = next(iter(inputs.values()))
         self.current_inputs = inputs
@@ -1256,23 +1271,34 @@ class ExecModel:
     def _weight_storages(self):
         return {t.untyped_storage().data_ptr() for t in (self.arena.master, self.arena.compute) if t is not None}
 
-    def _step_tensors(self, acts):
-        """Activations in memory of the step's own: not those that are views of the weights."""
+    def _eval_decide(self, entry):
+        """From an ordinary step: whether its signature gets a graph, and about how large that will be."""
         weights = self._weight_storages()
-        return [t for ts in acts.values() for t in ts
-                if torch.is_tensor(t) and t.untyped_storage().data_ptr() not in weights]
+        entry["bytes"] = storage_bytes([t for ts in self.acts.values() for t in ts if torch.is_tensor(t)
+                                        and t.untyped_storage().data_ptr() not in weights])
+        casts = sum(t.numel() for w in self.weights for t in w.handle._cache.values() if torch.is_tensor(t))
+        layers = sum(not getattr(l, "dead", False) for l in self.layers)
+        entry["eager"] = (casts > self._EVAL_GRAPH_CASTS or entry["bytes"] > self._EVAL_GRAPH_BYTES
+                          or entry["bytes"] > layers * self._EVAL_LAYER_BYTES)
 
-    def _capture_evaluation(self, entry, key, inputs, mode, gmb, offset):
-        """The step as a graph; None where it cannot or should not be one."""
+    def _eval_room(self, entry):
+        """Room for one more graph, from those that are idle."""
+        kept = [(k, e) for k, e in self._eval_graphs.items() if e["graph"] is not None]       # the oldest first
+        total, drop = sum(e["graph"].bytes for _, e in kept) + entry["bytes"], 0
+        while drop < len(kept) and (len(kept) - drop >= self._EVAL_GRAPHS or total > self._EVAL_GRAPH_BYTES):
+            if self._eval_steps - kept[drop][1]["used"] <= self._EVAL_IDLE:
+                return False
+            total -= kept[drop][1]["graph"].bytes
+            drop += 1
+        for k, _ in kept[:drop]:
+            del self._eval_graphs[k]
+        return True
+
+    def _capture_evaluation(self, inputs, mode, gmb, offset):
+        """The step as a graph; None where it cannot be one."""
         st = self.stats[mode]
         samples0, launches0 = st.samples, native.launches()
-        need = entry["bytes"]
-        for k in list(self._eval_graphs):
-            total = sum(e["graph"].bytes for e in self._eval_graphs.values() if e["graph"] is not None)
-            if k != key and total + need > self._EVAL_GRAPH_BYTES:
-                del self._eval_graphs[k]
-        if need > self._EVAL_GRAPH_BYTES or entry["casts"] > self._EVAL_GRAPH_CASTS:
-            return None
+        reserved0 = torch.cuda.memory_stats(self.device).get("reserved_bytes.all.current", 0)
         graph, static = None, {k: torch.empty_like(v) for k, v in inputs.items()}
         cuda_graph = torch.cuda.CUDAGraph()
         # the weights may change between replays: their 16-bit and packed copies are made inside
@@ -1283,8 +1309,9 @@ class ExecModel:
             with native.capture(cuda_graph, self.device):
                 out = self._evaluate_step_eager(static, mode, gmb, offset)
             acts, self.acts, self._mean_cache = self.acts, {}, {}
+            grown = torch.cuda.memory_stats(self.device).get("reserved_bytes.all.current", 0) - reserved0
             graph = EvaluationGraph(cuda_graph, static, out, acts, self._weight_storages(), self._global_mb,
-                                    native.launches() - launches0, storage_bytes(self._step_tensors(acts)))
+                                    native.launches() - launches0, grown + storage_bytes(static.values()))
         except Exception as e:      # something in this model cannot be captured
             torch.cuda.synchronize(self.device)
             print(f"WARNING: an evaluation step could not be captured as a CUDA graph ({e}); "
@@ -1293,7 +1320,7 @@ class ExecModel:
             w.handle.bump()
         st.samples = samples0
         native.count_launch(launches0 - native.launches())
-        return graph
+        return graph if graph is None or graph.bytes <= self._EVAL_GRAPH_BYTES else None
 
     # ------------------------------------------------------------------ reporting
     def reduce_statistics(self, mode: str):

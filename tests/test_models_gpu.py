@@ -460,3 +460,36 @@ def test_memory_freed_while_a_step_is_captured(training):
     assert any(e.get("graph") is not None for e in (m._graphs if training else m._eval_graphs).values())
     tr.shutdown()
     assert native.consume_status() == 0
+
+
+def test_which_evaluation_steps_keep_a_graph(monkeypatch):
+    """Limits of the captured evaluation steps: of their number, with and without an idle one to drop, of memory, of
+    what a replay would copy, of activations a layer, and of the signatures that are remembered."""
+    from lbann_b200.exec.model import ExecModel
+    tr, m = _switching_model(True)
+
+    def steps(rows, n=5):
+        for _ in range(n):
+            m.evaluate_step({"samples": torch.ones(rows, 24, device="cuda"),
+                             "responses": torch.ones(rows, 4, device="cuda")}, "validation", rows)
+        return {k[6][0][1][0] for k, e in m._eval_graphs.items() if e["graph"] is not None}
+
+    monkeypatch.setattr(ExecModel, "_EVAL_GRAPHS", 2)
+    monkeypatch.setattr(ExecModel, "_EVAL_IDLE", 12)
+    monkeypatch.setattr(ExecModel, "_EVAL_SIGNATURES", 5)
+    assert steps(1) == {1} and steps(2) == {1, 2}
+    assert steps(3) == {1, 2}                         # neither has been idle for long
+    assert steps(2) == {1, 2} and steps(3) == {2, 3}  # the first has
+    limits = (("_EVAL_LAYER_BYTES", 1), ("_EVAL_GRAPH_BYTES", 1), ("_EVAL_GRAPH_CASTS", -1))
+    for rows, (limit, value) in enumerate(limits, 4):
+        with monkeypatch.context() as mp:
+            mp.setattr(ExecModel, limit, value)
+            assert steps(rows, 20) == {2, 3}          # idle or not: nothing makes room for what gets no graph
+        assert len(m._eval_refused) == rows - 3
+    for rows in range(7, 15):
+        steps(rows, 1)
+    assert len(m._eval_graphs) == 5 and steps(3) == {2, 3}
+    held = sum(e["graph"].bytes for e in m._eval_graphs.values() if e["graph"] is not None)
+    assert (2 + 3) * (24 + 4) * 4 <= held <= ExecModel._EVAL_GRAPH_BYTES
+    tr.shutdown()
+    assert native.consume_status() == 0
