@@ -740,10 +740,17 @@ c10::intrusive_ptr<State> make_state(const optional<Tensor>& w, const optional<T
 
 }  // namespace
 
+// ``t.backward(gradient)``, which imports PyTorch's symbolic shapes (1.4 s) to compare two shapes.
+void backward(const Tensor& t, const Tensor& gradient) {
+  TORCH_CHECK(t.sizes() == gradient.sizes(), "gradient of another shape");
+  t.backward(gradient);
+}
+
 PYBIND11_MODULE(_lbann_autograd, m) {
   m.def("set_error_type", [](const py::object& t) { g_native_error = py::object(t).release().ptr(); });
   m.attr("abi_version") = LB_ABI_VERSION;
   m.def("launches", [] { return (long long)g_launches; });
+  m.def("backward", torch::wrap_pybind_function_no_gil(backward));
   m.def("splitk_offers", [] { return (long long)g_offers; });
   m.def("gemm", [](const Tensor& a, const Tensor& b, bool ta, bool tb, const optional<Tensor>& out, int64_t out_code,
                    double alpha, double beta, const optional<Tensor>& bias, bool per_row, int64_t act, double act_param,

@@ -836,7 +836,7 @@ class ExecModel:
                 local_obj.backward()
             elif self.device.type == "cuda":
                 # the scale as the objective's gradient: no host read of it, and no product
-                local_obj.backward(self._amp_device_state()[0].to(local_obj.dtype))
+                native.nodes().backward(local_obj, self._amp_device_state()[0].to(local_obj.dtype))
             else:
                 (local_obj * self._amp_scale_host).backward()
         self.arena.end_gradients()

@@ -2,6 +2,9 @@
 layer norm, softmax, fused softmax-cross-entropy, batch norm, fused optimizer) carry a few
 training steps of every model family."""
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -493,3 +496,45 @@ def test_which_evaluation_steps_keep_a_graph(monkeypatch):
     assert (2 + 3) * (24 + 4) * 4 <= held <= ExecModel._EVAL_GRAPH_BYTES
     tr.shutdown()
     assert native.consume_status() == 0
+
+
+def test_first_step_with_loss_scaling_imports_nothing_large():
+    """A training step with AMP in a process of its own; errors of Python functions in backward keep their type."""
+    code = """
+import sys, torch
+import lbann_b200 as lbann
+from lbann_b200.exec.trainer import ExecTrainer
+from lbann_b200.models.cosmoflow import construct_cosmoflow_model, synthetic_reader
+from lbann_b200.ops import native
+from lbann_b200.utils import options as opts
+opts.reset().set("default_dtype", "fp16")
+model = construct_cosmoflow_model(16, 4, 4, num_epochs=1, channels=(16, 32), pool_mode="max", conv_bias=False)
+model.amp = lbann.AmpOptions(enabled=True, init_scale=128.0)
+exp = lbann.proto.serialize.build_experiment(trainer=lbann.Trainer(mini_batch_size=2, random_seed=1), model=model,
+    data_reader=lbann.reader_pb2.DataReader(), optimizer=lbann.Adam(learn_rate=1e-4, beta1=0.9, beta2=0.99, eps=1e-8))
+import numpy as np
+from lbann_b200.data.readers import ArrayReader
+arrays = {"samples": np.zeros((1, 4, 16, 16, 16), np.float32), "responses": np.zeros((1, 4), np.float32)}
+m = ExecTrainer(exp, readers={"train": ArrayReader(arrays)}, background_io=False).build_model(exp.model)
+before = "sympy" in sys.modules
+m.train_step({"samples": torch.rand(2, 4, 16, 16, 16, device="cuda").half(), "responses": torch.rand(2, 4, device="cuda")})
+assert ("sympy" in sys.modules) == before, "sympy came in"
+assert native.consume_status() == 0 and any(w.gradient.any() for w in m.weights)
+class Bad(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x):
+        return x * 2
+    @staticmethod
+    def backward(ctx, g):
+        raise KeyError("mine")
+x = torch.ones((), device="cuda", requires_grad=True)
+try:
+    native.nodes().backward(Bad.apply(x), torch.ones((), device="cuda"))
+except KeyError as e:
+    assert "mine" in str(e)
+else:
+    raise AssertionError("no error")
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr[-2000:]
