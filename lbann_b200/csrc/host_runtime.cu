@@ -147,9 +147,9 @@ void* lb_status_ptr() { return lbhost::status_word(); }
 int lb_sm_count() { return lbhost::sm_count(); }
 
 // Lends scratch to the next GEMM / convolution launch of the calling thread (see
-// lbhost::SplitKOffer).  `ws` must be 16-byte aligned.
+// lbhost::SplitKOffer).  `ws` must be 32-byte aligned: partial sums are stored in whole sectors.
 int lb_splitk_offer(void* ws, long long ws_bytes) {
-  if ((reinterpret_cast<uintptr_t>(ws) & 15) || ws_bytes < 0) return -1;
+  if ((reinterpret_cast<uintptr_t>(ws) & 31) || ws_bytes < 0) return -1;
   lbhost::g_splitk_offer.ws = reinterpret_cast<float*>(ws);
   lbhost::g_splitk_offer.ws_bytes = ws_bytes;
   return 0;

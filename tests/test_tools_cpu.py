@@ -168,3 +168,17 @@ def test_autograd_nodes_belong_to_the_kernel_library_and_to_this_pytorch(monkeyp
     monkeypatch.setattr(torch, "__version__", torch.__version__ + ".other")
     _build.build_native()
     assert done == ["link", _build.NODES_SRC]
+
+
+def test_splitk_workspace_is_refused_off_32_bytes():
+    """Partial sums are stored 32 bytes at a time; nothing is launched here."""
+    import ctypes
+
+    from lbann_b200 import _build
+    from lbann_b200.ops import native
+    _build.build_native()
+    offer = native.cuda_lib().lb_splitk_offer
+    offer.restype, offer.argtypes = ctypes.c_int, [ctypes.c_void_p, ctypes.c_longlong]
+    base = 1 << 20
+    assert [offer(base + at, 4096) for at in (0, 4, 8, 16, 24, 32, 48)] == [0, -1, -1, -1, -1, 0, -1]
+    assert offer(base, -1) == -1 and offer(None, 0) == 0
