@@ -311,3 +311,37 @@ def test_conv_wgrad_from_slabs(case):
                     view = xp[:, a:a + Do, b:b + H, c:c + W].reshape(-1, C)
                     ref[:, :, a, b, c] = prev[:, :, a, b, c].double() + 0.5 * (dy.double().reshape(-1, K).t() @ view)
         assert float((got.double() - ref).norm() / ref.norm()) < 4.7e-6
+
+
+def test_filter_gradients_of_layers_in_turn():
+    """A thread's last tiling is kept between asking for the workspace and the launch: layers in turn, also by
+    threads of their own, give what each gives alone."""
+    import threading
+    torch.manual_seed(3)
+    cases = []
+    for n, ci, co, size, k in ((2, 32, 64, 20, 3), (1, 64, 32, 9, 1), (3, 16, 24, 17, 5)):
+        x = torch.randn(n, ci, size, size, device="cuda").half().contiguous(memory_format=torch.channels_last)
+        w = torch.randn(co, ci, k, k, device="cuda").requires_grad_(True)
+        wh = nn.WeightHandle(w, torch.zeros_like(w))
+        y = nn.convolution(x.requires_grad_(True), wh, None, (k, k), (k // 2,) * 2, (1, 1), (1, 1))
+        cases.append((x, wh, y, torch.randn_like(y)))
+
+    def grad(c):
+        x, wh, y, dy = c
+        wh.grad.zero_()
+        torch.autograd.grad(y, x, dy, retain_graph=True)
+        torch.cuda.synchronize()
+        return wh.grad.clone()
+
+    alone = [[grad(c) for _ in range(3)][-1] for c in cases]
+    got = [grad(cases[i]) for i in (0, 1, 2, 1, 0, 2)]
+    for i, g in zip((0, 1, 2, 1, 0, 2), got):
+        assert float((g - alone[i]).norm()) <= 1e-6 * float(alone[i].norm())
+    out = {}
+    threads = [threading.Thread(target=lambda i=i: out.__setitem__(i, [grad(cases[i]) for _ in range(5)])) for i in range(3)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    for i in range(3):
+        for g in out[i]:
+            assert float((g - alone[i]).norm()) <= 1e-6 * float(alone[i].norm())
+    assert native.consume_status() == 0
