@@ -5,7 +5,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from lbann_b200.ops import native
+from lbann_b200.ops import native, nn
 from lbann_b200.ops.conv import conv_fwd, pack_filter
 
 pytestmark = pytest.mark.gpu
