@@ -487,19 +487,23 @@ layer_norm_bwd_bands_kernel(const T* __restrict__ x, const T* __restrict__ dy, c
       rstd[u] = there ? __ldg(rstd_in + r + u) : 0.f;
     }
 #pragma unroll
-    for (int u = 0; u < R; ++u) {
-      const T* ex = reinterpret_cast<const T*>(&qx[u]);
-      const T* eg = reinterpret_cast<const T*>(&qg[u]);
-      s[2 * u] = s[2 * u + 1] = 0.f;
+    for (int u = 0; u < 2 * R; ++u) s[u] = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = (to_f32<T>(ex[j]) - mean[u]) * rstd[u], gy = to_f32<T>(eg[j]);
-        ds[j] += gy * xh;
-        db[j] += gy;
-        const float g = gy * c[j];
+    for (int j = 0; j < 8; ++j) {
+      // The band's first: a fourth of the terms in a row.  Two teams a block add up four times as many rows as
+      // eight did: 65536 x 1024, scale gradient 3.7e-7 off, so 3.4e-7, with eight 3.3e-7; both directions 171 -> 161 us.
+      float bs = 0.f, bb = 0.f;
+#pragma unroll
+      for (int u = 0; u < R; ++u) {
+        const float xh = (to_f32<T>(reinterpret_cast<const T*>(&qx[u])[j]) - mean[u]) * rstd[u];
+        const float gy = to_f32<T>(reinterpret_cast<const T*>(&qg[u])[j]), g = gy * c[j];
+        bs += gy * xh;
+        bb += gy;
         s[2 * u] += g;
         s[2 * u + 1] += g * xh;
       }
+      ds[j] += bs;
+      db[j] += bb;
     }
     ln_band_sum<2 * R>(s, W, tw, lane, team, sm[turn] + team * 2 * R * W);
     if (!on) continue;
