@@ -394,8 +394,7 @@ __device__ __forceinline__ void store_from_f32(void* p, long long i, float v, in
   else reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
 }
 
-// 2^x in one instruction (results below the normal range are zero; the form that keeps them scales before
-// and after).
+// 2^x by ex2.approx.ftz; results below the normal range are zero.
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));

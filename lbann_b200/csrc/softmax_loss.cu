@@ -144,9 +144,9 @@ __global__ void softmax_ce_bwd_kernel(const T* __restrict__ x, const long long* 
 // the two-pass scalar kernel above reads a row twice, two bytes a load.  A row of 4096 columns or more is
 // a block's, shorter ones a warp's.  Rows start anywhere (a vocabulary of 30522 words): the elements in front
 // of the first 16-byte boundary and behind the last are single ones.
-// Instructions are what is left of long rows: exponentials of one instruction instead of __expf's four
-// (terms below 2^-126 of the largest are zero).  Forward, bf16: 4096 x 50304 86 -> 78 us,
-// 16384 x 2048 34 -> 17 (a block for a row of 256 vectors is mostly its reductions).
+// Instructions are what is left of long rows: ex2.approx.ftz (terms below 2^-126 of the largest are zero).
+// Forward, bf16: 4096 x 50304 86 -> 78 us, 16384 x 2048 34 -> 17 (a block for a row of 256 vectors is
+// mostly its reductions).
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kCeBlockRow = 4096;                     // columns from which a row takes a block
 
