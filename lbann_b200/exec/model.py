@@ -165,7 +165,7 @@ class ExecModel:
         self._gen = None
         self.sync_layers = False       # debugging: synchronise after every layer
         self._graph_mode = None        # decided at the first training step
-        self._overwrite_cache = None   # (layers, handles), see _overwritten_gradients
+        self._overwrite_cache = None   # (what it was made from, handles), see _overwritten_gradients
         self._graphs = {}
         self._eval_graphs = OrderedDict()
         self._eval_steps, self._eval_refused = 0, set()
@@ -763,7 +763,7 @@ class ExecModel:
         if any(getattr(type(cb), h, None) is not getattr(ExecCallback, h) for cb in self.callbacks
                for h in self._IN_STEP_HOOKS):
             return []
-        key = tuple(id(l) for l in self.layers)
+        key = (self._layer_changes, list(self.layers), [w.handle for w in self.weights], self.arena.grad.data_ptr())
         if self._overwrite_cache is None or self._overwrite_cache[0] != key:
             uses = defaultdict(int)
             for l in self.layers:

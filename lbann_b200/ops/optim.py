@@ -275,10 +275,11 @@ class ParameterArena:
         not write after all."""
         if not handles:
             return self.zero_grad()
-        key = tuple(id(h) for h in handles)
+        spans = tuple((h.grad.storage_offset() - self.grad.storage_offset(), h.grad.numel()) for h in handles)
+        key = (self.grad.data_ptr(), spans)
         if self._begin_key != key:
             at, rest = 0, []
-            for lo, n in sorted((h.grad.storage_offset() - self.grad.storage_offset(), h.grad.numel()) for h in handles):
+            for lo, n in sorted(spans):
                 if lo > at:
                     rest.append(self.grad[at:lo])
                 at = lo + n

@@ -154,3 +154,54 @@ def test_compact_state_pack_gather_and_commit():
     back = a._unpack_state(a.state0)
     own = a.shard.owner_mask(want.numel(), "cpu")
     assert torch.equal(back[:a.total], torch.where(own, want, torch.zeros_like(want))[:a.total])
+
+
+def test_overwritten_gradients_follow_the_handles():
+    """What a step does not clear is where the handles' gradients are now, not where they were when it last asked."""
+    from lbann_b200.ops.nn import WeightHandle
+    from lbann_b200.ops.optim import ParameterArena
+    a = ParameterArena(torch.device("cpu"))
+    slots = [a.reserve(n, (300,)) for n in "xyz"]
+    a.materialise()
+    views = [a.view(a.grad, s) for s in slots]
+    h = WeightHandle(torch.zeros(300), views[0])
+    for at in (0, 2, 1):
+        h.grad = views[at]
+        a.grad.fill_(5.0)
+        a.begin_gradients([h])
+        assert [bool(v.any()) for v in views] == [i == at for i in range(3)]
+        a.end_gradients()                 # nobody wrote it: cleared
+        assert not a.grad.any()
+    a.grad = torch.full_like(a.grad, 5.0)
+    h.grad = a.view(a.grad, slots[1])
+    a.begin_gradients([h])
+    assert [bool(a.view(a.grad, s).any()) for s in slots] == [False, True, False]
+
+
+def test_overwritten_gradients_are_looked_up_again_for_a_new_handle(monkeypatch):
+    import numpy as np
+
+    import lbann_b200 as lbann
+    from lbann_b200.data.readers import ArrayReader
+    from lbann_b200.exec.model import ExecModel
+    from lbann_b200.exec.trainer import ExecTrainer
+    from lbann_b200.ops.nn import WeightHandle
+    from lbann_b200.utils import options as opts
+    opts.reset().set("disable_cuda", True)
+    x = lbann.Input(data_field="samples")
+    y = lbann.FullyConnected(x, num_neurons=4, has_bias=False, name="fc")
+    loss = lbann.MeanSquaredError(y, lbann.Input(data_field="responses"))
+    exp = lbann.proto.serialize.build_experiment(
+        trainer=lbann.Trainer(mini_batch_size=2),
+        model=lbann.Model(1, layers=lbann.traverse_layer_graph(x), objective_function=loss),
+        data_reader=lbann.reader_pb2.DataReader(), optimizer=lbann.SGD(learn_rate=0.1))
+    arrays = {"samples": np.zeros((2, 6), np.float32), "responses": np.zeros((2, 4), np.float32)}
+    m = ExecTrainer(exp, readers={"train": ArrayReader(arrays)}, background_io=False).build_model(exp.model)
+    monkeypatch.setattr(ExecModel, "_OVERWRITE_MIN", 1)
+    m.device = torch.device("cuda")           # nothing is launched
+    w = m.layer("fc").w
+    assert m._overwritten_gradients() == [w.handle] and m._overwritten_gradients() == [w.handle]
+    w.handle = WeightHandle(w.handle.master, w.handle.grad)
+    assert m._overwritten_gradients() == [w.handle]
+    m.layer("fc").transpose = True
+    assert m._overwritten_gradients() == []
