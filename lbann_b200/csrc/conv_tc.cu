@@ -21,7 +21,10 @@ namespace lb {
 template <int BN_>
 struct ConvFwdPolicy {
   static constexpr int BN = BN_;
-  static constexpr int kEpiGroups = BN == 32 ? 1 : 2;   // share a tile's columns (tc_pipeline.cuh)
+  // Groups share a tile's columns (tc_pipeline.cuh); tiles of 32 columns have one.  Against two that took tiles in
+  // turn: 3x3, 64 -> 32 channels, 32 x 56^2 11.3 / 11.2 us, 32 -> 32, 32 x 112^2 22.2 / 22.0, 27 taps, 64^3
+  // 23.2 / 23.3, 1x1, 32 -> 16, 16 x 112^2 24.0 / 17.4.
+  static constexpr int kEpiGroups = BN == 32 ? 1 : 2;
   using G = StageGeom<BN>;
   using HasSingleIssue = void;               // two boxes a slice, issued by one thread
 
