@@ -440,8 +440,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // delta[b][h][q] = scale * sum_d dO[b][q][h][d] * O[b][q][h][d]: 16 lanes of 16 bytes a row, two
 // rows of a warp at a time, four rounds in flight
 // ------------------------------------------------------------------------------------
-// 64 rows of a batch entry a block.  B = 2, H = 16, S = 2048, bf16: 6.4 us for 67 MB.  (64-bit divisions by run-time values for
-// every row, 11.5 us.)
+// 64 rows of a batch entry a block.  B = 2, H = 16, S = 2048, bf16: 6.4 us for 67 MB.  (64-bit divisions by
+// run-time values for every row, 11.5 us.)
 template <typename T>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __restrict__ delta, FastDiv heads, int exact,
@@ -497,9 +497,11 @@ attn_delta_kernel(const T* __restrict__ o, const T* __restrict__ dout, float* __
 // the rows of the last one are written.
 // B = 2, H = 16, S = 2048, bf16: causal 308 us as two kernels with one step in flight -> 161 with P and dS in
 // shared memory -> 153 with a CTA an item -> 142; not causal 242 -> 226.  What is left is a step's 16 MMAs of
-// N = 64, which read 128 rows of A for half the arithmetic (48-58 cycles for 32), and about 400 cycles from the
-// end of an accumulation to the scores that overwrite its operands: rows that do nothing leave 124 us.
-// (Waiting for P and dS separately: 143; scores read into registers first, P and dS elsewhere: 157; 16 row warps: no change.)
+// N = 64, which read 128 rows of A for half the arithmetic (48 cycles where 32 would do), and the wait from the
+// end of an accumulation to the scores that overwrite its operands: rows that do nothing leave 124 us.  The tensor
+// pipe is active for 47 % of the cycles.
+// (Waiting for P and dS separately: 143; scores read into registers first, P and dS elsewhere: 157; 16 row
+// warps: no change.)
 // ------------------------------------------------------------------------------------
 constexpr int kBwdCols = 64;                          // streamed rows (= score columns) per step
 constexpr int kBwdTile = kBwdCols * kAttD * 2;        // 16 KB: one streamed operand

@@ -491,7 +491,8 @@ layer_norm_bwd_bands_kernel(const T* __restrict__ x, const T* __restrict__ dy, c
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       // The band's first: a fourth of the terms in a row.  Two teams a block add up four times as many rows as
-      // eight did: 65536 x 1024, scale gradient 3.7e-7 off, so 3.4e-7, with eight 3.3e-7; both directions 171 -> 161 us.
+      // eight did: 65536 x 1024, scale gradient 3.7e-7 off, so 3.4e-7, with eight 3.3e-7; both directions
+      // 171 -> 161 us.
       float bs = 0.f, bb = 0.f;
 #pragma unroll
       for (int u = 0; u < R; ++u) {

@@ -1,7 +1,7 @@
 // What a step does with the values of its loss layers: their sum over the mini-batch, the objective's
-// scale, the gradient that goes back to them, and the running statistics of the mode.  A handful of numbers: the launches
-// are all that it costs, so there are three instead of the eleven of one operator each (1.2 to 2 us apiece in a
-// replayed step).
+// scale, the gradient that goes back to them, and the running statistics of the mode.  A handful of
+// numbers: the launches are all that it costs, so there are three instead of the eleven of one operator
+// each (1.2 to 2 us apiece in a replayed step).
 #include "common.cuh"
 
 namespace lb {
